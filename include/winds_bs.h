@@ -138,23 +138,26 @@ int winds_bs_length_device(const double *F1, const double *F2, const long long d
 int winds_bs_last_stats(double *main_ms, int *launches, long long *near_pairs);
 
 /* How many pairs of the last winds_bs_eval_host / winds_bs_eval_device call's
- * FP32c direct sum took the core-free form, where leaving the core out
- * changes the pair term by less than FP32's unit roundoff 2^-24 (one-sided):
- * Vatistas, targets at least 54 core radii from the filament's line (the
- * factor 1/sqrt(1 + (rc/h)^4) is within 5.9e-8 of 1); cut-off, targets at
- * least r from the segment with r^4 >= 2^24 d |L|^2. A screen of 32
- * filaments against a warp's targets decides. 0 for the FP64 path. */
+ * FP32c direct sum took the core-free form, where leaving the core out moves
+ * the pair term by no more than the FP32 rounding of forming it: Vatistas,
+ * targets at h from the filament's line and r from the segment with
+ * h^3 max(h, r) >= (54 rc)^4 (54 core radii, or fewer where r is larger);
+ * cut-off, targets at least r from the segment with r^4 >= 2^24 d |L|^2. A
+ * screen of 32 filaments against a warp's targets decides; the form also wants
+ * the filament 1.5 radii of the ball of the warp's targets away. 0 for the
+ * FP64 path. */
 int winds_bs_last_core_free(long long *pairs);
 
 /* 1 when the last winds_bs_eval_host / winds_bs_eval_device call's FP32c
  * direct sum ran on the chained filament stream, else 0. The chained stream
- * lays each line of connected filaments (the shed call's along the span, the
- * trailing call's along the wake age: BiotSavart calls of WInDS.m:150,153)
- * along one lane of consecutive pair records, so that each interaction takes
- * its second endpoint's inverse distance from the previous filament's first
- * one (one rsqrt fewer); the autotuner picks it or the input order per size
- * bucket together with the tiling (no reference counterpart: the reference's
- * kernel evaluates every filament on its own, BiotSavartMex.cu:131-193). */
+ * lays each family out along the index with more connected filaments (the shed
+ * call's along the span, the trailing call's along the wake age: BiotSavart
+ * calls of WInDS.m:150,153), so that each interaction takes its second
+ * endpoint's inverse distance from the previous filament's first one (one
+ * rsqrt fewer); input order does so only where consecutive filaments of the
+ * input are connected. The autotuner picks one of the two per size bucket
+ * together with the tiling (no reference counterpart: the reference's kernel
+ * evaluates every filament on its own, BiotSavartMex.cu:131-193). */
 int winds_bs_last_chained(int *chained);
 
 /* Synchronises `stream` (NULL: the library's stream) and reports a device-side
@@ -164,12 +167,13 @@ int winds_bs_sync(void *stream);
 
 /* Autotuner control. The first FP32 evaluation of a (core model, log2 targets,
  * log2 filaments) bucket on the library's own stream times the candidate
- * tilings (targets per thread T in {2,3,4}, filaments per tile KF in {32,64,128},
- * work-queue depth: items per resident warp) on both filament stream layouts
- * (input order and chained) and caches the fastest tiling and layout (T = 8
- * is settable). Evaluations on another stream, or with the autotuner off, use
- * the cached choice or the untuned default (T = 4, or 2 below 2048 targets;
- * KF = 64; input order).
+ * tilings (T in {2,3,4}: 2, 6 or 4 targets per lane; filaments per tile KF in
+ * {32,64}; work-queue depth: items per resident warp) on both filament stream
+ * layouts (input order and chained) and caches the fastest tiling and layout
+ * (T = 8, eight targets per lane, and KF = 128, which runs as 64, are
+ * settable). Evaluations on another stream, or with the autotuner off, use
+ * the cached choice or the untuned default (T = 4, 2 below 2048 targets, 3 from
+ * 49152; KF = 64; input order).
  * set_tuning / get_tuning read and write that cache directly (e.g. to restore
  * a saved choice). */
 int winds_bs_set_autotune(int on);

@@ -168,11 +168,6 @@ __device__ __forceinline__ void bbox_accumulate(const float lo[3], const float h
 }
 
 // ------------------------------------------------------- filament packing
-// Field q of filament f in the pair-record layout (bs_types.h).
-__device__ __forceinline__ float &pk_field(float4 *pk, long long f, int q) {
-  return reinterpret_cast<float *>(pk)[(f >> 1) * 32 + 2 * q + (f & 1)];
-}
-
 // Writes filament f in the packed layout (see bs_types.h): FP32 hi/lo x1,
 // |L|^2, near-singular radius Rn^2 = max(|L|^2, 9 rc^2), L, the core term and
 // K L (K = gamma/4pi), plus the FP64 copy. A NaN/Inf ubar is zeroed by the
@@ -183,10 +178,6 @@ __device__ __forceinline__ float &pk_field(float4 *pk, long long f, int q) {
 // Vatistas n=2 in FP32: with c = K L x r1, the core factor
 // |L x r1|^2 / sqrt(|L x r1|^4 + (rc^2 |L|^2)^2) equals |c|^2 / sqrt(|c|^4 + D)
 // for D = (K^2 rc^2 |L|^2)^2, so the kernel never multiplies by K.
-//
-// filament_fields computes the 16 FP32 fields; pack_filament writes them one
-// float at a time, store_pair_fields lets the two lanes of a pair write the
-// 128-byte record with four 16-byte stores each.
 __device__ __forceinline__ void filament_fields(double x1, double y1, double z1, double x2,
                                                 double y2, double z2, double g, double r,
                                                 int model, double dcut, float v[16]) {
@@ -212,12 +203,21 @@ __device__ __forceinline__ void filament_fields(double x1, double y1, double z1,
   if (!(Rn2 > 1e-20)) Rn2 = 1e-20;
   const float hx = (float)x1, hy = (float)y1, hz = (float)z1;
   v[0] = hx, v[1] = hy, v[2] = hz, v[3] = (float)L2;
-  v[4] = (float)(x1 - (double)hx), v[5] = (float)(y1 - (double)hy);
-  v[6] = (float)(z1 - (double)hz), v[7] = (float)Rn2;
-  v[8] = (float)Lx, v[9] = (float)Ly, v[10] = (float)Lz, v[11] = (float)D;
-  v[12] = (float)(K * Lx), v[13] = (float)(K * Ly), v[14] = (float)(K * Lz);
+  v[4] = (float)(K * Lx), v[5] = (float)(K * Ly), v[6] = (float)(K * Lz);
   // the core radius, for the kernel's screen of pairs whose core factor is 1
-  v[15] = model == kCoreVatistas && K != 0.0 ? (float)sqrt(fmax(r, 0.0)) : 0.f;
+  v[7] = model == kCoreVatistas && K != 0.0 ? (float)sqrt(fmax(r, 0.0)) : 0.f;
+  v[8] = (float)(x1 - (double)hx), v[9] = (float)(y1 - (double)hy);
+  v[10] = (float)(z1 - (double)hz), v[11] = (float)Rn2;
+  v[12] = (float)Lx, v[13] = (float)Ly, v[14] = (float)Lz, v[15] = (float)D;
+}
+
+// Stores the 16 fields as record f: chunk q of four floats at (q ^ ((f >> 2) & 3)).
+__device__ __forceinline__ void store_record(float4 *pk, long long f, const float v[16]) {
+  float4 *r = pk + 4 * f;
+  const int sw = (int)(f >> 2) & 3;
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+    r[q ^ sw] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
 }
 
 // Fields of an inert filament (far away, zero length, zero circulation) for padding.
@@ -226,54 +226,35 @@ __device__ __forceinline__ void inert_fields(float v[16]) {
 #pragma unroll
   for (int q = 0; q < 16; ++q) v[q] = 0.f;
   v[0] = v[1] = v[2] = far;
-  v[11] = 1.f;
+  v[3] = -0.f;  // a head: an infinite 1/r of the filament before must not reach it
+  v[15] = 1.f;
 }
 constexpr double kInertFar = 1e18;
 
+// rev: the FP32 record starts at x2 (x1 and x2 exchanged with the sign of the
+// circulation, the same term), for chains that share x1 with their predecessor.
+// head: its x2 is not the x1 of the record before (the sign of |L|^2).
 __device__ __forceinline__ void pack_filament(long long f, double x1, double y1, double z1,
                                               double x2, double y2, double z2, double g, double r,
-                                              int model, double dcut, float4 *pk, double4 *ra,
-                                              double4 *rb) {
+                                              bool rev, bool head, int model, double dcut,
+                                              float4 *pk, double4 *ra, double4 *rb) {
   ra[f] = make_double4(x1, y1, z1, g);
   rb[f] = make_double4(x2, y2, z2, r);
   float v[16];
-  filament_fields(x1, y1, z1, x2, y2, z2, g, r, model, dcut, v);
-#pragma unroll
-  for (int q = 0; q < 16; ++q) pk_field(pk, f, q) = v[q];
+  if (rev)
+    filament_fields(x2, y2, z2, x1, y1, z1, -g, r, model, dcut, v);
+  else
+    filament_fields(x1, y1, z1, x2, y2, z2, g, r, model, dcut, v);
+  if (head) v[3] = -v[3];
+  store_record(pk, f, v);
 }
 
 __device__ __forceinline__ void pack_inert(long long f, float4 *pk, double4 *ra, double4 *rb) {
   float v[16];
   inert_fields(v);
-#pragma unroll
-  for (int q = 0; q < 16; ++q) pk_field(pk, f, q) = v[q];
+  store_record(pk, f, v);
   ra[f] = make_double4(kInertFar, kInertFar, kInertFar, 0.0);
   rb[f] = make_double4(kInertFar, kInertFar, kInertFar, 0.0);
-}
-
-// Pair record of filaments f and f ^ 1 from the two lanes holding them (f even
-// on the even lane of the pair): every lane of the warp calls this; a lane
-// with `active` false stores nothing (its pair partner must be inactive too).
-// Float4 k of the record is {e[2k], o[2k], e[2k+1], o[2k+1]} (e, o the even
-// and odd filament's fields); the even lane stores k = 0..3, the odd lane 4..7.
-__device__ __forceinline__ void store_pair_fields(float4 *pk, long long f, const float v[16],
-                                                  bool active) {
-  const bool odd = (threadIdx.x & 1) != 0;
-  // x: the partner's fields this lane stores -- the odd filament's 0..7 on
-  // the even lane, the even filament's 8..15 on the odd lane
-  float x[8];
-#pragma unroll
-  for (int q = 0; q < 8; ++q) x[q] = __shfl_xor_sync(0xffffffffu, odd ? v[q] : v[q + 8], 1);
-  if (!active) return;
-  float4 *rec = pk + (f >> 1) * 8;
-  if (!odd) {
-#pragma unroll
-    for (int k = 0; k < 4; ++k) rec[k] = make_float4(v[2 * k], x[2 * k], v[2 * k + 1], x[2 * k + 1]);
-  } else {
-#pragma unroll
-    for (int k = 4; k < 8; ++k)
-      rec[k] = make_float4(x[2 * k - 8], v[2 * k], x[2 * k - 7], v[2 * k + 1]);
-  }
 }
 
 // ---------------------------------------------------- FP64 reference pair term

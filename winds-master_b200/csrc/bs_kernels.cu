@@ -3,22 +3,21 @@
 // BiotSavart_sh kernels of cuda/source/BiotSavartMex.cu:131-193.
 //
 // Kernels
-//   bs_pack_filaments  MATLAB-layout F1/F2/gamma/rc -> packed SoA float4 tiles
-//                      (+ FP64 copies), the device-side replacement of the host
-//                      crunch_f / crunch_rg packing (BiotSavartMex.cu:316-357)
-//   bs_chain_count,    the same records laid out along the wake's lines of
-//   bs_pack_chains     filaments (each lane of a record continuing the lane of
-//                      the record before: x2 = previous x1), with a head bit per
-//                      record where a line starts or the input has no link
+//   bs_chain_count,    MATLAB-layout F1/F2/gamma/rc -> 64-byte records (+ FP64
+//   bs_pack_filaments  copies), the device-side replacement of the host crunch_f
+//                      / crunch_rg packing (BiotSavartMex.cu:316-357), in input
+//                      order or laid out along the wake's lines of filaments
+//                      (x2 of a record = x1 of the one before, but for marked
+//                      heads where a line starts or the input has no link)
 //   bs_pack_targets    MATLAB-layout P -> double4 targets (crunch_p, :361-379)
 //   bs_f32c            persistent FP32 direct sum on independent warp workers:
 //                      each warp stages its filament tiles into its own shared
 //                      memory by bulk copies (cp.async.bulk + mbarrier), keeps
 //                      T register-resident targets per lane, Kahan-compensates
 //                      the per-target sums, and recomputes the near-singular
-//                      pairs in FP64 with all 32 lanes; on a chained stream
-//                      (CHAIN) each interaction reuses the previous record's
-//                      endpoint rsqrt
+//                      pairs in FP64 with all 32 lanes; each interaction
+//                      reuses the previous record's endpoint rsqrt, and groups
+//                      distant from the warp's targets run in an expanded form
 //   bs_f64             plain FP64 direct sum (the comparison GPU path)
 //   bs_reduce          deterministic sum of the per-chunk partials, written in
 //                      MATLAB layout (reassem_uind, :383-401)
@@ -43,47 +42,17 @@ __global__ void bs_bbox_init(BBox *bb) {
   }
 }
 
-__global__ void bs_pack_filaments(const double *__restrict__ F1, const double *__restrict__ F2,
-                                  const double *__restrict__ gam, const double *__restrict__ rc,
-                                  long long d0, long long nf, long long off, int model, double dcut,
-                                  float4 *pk, double4 *ra,
-                                  double4 *rb, BBox *bb) {
-  const long long f = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
-  if (f < nf) {
-    const long long j = f / d0, i = f - j * d0;
-    const long long b = i + d0 * 3 * j;
-    const double x1 = F1[b], y1 = F1[b + d0], z1 = F1[b + 2 * d0];
-    const double x2 = F2[b], y2 = F2[b + d0], z2 = F2[b + 2 * d0];
-    const double g = gam[f], r = rc[f];
-    pack_filament(off + f, x1, y1, z1, x2, y2, z2, g, r, model, dcut, pk, ra, rb);
-    lo[0] = (float)fmin(x1, x2), lo[1] = (float)fmin(y1, y2), lo[2] = (float)fmin(z1, z2);
-    hi[0] = (float)fmax(x1, x2), hi[1] = (float)fmax(y1, y2), hi[2] = (float)fmax(z1, z2);
-  }
-  bbox_accumulate(lo, hi, bb->fmin, bb->fmax);
-}
-
-// Inert filaments filling [from, to): far away, zero length, zero circulation.
-__global__ void bs_pad_filaments(long long from, long long to, float4 *pk, double4 *ra,
-                                 double4 *rb) {
-  const long long f = from + (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= to) return;
-  pack_inert(f, pk, ra, rb);
-}
-
-// ------------------------------------------------------- chained packing
 // WInDS's filaments meet at the wake's nodes: the shed call's F2(i) is its
 // F1(i+1) (WInDS.m:150, along the first index) and the trailing call's
-// F2(:,:,j) is its F1(:,:,j-1) (WInDS.m:153, along the third). Laid out so that
-// each lane of a pair record follows one such line -- x2 of record r equal to
-// x1 of record r - 1 -- the FP32 kernel reuses the previous record's endpoint
-// term (interact_chain). bs_chain_count counts, per family, the filaments
-// whose end is bitwise the start of their neighbour along each index;
-// bs_pack_chains lays the family out along the index with more such links,
-// lines paired in the two lanes of the records, and flags every record where
-// either lane does not continue its predecessor (a head). Any layout of the
-// input is evaluated correctly: a filament that does not continue a chain is
-// a head, which the kernel evaluates from its own L.
+// F2(:,:,j) is its F1(:,:,j-1) (WInDS.m:153, along the third). The FP32 records
+// go along such a line, each with the end it shares with its predecessor as its
+// second end, so that the kernel reuses the predecessor's endpoint term
+// (interact). Two orders: the input's own (a chain along the first index), and,
+// where the family has more links along the third index, line by line along
+// that one. bs_chain_count counts, per family, the filaments whose end is
+// bitwise the start of their neighbour along each index. A record whose end is
+// not its predecessor's is a head (marked in the record): the kernel evaluates
+// the end from its own L, so any input is evaluated correctly.
 __device__ __forceinline__ bool same_point(const double *__restrict__ F2, long long b2,
                                            const double *__restrict__ F1, long long b1,
                                            long long d0) {
@@ -109,81 +78,45 @@ __global__ void bs_chain_count(const double *__restrict__ F1, const double *__re
   }
 }
 
-// Records of nl lines of len filaments: pairs of lines side by side, and an
-// odd last line split in two halves side by side.
-__host__ __device__ __forceinline__ long long chain_layout_records(long long nl, long long len) {
-  return nl / 2 * len + (nl & 1) * ((len + 1) / 2);
-}
-
-// One thread per lane slot of the family's nrec records from record rec_off:
-// slot 2 r + h is lane h of record r. Order along the third index when cnt[1]
-// > cnt[0] (lines (i, b), position k = j), else along the first (lines (j, b),
-// position k = d0 - 1 - i). Line 2 m + h fills lane h of the m-th run of `len`
-// records; an odd last line fills lane 0 with its first (len + 1) / 2
-// positions and lane 1 with the rest. Slots past the lines are inert heads.
-__global__ void bs_pack_chains(const double *__restrict__ F1, const double *__restrict__ F2,
-                               const double *__restrict__ gam, const double *__restrict__ rc,
-                               long long d0, long long d2, long long d3, long long rec_off,
-                               long long nrec, const unsigned long long *__restrict__ cnt,
-                               int model, double dcut, float4 *pk, double4 *ra, double4 *rb,
-                               unsigned *heads, BBox *bb) {
-  const long long slot = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+// One thread per filament of the family, in input order; its record goes to
+// slot off + f, or (cnt given and cnt[1] > cnt[0]) to its place along the third
+// index.
+__global__ void bs_pack_filaments(const double *__restrict__ F1, const double *__restrict__ F2,
+                                  const double *__restrict__ gam, const double *__restrict__ rc,
+                                  long long d0, long long d2, long long nf, long long off,
+                                  const unsigned long long *__restrict__ cnt, int model,
+                                  double dcut, float4 *pk, double4 *ra, double4 *rb, BBox *bb) {
+  const long long f = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
-  if (slot < 2 * nrec) {
-    const bool along3 = cnt[1] > cnt[0];
-    const long long nl = along3 ? d0 * d3 : d2 * d3;
-    const long long len = along3 ? d2 : d0;
-    const long long r = slot >> 1;
-    const long long h = slot & 1;
-    const long long f = 2 * rec_off + slot;  // packed filament index
-    long long k = 0, run = 0, line = -1;      // position in the line, in this lane's run
-    const long long full = nl / 2 * len, half = (len + 1) / 2;
-    if (r < full) {
-      const long long m = r / len;
-      run = k = r - m * len;
-      line = 2 * m + h;
-    } else if ((nl & 1) && r < full + half) {
-      run = r - full;
-      k = run + h * half;
-      if (k < len) line = nl - 1;
-    }
+  if (f < nf) {
+    const bool along3 = cnt && cnt[1] > cnt[0];
+    const long long jb = f / d0, i = f - jb * d0;
+    const long long b = i + d0 * 3 * jb;
+    const double x1 = F1[b], y1 = F1[b + d0], z1 = F1[b + 2 * d0];
+    const double x2 = F2[b], y2 = F2[b + d0], z2 = F2[b + 2 * d0];
+    long long slot = off + f;
     bool head;
-    if (line >= 0 && line < nl) {
-      long long i, jb;
-      if (along3) {
-        const long long bl = line / d0;
-        i = line - bl * d0;
-        jb = k + d2 * bl;
-      } else {
-        i = d0 - 1 - k;
-        jb = line;
-      }
-      const long long b = i + d0 * 3 * jb;
-      const double x1 = F1[b], y1 = F1[b + d0], z1 = F1[b + 2 * d0];
-      const double x2 = F2[b], y2 = F2[b + d0], z2 = F2[b + 2 * d0];
-      const long long src = i + d0 * jb;
-      pack_filament(f, x1, y1, z1, x2, y2, z2, gam[src], rc[src], model, dcut, pk, ra, rb);
-      lo[0] = (float)fmin(x1, x2), lo[1] = (float)fmin(y1, y2), lo[2] = (float)fmin(z1, z2);
-      hi[0] = (float)fmax(x1, x2), hi[1] = (float)fmax(y1, y2), hi[2] = (float)fmax(z1, z2);
-      // the predecessor in the line is (i, j-1) along the third index, (i+1, j) along the first
-      head = run == 0 || !(along3 ? same_point(F2, b, F1, b - 3 * d0, d0)
-                                  : same_point(F2, b, F1, b + 1, d0));
+    if (along3) {
+      const long long bl = jb / d2, j = jb - bl * d2;
+      slot = off + j + d2 * (i + d0 * bl);
+      head = !(j >= 1 && same_point(F2, b, F1, b - 3 * d0, d0));
     } else {
-      pack_inert(f, pk, ra, rb);
-      head = true;  // never continues a real lane (its x2 would not be its own)
+      head = !(i >= 1 && same_point(F2, b - 1, F1, b, d0));
     }
-    if (head) atomicOr(heads + (f >> 6), 1u << ((f >> 1) & 31));
+    pack_filament(slot, x1, y1, z1, x2, y2, z2, gam[f], rc[f], !along3, head, model, dcut, pk, ra,
+                  rb);
+    lo[0] = (float)fmin(x1, x2), lo[1] = (float)fmin(y1, y2), lo[2] = (float)fmin(z1, z2);
+    hi[0] = (float)fmax(x1, x2), hi[1] = (float)fmax(y1, y2), hi[2] = (float)fmax(z1, z2);
   }
   bbox_accumulate(lo, hi, bb->fmin, bb->fmax);
 }
 
-// Inert filaments filling [from, to) of a chained stream, their records heads.
-__global__ void bs_pad_chains(long long from, long long to, float4 *pk, double4 *ra, double4 *rb,
-                              unsigned *heads) {
+// Inert filaments filling [from, to): far away, zero length, zero circulation.
+__global__ void bs_pad_filaments(long long from, long long to, float4 *pk, double4 *ra,
+                                 double4 *rb) {
   const long long f = from + (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= to) return;
   pack_inert(f, pk, ra, rb);
-  atomicOr(heads + (f >> 6), 1u << ((f >> 1) & 31));
 }
 
 __global__ void bs_pack_targets(const double *__restrict__ P, long long ns, long long np,
@@ -213,23 +146,55 @@ __device__ __forceinline__ unsigned long long spread3(unsigned v) {
   return x;
 }
 
-// Sort key of a target: group id above a 30-bit Morton code of its position
-// in the targets' bounding box (bit 31: the target is unused).
+// Distance along a 3-D Hilbert curve of 10 bits a coordinate (Skilling's
+// transpose algorithm, "Programming the Hilbert curve", AIP Conf. Proc. 707,
+// 2004). Consecutive targets on it are neighbours in space without exception,
+// where a Morton code jumps at every power of two: on the large wake the
+// radius of 96 consecutive targets is 9.1 m (median; largest 34 m) instead of
+// 10.1 m (82 m).
+__device__ __forceinline__ unsigned long long hilbert30(unsigned x, unsigned y, unsigned z) {
+  unsigned X[3] = {x, y, z};
+#pragma unroll
+  for (unsigned Q = 512u; Q > 1u; Q >>= 1) {
+    const unsigned m = Q - 1u;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      if (X[c] & Q) {
+        X[0] ^= m;
+      } else {
+        const unsigned t = (X[0] ^ X[c]) & m;
+        X[0] ^= t;
+        X[c] ^= t;
+      }
+    }
+  }
+  X[1] ^= X[0];
+  X[2] ^= X[1];
+  unsigned t = 0;
+#pragma unroll
+  for (unsigned Q = 512u; Q > 1u; Q >>= 1)
+    if (X[2] & Q) t ^= Q - 1u;
+  return spread3(X[0] ^ t) << 2 | spread3(X[1] ^ t) << 1 | spread3(X[2] ^ t);
+}
+
+// Sort key of a target: group id above the 30-bit Hilbert position in the
+// targets' bounding box (bit 31: the target is unused).
 __global__ void bs_target_keys(const double4 *__restrict__ tp, const int *__restrict__ tgroup,
                                long long n, const BBox *bb, unsigned long long *keys, int *vals) {
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
   const double4 p = tp[t];
   const double q[3] = {p.x, p.y, p.z};
-  unsigned long long code = 0;
+  unsigned cell[3];
   for (int c = 0; c < 3; ++c) {
     const double lo = key_float(bb->tmin[c]), hi = key_float(bb->tmax[c]);
     const double w = hi > lo ? hi - lo : 1.0;
     double u = (q[c] - lo) / w * 1023.999;
     if (!(u >= 0.0)) u = 0.0;  // also catches NaN
     if (u > 1023.0) u = 1023.0;
-    code |= spread3((unsigned)u) << c;
+    cell[c] = (unsigned)u;
   }
+  unsigned long long code = hilbert30(cell[0], cell[1], cell[2]);
   // a target marked unused (w != 0: past a growing wake's live columns) sorts
   // after every live target of its group
   if (p.w != 0.0) code |= 1ull << 31;
@@ -280,23 +245,40 @@ constexpr uint64_t kDefaultWaitNs = 2000000000ull;  // 2 s per tile: far above a
 
 template <int KF>
 struct StageSmem {
-  static constexpr int kBytes = KF * 64;  // KF/2 pair records of 128 B
-  // stages in flight: a warp's tile takes ~10-50 us, a bulk copy ~2 us, so
-  // one stage ahead suffices; three for the short 32-filament tiles
-  static constexpr int kStages = KF >= 64 ? 2 : 3;
-  // tiles per Kahan fold: the FP32 partial sums span 128 filaments
-  static constexpr int kFold = KF >= 128 ? 1 : 128 / KF;
+  static constexpr int kBytes = KF * 64;
+  // two stages: a warp's tile takes ~5-50 us, a bulk copy ~2 us
+  static constexpr int kStages = 2;
+  // tiles per Kahan fold: the FP32 partial sums span 64 filaments
+static constexpr int kFold = 64 / KF;
 };
 
 // Shared memory of one worker: its filament stages, the Kahan state of its
-// targets (sum, compensation) x 3 components as floats, the near-singular bit
-// words of the current tile (KF/4 words per lane), its full[s] barriers
-// (bytes landed) and its target ball (centre, radius, threshold).
+// targets (sum, compensation) x 3 components as floats, the targets themselves
+// relative to their lane's centre (component c of the lane's target t at
+// (c T + t) 32 + lane), the near-singular bits of the current tile (a word per
+// lane and group of four filaments), its full[s] barriers (bytes landed) and its target ball
+// (centre, radius, threshold).
+template <int T>
+struct NearBits {
+  using type = unsigned;  // bit 8 j + t: filament j of the group, target t
+  static constexpr int kPer = 8;
+};
+template <>
+struct NearBits<2> {
+  using type = unsigned short;
+  static constexpr int kPer = 4;
+};
+template <>
+struct NearBits<4> {
+  using type = unsigned short;
+  static constexpr int kPer = 4;
+};
+
 template <int T, int KF>
 __host__ __device__ constexpr size_t warp_smem_bytes() {
   constexpr int S = StageSmem<KF>::kStages;
-  return ((size_t)S * StageSmem<KF>::kBytes + (size_t)6 * 32 * T * sizeof(float) +
-          (size_t)(KF / 4) * 32 * sizeof(unsigned) + S * sizeof(uint64_t) + 8 * sizeof(float) +
+  return ((size_t)S * StageSmem<KF>::kBytes + (size_t)9 * 32 * T * sizeof(float) +
+          (size_t)(KF / 4) * 32 * sizeof(typename NearBits<T>::type) + S * sizeof(uint64_t) + 8 * sizeof(float) +
           127) / 128 * 128;
 }
 
@@ -318,7 +300,7 @@ template <int KF>
 __device__ __forceinline__ void issue_stage(const F32cArgs &a, unsigned char *stage, uint64_t *bar,
                                             int f0) {
   mbar_arrive_expect_tx(bar, StageSmem<KF>::kBytes);
-  bulk_g2s(stage, a.pk + (size_t)(f0 / 2) * 8, KF * 64, bar);
+  bulk_g2s(stage, a.pk + (size_t)f0 * 4, KF * 64, bar);
 }
 
 // Orders this thread's earlier shared-memory accesses (generic proxy) before
@@ -328,12 +310,15 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
 }
 
 // ----------------------------------------------------- packed FP32 arithmetic
-// The direct sum runs on pairs of filaments: every FP32 operation is a packed
-// f32x2 instruction (two independent IEEE operations, round to nearest) on the
-// two filaments of a pair record, so one issue slot does two interactions'
-// worth of arithmetic; the FMA pipe, not instruction issue, bounds the loop.
-__device__ __forceinline__ float2 lo2(const float4 v) { return make_float2(v.x, v.y); }
-__device__ __forceinline__ float2 hi2(const float4 v) { return make_float2(v.z, v.w); }
+// The direct sum runs on pairs of targets: every FP32 operation is a packed
+// f32x2 instruction (two independent IEEE operations, round to nearest) on two
+// of a lane's targets, so one issue slot does two interactions' worth of
+// arithmetic. A filament's field goes to both halves of the instruction from
+// one register (bc costs no instruction), and a target holds 12 registers: with
+// the filaments in the two halves instead, the broadcast targets and the
+// double sums took 24 a target and capped the kernel at three warps a
+// scheduler, where latency, not the FMA pipe, bounded it.
+__device__ __forceinline__ float2 bc(const float v) { return make_float2(v, v); }
 __device__ __forceinline__ float2 neg2(const float2 v) { return make_float2(-v.x, -v.y); }
 __device__ __forceinline__ float2 rsqrt2(const float2 v) {
   return make_float2(rsqrt_approx(v.x), rsqrt_approx(v.y));
@@ -342,74 +327,63 @@ __device__ __forceinline__ float2 rcp2(const float2 v) {
   return make_float2(rcp_approx(v.x), rcp_approx(v.y));
 }
 
-// One filament pair of a stage, relative to this thread's centre c.
-struct Fil2 {
-  float2 qx, qy, qz;  // x1 - c (from the hi/lo split)
-  float2 Lx, Ly, Lz, L2, D;
-  float2 Mx, My, Mz;  // K L, K = gamma/4pi
-  float2 Rn2;         // near-singular threshold (careful path)
+// One filament of a stage, relative to this lane's centre c.
+struct Fil {
+  float qx, qy, qz;  // x1 - c (from the hi/lo split)
+  float Lx, Ly, Lz, L2, D;
+  float Mx, My, Mz;  // K L, K = gamma/4pi
+  float Rn2;         // near-singular threshold (careful path)
 };
 
-// Pair record r (8 float4, layout in bs_types.h) into registers.
-__device__ __forceinline__ void load_pair(const float4 *r, float2 ncx, float2 ncy, float2 ncz,
-                                          Fil2 &f) {
-  const float4 a0 = r[0], a1 = r[1], b0 = r[2], b1 = r[3];
-  const float4 l0 = r[4], l1 = r[5], m0 = r[6], m1 = r[7];
-  f.qx = __fadd2_rn(__fadd2_rn(lo2(a0), ncx), lo2(b0));
-  f.qy = __fadd2_rn(__fadd2_rn(hi2(a0), ncy), hi2(b0));
-  f.qz = __fadd2_rn(__fadd2_rn(lo2(a1), ncz), lo2(b1));
-  f.L2 = hi2(a1);
-  f.Rn2 = hi2(b1);
-  f.Lx = lo2(l0);
-  f.Ly = hi2(l0);
-  f.Lz = lo2(l1);
-  f.D = hi2(l1);
-  f.Mx = lo2(m0);
-  f.My = hi2(m0);
-  f.Mz = lo2(m1);
+// Filament record (4 float4, layout in bs_types.h) whose chunk q is at r[q ^ sw].
+__device__ __forceinline__ Fil load_filament(const float4 *r, int sw, float cx, float cy,
+                                             float cz) {
+  const float4 a = r[0 ^ sw], b = r[1 ^ sw], c = r[2 ^ sw], d = r[3 ^ sw];
+  Fil f;
+  f.qx = (a.x - cx) + c.x;
+  f.qy = (a.y - cy) + c.y;
+  f.qz = (a.z - cz) + c.z;
+  f.L2 = fabsf(a.w);
+  f.Mx = b.x, f.My = b.y, f.Mz = b.z;
+  f.Rn2 = c.w;
+  f.Lx = d.x, f.Ly = d.y, f.Lz = d.z, f.D = d.w;
+  return f;
 }
 
-// Internal form code of interact2: the pair term with its core left out,
-// (i1 + i2) i1 i2 / e, for pairs where the core changes it by less than
-// FP32's unit roundoff 2^-24. Vatistas: the warp screen places the targets
-// at least kCoreFreeRatio core radii from the filament's line, where the
-// factor 1/sqrt(1 + (rc/h)^4) is within (1/54)^4 / 2 = 5.9e-8 of 1.
-// Cut-off: the targets are at least r from the segment with
-// r^4 >= 2^24 d |L|^2, so the denominator's d |L|^2 gg^2 <= 2^-24 <= 2^-24 e
-// (e >= 1 on the far path, where r1.r2 > 0).
-constexpr int kCoreFree = 2;
-constexpr float kCoreFreeRatio = 54.f;
-constexpr float kCutoffFreeSq = 4096.f;  // r^2 >= 4096 sqrt(d |L|^2) is r^4 >= 2^24 d |L|^2
-
-// One target against one filament pair, accumulated into the packed sums
-// (ax, ay, az) (one lane per filament of the pair). (npx, npy, npz) = -(P - c)
-// broadcast to both lanes. With NEAR it also tests r1.r2 < Rn^2 per lane: such
-// terms are zeroed and recorded in `bits` (bit0 for the pair's first
-// filament, bit1 for its second); they are redone in FP64 after the tile.
-template <int MODEL, bool CO, bool NEAR>
-__device__ __forceinline__ void interact2(float2 npx, float2 npy, float2 npz, const Fil2 &f,
-                                          float2 Rn2, float co2, float2 &ax, float2 &ay,
-                                          float2 &az, unsigned &bits, unsigned bit0,
-                                          unsigned bit1) {
-  const float2 nx = __fadd2_rn(f.qx, npx);  // x1 - P = -r1
-  const float2 ny = __fadd2_rn(f.qy, npy);
-  const float2 nz = __fadd2_rn(f.qz, npz);
+// Two targets against one filament, added to (ax, ay, az) (one half per
+// target). (npx, npy, npz) = -(P - c). Terms with r1.r2 < Rn2 are zeroed and
+// recorded in `bits` (bit0 for the pair's first target, bit1 for its second);
+// they are redone in FP64 after the tile. So are zeroed, for good, the terms
+// beyond the reach cut-off (both ends farther than co2, squared).
+//
+// The filaments form chains: x2 of a record is x1 of the record before it --
+// the wake's filaments meet at its nodes -- so 1/|x2 - P| is the previous
+// record's 1/|x1 - P|, carried in `ti`, and a record needs no rsqrt for it.
+// Before a record that starts a chain, chain_start puts 1/|x2 - P| into the
+// carry. 1/|x1 - P| is left there for the next record.
+template <int MODEL>
+__device__ __forceinline__ void interact(float2 npx, float2 npy, float2 npz, const Fil &f,
+                                         float Rn2, float co2, float2 &ax, float2 &ay, float2 &az,
+                                         unsigned &bits, unsigned bit0, unsigned bit1, float2 &ti) {
+  const float2 nx = __fadd2_rn(bc(f.qx), npx);  // x1 - P = -r1
+  const float2 ny = __fadd2_rn(bc(f.qy), npy);
+  const float2 nz = __fadd2_rn(bc(f.qz), npz);
   float2 r1s = __fmul2_rn(nx, nx);
   r1s = __ffma2_rn(ny, ny, r1s);
   r1s = __ffma2_rn(nz, nz, r1s);
-  float2 ld = __fmul2_rn(f.Lx, nx);  // -L.r1
-  ld = __ffma2_rn(f.Ly, ny, ld);
-  ld = __ffma2_rn(f.Lz, nz, ld);
-  const float2 dot = __fadd2_rn(r1s, ld);                   // r1 . r2
-  const float2 r2s = __fadd2_rn(dot, __fadd2_rn(f.L2, ld));  // |r1 - L|^2
-  const float2 i1 = rsqrt2(r1s), i2 = rsqrt2(r2s);
+  float2 ld = __fmul2_rn(bc(f.Lx), nx);  // -L.r1
+  ld = __ffma2_rn(bc(f.Ly), ny, ld);
+  ld = __ffma2_rn(bc(f.Lz), nz, ld);
+  const float2 dot = __fadd2_rn(r1s, ld);                        // r1 . r2
+  const float2 r2s = __fadd2_rn(dot, __fadd2_rn(bc(f.L2), ld));  // |r1 - L|^2
+  const float2 i1 = rsqrt2(r1s), i2 = ti;
   const float2 gg = __fmul2_rn(i1, i2);
-  const float2 e = __ffma2_rn(dot, gg, make_float2(1.f, 1.f));  // 1 + cos(theta)
+  const float2 e = __ffma2_rn(dot, gg, bc(1.f));  // 1 + cos(theta)
   // K (r1 x r2) = K L x r1 = (x1 - P) x (K L): no cancellation for far or
   // collinear points
-  const float2 cx = __ffma2_rn(ny, f.Mz, __fmul2_rn(nz, neg2(f.My)));
-  const float2 cy = __ffma2_rn(nz, f.Mx, __fmul2_rn(nx, neg2(f.Mz)));
-  const float2 cz = __ffma2_rn(nx, f.My, __fmul2_rn(ny, neg2(f.Mx)));
+  const float2 cx = __ffma2_rn(ny, bc(f.Mz), __fmul2_rn(nz, bc(-f.My)));
+  const float2 cy = __ffma2_rn(nz, bc(f.Mx), __fmul2_rn(nx, bc(-f.Mz)));
+  const float2 cz = __ffma2_rn(nx, bc(f.My), __fmul2_rn(ny, bc(-f.Mx)));
   float2 ub;
   if (MODEL == kCoreVatistas) {
     // Cnu / (r1 r2 (r1 r2 + r1.r2)) with h^2 = |L x r1|^2/|L|^2 and rc^4 folded:
@@ -417,98 +391,23 @@ __device__ __forceinline__ void interact2(float2 npx, float2 npy, float2 npz, co
     float2 c2 = __fmul2_rn(cx, cx);
     c2 = __ffma2_rn(cy, cy, c2);
     c2 = __ffma2_rn(cz, cz, c2);
-    const float2 q = __ffma2_rn(c2, c2, f.D);
+    const float2 q = __ffma2_rn(c2, c2, bc(f.D));
     const float2 w = __fmul2_rn(__fmul2_rn(__fadd2_rn(i1, i2), gg), c2);
     ub = __fmul2_rn(w, rsqrt2(__fmul2_rn(__fmul2_rn(e, e), q)));
-  } else if (MODEL == kCoreFree) {
-    // (r1+r2)/(r1r2(r1r2+r1.r2)) = (i1+i2) gg / e
-    ub = __fmul2_rn(__fmul2_rn(__fadd2_rn(i1, i2), gg), rcp2(e));
   } else {
     // (r1+r2)/(r1r2(r1r2+r1.r2) + d|L|^2) = (i1+i2) gg / (e + d|L|^2 gg^2)
     ub = __fmul2_rn(__fmul2_rn(__fadd2_rn(i1, i2), gg),
-                    rcp2(__ffma2_rn(f.D, __fmul2_rn(gg, gg), e)));
+                    rcp2(__ffma2_rn(bc(f.D), __fmul2_rn(gg, gg), e)));
   }
-  if (NEAR) {
-    if (dot.x < Rn2.x) {
-      bits |= bit0;
-      ub.x = 0.f;
-    }
-    if (dot.y < Rn2.y) {
-      bits |= bit1;
-      ub.y = 0.f;
-    }
+  if (fminf(r1s.x, r2s.x) > co2) ub.x = 0.f;
+  if (fminf(r1s.y, r2s.y) > co2) ub.y = 0.f;
+  if (dot.x < Rn2) {
+    bits |= bit0;
+    ub.x = 0.f;
   }
-  if (CO) {
-    if (fminf(r1s.x, r2s.x) > co2) ub.x = 0.f;
-    if (fminf(r1s.y, r2s.y) > co2) ub.y = 0.f;
-  }
-  ax = __ffma2_rn(ub, cx, ax);
-  ay = __ffma2_rn(ub, cy, ay);
-  az = __ffma2_rn(ub, cz, az);
-}
-
-// interact2 on chained pair records. In a chained stream the second endpoint
-// of each filament (per lane of the record) is the first endpoint of the same
-// lane's filament in the previous record -- the wake's filaments meet at its
-// nodes -- so 1/|x2 - P| is the previous record's 1/|x1 - P|, carried in `ti`:
-// a chained record needs neither |r2|^2 nor its rsqrt (two FP32 operations and
-// one MUFU result fewer per interaction). A record that starts a chain (HEAD)
-// forms them from L as interact2 does. Either way 1/|x1 - P| is left in `ti`
-// for the next record.
-template <int MODEL, bool CO, bool NEAR, bool HEAD>
-__device__ __forceinline__ void interact_chain(float2 npx, float2 npy, float2 npz, const Fil2 &f,
-                                               float2 Rn2, float co2, float2 &ax, float2 &ay,
-                                               float2 &az, unsigned &bits, unsigned bit0,
-                                               unsigned bit1, float2 &ti) {
-  const float2 nx = __fadd2_rn(f.qx, npx);  // x1 - P = -r1
-  const float2 ny = __fadd2_rn(f.qy, npy);
-  const float2 nz = __fadd2_rn(f.qz, npz);
-  float2 r1s = __fmul2_rn(nx, nx);
-  r1s = __ffma2_rn(ny, ny, r1s);
-  r1s = __ffma2_rn(nz, nz, r1s);
-  float2 ld = __fmul2_rn(f.Lx, nx);  // -L.r1
-  ld = __ffma2_rn(f.Ly, ny, ld);
-  ld = __ffma2_rn(f.Lz, nz, ld);
-  const float2 dot = __fadd2_rn(r1s, ld);  // r1 . r2
-  float2 r2s, i2;
-  if (HEAD || CO) r2s = __fadd2_rn(dot, __fadd2_rn(f.L2, ld));  // |r1 - L|^2
-  if (HEAD)
-    i2 = rsqrt2(r2s);
-  else
-    i2 = ti;
-  const float2 i1 = rsqrt2(r1s);
-  const float2 gg = __fmul2_rn(i1, i2);
-  const float2 e = __ffma2_rn(dot, gg, make_float2(1.f, 1.f));  // 1 + cos(theta)
-  const float2 cx = __ffma2_rn(ny, f.Mz, __fmul2_rn(nz, neg2(f.My)));
-  const float2 cy = __ffma2_rn(nz, f.Mx, __fmul2_rn(nx, neg2(f.Mz)));
-  const float2 cz = __ffma2_rn(nx, f.My, __fmul2_rn(ny, neg2(f.Mx)));
-  float2 ub;
-  if (MODEL == kCoreVatistas) {
-    float2 c2 = __fmul2_rn(cx, cx);
-    c2 = __ffma2_rn(cy, cy, c2);
-    c2 = __ffma2_rn(cz, cz, c2);
-    const float2 q = __ffma2_rn(c2, c2, f.D);
-    const float2 w = __fmul2_rn(__fmul2_rn(__fadd2_rn(i1, i2), gg), c2);
-    ub = __fmul2_rn(w, rsqrt2(__fmul2_rn(__fmul2_rn(e, e), q)));
-  } else if (MODEL == kCoreFree) {
-    ub = __fmul2_rn(__fmul2_rn(__fadd2_rn(i1, i2), gg), rcp2(e));
-  } else {
-    ub = __fmul2_rn(__fmul2_rn(__fadd2_rn(i1, i2), gg),
-                    rcp2(__ffma2_rn(f.D, __fmul2_rn(gg, gg), e)));
-  }
-  if (NEAR) {
-    if (dot.x < Rn2.x) {
-      bits |= bit0;
-      ub.x = 0.f;
-    }
-    if (dot.y < Rn2.y) {
-      bits |= bit1;
-      ub.y = 0.f;
-    }
-  }
-  if (CO) {
-    if (fminf(r1s.x, r2s.x) > co2) ub.x = 0.f;
-    if (fminf(r1s.y, r2s.y) > co2) ub.y = 0.f;
+  if (dot.y < Rn2) {
+    bits |= bit1;
+    ub.y = 0.f;
   }
   ax = __ffma2_rn(ub, cx, ax);
   ay = __ffma2_rn(ub, cy, ay);
@@ -516,34 +415,145 @@ __device__ __forceinline__ void interact_chain(float2 npx, float2 npy, float2 np
   ti = i1;
 }
 
-// One chained pair record against the lane's T targets, in form FORM
-// (kCoreFree, or the kernel's model), the record starting a chain or not.
-template <int T, int FORM, bool CO, bool NEAR>
-__device__ __forceinline__ void chain_record(const float4 *rec, bool head, float2 ncx, float2 ncy,
-                                             float2 ncz, const float2 (&npx)[T],
-                                             const float2 (&npy)[T], const float2 (&npz)[T],
-                                             float S2, float co2, float2 (&ax)[T],
-                                             float2 (&ay)[T], float2 (&az)[T], float2 (&ti)[T],
-                                             unsigned &nbits, int j) {
-  Fil2 f;
-  load_pair(rec, ncx, ncy, ncz, f);
-  // near-singular threshold, raised for threads whose targets spread far
-  // from their centre (as in the unchained careful path)
-  const float2 Rn2 = NEAR ? make_float2(fmaxf(f.Rn2.x, S2), fmaxf(f.Rn2.y, S2)) : f.Rn2;
-  if (head) {
+// The carry of a record that starts a chain: 1/|x2 - P| from its own x1 and L.
+template <int NP>
+__device__ __forceinline__ void chain_start(const Fil &f, const float2 (&npx)[NP],
+                                            const float2 (&npy)[NP], const float2 (&npz)[NP],
+                                            float2 (&ti)[NP]) {
+  const float ex = f.qx + f.Lx, ey = f.qy + f.Ly, ez = f.qz + f.Lz;
 #pragma unroll
-    for (int t = 0; t < T; ++t)
-      interact_chain<FORM, CO, NEAR, true>(npx[t], npy[t], npz[t], f, Rn2, co2, ax[t], ay[t],
-                                           az[t], nbits, 1u << (8 * (2 * j) + t),
-                                           1u << (8 * (2 * j + 1) + t), ti[t]);
-  } else {
-#pragma unroll
-    for (int t = 0; t < T; ++t)
-      interact_chain<FORM, CO, NEAR, false>(npx[t], npy[t], npz[t], f, Rn2, co2, ax[t], ay[t],
-                                            az[t], nbits, 1u << (8 * (2 * j) + t),
-                                            1u << (8 * (2 * j + 1) + t), ti[t]);
+  for (int p = 0; p < NP; ++p) {
+    const float2 nx = __fadd2_rn(bc(ex), npx[p]), ny = __fadd2_rn(bc(ey), npy[p]),
+                 nz = __fadd2_rn(bc(ez), npz[p]);
+    float2 r2s = __fmul2_rn(nx, nx);
+    r2s = __ffma2_rn(ny, ny, r2s);
+    r2s = __ffma2_rn(nz, nz, r2s);
+    ti[p] = rsqrt2(r2s);
   }
 }
+
+// ------------------------------------------------------------ distant form
+// A filament is distant when its endpoints are at least kDistantRatio radii
+// from the centre w of the ball of the warp's targets (and it is far, as the
+// screen defines it). Everything is then expanded about w. With q = x1 - w,
+// p = P - w, r1 = |x1 - P|, r2 = |x2 - P|, M = K L:
+//     |x1 - P|^2  = |q|^2 + |p|^2 - 2 q.p                       (4 operations)
+//     r1r2 + r1.r2 = ((r1 + r2)^2 - |L|^2) / 2                  (no dot product)
+//     K L x r1     = q x M - p x M
+// |q|^2, q x M and the rest are per filament and warp, not per lane: each lane
+// prepares one filament of the 32 it screens, in place of the record's fields
+// that the loop no longer needs.
+//
+// Core-free filaments, whose core changes no term by more than the roundoff
+// that forming the term has anyway, go further: the sum over filaments of
+// ub (x1 - P) x M is  B - p x A  with A = sum ub M, B = sum ub (q x M), so the
+// cross product leaves the pair loop, and an interaction costs 16 FP32
+// operations and two MUFU results, against 33 and 6 per filament and lane in
+// the form above. With the core it costs 28 (Vatistas, whose factor needs
+// |K L x r1|^2) or 17 (cut-off).
+//   Vatistas  the factor 1/sqrt(1 + (rc/h)^4), h the distance from the
+//             filament's line, is short of 1 by at most (rc/h)^4 / 2 and the
+//             term's cross product is |M| h, so leaving it out moves the term
+//             by ub |M| rc^4 / (2 h^3), where rounding moves it by about
+//             2^-24 ub |M| r: kCoreFree4 rc^4 <= h^3 max(h, r) (54^4 is 2^23).
+//   cut-off   every target is at least r from it with r^4 >= 2^24 d |L|^2, so
+//             the denominator's d |L|^2 gg^2 <= 2^-24 <= 2^-24 e (e >= 1 there).
+// Rounding: |x1 - P|^2 is formed from terms of at most |q|^2 + 2|q||p| + |p|^2
+// with |p| <= |q| / kDistantRatio. Error against FP64 over the wakes of 6k to
+// 175k filaments (2-norm, all targets): 4.3e-8 to 5.0e-8, as without this form.
+constexpr float kDistantRatio = 1.5f;
+// squared distances for which no product of the form leaves FP32's range, and
+// |M|^2 |q|^2 for which the fourth power of the cross product does not
+constexpr float kDistantMinSq = 1e-12f, kDistantMaxSq = 1e16f, kDistantMaxMq = 1e17f;
+constexpr float kCoreFree4 = 54.f * 54.f * 54.f * 54.f;
+constexpr float kCutoffFreeSq = 4096.f;  // r^2 >= 4096 sqrt(d |L|^2) is r^4 >= 2^24 d |L|^2
+
+// One prepared filament against the lane's 2 NP targets: (mx, my, mz) = -2 p,
+// p2 = |p|^2. a = q, |q|^2; c = 2 q x M; b = 2 M, -|L|^2, but for the Vatistas
+// core M, -|L|^2; D = 16 (K^2 rc^2 |L|^2)^2 or 2 d |L|^2. (Ax, Ay, Az) = A, B is
+// added to (ax, ay, az). Carry: 1/r1, r1. CORE: kNoCore or the kernel's model.
+constexpr int kNoCore = 2;
+template <int NP, int CORE>
+__device__ __forceinline__ void distant_filament(const float4 a, const float4 b, const float4 c,
+                                                 const float D, const float2 (&mx)[NP],
+                                                 const float2 (&my)[NP], const float2 (&mz)[NP],
+                                                 const float2 (&p2)[NP], float2 (&ax)[NP],
+                                                 float2 (&ay)[NP], float2 (&az)[NP],
+                                                 float2 (&Ax)[NP], float2 (&Ay)[NP],
+                                                 float2 (&Az)[NP], float2 (&ti)[NP],
+                                                 float2 (&tr)[NP]) {
+#pragma unroll
+  for (int p = 0; p < NP; ++p) {
+    float2 r1s = __fadd2_rn(bc(a.w), p2[p]);
+    r1s = __ffma2_rn(bc(a.x), mx[p], r1s);
+    r1s = __ffma2_rn(bc(a.y), my[p], r1s);
+    r1s = __ffma2_rn(bc(a.z), mz[p], r1s);
+    const float2 i1 = rsqrt2(r1s);
+    const float2 r1 = __fmul2_rn(r1s, i1);
+    const float2 s = __fadd2_rn(r1, tr[p]);
+    const float2 y = __ffma2_rn(s, s, bc(b.w));  // 2 (r1r2 + r1.r2)
+    const float2 gg = __fmul2_rn(i1, ti[p]);
+    ti[p] = i1;
+    tr[p] = r1;
+    if (CORE == kCoreVatistas) {
+      // 2 K L x r1 and its squared length; s gg^2 / (y gg) |c|^2 / sqrt(|c|^4 + D)
+      const float2 cx = __ffma2_rn(my[p], bc(b.z), __ffma2_rn(mz[p], bc(-b.y), bc(c.x)));
+      const float2 cy = __ffma2_rn(mz[p], bc(b.x), __ffma2_rn(mx[p], bc(-b.z), bc(c.y)));
+      const float2 cz = __ffma2_rn(mx[p], bc(b.y), __ffma2_rn(my[p], bc(-b.x), bc(c.z)));
+      float2 c2 = __fmul2_rn(cx, cx);
+      c2 = __ffma2_rn(cy, cy, c2);
+      c2 = __ffma2_rn(cz, cz, c2);
+      const float2 q = __ffma2_rn(c2, c2, bc(D));
+      const float2 yg = __fmul2_rn(y, gg);
+      const float2 ub = __fmul2_rn(__fmul2_rn(__fmul2_rn(s, gg), __fmul2_rn(gg, c2)),
+                                   rsqrt2(__fmul2_rn(__fmul2_rn(yg, yg), q)));
+      ax[p] = __ffma2_rn(ub, cx, ax[p]);
+      ay[p] = __ffma2_rn(ub, cy, ay[p]);
+      az[p] = __ffma2_rn(ub, cz, az[p]);
+    } else {
+      const float2 den = CORE == kCoreCutoff ? __ffma2_rn(bc(D), gg, y) : y;
+      const float2 ub = __fmul2_rn(__fmul2_rn(s, gg), rcp2(den));
+      Ax[p] = __ffma2_rn(ub, bc(b.x), Ax[p]);
+      Ay[p] = __ffma2_rn(ub, bc(b.y), Ay[p]);
+      Az[p] = __ffma2_rn(ub, bc(b.z), Az[p]);
+      ax[p] = __ffma2_rn(ub, bc(c.x), ax[p]);
+      ay[p] = __ffma2_rn(ub, bc(c.y), ay[p]);
+      az[p] = __ffma2_rn(ub, bc(c.z), az[p]);
+    }
+  }
+}
+
+// The carry of a prepared filament that starts a chain: 1/r2 and r2 of its own
+// second endpoint q + L.
+template <int NP>
+__device__ __forceinline__ void distant_start(const float4 a, const float4 d,
+                                              const float2 (&mx)[NP], const float2 (&my)[NP],
+                                              const float2 (&mz)[NP], const float2 (&p2)[NP],
+                                              float2 (&ti)[NP], float2 (&tr)[NP]) {
+  const float ex = a.x + d.x, ey = a.y + d.y, ez = a.z + d.z;
+  const float e2 = fmaf(ex, ex, fmaf(ey, ey, ez * ez));
+#pragma unroll
+  for (int p = 0; p < NP; ++p) {
+    float2 r2s = __fadd2_rn(bc(e2), p2[p]);
+    r2s = __ffma2_rn(bc(ex), mx[p], r2s);
+    r2s = __ffma2_rn(bc(ey), my[p], r2s);
+    r2s = __ffma2_rn(bc(ez), mz[p], r2s);
+    ti[p] = rsqrt2(r2s);
+    tr[p] = __fmul2_rn(r2s, ti[p]);
+  }
+}
+
+// Bits 0, 4, ..., 28 of x gathered into bits 0 .. 7.
+__device__ __forceinline__ unsigned gather_nibbles(unsigned x) {
+  x = (x | (x >> 3)) & 0x03030303u;
+  x = (x | (x >> 6)) & 0x000f000fu;
+  return (x | (x >> 12)) & 0xffu;
+}
+__device__ __forceinline__ unsigned nibble_any(unsigned m) {
+  m |= m >> 2;
+  return gather_nibbles((m | (m >> 1)) & 0x11111111u);
+}
+__device__ __forceinline__ unsigned nibble_all(unsigned m) { return nibble_any(~m) ^ 0xffu; }
 
 // A near-singular pair of a tile, listed in the tile's consumed stage: the
 // FP64 reference term `u` of filament `fidx` at the owner's target `slot`.
@@ -552,23 +562,25 @@ struct NearEntry {
   int fidx, slot;
 };
 
-// One item: the lane's T targets against filaments [it.f_begin, it.f_end),
-// streamed through the warp's S stages (tile g of the warp in stage g % S).
-// Returns false, for the whole warp, when a bounded wait ran out (the item is
-// abandoned after the copies in flight have landed).
-template <int T, int KF, int MODEL, bool CO, bool CHAIN>
+// One item: the lane's T targets (T even) against filaments [it.f_begin,
+// it.f_end), streamed through the warp's S stages (tile g of the warp in stage
+// g % S). Returns false, for the whole warp, when a bounded wait ran out (the
+// item is abandoned after the copies in flight have landed).
+template <int T, int KF, int MODEL>
 __device__ __forceinline__ bool f32c_item(const F32cArgs &a, const Item &it, unsigned char *stages,
-                                          uint64_t *full, float *s_k, unsigned *s_nb,
-                                          unsigned &gt, float2 (&npx)[T], float2 (&npy)[T],
-                                          float2 (&npz)[T], float2 ncx, float2 ncy, float2 ncz,
-                                          float S2, const float *ws, unsigned &near_cnt,
-                                          unsigned long long &free_cnt,
+                                          uint64_t *full, float *s_k, const float *s_p,
+                                          typename NearBits<T>::type *s_nb, unsigned &gt, float cx, float cy,
+                                          float cz, float S2, const float *ws, bool co_on,
+                                          unsigned &near_cnt, unsigned long long &free_cnt,
                                           const Tile &tl) {
   constexpr int S = StageSmem<KF>::kStages;
   constexpr int kB = StageSmem<KF>::kBytes;
+  constexpr int NP = T / 2;
+  constexpr int kPer = NearBits<T>::kPer;
+  constexpr unsigned kGroups = (1u << (KF / 4)) - 1u;
   const int lane = threadIdx.x & 31;
   const int ntiles = (it.f_end - it.f_begin) / KF;
-  const float co2 = (float)(a.co * a.co);
+  const float co2 = co_on ? (float)(a.co * a.co) : FLT_MAX;
   const int nslots = tl.t_count - lane * T;  // this lane's targets in the tile
   const unsigned live_slots = (unsigned)(nslots < 0 ? 0 : (nslots > T ? T : nslots));
   RefParams rp;
@@ -582,9 +594,9 @@ __device__ __forceinline__ bool f32c_item(const F32cArgs &a, const Item &it, uns
   if (lane == 0)
     for (int j = 0; j < issued; ++j)
       issue_stage<KF>(a, stages + ((gt + j) % S) * kB, &full[(gt + j) % S], it.f_begin + j * KF);
-  float2 ax[T], ay[T], az[T];
+  float2 ax[NP], ay[NP], az[NP];
 #pragma unroll
-  for (int t = 0; t < T; ++t) ax[t] = ay[t] = az[t] = make_float2(0.f, 0.f);
+  for (int p = 0; p < NP; ++p) ax[p] = ay[p] = az[p] = make_float2(0.f, 0.f);
 
   int i = 0;
   for (; i < ntiles; ++i) {
@@ -592,180 +604,199 @@ __device__ __forceinline__ bool f32c_item(const F32cArgs &a, const Item &it, uns
     const int st = g % S;
     const bool landed = mbar_wait_bounded(&full[st], (g / S) & 1u, a.err, a.wait_limit_ns);
     if (!__all_sync(0xffffffffu, landed)) break;
-    const unsigned char *stage = stages + st * kB;
-    const float4 *sP = reinterpret_cast<const float4 *>(stage);  // KF/2 pair records
-    const float *sF = reinterpret_cast<const float *>(stage);
-    // Hot loop: filaments in groups of 4 (two pair records). A warp-level
-    // screen (one filament per lane, every 32 filaments) sends groups that are
-    // far from all of the warp's targets down the plain path; the others test
-    // every pair and put their near-singular bits (bit 8*j + t: filament
-    // 4*kk+j, target t) in shared memory as one word. `careful` has bit g for
-    // every such group g. A far group whose four filaments all leave every
-    // target of the warp outside their core's reach (Vatistas: lines at least
-    // kCoreFreeRatio core radii away; cut-off: segments far enough that the
-    // d |L|^2 term is below FP32 resolution) takes the core-free form (`mf`
-    // has a bit per such filament).
-    unsigned careful = 0u;
+    unsigned char *stage = stages + st * kB;
+    float4 *sP = reinterpret_cast<float4 *>(stage);  // KF records of 4
+    // Filaments go in groups of 4; bit g of these masks is group g of the tile.
+    // A warp-level screen (one filament per lane, every 32 filaments) sorts the
+    // groups: all four filaments distant (above), core-free or not, and of the
+    // others those near some target, whose near-singular bits (NearBits) go to
+    // shared memory as one word for the FP64 pass. With the reach cut-off in
+    // play every group is of the last kind.
+    // Bit f of hm: filament f starts a chain (the sign of its |L|^2).
+    unsigned careful = 0u, gfree = 0u, gdist = 0u;
+    unsigned long long hm = 0;
+    if (co_on) {
+      careful = kGroups;
 #pragma unroll 1
-    for (int w = 0; w < KF / 32; ++w) {
-      unsigned m, mf = 0u;
-      if (CO) {
-        m = 0xffffffffu;
-      } else {
+      for (int w = 0; w < KF / 32; ++w) {
         const int k = 32 * w + lane;
-        const float *f = sF + (k >> 1) * 32 + (k & 1);  // field j of filament k at f[2 j]
+        const unsigned h = __ballot_sync(0xffffffffu, signbit(sP[4 * k + ((k >> 2) & 3)].w));
+        hm |= (unsigned long long)h << (32 * w);
+      }
+    } else {
+#pragma unroll 1
+      for (int w = 0; w < KF / 32; ++w) {
+        const int k = 32 * w + lane;
+        float4 *r = sP + 4 * k;
+        const int sw = (k >> 2) & 3;
+        float4 A = r[0 ^ sw], B = r[1 ^ sw], C = r[2 ^ sw];
+        const float4 D = r[3 ^ sw];
         // the warp's target ball (centre, radius, largest S2), kept in shared
-        // memory so it holds no registers across the hot loop
+        // memory so it holds no registers across the hot loops
         const float wcx = ws[0], wcy = ws[1], wcz = ws[2], wr = ws[3], rn_floor = ws[4];
         const float big = fabsf(wcx) + fabsf(wcy) + fabsf(wcz);
-        const float Ax = f[0], Ay = f[2], Az = f[4], L2 = f[6];
-        const float mx = (Ax - wcx) + fmaf(0.5f, f[16], f[8]);
-        const float my = (Ay - wcy) + fmaf(0.5f, f[18], f[10]);
-        const float mz = (Az - wcz) + fmaf(0.5f, f[20], f[12]);
+        const float L2 = fabsf(A.w);
+        hm |= (unsigned long long)__ballot_sync(0xffffffffu, signbit(A.w)) << (32 * w);
+        const float dx = (A.x - wcx) + C.x, dy = (A.y - wcy) + C.y, dz = (A.z - wcz) + C.z;
+        const float mx = fmaf(0.5f, D.x, dx), my = fmaf(0.5f, D.y, dy), mz = fmaf(0.5f, D.z, dz);
         const float d2 = mx * mx + my * my + mz * mz;
-        const float reach = sqrtf(fmaf(0.25f, L2, fmaxf(f[14], rn_floor)));
+        const float reach = sqrtf(fmaf(0.25f, L2, fmaxf(C.w, rn_floor)));
         const float slack =
-            1e-5f * (big + fabsf(Ax) + fabsf(Ay) + fabsf(Az)) + 1e-3f * (reach + wr);
+            1e-5f * (big + fabsf(A.x) + fabsf(A.y) + fabsf(A.z)) + 1e-3f * (reach + wr);
         const float lim = wr + reach + slack;
-        m = __ballot_sync(0xffffffffu, !(d2 > lim * lim));
+        const bool far = d2 > lim * lim;
+        // nearest approach of a warp target to the segment: its midpoint
+        // distance less wr and |L|/2
+        const float rmin = sqrtf(d2) - wr - 0.5f * sqrtf(L2) - slack;
+        bool free_;
         if (MODEL == kCoreVatistas) {
           // distance of the ball centre from the filament's line: |L x (x1 - c)| / |L|;
           // every target of the warp is at least that less wr from it
-          const float Lx = f[16], Ly = f[18], Lz = f[20], rc = f[30];
-          const float dx = Ax - wcx, dy = Ay - wcy, dz = Az - wcz;
-          const float cx = Ly * dz - Lz * dy, cy = Lz * dx - Lx * dz, cz = Lx * dy - Ly * dx;
-          const float R = fmaf(kCoreFreeRatio, rc, wr + slack);
+          const float hx = D.y * dz - D.z * dy, hy = D.z * dx - D.x * dz, hz = D.x * dy - D.y * dx;
+          const float h = sqrtf((hx * hx + hy * hy + hz * hz) / L2) - wr - slack;
+          const float rc2 = B.w * B.w;
           // zero length: the pair term is zero on either form; rc = 0 (no core,
           // or K = 0 and a zero term): the factor is 1
-          const bool free_ =
-              !(L2 > 0.f) || rc == 0.f || cx * cx + cy * cy + cz * cz >= R * R * L2;
-          mf = __ballot_sync(0xffffffffu, free_);
-        } else {
-          // nearest approach of a warp target to the segment: its midpoint
-          // distance less wr and |L|/2; D = d |L|^2 (record field 11)
-          const float rmin = sqrtf(d2) - wr - 0.5f * sqrtf(L2) - slack;
-          const bool free_ = rmin > 0.f && rmin * rmin >= kCutoffFreeSq * sqrtf(f[22]);
-          mf = __ballot_sync(0xffffffffu, free_);
+          free_ = !(L2 > 0.f) || B.w == 0.f ||
+                  (h > 0.f && h * h * h * fmaxf(h, rmin) >= kCoreFree4 * rc2 * rc2);
+        } else {  // D.w = d |L|^2
+          free_ = rmin > 0.f && rmin * rmin >= kCutoffFreeSq * sqrtf(D.w);
         }
-      }
-      if constexpr (CHAIN) {
-        // Chained records: bit j of hm is set when record j of the word starts
-        // a chain (the word's first record always does: no carry crosses a
-        // word). The carry holds the previous record's x1 - P and 1/|x1 - P|.
-        const unsigned r0 = (unsigned)((it.f_begin + i * KF + 32 * w) >> 1);
-        const unsigned hm = ((__ldg(a.heads + (r0 >> 5)) >> (r0 & 31u)) & 0xffffu) | 1u;
-        float2 ti[T];
-        unsigned unused = 0;
-        if (m == 0u && mf == 0xffffffffu) {
-          free_cnt += 32u * live_slots;
-#pragma unroll 2
-          for (int j = 0; j < 16; ++j)
-            chain_record<T, kCoreFree, false, false>(sP + (16 * w + j) * 8, (hm >> j) & 1u, ncx,
-                                                     ncy, ncz, npx, npy, npz, S2, co2, ax, ay, az,
-                                                     ti, unused, 0);
-          continue;
-        }
-#pragma unroll 1
-        for (int g = 0; g < 8; ++g) {
-          const int kk = 32 * w + 4 * g;
-          const unsigned hg = hm >> (2 * g);
-          if (((m >> (4 * g)) & 0xfu) == 0u && ((mf >> (4 * g)) & 0xfu) == 0xfu) {
-            free_cnt += 4u * live_slots;
-#pragma unroll
-            for (int j = 0; j < 2; ++j)
-              chain_record<T, kCoreFree, false, false>(sP + (kk / 2 + j) * 8, (hg >> j) & 1u, ncx,
-                                                       ncy, ncz, npx, npy, npz, S2, co2, ax, ay,
-                                                       az, ti, unused, j);
-          } else if (((m >> (4 * g)) & 0xfu) == 0u) {
-#pragma unroll
-            for (int j = 0; j < 2; ++j)
-              chain_record<T, MODEL, false, false>(sP + (kk / 2 + j) * 8, (hg >> j) & 1u, ncx,
-                                                   ncy, ncz, npx, npy, npz, S2, co2, ax, ay, az,
-                                                   ti, unused, j);
+        // both endpoints kDistantRatio ball radii from the centre, all in range
+        const float q1 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+        const float ex = dx + D.x, ey = dy + D.y, ez = dz + D.z;
+        const float q2 = ex * ex + ey * ey + ez * ez;
+        const float dmin = fmaxf(kDistantRatio * kDistantRatio * wr * wr, kDistantMinSq);
+        const float qmax = fmaxf(q1, q2);
+        const bool dist = far && fminf(q1, q2) >= dmin && qmax <= kDistantMaxSq;
+        const bool cored = qmax * (B.x * B.x + B.y * B.y + B.z * B.z) <= kDistantMaxMq;
+        careful |= nibble_any(__ballot_sync(0xffffffffu, !far)) << (8 * w);
+        const unsigned gf = nibble_all(__ballot_sync(0xffffffffu, free_ && far));
+        const unsigned gd = nibble_all(__ballot_sync(0xffffffffu, dist)) &
+                            (gf | nibble_all(__ballot_sync(0xffffffffu, cored)));
+        free_cnt += 4u * live_slots * __popc(gd & gf);
+        gfree |= (gd & gf) << (8 * w);
+        gdist |= gd << (8 * w);
+        if ((gd >> (lane >> 2)) & 1u) {
+          const float nx = 2.f * B.x, ny = 2.f * B.y, nz = 2.f * B.z;
+          r[0 ^ sw] = make_float4(dx, dy, dz, q1);
+          r[2 ^ sw] = make_float4(dy * nz - dz * ny, dz * nx - dx * nz, dx * ny - dy * nx, 0.f);
+          if (MODEL == kCoreVatistas && !((gf >> (lane >> 2)) & 1u)) {
+            r[1 ^ sw] = make_float4(B.x, B.y, B.z, -L2);
+            r[3 ^ sw] = make_float4(D.x, D.y, D.z, 16.f * D.w);
           } else {
-            careful |= 1u << (8 * w + g);
-            unsigned nbits = 0;
-#pragma unroll
-            for (int j = 0; j < 2; ++j)
-              chain_record<T, MODEL, CO, true>(sP + (kk / 2 + j) * 8, (hg >> j) & 1u, ncx, ncy,
-                                               ncz, npx, npy, npz, S2, co2, ax, ay, az, ti,
-                                               nbits, j);
-            s_nb[(kk / 4) * 32 + lane] = nbits;
+            r[1 ^ sw] = make_float4(nx, ny, nz, -L2);
+            r[3 ^ sw] = make_float4(D.x, D.y, D.z, 2.f * D.w);
           }
         }
-        continue;
       }
-      if (m == 0u && mf == 0xffffffffu) {
-        // the whole word far and core-free: one loop over its 16 pairs
-        free_cnt += 32u * live_slots;
-#pragma unroll 2
-        for (int j = 0; j < 16; ++j) {
-          Fil2 f;
-          load_pair(sP + (16 * w + j) * 8, ncx, ncy, ncz, f);
-          unsigned unused = 0;
+      __syncwarp();
+    }
+    // the first filament after a group of another form starts a chain too
+    const auto group_heads = [&](int gr) { return (unsigned)(hm >> (4 * gr)) & 15u; };
+    if (gdist) {
+      float2 mx[NP], my[NP], mz[NP], p2[NP], Ax[NP], Ay[NP], Az[NP], ti[NP], tr[NP];
+      const float ox = cx - ws[0], oy = cy - ws[1], oz = cz - ws[2];
 #pragma unroll
-          for (int t = 0; t < T; ++t)
-            interact2<kCoreFree, false, false>(npx[t], npy[t], npz[t], f, f.Rn2, co2, ax[t],
-                                               ay[t], az[t], unused, 0u, 0u);
-        }
-        continue;
+      for (int p = 0; p < NP; ++p) {
+        const float2 x = make_float2(s_p[2 * p * 32 + lane] + ox, s_p[(2 * p + 1) * 32 + lane] + ox);
+        const float2 y = make_float2(s_p[(T + 2 * p) * 32 + lane] + oy,
+                                     s_p[(T + 2 * p + 1) * 32 + lane] + oy);
+        const float2 z = make_float2(s_p[(2 * T + 2 * p) * 32 + lane] + oz,
+                                     s_p[(2 * T + 2 * p + 1) * 32 + lane] + oz);
+        p2[p] = __ffma2_rn(x, x, __ffma2_rn(y, y, __fmul2_rn(z, z)));
+        mx[p] = __fmul2_rn(bc(-2.f), x);
+        my[p] = __fmul2_rn(bc(-2.f), y);
+        mz[p] = __fmul2_rn(bc(-2.f), z);
+        Ax[p] = Ay[p] = Az[p] = make_float2(0.f, 0.f);
       }
+      int last = -2;
 #pragma unroll 1
-      for (int g = 0; g < 8; ++g) {
-        const int kk = 32 * w + 4 * g;
-        if (((m >> (4 * g)) & 0xfu) == 0u && ((mf >> (4 * g)) & 0xfu) == 0xfu) {
-          free_cnt += 4u * live_slots;
+      for (unsigned gm = gdist; gm; gm &= gm - 1u) {
+        const int gr = __ffs(gm) - 1;
+        const unsigned hg = group_heads(gr) | (gr != last + 1 ? 1u : 0u);
+        last = gr;
+        const float4 *rec = sP + 16 * gr;
+        const int sw = gr & 3;
+        if (hg & 1u) distant_start<NP>(rec[0 ^ sw], rec[3 ^ sw], mx, my, mz, p2, ti, tr);
+        if (((gfree >> gr) & 1u) && !(hg & 14u)) {
 #pragma unroll
-          for (int j = 0; j < 2; ++j) {
-            Fil2 f;
-            load_pair(sP + (kk / 2 + j) * 8, ncx, ncy, ncz, f);
-            unsigned unused = 0;
-#pragma unroll
-            for (int t = 0; t < T; ++t)
-              interact2<kCoreFree, false, false>(npx[t], npy[t], npz[t], f, f.Rn2, co2, ax[t],
-                                                 ay[t], az[t], unused, 0u, 0u);
-          }
-        } else if (((m >> (4 * g)) & 0xfu) == 0u) {
-#pragma unroll
-          for (int j = 0; j < 2; ++j) {
-            Fil2 f;
-            load_pair(sP + (kk / 2 + j) * 8, ncx, ncy, ncz, f);
-            unsigned unused = 0;
-#pragma unroll
-            for (int t = 0; t < T; ++t)
-              interact2<MODEL, false, false>(npx[t], npy[t], npz[t], f, f.Rn2, co2, ax[t], ay[t],
-                                             az[t], unused, 0u, 0u);
-          }
+          for (int j = 0; j < 4; ++j)
+            distant_filament<NP, kNoCore>(rec[4 * j + (0 ^ sw)], rec[4 * j + (1 ^ sw)],
+                                          rec[4 * j + (2 ^ sw)], 0.f, mx, my, mz, p2, ax, ay, az,
+                                          Ax, Ay, Az, ti, tr);
         } else {
-          careful |= 1u << (8 * w + g);
-          unsigned nbits = 0;
-#pragma unroll
-          for (int j = 0; j < 2; ++j) {
-            Fil2 f;
-            load_pair(sP + (kk / 2 + j) * 8, ncx, ncy, ncz, f);
-            // near-singular threshold, raised for threads whose targets spread
-            // far from their centre (the FP32 differences lose ~eps * spread / |r1|)
-            const float2 Rn2 = make_float2(fmaxf(f.Rn2.x, S2), fmaxf(f.Rn2.y, S2));
-#pragma unroll
-            for (int t = 0; t < T; ++t)
-              interact2<MODEL, CO, true>(npx[t], npy[t], npz[t], f, Rn2, co2, ax[t], ay[t],
-                                         az[t], nbits, 1u << (8 * (2 * j) + t),
-                                         1u << (8 * (2 * j + 1) + t));
+          const bool core = !((gfree >> gr) & 1u);
+#pragma unroll 1
+          for (int j = 0; j < 4; ++j) {
+            const float4 qa = rec[4 * j + (0 ^ sw)], qd = rec[4 * j + (3 ^ sw)];
+            const float4 qb = rec[4 * j + (1 ^ sw)], qc = rec[4 * j + (2 ^ sw)];
+            if (j > 0 && ((hg >> j) & 1u)) distant_start<NP>(qa, qd, mx, my, mz, p2, ti, tr);
+            if (MODEL == kCoreCutoff || core)
+              distant_filament<NP, MODEL>(qa, qb, qc, qd.w, mx, my, mz, p2, ax, ay, az, Ax, Ay, Az,
+                                          ti, tr);
+            else
+              distant_filament<NP, kNoCore>(qa, qb, qc, 0.f, mx, my, mz, p2, ax, ay, az, Ax, Ay, Az,
+                                            ti, tr);
           }
-          s_nb[(kk / 4) * 32 + lane] = nbits;
         }
+      }
+#pragma unroll
+      for (int p = 0; p < NP; ++p) {  // - p x A
+        ax[p] = __ffma2_rn(bc(0.5f), __ffma2_rn(my[p], Az[p], neg2(__fmul2_rn(mz[p], Ay[p]))), ax[p]);
+        ay[p] = __ffma2_rn(bc(0.5f), __ffma2_rn(mz[p], Ax[p], neg2(__fmul2_rn(mx[p], Az[p]))), ay[p]);
+        az[p] = __ffma2_rn(bc(0.5f), __ffma2_rn(mx[p], Ay[p], neg2(__fmul2_rn(my[p], Ax[p]))), az[p]);
+      }
+    }
+    if (gdist != kGroups) {
+      float2 npx[NP], npy[NP], npz[NP], ti[NP];  // -(P - c)
+#pragma unroll
+      for (int p = 0; p < NP; ++p) {
+        npx[p] = make_float2(-s_p[2 * p * 32 + lane], -s_p[(2 * p + 1) * 32 + lane]);
+        npy[p] = make_float2(-s_p[(T + 2 * p) * 32 + lane], -s_p[(T + 2 * p + 1) * 32 + lane]);
+        npz[p] = make_float2(-s_p[(2 * T + 2 * p) * 32 + lane],
+                             -s_p[(2 * T + 2 * p + 1) * 32 + lane]);
+        ti[p] = make_float2(0.f, 0.f);
+      }
+      int last = -2;
+#pragma unroll 1
+      for (unsigned gm = ~gdist & kGroups; gm; gm &= gm - 1u) {
+        const int gr = __ffs(gm) - 1;
+        const unsigned hg = group_heads(gr) | (gr != last + 1 ? 1u : 0u);
+        last = gr;
+        const bool near_some = (careful >> gr) & 1u;
+        const float4 *rec = sP + 16 * gr;
+        unsigned nbits = 0;
+#pragma unroll 1
+        for (int j = 0; j < 4; ++j) {
+          const Fil f = load_filament(rec + 4 * j, gr & 3, cx, cy, cz);
+          // near-singular threshold, raised for threads whose targets spread far
+          // from their centre (the FP32 differences lose ~eps * spread / |r1|)
+          const float Rn2 = near_some ? fmaxf(f.Rn2, S2) : -FLT_MAX;
+          if ((hg >> j) & 1u) chain_start<NP>(f, npx, npy, npz, ti);
+          unsigned m = 0;
+#pragma unroll
+          for (int p = 0; p < NP; ++p)
+            interact<MODEL>(npx[p], npy[p], npz[p], f, Rn2, co2, ax[p], ay[p], az[p], m,
+                            1u << (2 * p), 2u << (2 * p), ti[p]);
+          nbits |= m << (kPer * j);
+        }
+        if (near_some) s_nb[gr * 32 + lane] = (typename NearBits<T>::type)nbits;
       }
     }
     __syncwarp();
-    // Kahan-fold the partial sums into the per-target totals every 128 filaments.
+    // Kahan-fold the partial sums into the per-target totals every 64 filaments.
     if ((i + 1) % StageSmem<KF>::kFold == 0 || i + 1 == ntiles) {
 #pragma unroll
-      for (int t = 0; t < T; ++t) {
-        const int sl = lane * T + t;
-        kahan_add(s_k[0 * 32 * T + sl], s_k[1 * 32 * T + sl], ax[t].x + ax[t].y);
-        kahan_add(s_k[2 * 32 * T + sl], s_k[3 * 32 * T + sl], ay[t].x + ay[t].y);
-        kahan_add(s_k[4 * 32 * T + sl], s_k[5 * 32 * T + sl], az[t].x + az[t].y);
-        ax[t] = ay[t] = az[t] = make_float2(0.f, 0.f);
+      for (int p = 0; p < NP; ++p) {
+        const int sl = lane * T + 2 * p;
+        kahan_add(s_k[0 * 32 * T + sl], s_k[1 * 32 * T + sl], ax[p].x);
+        kahan_add(s_k[2 * 32 * T + sl], s_k[3 * 32 * T + sl], ay[p].x);
+        kahan_add(s_k[4 * 32 * T + sl], s_k[5 * 32 * T + sl], az[p].x);
+        kahan_add(s_k[0 * 32 * T + sl + 1], s_k[1 * 32 * T + sl + 1], ax[p].y);
+        kahan_add(s_k[2 * 32 * T + sl + 1], s_k[3 * 32 * T + sl + 1], ay[p].y);
+        kahan_add(s_k[4 * 32 * T + sl + 1], s_k[5 * 32 * T + sl + 1], az[p].y);
+        ax[p] = ay[p] = az[p] = make_float2(0.f, 0.f);
       }
     }
     // Near-singular pairs of this tile: the reference formula in FP64, added to
@@ -777,7 +808,7 @@ __device__ __forceinline__ bool f32c_item(const F32cArgs &a, const Item &it, uns
       constexpr int kCap = kB / (int)sizeof(NearEntry);
       NearEntry *ne = reinterpret_cast<NearEntry *>(stages + st * kB);
       int cnt = 0;
-      for (unsigned cg = careful; cg; cg &= cg - 1u) cnt += __popc(s_nb[(__ffs(cg) - 1) * 32 + lane]);
+      for (unsigned cg = careful; cg; cg &= cg - 1u) cnt += __popc((unsigned)s_nb[(__ffs(cg) - 1) * 32 + lane]);
       int incl = cnt;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
@@ -796,8 +827,8 @@ __device__ __forceinline__ bool f32c_item(const F32cArgs &a, const Item &it, uns
             for (unsigned bits = s_nb[w * 32 + lane]; bits && k < end; bits &= bits - 1u, ++k) {
               if (k < base) continue;
               const int b = __ffs(bits) - 1;
-              ne[k - base].fidx = it.f_begin + i * KF + 4 * w + (b >> 3);
-              ne[k - base].slot = lane * T + (b & 7);
+              ne[k - base].fidx = it.f_begin + i * KF + 4 * w + b / kPer;
+              ne[k - base].slot = lane * T + b % kPer;
             }
           }
         }
@@ -832,12 +863,14 @@ __device__ __forceinline__ bool f32c_item(const F32cArgs &a, const Item &it, uns
       }
     }
     // Every lane is done with the stage (tile and near list): refill it with
-    // tile i + S.
+    // tile i + S. Lanes wrote to it (prepared records, near list): each orders
+    // its own accesses before the copy.
+    if (issued < ntiles) fence_proxy_async_smem();
+    __syncwarp();
     if (lane == 0 && issued < ntiles) {
-      fence_proxy_async_smem();
       issue_stage<KF>(a, stages + st * kB, &full[st], it.f_begin + issued * KF);
-      ++issued;
     }
+    if (issued < ntiles) ++issued;
     __syncwarp();
   }
   if (i < ntiles) {
@@ -856,28 +889,27 @@ __device__ __forceinline__ bool f32c_item(const F32cArgs &a, const Item &it, uns
   return true;
 }
 
-// Resident CTAs per SM the register allocation is capped for: 6 for T = 2
-// (80 registers), 5 for T = 3 (96), 4 for T = 4 (128), 2 for T = 8 (255). The
-// packed loop keeps each target as broadcast pairs and its sums as pairs (12
-// registers a target). The chained kernel carries one more pair a target: 5
-// for T = 2 (96), 4 for T = 3 and T = 4 (128; T = 4 then spills ~100 bytes,
-// and measured faster so than at 3 CTAs with 168 registers on the cut-off
-// core, slower on the Vatistas core, where T = 3 wins).
-template <int T, bool CHAIN>
+// Resident CTAs per SM the register allocation is capped for. The loops want
+// registers for four filaments in flight more than they want warps: with six
+// targets a lane, 3 CTAs (168 registers) run the large wake at 1289 Gint/s, 4
+// CTAs (128, spills) at 1159, 2 CTAs at 1184; with four targets 4 CTAs run the
+// 60k-filament cut-off wake at 1193, 3 at 1148, 5 at 1072.
+template <int T>
 struct MinBlocks {
-  static constexpr int value = CHAIN ? (T <= 2 ? 5 : (T <= 4 ? 4 : 2))
-                                     : (T <= 2 ? 6 : (T == 3 ? 5 : (T <= 4 ? 4 : 2)));
+  static constexpr int value = T <= 2 ? 5 : (T == 4 ? 4 : (T == 6 ? 3 : 2));
 };
 
-template <int T, int KF, int MODEL, bool CHAIN>
-__global__ void __launch_bounds__(kThreads, MinBlocks<T, CHAIN>::value) bs_f32c(const F32cArgs a) {
-  static_assert(KF % 32 == 0 && KF / 4 <= 32, "one screen word per 32 filaments, one bit per group");
+template <int T, int KF, int MODEL>
+__global__ void __launch_bounds__(kThreads, MinBlocks<T>::value) bs_f32c(const F32cArgs a) {
+  static_assert(KF % 32 == 0 && KF <= 64, "one screen word per 32 filaments, a head bit per filament");
+  static_assert(T % 2 == 0 && T <= 8, "targets go in pairs, near-singular bits eight to a filament");
   constexpr int S = StageSmem<KF>::kStages;
   extern __shared__ __align__(128) unsigned char smem[];
   const int lane = threadIdx.x & 31;
   unsigned char *stages = smem + (threadIdx.x >> 5) * warp_smem_bytes<T, KF>();
   float *s_k = reinterpret_cast<float *>(stages + S * StageSmem<KF>::kBytes);
-  unsigned *s_nb = reinterpret_cast<unsigned *>(s_k + 6 * 32 * T);
+  float *s_p = s_k + 6 * 32 * T;
+  auto *s_nb = reinterpret_cast<typename NearBits<T>::type *>(s_p + 3 * 32 * T);
   uint64_t *full = reinterpret_cast<uint64_t *>(s_nb + (KF / 4) * 32);
   float *ws = reinterpret_cast<float *>(full + S);
   if (lane == 0) {
@@ -918,20 +950,13 @@ __global__ void __launch_bounds__(kThreads, MinBlocks<T, CHAIN>::value) bs_f32c(
       py[t] = (float)(p.y - (double)cy);
       pz[t] = (float)(p.z - (double)cz);
       spread2 = fmaxf(spread2, px[t] * px[t] + py[t] * py[t] + pz[t] * pz[t]);
+      s_p[t * 32 + lane] = px[t];
+      s_p[(T + t) * 32 + lane] = py[t];
+      s_p[(2 * T + t) * 32 + lane] = pz[t];
 #pragma unroll
       for (int c = 0; c < 6; ++c) s_k[c * 32 * T + lane * T + t] = 0.f;
     }
     const float S2 = 0.09f * spread2;  // pairs closer than 0.3 x spread go to FP64
-    // -(P - c) in both lanes of a packed register, and -c likewise
-    float2 npx[T], npy[T], npz[T];
-#pragma unroll
-    for (int t = 0; t < T; ++t) {
-      npx[t] = make_float2(-px[t], -px[t]);
-      npy[t] = make_float2(-py[t], -py[t]);
-      npz[t] = make_float2(-pz[t], -pz[t]);
-    }
-    const float2 ncx = make_float2(-cx, -cx), ncy = make_float2(-cy, -cy),
-                 ncz = make_float2(-cz, -cz);
     // The warp's targets lie in the ball (wc, wr) around the centre of their
     // bounding box. As r1.r2 = |P - m|^2 - |L|^2/4 (m the filament midpoint),
     // a filament whose midpoint is farther than wr + sqrt(|L|^2/4 + Rn^2)
@@ -974,14 +999,8 @@ __global__ void __launch_bounds__(kThreads, MinBlocks<T, CHAIN>::value) bs_f32c(
       ws[4] = rn_floor;
     }
     __syncwarp();
-    bool ok;
-    if (co_on)
-      ok = f32c_item<T, KF, MODEL, true, CHAIN>(a, it, stages, full, s_k, s_nb, gt, npx, npy, npz,
-                                                ncx, ncy, ncz, S2, ws, near_cnt, free_cnt, tl);
-    else
-      ok = f32c_item<T, KF, MODEL, false, CHAIN>(a, it, stages, full, s_k, s_nb, gt, npx, npy,
-                                                 npz, ncx, ncy, ncz, S2, ws, near_cnt, free_cnt,
-                                                 tl);
+    const bool ok = f32c_item<T, KF, MODEL>(a, it, stages, full, s_k, s_p, s_nb, gt, cx, cy, cz, S2,
+                                            ws, co_on, near_cnt, free_cnt, tl);
     if (!ok) break;
     double *part = a.part + (size_t)item_id * 3 * a.tile_cap;
 #pragma unroll
@@ -1148,59 +1167,50 @@ __global__ void bs_wait_selftest(unsigned *err, unsigned long long limit_ns) {
 
 // ============================================================ host launchers
 namespace {
-template <int T, int KF, int MODEL, bool CH>
+template <int T, int KF, int MODEL>
 cudaError_t launch_f32c_t(const F32cArgs &a, int grid, cudaStream_t s) {
   const size_t smem = f32c_smem_bytes_t<T, KF>();
   static unsigned attr_set = 0;  // one bit per device: the attribute is per context
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 32 || !(attr_set & (1u << dev))) {
-    cudaError_t e = cudaFuncSetAttribute(bs_f32c<T, KF, MODEL, CH>,
+    cudaError_t e = cudaFuncSetAttribute(bs_f32c<T, KF, MODEL>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(bs_f32c<T, KF, MODEL, CH>,
-                             cudaFuncAttributePreferredSharedMemoryCarveout,
+    e = cudaFuncSetAttribute(bs_f32c<T, KF, MODEL>, cudaFuncAttributePreferredSharedMemoryCarveout,
                              (int)cudaSharedmemCarveoutMaxShared);
     if (e != cudaSuccess) return e;
     if (dev < 32) attr_set |= (1u << dev);
   }
   // `grid` counts workers (warps); kWarps of them per CTA
-  bs_f32c<T, KF, MODEL, CH><<<(grid + kWarps - 1) / kWarps, kThreads, smem, s>>>(a);
+  bs_f32c<T, KF, MODEL><<<(grid + kWarps - 1) / kWarps, kThreads, smem, s>>>(a);
   return cudaGetLastError();
 }
 
-template <int T, int KF, int MODEL, bool CH>
+template <int T, int KF, int MODEL>
 int occupancy_t() {
   const size_t smem = f32c_smem_bytes_t<T, KF>();
-  cudaFuncSetAttribute(bs_f32c<T, KF, MODEL, CH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  cudaFuncSetAttribute(bs_f32c<T, KF, MODEL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)smem);
-  cudaFuncSetAttribute(bs_f32c<T, KF, MODEL, CH>, cudaFuncAttributePreferredSharedMemoryCarveout,
+  cudaFuncSetAttribute(bs_f32c<T, KF, MODEL>, cudaFuncAttributePreferredSharedMemoryCarveout,
                        (int)cudaSharedmemCarveoutMaxShared);
   int n = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, bs_f32c<T, KF, MODEL, CH>, kThreads, smem) !=
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, bs_f32c<T, KF, MODEL>, kThreads, smem) !=
       cudaSuccess)
     return kWarps;
   return (n > 0 ? n : 1) * kWarps;  // resident workers per SM
 }
 
 #define WINDS_F32C_CASE(FN, M, TT, KK, ...) \
-  case M * 1000 + TT * 100 + KK / 32: return FN<TT, KK, M, CH>(__VA_ARGS__);
-#define WINDS_F32C_DISPATCH(FN, ...)                                                    \
-  switch (model * 1000 + T * 100 + KF / 32) {                                          \
-    WINDS_F32C_CASE(FN, 0, 2, 32, __VA_ARGS__) WINDS_F32C_CASE(FN, 0, 2, 64, __VA_ARGS__) \
-    WINDS_F32C_CASE(FN, 0, 2, 128, __VA_ARGS__) WINDS_F32C_CASE(FN, 0, 3, 32, __VA_ARGS__) \
-    WINDS_F32C_CASE(FN, 0, 3, 64, __VA_ARGS__) WINDS_F32C_CASE(FN, 0, 3, 128, __VA_ARGS__) \
-    WINDS_F32C_CASE(FN, 0, 4, 32, __VA_ARGS__) \
-    WINDS_F32C_CASE(FN, 0, 4, 64, __VA_ARGS__) WINDS_F32C_CASE(FN, 0, 4, 128, __VA_ARGS__) \
-    WINDS_F32C_CASE(FN, 0, 8, 32, __VA_ARGS__) WINDS_F32C_CASE(FN, 0, 8, 64, __VA_ARGS__) \
-    WINDS_F32C_CASE(FN, 0, 8, 128, __VA_ARGS__) WINDS_F32C_CASE(FN, 1, 2, 32, __VA_ARGS__) \
-    WINDS_F32C_CASE(FN, 1, 2, 64, __VA_ARGS__) WINDS_F32C_CASE(FN, 1, 2, 128, __VA_ARGS__) \
-    WINDS_F32C_CASE(FN, 1, 3, 32, __VA_ARGS__) WINDS_F32C_CASE(FN, 1, 3, 64, __VA_ARGS__) \
-    WINDS_F32C_CASE(FN, 1, 3, 128, __VA_ARGS__) \
-    WINDS_F32C_CASE(FN, 1, 4, 32, __VA_ARGS__) WINDS_F32C_CASE(FN, 1, 4, 64, __VA_ARGS__) \
-    WINDS_F32C_CASE(FN, 1, 4, 128, __VA_ARGS__) WINDS_F32C_CASE(FN, 1, 8, 32, __VA_ARGS__) \
-    WINDS_F32C_CASE(FN, 1, 8, 64, __VA_ARGS__) WINDS_F32C_CASE(FN, 1, 8, 128, __VA_ARGS__) \
-    default: break;                                                                     \
+  case M * 1000 + TT * 100 + KK / 32: return FN<TT, KK, M>(__VA_ARGS__);
+#define WINDS_F32C_KF(FN, M, TT, ...) \
+  WINDS_F32C_CASE(FN, M, TT, 32, __VA_ARGS__) WINDS_F32C_CASE(FN, M, TT, 64, __VA_ARGS__)
+#define WINDS_F32C_T(FN, M, ...)                                              \
+  WINDS_F32C_KF(FN, M, 2, __VA_ARGS__) WINDS_F32C_KF(FN, M, 4, __VA_ARGS__) \
+  WINDS_F32C_KF(FN, M, 6, __VA_ARGS__) WINDS_F32C_KF(FN, M, 8, __VA_ARGS__)
+#define WINDS_F32C_DISPATCH(FN, ...)                                           \
+  switch (model * 1000 + f32c_targets(T) * 100 + (KF < 64 ? KF : 64) / 32) {  \
+    WINDS_F32C_T(FN, 0, __VA_ARGS__) WINDS_F32C_T(FN, 1, __VA_ARGS__) default: break; \
   }
 }  // namespace
 
@@ -1208,32 +1218,21 @@ bool f32c_config_supported(int T, int KF) {
   return (T == 2 || T == 3 || T == 4 || T == 8) && (KF == 32 || KF == 64 || KF == 128);
 }
 
-int f32c_threads() { return 32; }  // lanes of one worker: a tile holds 32 x T targets
+// Targets per lane of a choice: they go in pairs, T = 3 (three pairs) runs with
+// six. KF = 128 runs as 64.
+int f32c_targets(int T) { return T == 3 ? 6 : T; }
+int f32c_tile(int T) { return 32 * f32c_targets(T); }
 int f64_threads() { return kF64Threads; }
 int f64_tile() { return kF64Tile; }
 
-namespace {
-template <bool CH>
-cudaError_t launch_f32c_ch(const F32cArgs &a, int model, int T, int KF, int grid, cudaStream_t s) {
+cudaError_t launch_f32c(const F32cArgs &a, int model, int T, int KF, int grid, cudaStream_t s) {
   WINDS_F32C_DISPATCH(launch_f32c_t, a, grid, s)
   return cudaErrorInvalidValue;
 }
 
-template <bool CH>
-int f32c_occupancy_ch(int model, int T, int KF) {
+int f32c_occupancy(int model, int T, int KF) {
   WINDS_F32C_DISPATCH(occupancy_t)
   return 1;
-}
-}  // namespace
-
-// a.heads set: the filament stream is chained (bs_pack_chains)
-cudaError_t launch_f32c(const F32cArgs &a, int model, int T, int KF, int grid, cudaStream_t s) {
-  return a.heads ? launch_f32c_ch<true>(a, model, T, KF, grid, s)
-                 : launch_f32c_ch<false>(a, model, T, KF, grid, s);
-}
-
-int f32c_occupancy(int model, int T, int KF, bool chain) {
-  return chain ? f32c_occupancy_ch<true>(model, T, KF) : f32c_occupancy_ch<false>(model, T, KF);
 }
 
 int f64_occupancy() {
@@ -1254,14 +1253,21 @@ cudaError_t launch_bbox_init(BBox *bb, cudaStream_t s) {
 }
 
 cudaError_t launch_pack_filaments(const double *F1, const double *F2, const double *gam,
-                                  const double *rc, long long d0, long long nf, long long off,
-                                  int model, double dcut, const PackedFilaments &pf, BBox *bb,
-                                  cudaStream_t s) {
+                                  const double *rc, const long long d[4], long long off,
+                                  unsigned long long *cnt, int model, double dcut,
+                                  const PackedFilaments &pf, BBox *bb, cudaStream_t s) {
+  const long long nf = d[0] * d[2] * d[3];
   if (nf <= 0) return cudaSuccess;
   const int bs = 256;
-  const long long grid = (nf + bs - 1) / bs;
-  bs_pack_filaments<<<(unsigned)grid, bs, 0, s>>>(F1, F2, gam, rc, d0, nf, off, model, dcut, pf.pk,
-                                                 pf.ra, pf.rb, bb);
+  const unsigned grid = (unsigned)((nf + bs - 1) / bs);
+  cudaError_t e;
+  if (cnt) {
+    if ((e = cudaMemsetAsync(cnt, 0, 2 * sizeof(unsigned long long), s)) != cudaSuccess) return e;
+    bs_chain_count<<<grid, bs, 0, s>>>(F1, F2, d[0], d[2], nf, cnt);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  }
+  bs_pack_filaments<<<grid, bs, 0, s>>>(F1, F2, gam, rc, d[0], d[2], nf, off, cnt, model, dcut,
+                                        pf.pk, pf.ra, pf.rb, bb);
   return cudaGetLastError();
 }
 
@@ -1271,42 +1277,6 @@ cudaError_t launch_pad_filaments(long long from, long long to, const PackedFilam
   const int bs = 256;
   const long long grid = (to - from + bs - 1) / bs;
   bs_pad_filaments<<<(unsigned)grid, bs, 0, s>>>(from, to, pf.pk, pf.ra, pf.rb);
-  return cudaGetLastError();
-}
-
-// Records of a [d0,3,d2,d3] family in a chained stream: room for the layout
-// along either index (the device picks one; the rest of the room is inert).
-long long chain_records(long long d0, long long d2, long long d3) {
-  if (d0 <= 0 || d2 <= 0 || d3 <= 0) return 0;
-  const long long a = chain_layout_records(d2 * d3, d0), b = chain_layout_records(d0 * d3, d2);
-  return a > b ? a : b;
-}
-
-cudaError_t launch_pack_chains(const double *F1, const double *F2, const double *gam,
-                               const double *rc, const long long d[4], long long rec_off,
-                               unsigned long long *cnt, int model, double dcut,
-                               const PackedFilaments &pf, unsigned *heads, BBox *bb,
-                               cudaStream_t s) {
-  const long long nf = d[0] * d[2] * d[3];
-  const long long nrec = chain_records(d[0], d[2], d[3]);
-  if (nf <= 0 || nrec <= 0) return cudaSuccess;
-  const int bs = 256;
-  cudaError_t e = cudaMemsetAsync(cnt, 0, 2 * sizeof(unsigned long long), s);
-  if (e != cudaSuccess) return e;
-  bs_chain_count<<<(unsigned)((nf + bs - 1) / bs), bs, 0, s>>>(F1, F2, d[0], d[2], nf, cnt);
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  bs_pack_chains<<<(unsigned)((2 * nrec + bs - 1) / bs), bs, 0, s>>>(
-      F1, F2, gam, rc, d[0], d[2], d[3], rec_off, nrec, cnt, model, dcut, pf.pk, pf.ra, pf.rb,
-      heads, bb);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_pad_chains(long long from, long long to, const PackedFilaments &pf,
-                              unsigned *heads, cudaStream_t s) {
-  if (to <= from) return cudaSuccess;
-  const int bs = 256;
-  bs_pad_chains<<<(unsigned)((to - from + bs - 1) / bs), bs, 0, s>>>(from, to, pf.pk, pf.ra, pf.rb,
-                                                                     heads);
   return cudaGetLastError();
 }
 

@@ -8,7 +8,7 @@
 namespace winds {
 
 struct PackedFilaments {
-  float4 *pk;  // pair records: 4 float4 per filament (layout in bs_types.h)
+  float4 *pk;  // records: 4 float4 per filament (layout in bs_types.h)
   double4 *ra, *rb;
 };
 
@@ -17,34 +17,26 @@ struct PackedFilaments {
 constexpr int kFilamentPad = 128;
 
 bool f32c_config_supported(int T, int KF);
-// FP32c work runs on independent warp workers: a tile holds f32c_threads() * T
+// FP32c work runs on independent warp workers: a tile holds f32c_tile(T)
 // targets, f32c_occupancy() counts resident workers per SM, and launch_f32c's
 // grid counts workers.
-int f32c_threads();
+int f32c_targets(int T);  // targets per lane that a choice of T runs with
+int f32c_tile(int T);
 int f64_threads();
 int f64_tile();
-int f32c_occupancy(int model, int T, int KF, bool chain = false);
+int f32c_occupancy(int model, int T, int KF);
 int f64_occupancy();
 unsigned long long default_wait_limit_ns();
 
 cudaError_t launch_bbox_init(BBox *bb, cudaStream_t s);
+// Packs a [d0,3,d2,d3] family from slot off on, in input order or (cnt: 2 device
+// words of scratch) in the order with more links between neighbours.
 cudaError_t launch_pack_filaments(const double *F1, const double *F2, const double *gam,
-                                  const double *rc, long long d0, long long nf, long long off,
-                                  int model, double dcut, const PackedFilaments &pf, BBox *bb,
-                                  cudaStream_t s);
+                                  const double *rc, const long long d[4], long long off,
+                                  unsigned long long *cnt, int model, double dcut,
+                                  const PackedFilaments &pf, BBox *bb, cudaStream_t s);
 cudaError_t launch_pad_filaments(long long from, long long to, const PackedFilaments &pf,
                                  cudaStream_t s);
-// Chained filament stream (the FP32c path): records per [d0,3,d2,d3] family,
-// and the packing of one family from record rec_off (cnt: 2 device words of
-// scratch per family; heads zeroed beforehand, one bit per record).
-long long chain_records(long long d0, long long d2, long long d3);
-cudaError_t launch_pack_chains(const double *F1, const double *F2, const double *gam,
-                               const double *rc, const long long d[4], long long rec_off,
-                               unsigned long long *cnt, int model, double dcut,
-                               const PackedFilaments &pf, unsigned *heads, BBox *bb,
-                               cudaStream_t s);
-cudaError_t launch_pad_chains(long long from, long long to, const PackedFilaments &pf,
-                              unsigned *heads, cudaStream_t s);
 cudaError_t launch_pack_targets(const double *P, long long ns, long long np, long long off,
                                 int group, double4 *tp, int *tgroup, BBox *bb, cudaStream_t s);
 cudaError_t launch_target_keys(const double4 *tp, const int *tgroup, long long n, const BBox *bb,

@@ -2,25 +2,24 @@
 //
 // HBM layout of one evaluation (all per-context, grow-only buffers):
 //   packed filaments, padded to the filament tile (KF) with inert entries, as
-//   pair records: filaments 2j and 2j+1 share 32 floats (8 float4), field q of
-//   filament 2j+h at float 2q+h, so every float4 holds two fields of both:
-//     fields  0-3   x1_hi.x, x1_hi.y, x1_hi.z, |L|^2
-//             4-7   x1_lo.x, x1_lo.y, x1_lo.z, Rn^2   (x1 = hi + lo to ~2^-48)
-//             8-11  L.x, L.y, L.z, D                  (L = x2 - x1)
-//            12-15  K L.x, K L.y, K L.z, rc           (K = gamma/4pi; rc the core
-//                                                       radius, Vatistas with K != 0, else 0)
+//   64-byte records of four float4 chunks:
+//     chunk 0   x1_hi.x, x1_hi.y, x1_hi.z, |L|^2
+//           1   K L.x, K L.y, K L.z, rc       (K = gamma/4pi; rc the core radius,
+//                                              Vatistas with K != 0, else 0)
+//           2   x1_lo.x, x1_lo.y, x1_lo.z, Rn^2   (x1 = hi + lo to ~2^-48)
+//           3   L.x, L.y, L.z, D              (L = x2 - x1)
 //   with D = (K^2 rc^2 |L|^2)^2 (Vatistas: the core term scaled like |K L x r1|^4,
 //   so K cancels from the core factor and enters only through K L) or d |L|^2
-//   (cut-off)
-//   For the FP32c evaluations the records form a chained stream: the lines of
-//   filaments of each family (the shed call's along the span, the trailing
-//   call's along the wake age) fill the two lanes of consecutive records so
-//   that x2 of a lane is x1 of the same lane one record earlier, except at the
-//   records flagged in a head bit array (F32cArgs::heads).
+//   (cut-off). Chunk q of record f lies at position q ^ ((f >> 2) & 3): the
+//   warp's screen, which reads a record per lane, then meets two-way bank
+//   conflicts instead of four-way, and a group of four records, which the pair
+//   loops read together, has one swizzle.
+//   The records form chains: x2 of a record is x1 of the one before it, except
+//   at heads, whose |L|^2 has the sign bit set.
 //   raw FP64 filaments for near-singular terms and the FP64 path
 //     ra[f] = (x1, y1, z1, gamma)  rb[f] = (x2, y2, z2, rc^2)   double4
-//   targets  tp[t] = (x, y, z, 0) double4, sorted by (group, Morton code of the
-//            position) so the T targets of a thread are close together;
+//   targets  tp[t] = (x, y, z, 0) double4, sorted by (group, place on a Hilbert
+//            curve) so the targets of a lane, and of a warp, are close together;
 //            perm[t] = index of sorted target t in the packed input order
 //   partial sums per work item: part[item][3][tile_cap] double
 #pragma once
@@ -79,7 +78,7 @@ struct BBox {           // ordered-int keys of float bounds (see float_key)
 };
 
 struct F32cArgs {
-  const float4 *pk;  // pair records, 8 float4 per two filaments
+  const float4 *pk;  // records, 4 float4 per filament
   const double4 *ra, *rb;
   const double4 *tp;
   const Group *groups;
@@ -87,10 +86,6 @@ struct F32cArgs {
   const Item *items;
   const int *order;  // work queue: queue position -> item (nullptr: identity)
   const GroupLive *live = nullptr;  // per group (nullptr: every tile and item is live)
-  // Chained stream (nullptr: unchained): bit (r & 31) of heads[r >> 5] is set
-  // when pair record r starts a chain, i.e. when either of its filaments does
-  // not end where the same lane's filament of record r - 1 begins.
-  const unsigned *heads = nullptr;
   int n_items;
   int tile_cap;
   double *part;

@@ -165,7 +165,7 @@ void shutdown_all() {
     for (DevBuf *b : {&c->pk, &c->ra, &c->rb, &c->tp, &c->tp_raw,
                       &c->tgroup, &c->keys, &c->vals, &c->perm, &c->sort_tmp, &c->groups,
                       &c->tiles, &c->items, &c->order, &c->part, &c->bbox, &c->ctr, &c->err,
-                      &c->nearctr,
+                      &c->nearctr, &c->chaincnt,
                       &c->in_P, &c->in_F, &c->out_u})
       b->release();
     c->htab.release();
@@ -292,19 +292,14 @@ int upload_plan(Context *c, const Plan &pl, cudaStream_t s) {
 }
 
 // ------------------------------------------------------------- packing
-// chain: lay the filaments out as a chained stream (the FP32c kernel's
-// faster form; bs_pack_chains), else in input order.
+// chain: order each family along the index with more links between neighbours
+// (bs_pack_filaments), else in input order.
 int pack_inputs(Context *c, const winds_bs_family *fams, int nfam,
                 const std::vector<TargetSpec> &tsets, int model, double dcut, cudaStream_t s,
                 long long *nf_real, long long *nf_pad, long long *nt_total, bool chain) {
-  long long nf = 0, nrec = 0;
-  for (int k = 0; k < nfam; ++k) {
-    const long long *d = fams[k].dims;
-    nf += d[0] * d[2] * d[3];
-    nrec += chain_records(d[0], d[2], d[3]);
-  }
-  const long long nfp =
-      std::max<long long>(round_up(chain ? 2 * nrec : nf, kFilamentPad), kFilamentPad);
+  long long nf = 0;
+  for (int k = 0; k < nfam; ++k) nf += fams[k].dims[0] * fams[k].dims[2] * fams[k].dims[3];
+  const long long nfp = std::max<long long>(round_up(nf, kFilamentPad), kFilamentPad);
   long long nt = 0;
   for (const TargetSpec &t : tsets) nt += t.count;
   int rc;
@@ -318,8 +313,7 @@ int pack_inputs(Context *c, const winds_bs_family *fams, int nfam,
       (rc = c->vals.ensure(std::max<long long>(nt, 1) * sizeof(int), s)) ||
       (rc = c->perm.ensure(std::max<long long>(nt, 1) * sizeof(int), s)))
     return rc;
-  if (chain && ((rc = c->heads.ensure((nfp / 64 + 1) * sizeof(unsigned), s)) ||
-                (rc = c->chaincnt.ensure(std::max(nfam, 1) * 2 * sizeof(unsigned long long), s))))
+  if ((rc = c->chaincnt.ensure(std::max(nfam, 1) * 2 * sizeof(unsigned long long), s)))
     return rc;
   size_t sort_bytes = 0;
   if (sort_target_keys(nullptr, &sort_bytes, nullptr, nullptr, nullptr, nullptr, nt, s) !=
@@ -330,36 +324,19 @@ int pack_inputs(Context *c, const winds_bs_family *fams, int nfam,
   cudaError_t e = launch_bbox_init((BBox *)c->bbox.p, s);
   c->launches += 1;
   c->chained = chain;
-  if (chain) {
-    unsigned *heads = (unsigned *)c->heads.p;
-    if (e == cudaSuccess) e = cudaMemsetAsync(heads, 0, (nfp / 64 + 1) * sizeof(unsigned), s);
-    long long roff = 0;
-    for (int k = 0; k < nfam && e == cudaSuccess; ++k) {
-      const long long *d = fams[k].dims;
-      e = launch_pack_chains(fams[k].F1, fams[k].F2, fams[k].gamma, fams[k].rc, d,
-                             roff, (unsigned long long *)c->chaincnt.p + 2 * k, model, dcut, pf,
-                             heads, (BBox *)c->bbox.p, s);
-      c->launches += d[0] * d[2] * d[3] > 0 ? 2 : 0;
-      roff += chain_records(d[0], d[2], d[3]);
-    }
-    if (e == cudaSuccess) {
-      e = launch_pad_chains(2 * nrec, nfp, pf, heads, s);
-      c->launches += nfp > 2 * nrec;
-    }
-  } else {
-    long long off = 0;
-    for (int k = 0; k < nfam && e == cudaSuccess; ++k) {
-      const long long *d = fams[k].dims;
-      const long long n = d[0] * d[2] * d[3];
-      e = launch_pack_filaments(fams[k].F1, fams[k].F2, fams[k].gamma, fams[k].rc, d[0], n, off,
-                                model, dcut, pf, (BBox *)c->bbox.p, s);
-      c->launches += n > 0;
-      off += n;
-    }
-    if (e == cudaSuccess) {
-      e = launch_pad_filaments(nf, nfp, pf, s);
-      c->launches += nfp > nf;
-    }
+  long long off = 0;
+  for (int k = 0; k < nfam && e == cudaSuccess; ++k) {
+    const long long *d = fams[k].dims;
+    const long long n = d[0] * d[2] * d[3];
+    e = launch_pack_filaments(fams[k].F1, fams[k].F2, fams[k].gamma, fams[k].rc, d, off,
+                              chain ? (unsigned long long *)c->chaincnt.p + 2 * k : nullptr, model,
+                              dcut, pf, (BBox *)c->bbox.p, s);
+    c->launches += n > 0 ? (chain ? 2 : 1) : 0;
+    off += n;
+  }
+  if (e == cudaSuccess) {
+    e = launch_pad_filaments(nf, nfp, pf, s);
+    c->launches += nfp > nf;
   }
   long long toff = 0;
   int gid = 0;
@@ -370,7 +347,7 @@ int pack_inputs(Context *c, const winds_bs_family *fams, int nfam,
     c->launches += t.count > 0;
     toff += t.count;
   }
-  // Sort targets by (set, Morton code) so each thread's targets lie close together.
+  // Sort targets by (set, Hilbert position) so each thread's targets lie close together.
   unsigned long long *k0 = (unsigned long long *)c->keys.p, *k1 = k0 + std::max<long long>(nt, 1);
   if (e == cudaSuccess)
     e = launch_target_keys((const double4 *)c->tp_raw.p, (const int *)c->tgroup.p, nt,
@@ -410,12 +387,14 @@ static int log2_bucket(long long n) {
   return b;
 }
 
-// Untuned tiling: 4 targets per thread (2 for small sets). T = 8 unrolls
-// twice as much code per path; where warps alternate between the screened
-// far path and the careful path it runs ~35% slower (64-case wake batch).
+// Untuned tiling: more targets per lane spread a filament's loads and the
+// screen over more pairs, fewer keep the warp's ball of targets small. Measured
+// in input order or chained: 2 against 4 targets per lane 82 against 82 us on
+// 3.2k targets, 4 against 6 (T = 3) 1.51 against 1.52 ms on 30k targets and
+// 13.1 against 12.1 ms on 89k.
 TuneChoice default_choice(long long nt) {
   TuneChoice ch;
-  ch.T = nt >= 2048 ? 4 : 2;
+  ch.T = nt >= 49152 ? 3 : (nt >= 2048 ? 4 : 2);
   ch.KF = 64;
   ch.waves = 32.0;
   return ch;
@@ -446,8 +425,8 @@ int run_direct_sum(Context *c, const std::vector<GroupSpec> &gs, int model, doub
     quantum = f64_tile();
   } else {
     if (!f32c_config_supported(ch.T, ch.KF)) return fail(WINDS_BS_ERR_ARG, "bad tile choice");
-    tile_cap = f32c_threads() * ch.T;
-    resident = f32c_occupancy(model, ch.T, ch.KF, c->chained) * c->num_sms;
+    tile_cap = f32c_tile(ch.T);
+    resident = f32c_occupancy(model, ch.T, ch.KF) * c->num_sms;
     quantum = kFilamentPad;
   }
   // sequential: one chunk per tile, so every target sums its filaments in order
@@ -500,7 +479,6 @@ int run_direct_sum(Context *c, const std::vector<GroupSpec> &gs, int model, doub
   a.n = n;
   a.co = co;
   a.wait_limit_ns = default_wait_limit_ns();
-  a.heads = precision == WINDS_PREC_F32C && c->chained ? (const unsigned *)c->heads.p : nullptr;
   cudaError_t e = cudaMemsetAsync(c->ctr.p, 0, sizeof(unsigned), s);
   // near-singular pairs are counted per evaluation
   if (e == cudaSuccess) e = cudaMemsetAsync(c->nearctr.p, 0, 2 * sizeof(unsigned long long), s);
@@ -628,9 +606,10 @@ int eval_device(Context *c, const winds_bs_family *fams, int nfam,
 // packed and returns the fastest with its time.
 int autotune(Context *c, const std::vector<GroupSpec> &gs, int model, double dcut, double n,
              double co, TuneChoice *best, float *best_ms_out) {
-  // T = 8 (supported, settable) is left out: its unrolled paths run slower
+  // T = 8 (supported, settable) is left out: its target balls are too wide
+  // (6 targets per lane 1.52 ms, 8 1.67 ms on the 60k-filament wake)
   const int Ts[3] = {2, 3, 4};
-  const int KFs[3] = {32, 64, 128};
+  const int KFs[2] = {32, 64};
   const double Ws[3] = {16.0, 32.0, 64.0};
   float best_ms = 1e30f;
   TuneChoice bc;

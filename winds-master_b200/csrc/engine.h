@@ -66,9 +66,8 @@ struct Context {
   DevBuf groups, tiles, items, order, part;
   // small words
   DevBuf bbox, ctr, err, nearctr;
-  // chained filament stream (FP32c path): head bit per pair record, and the
-  // per-family link counts that choose each family's layout
-  DevBuf heads, chaincnt;
+  // per-family link counts that choose each family's order
+  DevBuf chaincnt;
   bool chained = false;  // the packed filaments are a chained stream
   // device copies of host inputs/outputs (host API)
   DevBuf in_P, in_F, out_u;

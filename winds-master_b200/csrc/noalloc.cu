@@ -159,7 +159,7 @@ extern "C" int winds_bs_eval_device_noalloc(const winds_bs_family *fams, int nfa
     resident = f64_occupancy() * sms;
     quantum = f64_tile();
   } else {
-    tile_cap = f32c_threads() * ch.T;
+    tile_cap = f32c_tile(ch.T);
     resident = f32c_occupancy(model, ch.T, ch.KF) * sms;
     quantum = kFilamentPad;
   }
@@ -188,6 +188,7 @@ extern "C" int winds_bs_eval_device_noalloc(const winds_bs_family *fams, int nfa
   unsigned *err = cv.take<unsigned>(4);
   unsigned long long *nearc = cv.take<unsigned long long>(2);  // near, core-free pairs
   PackedFilaments pf{cv.take<float4>(nfp * 4), cv.take<double4>(nfp), cv.take<double4>(nfp)};
+  unsigned long long *chaincnt = cv.take<unsigned long long>(2);
   double4 *tp = cv.take<double4>(nt);
   double4 *tp_raw = cv.take<double4>(nt);
   int *tgroup = cv.take<int>(nt);
@@ -216,8 +217,9 @@ extern "C" int winds_bs_eval_device_noalloc(const winds_bs_family *fams, int nfa
   for (int k = 0; k < nfam && e == cudaSuccess; ++k) {
     const long long *d = fams[k].dims;
     const long long m = d[0] * d[2] * d[3];
-    e = launch_pack_filaments(fams[k].F1, fams[k].F2, fams[k].gamma, fams[k].rc, d[0], m, off,
-                              model, dcut, pf, bbox, s);
+    e = launch_pack_filaments(fams[k].F1, fams[k].F2, fams[k].gamma, fams[k].rc, d, off,
+                              prec == WINDS_PREC_F32C ? chaincnt : nullptr, model, dcut, pf, bbox,
+                              s);
     off += m;
   }
   if (e == cudaSuccess) e = launch_pad_filaments(nf, nfp, pf, s);

@@ -166,7 +166,7 @@ int build_plans(winds_wake_batch *b) {
     resident = f64_occupancy() * sms;
     quantum = f64_tile();
   } else {
-    b->tile_cap = f32c_threads() * b->ch.T;
+    b->tile_cap = f32c_tile(b->ch.T);
     resident = f32c_occupancy(b->model, b->ch.T, b->ch.KF) * sms;
     quantum = kFilamentPad;
   }
@@ -1289,7 +1289,7 @@ int winds_wake_set_kj(winds_wake_batch *b, const winds_kj_case *kj, const winds_
     resident = f64_occupancy() * sms;
     quantum = f64_tile();
   } else {
-    b->kj_tile_cap = f32c_threads() * b->kj_T;
+    b->kj_tile_cap = f32c_tile(b->kj_T);
     resident = f32c_occupancy(b->model, b->kj_T, b->kj_KF) * sms;
     quantum = kFilamentPad;
   }

@@ -16,7 +16,9 @@
 // wake.domain{p} of core/initials.m:44-51 is live_cols = min(2 + s, na)).
 // Memory is addressed with the capacity's strides; the packed filaments of
 // the direct sum are numbered over the live columns only (shed, then
-// trailing), so the live ones are the first of the case's range.
+// trailing: shed along the span, trailing along the wake age, the lines of
+// connected filaments that the direct sum follows), so the live ones are the
+// first of the case's range.
 #include "bs_device.cuh"
 #include "wake_launch.h"
 #include "wake_types.h"
@@ -132,13 +134,14 @@ __global__ void wake_filaments(const WakeCase *cases, const int *step, int step_
   const WakeCase c = cases[blockIdx.y];
   const long long f = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
-  float v[16];
   const int ns = c.nst - 1;
   const int s = *step + step_add;
   const int na_l = live_cols(c, s);
   const long long nsh = (long long)ns * na_l * c.nb;
-  if (f < live_filaments(c, na_l)) {
+  const long long nlive = live_filaments(c, na_l);
+  if (f < nlive) {
     int i, j, b, m;
+    long long place = f;
     double x1, y1, z1, x2, y2, z2, g, age;
     long long slot;
     const double *lold;
@@ -164,6 +167,8 @@ __global__ void wake_filaments(const WakeCase *cases, const int *step, int step_
       j = q % (na_l - 1);
       b = q / (na_l - 1);
       m = na_l - 1;
+      // along the wake age; threads run along the span, as the arrays do
+      place = nsh + j + (na_l - 1) * ((long long)i + (long long)c.nst * b);
       x1 = node_comp(dom, c, i, 0, j + 1, b), y1 = node_comp(dom, c, i, 1, j + 1, b);
       z1 = node_comp(dom, c, i, 2, j + 1, b);
       x2 = node_comp(dom, c, i, 0, j, b), y2 = node_comp(dom, c, i, 1, j, b);
@@ -191,21 +196,13 @@ __global__ void wake_filaments(const WakeCase *cases, const int *step, int step_
       lnew[slot] = L;
       if (rcout) rcout[slot] = rc;
     }
-    pf.ra[c.fil_off + f] = make_double4(x1, y1, z1, g);
-    pf.rb[c.fil_off + f] = make_double4(x2, y2, z2, rc);
-    filament_fields(x1, y1, z1, x2, y2, z2, g, rc, model, dcut, v);
+    pack_filament(c.fil_off + place, x1, y1, z1, x2, y2, z2, g, rc, f < nsh,
+                  f < nsh ? i == 0 : j == 0, model, dcut, pf.pk, pf.ra, pf.rb);
     lo[0] = (float)fmin(x1, x2), lo[1] = (float)fmin(y1, y2), lo[2] = (float)fmin(z1, z2);
     hi[0] = (float)fmax(x1, x2), hi[1] = (float)fmax(y1, y2), hi[2] = (float)fmax(z1, z2);
-  } else {
-    inert_fields(v);
-    if (f < c.fil_pad) {
-      pf.ra[c.fil_off + f] = make_double4(kInertFar, kInertFar, kInertFar, 0.0);
-      pf.rb[c.fil_off + f] = make_double4(kInertFar, kInertFar, kInertFar, 0.0);
-    }
+  } else if (f < c.fil_pad) {
+    pack_inert(c.fil_off + f, pf.pk, pf.ra, pf.rb);
   }
-  // fil_off and fil_pad are multiples of kFilamentPad, so both filaments of a
-  // pair are in this warp and both are stored (real or inert) or neither is
-  store_pair_fields(pf.pk, c.fil_off + f, v, f < c.fil_pad);
   bbox_accumulate(lo, hi, bb->fmin, bb->fmax);
 }
 
@@ -248,7 +245,7 @@ __global__ void wake_filaments_bound_cols(const WakeCase *cases, const int *step
     b = u / c.nst;
     i = u - b * c.nst;
     const long long slot = c.trail_off + i + (long long)c.nst * ((long long)(c.na - 1) * b);
-    f = (long long)ns * na_l * c.nb + i + (long long)c.nst * ((long long)(na_l - 1) * b);
+    f = (long long)ns * na_l * c.nb + (na_l - 1) * ((long long)i + (long long)c.nst * b);
     x1 = node_comp(dom, c, i, 0, 1, b), y1 = node_comp(dom, c, i, 1, 1, b);
     z1 = node_comp(dom, c, i, 2, 1, b);
     x2 = node_comp(dom, c, i, 0, 0, b), y2 = node_comp(dom, c, i, 1, 0, b);
@@ -256,7 +253,8 @@ __global__ void wake_filaments_bound_cols(const WakeCase *cases, const int *step
     g = trail[slot];
     rc = rc_in_t[slot];
   }
-  pack_filament(c.fil_off + f, x1, y1, z1, x2, y2, z2, g, rc, model, dcut, pf.pk, pf.ra, pf.rb);
+  pack_filament(c.fil_off + f, x1, y1, z1, x2, y2, z2, g, rc, t < n_shed,
+                t < n_shed ? i == 0 : true, model, dcut, pf.pk, pf.ra, pf.rb);
 }
 
 // One thread per node slot of the case: nodes of the live columns of step
