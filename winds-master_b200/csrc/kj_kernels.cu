@@ -1,13 +1,18 @@
 // kj_kernels.cu -- device kernels of the Kutta-Joukowski fixed point
 // (core/KuttaJoukowski.m:42-49 and kj(), :173-298) for every case of a batch.
 //   kj_targets   lifting-line points of step s -> direct-sum targets (:216-219)
-//   kj_update    blade-frame transform (:241-246), aoa (:258), interp1 of the
-//                airfoil tables (:262-269), Γ = ½|V|c Cl (:277), relaxed update
-//                (:281), relative residual in FP64 (:290), per station
-//   kj_check     per case: converged when max |residual| <= tol (:45)
+//   kj_solve     the fixed point: every iteration of every case in one launch,
+//                per station the blade-frame transform (:241-246), aoa (:258),
+//                interp1 of the airfoil tables (:262-269), Γ = ½|V|c Cl (:277),
+//                the relaxed update (:281) and the relative residual in FP64
+//                (:290); a case stops when max |residual| <= tol (:45)
+//   kj_finish    the batch's iteration count and the last induced velocities
 //   kj_features, kj_apply_guess   inputs and result of the bound-circulation
 //                MLP that replaces the previous-step start value (WInDS.m:131)
 //   kj_loads     rotor thrust, torque and power (postproc/perform.m:18-62)
+#include <cooperative_groups.h>
+
+#include <algorithm>
 #include <cmath>
 
 #include "bs_device.cuh"
@@ -33,60 +38,298 @@ __global__ void kj_targets(const WakeCase *cases, const KJCase *kc, const int *s
   bbox_accumulate(lo, hi, bb->tmin, bb->tmax);
 }
 
-// MATLAB interp1(x, y, xi): linear, NaN outside [x(1), x(end)].
-__device__ double interp1(const double *x, const double *y, int n, double xi) {
-  if (!(xi >= x[0] && xi <= x[n - 1])) return NAN;
+// MATLAB interp1(x, y, xi) of two tables: linear, NaN outside [x(1), x(end)].
+__device__ void interp1(const double *x, const double *y, const double *z, int n, double xi,
+                        double &yi, double &zi) {
+  if (!(xi >= x[0] && xi <= x[n - 1])) {
+    yi = zi = NAN;
+    return;
+  }
   int lo = 0, hi = n - 1;
   while (hi - lo > 1) {
     const int mid = (lo + hi) >> 1;
     if (x[mid] <= xi) lo = mid; else hi = mid;
   }
   const double t = (xi - x[lo]) / (x[hi] - x[lo]);
-  return y[lo] + t * (y[hi] - y[lo]);
+  yi = y[lo] + t * (y[hi] - y[lo]);
+  zi = z[lo] + t * (z[hi] - z[lo]);
 }
 
-__global__ void kj_update(const WakeCase *cases, const KJCase *kc, const int *step,
-                          const double *uindb, const double *bxn, const double *byn,
-                          const double *bzn, const double *vblade, const double *chord,
-                          const int *foil, const int *foil_off, const double *aoa_t,
-                          const double *cl_t, const double *cd_t, double relax, double *bound,
-                          const int *converged, unsigned long long *res_max, int *diverged,
-                          double *cl_out, double *cd_out, double *aoa_out) {
-  const int ci = blockIdx.y;
-  const WakeCase c = cases[ci];
-  const KJCase k = kc[ci];
+// ---------------------------------------------------------------- kj_solve
+// The iteration's Biot-Savart calls (KuttaJoukowski.m:216,218) differ from one
+// iteration to the next only in the circulation of the filaments that follow
+// the bound iterate -- shed columns 0 and 1 and trailing column 0, nb (2 ns +
+// nst) "own" filaments -- and the velocity is linear in it. So the direct sum
+// over all other filaments runs once per step (u_fix), and an iteration adds
+// the own filaments' influence: a matrix of unit-circulation terms in FP64,
+// formed once, times their circulation. Before, each iteration was six
+// launches over every filament: 89 us for one rotor of 17 x 60 (23 us of it
+// the sum), 30 iterations of it most of the step.
+//
+// A cluster of kCluster CTAs runs a case. Each CTA owns a slice of the
+// lifting-line points: it forms their rows of the matrix in its shared memory
+// (16 points x 363 filaments x 24 B on 41 nodes; beyond the limit the rows go to
+// the global scratch, and with no scratch each term is formed again in each
+// iteration), and every iteration a warp per point sums its row, updates its
+// station and sends the new circulation to all CTAs of the cluster. One cluster
+// barrier per iteration; each CTA then forms all own circulations by itself.
+// Latency bounds it: the barrier, the span sums and the station update are
+// chains. Every loop ends after maxiter iterations.
+namespace cg = cooperative_groups;
+constexpr int kCluster = 8;
+constexpr int kSolveThreads = 512;
+constexpr int kSolveWarps = kSolveThreads / 32;
+
+// Endpoints, squared core and index of own filament f of case c: shed columns 0
+// and 1 of each blade (b, j, i), then trailing column 0 (b, i).
+struct OwnFilament {
+  double4 A, B;
+};
+__device__ __forceinline__ OwnFilament own_filament(const WakeCase &c, const double *dom,
+                                                    const double *rc_s, const double *rc_t, int f) {
+  const int ns = c.nst - 1, n_shed = c.nb * 2 * ns;
+  int i, j, b, j1, j2, i2;
+  double rc;
+  if (f < n_shed) {
+    b = f / (2 * ns);
+    const int r = f - b * 2 * ns;
+    j = r / ns;
+    i = r - j * ns;
+    j1 = j2 = j;
+    i2 = i + 1;
+    rc = rc_s[c.shed_off + i + (long long)ns * (j + (long long)c.na * b)];
+  } else {
+    const int u = f - n_shed;
+    b = u / c.nst;
+    i = i2 = u - b * c.nst;
+    j1 = 1, j2 = 0;
+    rc = rc_t[c.trail_off + i + (long long)c.nst * ((long long)(c.na - 1) * b)];
+  }
+  const double *p1 = dom + c.node_off * 3 + i + (long long)c.nst * 3 * (j1 + (long long)c.na * b);
+  const double *p2 = dom + c.node_off * 3 + i2 + (long long)c.nst * 3 * (j2 + (long long)c.na * b);
+  OwnFilament o;
+  o.A = make_double4(p1[0], p1[c.nst], p1[2 * c.nst], 1.0);
+  o.B = make_double4(p2[0], p2[c.nst], p2[2 * c.nst], rc);
+  return o;
+}
+
+// Station (i, b) of the case with induced velocity u: writes cl, cd, aoa and
+// returns the updated circulation; the residual's bits in *res (0, and the
+// circulation unchanged, where Cl is NaN).
+__device__ double station_update(const KJSolveArgs &a, const WakeCase &c, const KJCase &k, int ci,
+                                 int s, int i, int b, const double u[3], double bound,
+                                 unsigned long long *res) {
   const int ns = c.nst - 1;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= ns * c.nb || converged[ci]) return;
-  const int i = t % ns, b = t / ns;
-  const int s = *step;
   const long long fo = k.frame_off + i + (long long)ns * (3 * (s + (long long)c.nsteps * b));
-  const double *u = uindb + 3 * k.t_off + i + (long long)ns * 3 * b;  // [ns,3,nb] of this case
   double rot[3];
-  const double *fr[3] = {bxn, byn, bzn};
-  for (int a = 0; a < 3; ++a)
-    rot[a] = fr[a][fo] * u[0] + fr[a][fo + ns] * u[ns] + fr[a][fo + 2 * ns] * u[2 * ns];
-  const double vb0 = vblade[fo], vb1 = vblade[fo + ns], vb2 = vblade[fo + 2 * ns];
+  const double *fr[3] = {a.bxn, a.byn, a.bzn};
+#pragma unroll
+  for (int q = 0; q < 3; ++q)
+    rot[q] = fr[q][fo] * u[0] + fr[q][fo + ns] * u[1] + fr[q][fo + 2 * ns] * u[2];
+  const double vb0 = a.vblade[fo], vb1 = a.vblade[fo + ns], vb2 = a.vblade[fo + 2 * ns];
   const double tu = vb0 + rot[0], tv = vb1 + rot[1];
   const double Vinf = sqrt(vb0 * vb0 + vb1 * vb1 + vb2 * vb2);
   const double aoa = atan2(-tv, tu) * (180.0 / kPi);
-  const int f = foil[k.station_off + i];
-  const int o0 = foil_off[k.foil_base + f], o1 = foil_off[k.foil_base + f + 1];
-  const double cl = interp1(aoa_t + o0, cl_t + o0, o1 - o0, aoa);
-  const double cd = interp1(aoa_t + o0, cd_t + o0, o1 - o0, aoa);
+  const int f = a.foil[k.station_off + i];
+  const int o0 = a.foil_off[k.foil_base + f], o1 = a.foil_off[k.foil_base + f + 1];
+  double cl, cd;
+  interp1(a.aoa_t + o0, a.cl_t + o0, a.cd_t + o0, o1 - o0, aoa, cl, cd);
   const long long q = c.bound_off + i + (long long)ns * b;  // station slot of the case
-  cl_out[q] = cl;
-  cd_out[q] = cd;
-  aoa_out[q] = aoa;
+  a.cl_out[q] = cl;
+  a.cd_out[q] = cd;
+  a.aoa_out[q] = aoa;
+  *res = 0ull;
   if (isnan(cl)) {
-    atomicOr(&diverged[ci], 1);
-    return;
+    atomicOr(&a.diverged[ci], 1);
+    return bound;
   }
-  const double gamma = 0.5 * Vinf * chord[k.station_off + i] * cl;
-  const double dg = gamma - bound[q];
-  bound[q] = bound[q] + relax * dg;
-  const double r = fabs(dg / (fabs(gamma) + 1.0));
-  atomicMax(&res_max[ci], (unsigned long long)__double_as_longlong(r));
+  const double gamma = 0.5 * Vinf * a.chord[k.station_off + i] * cl;
+  const double dg = gamma - bound;
+  *res = (unsigned long long)__double_as_longlong(fabs(dg / (fabs(gamma) + 1.0)));
+  return bound + a.relax * dg;
+}
+
+__global__ void __launch_bounds__(kSolveThreads) kj_solve(const KJSolveArgs a) {
+  extern __shared__ __align__(16) double kj_smem[];
+  cg::cluster_group cl = cg::this_cluster();
+  const int ci = blockIdx.x / kCluster, rank = blockIdx.x % kCluster;
+  const WakeCase c = a.cases[ci];
+  const KJCase k = a.kc[ci];
+  const int s = *a.step;
+  if (s < c.kj_from) return;  // the start-up's first step has no iteration
+  const int ns = c.nst - 1, nt = ns * c.nb, n_shed = c.nb * 2 * ns, own = n_shed + c.nb * c.nst;
+  const int per = (nt + kCluster - 1) / kCluster;
+  const int t0 = rank * per;
+  const int cnt = max(0, min(per, nt - t0));
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  // shared or (vectors too long for it) global working vectors: the bound
+  // iterate and the residuals of all points, twice; the own circulations; the
+  // part of shed column 1 that stays
+  double *vec = a.vec_smem ? kj_smem : a.vec_scratch + ((long long)ci * kCluster + rank) * a.vec_stride;
+  double *sB[2] = {vec, vec + nt};
+  unsigned long long *sR[2] = {reinterpret_cast<unsigned long long *>(vec + 2 * nt),
+                               reinterpret_cast<unsigned long long *>(vec + 3 * nt)};
+  double *sG = vec + 4 * nt, *sC = sG + own;
+  double *mat = a.mat_smem      ? kj_smem + (a.vec_smem ? a.vec_stride : 0)
+                : a.mat_scratch ? a.mat_scratch + ((long long)ci * kCluster + rank) * a.mat_stride
+                                : nullptr;
+  RefParams rp;
+  rp.model = a.model;
+  rp.d = a.d;
+  rp.n = a.n;
+  rp.co = a.co;
+  const auto term = [&](int tt, int f, double u[3]) {
+    const double4 p = a.tp[k.t_off + t0 + tt];
+    const OwnFilament o = own_filament(c, a.dom, a.rc_s, a.rc_t, f);
+    u[0] = u[1] = u[2] = 0.0;
+    ref_pair(o.A, o.B, p.x, p.y, p.z, rp, u[0], u[1], u[2]);
+  };
+  if (mat)
+    for (int idx = tid; idx < cnt * own; idx += kSolveThreads) {
+      const int tt = idx / own, f = idx - tt * own;
+      double u[3];
+      term(tt, f, u);
+#pragma unroll
+      for (int q = 0; q < 3; ++q) mat[(long long)(3 * tt + q) * own + f] = u[q];
+    }
+  for (int t = tid; t < nt; t += kSolveThreads) sB[0][t] = a.bound[c.bound_off + t];
+  // shed(:, 1) = C_1 - C_0 (WInDS.m:139-140): C_1, of the previous step's
+  // trailing column 0, stays; summed as wake_bookkeep does
+  const int m = live_cols(c, s) - 1;
+  for (int b = tid; b < c.nb; b += kSolveThreads) {
+    double cum = 0.0;
+    const double *tp = a.trail_prev + c.trail_off + (long long)c.nst * ((long long)(c.na - 1) * b);
+    for (int i = 0; i < ns; ++i) {
+      if (m > 1) cum += tp[i];
+      sC[i + ns * b] = cum;
+    }
+  }
+  cl.sync();
+  // the own circulations of iterate B; a non-finite one adds nothing, as its
+  // terms are zeroed in the direct sum (BiotSavart.m:111)
+  const auto circulation = [&](const double *B) {
+    const auto put = [&](int f, double g) { sG[f] = isfinite(g) ? g : 0.0; };
+    for (int t = tid; t < c.nb * c.nst; t += kSolveThreads) {
+      const int b = t / c.nst, i = t - b * c.nst;
+      const double hi = i < ns ? B[i + ns * b] : 0.0, lo = i > 0 ? B[i - 1 + ns * b] : 0.0;
+      put(n_shed + t, hi - lo);
+      if (i < ns) put(2 * ns * b + i, hi);
+    }
+    if (lane == 0)  // one warp per blade: the span sums are chains
+      for (int b = warp; b < c.nb; b += kSolveWarps) {
+        double cum = 0.0, lo = 0.0;
+        for (int i = 0; i < ns; ++i) {
+          const double hi = B[i + ns * b];
+          cum += hi - lo;
+          lo = hi;
+          put(2 * ns * b + ns + i, sC[i + ns * b] - cum);
+        }
+      }
+    __syncthreads();
+  };
+  // velocity at point tt of this CTA, in every lane of the warp
+  const auto velocity = [&](int tt, double u[3]) {
+    double v[3] = {0.0, 0.0, 0.0};
+    if (mat) {
+      const double *r = mat + (long long)3 * tt * own;
+      for (int f = lane; f < own; f += 32) {
+        const double g = sG[f];
+        v[0] = fma(r[f], g, v[0]);
+        v[1] = fma(r[own + f], g, v[1]);
+        v[2] = fma(r[2 * own + f], g, v[2]);
+      }
+    } else {
+      for (int f = lane; f < own; f += 32) {
+        double w[3];
+        term(tt, f, w);
+        const double g = sG[f];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) v[q] = fma(w[q], g, v[q]);
+      }
+    }
+    const int t = t0 + tt, b = t / ns, i = t - b * ns;
+    const double *fix = a.u_fix + 3 * k.t_off + i + (long long)ns * 3 * b;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_xor_sync(0xffffffffu, v[q], o);
+      u[q] = fix[q * ns] + v[q];
+    }
+  };
+  int it = 0;
+  bool done = false;
+  double res = 0.0;
+  while (it < a.maxiter && !done) {
+    const int cur = it & 1, nxt = cur ^ 1;
+    circulation(sB[cur]);
+    for (int tt = warp; tt < cnt; tt += kSolveWarps) {
+      double u[3];
+      velocity(tt, u);
+      const int t = t0 + tt, b = t / ns, i = t - b * ns;
+      double g = 0.0;
+      unsigned long long r = 0ull;
+      if (lane == 0) {
+        g = station_update(a, c, k, ci, s, i, b, u, sB[cur][t], &r);
+        double *o = a.uindb + 3 * k.t_off + i + (long long)ns * 3 * b;  // [ns,3,nb] of this case
+#pragma unroll
+        for (int q = 0; q < 3; ++q) o[q * ns] = u[q];
+      }
+      g = __shfl_sync(0xffffffffu, g, 0);
+      r = __shfl_sync(0xffffffffu, r, 0);
+      if (lane < kCluster) {
+        if (a.vec_smem) {
+          *cl.map_shared_rank(sB[nxt] + t, lane) = g;
+          *cl.map_shared_rank(sR[nxt] + t, lane) = r;
+        } else {
+          const long long o = ((long long)lane - rank) * a.vec_stride;
+          sB[nxt][o + t] = g;
+          sR[nxt][o + t] = r;
+        }
+      }
+    }
+    cl.sync();
+    unsigned long long r = 0ull;  // largest residual: the bits of non-negative doubles order them
+    for (int t = lane; t < nt; t += 32) r = max(r, sR[nxt][t]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) r = max(r, __shfl_xor_sync(0xffffffffu, r, o));
+    res = __longlong_as_double((long long)r);
+    done = res <= a.tol;
+    ++it;
+  }
+  for (int t = t0 + tid; t < t0 + cnt; t += kSolveThreads) a.bound[c.bound_off + t] = sB[it & 1][t];
+  if (done) {
+    // the velocities of the converged circulation, for kj_finish
+    circulation(sB[it & 1]);
+    for (int tt = warp; tt < cnt; tt += kSolveWarps) {
+      double u[3];
+      velocity(tt, u);
+      const int t = t0 + tt, b = t / ns, i = t - b * ns;
+      double *o = a.uindb_conv + 3 * k.t_off + i + (long long)ns * 3 * b;
+      if (lane == 0)
+#pragma unroll
+        for (int q = 0; q < 3; ++q) o[q * ns] = u[q];
+    }
+  }
+  if (rank == 0 && tid == 0) {
+    a.iters[ci] = it;
+    a.converged[ci] = done;
+    a.res_last[ci] = res;
+    atomicMax(a.it_max, it);
+  }
+  cl.sync();  // no CTA leaves while another may still read or write its shared memory
+}
+
+// A case that converged before the batch's last iteration ends with the
+// induced velocity of its converged circulation, as if it had been evaluated
+// with the others to the end.
+__global__ void kj_finish(const WakeCase *cases, const KJCase *kc, const int *iters,
+                          const int *converged, const int *it_max, const double *uindb_conv,
+                          double *uindb) {
+  const int ci = blockIdx.y;
+  const int n = 3 * (cases[ci].nst - 1) * cases[ci].nb;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= n || !converged[ci] || iters[ci] >= *it_max) return;
+  uindb[3 * kc[ci].t_off + t] = uindb_conv[3 * kc[ci].t_off + t];
 }
 
 // The inflow features are the station's total inflow in the blade frame at
@@ -224,69 +467,6 @@ __global__ void kj_sum_loads(const WakeCase *cases, const KJCase *kc, int ncases
   for (int a = 0; a < 3; ++a) out[3 * ci + a] = tot[a];
 }
 
-// One thread per case: a case converged in this iteration stops updating.
-__global__ void kj_check(int ncases, double tol, int *converged, int *iters,
-                         unsigned long long *res_max, double *res_last, int *active) {
-  const int ci = blockIdx.x * blockDim.x + threadIdx.x;
-  if (ci == 0) *active = 0;
-  __syncthreads();
-  if (ci >= ncases || converged[ci]) return;
-  const double r = __longlong_as_double((long long)res_max[ci]);
-  res_max[ci] = 0ull;
-  res_last[ci] = r;
-  iters[ci] += 1;
-  if (r <= tol) converged[ci] = 1; else atomicOr(active, 1);
-}
-
-// kj_check inside a graph's conditional WHILE node: the same per-case update,
-// then one thread sets the loop condition -- continue while any case is active
-// and fewer than maxiter iterations ran (the counter makes the loop finite).
-__global__ void kj_check_cond(int ncases, double tol, int *converged, int *iters,
-                              unsigned long long *res_max, double *res_last, int *active,
-                              int *it_ctr, int maxiter, cudaGraphConditionalHandle h) {
-  __shared__ int any;
-  if (threadIdx.x == 0) any = 0;
-  __syncthreads();
-  for (int ci = threadIdx.x; ci < ncases; ci += blockDim.x) {
-    if (converged[ci]) continue;
-    const double r = __longlong_as_double((long long)res_max[ci]);
-    res_max[ci] = 0ull;
-    res_last[ci] = r;
-    iters[ci] += 1;
-    if (r <= tol) converged[ci] = 1; else atomicOr(&any, 1);
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    *active = any;
-    const int it = *it_ctr + 1;
-    *it_ctr = it;
-    cudaGraphSetConditional(h, (any && it < maxiter) ? 1u : 0u);
-  }
-}
-
-// Upstream of a graph's WHILE node: no iteration at a step before the one the
-// iteration starts at (WakeCase::kj_from, the same for every case; the
-// reference's first step is core/initials.m's, which has none).
-__global__ void kj_gate_cond(const WakeCase *cases, const int *step, cudaGraphConditionalHandle h) {
-  if (threadIdx.x == 0 && *step < cases[0].kj_from) cudaGraphSetConditional(h, 0u);
-}
-
-cudaError_t launch_kj_gate_cond(const WakeCase *cases, const int *step,
-                                cudaGraphConditionalHandle h, cudaStream_t s) {
-  kj_gate_cond<<<1, 32, 0, s>>>(cases, step, h);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_kj_check_cond(int ncases, double tol, int *converged, int *iters,
-                                 unsigned long long *res_max, double *res_last, int *active,
-                                 int *it_ctr, int maxiter, cudaGraphConditionalHandle h,
-                                 cudaStream_t s) {
-  const int bs = ncases <= 1024 ? ((ncases + 31) / 32) * 32 : 1024;
-  kj_check_cond<<<1, bs, 0, s>>>(ncases, tol, converged, iters, res_max, res_last, active, it_ctr,
-                                 maxiter, h);
-  return cudaGetLastError();
-}
-
 cudaError_t launch_kj_targets(const WakeCase *cases, const KJCase *kc, int ncases, int max_st,
                               const int *step, const double *ll, double4 *tp, BBox *bb,
                               cudaStream_t s) {
@@ -294,17 +474,41 @@ cudaError_t launch_kj_targets(const WakeCase *cases, const KJCase *kc, int ncase
   return cudaGetLastError();
 }
 
-cudaError_t launch_kj_update(const WakeCase *cases, const KJCase *kc, int ncases, int max_st,
-                             const int *step, const double *uindb, const double *bxn,
-                             const double *byn, const double *bzn, const double *vblade,
-                             const double *chord, const int *foil, const int *foil_off,
-                             const double *aoa_t, const double *cl_t, const double *cd_t,
-                             double relax, double *bound, const int *converged,
-                             unsigned long long *res_max, int *diverged, double *cl_out,
-                             double *cd_out, double *aoa_out, cudaStream_t s) {
-  kj_update<<<dim3((max_st + 127) / 128, ncases), 128, 0, s>>>(
-      cases, kc, step, uindb, bxn, byn, bzn, vblade, chord, foil, foil_off, aoa_t, cl_t, cd_t,
-      relax, bound, converged, res_max, diverged, cl_out, cd_out, aoa_out);
+// Doubles of a CTA's working vectors and matrix rows for a case of ns stations
+// and nb blades.
+long long kj_vec_doubles(int ns, int nb) {
+  return 4LL * ns * nb + (long long)nb * (3 * ns + 1) + (long long)ns * nb;
+}
+long long kj_mat_doubles(int ns, int nb) {
+  return (long long)(ns * nb + kCluster - 1) / kCluster * 3 * nb * (3 * ns + 1);
+}
+int kj_cluster() { return kCluster; }
+
+cudaError_t launch_kj_solve(const KJSolveArgs &a, int ncases, cudaStream_t s) {
+  const size_t smem = (size_t)((a.vec_smem ? a.vec_stride : 0) + (a.mat_smem ? a.mat_stride : 0)) *
+                      sizeof(double);
+  cudaError_t e = cudaFuncSetAttribute(kj_solve, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)kKJSmemBytes);
+  if (e != cudaSuccess) return e;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)ncases * kCluster);
+  cfg.blockDim = dim3(kSolveThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = kCluster;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kj_solve, a);
+}
+
+cudaError_t launch_kj_finish(const WakeCase *cases, const KJCase *kc, int ncases, int max_st,
+                             const int *iters, const int *converged, const int *it_max,
+                             const double *uindb_conv, double *uindb, cudaStream_t s) {
+  kj_finish<<<dim3((3 * max_st + 127) / 128, ncases), 128, 0, s>>>(cases, kc, iters, converged,
+                                                                   it_max, uindb_conv, uindb);
   return cudaGetLastError();
 }
 
@@ -342,15 +546,6 @@ cudaError_t launch_kj_loads(const WakeCase *cases, const KJCase *kc, int ncases,
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   kj_sum_loads<<<(ncases + 127) / 128, 128, 0, s>>>(cases, kc, ncases, dl, out);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_kj_check(int ncases, double tol, int *converged, int *iters,
-                            unsigned long long *res_max, double *res_last, int *active,
-                            cudaStream_t s) {
-  const int bs = ncases <= 1024 ? ((ncases + 31) / 32) * 32 : 1024;
-  if (ncases > 1024) return cudaErrorInvalidValue;
-  kj_check<<<1, bs, 0, s>>>(ncases, tol, converged, iters, res_max, res_last, active);
   return cudaGetLastError();
 }
 

@@ -31,14 +31,37 @@ constexpr int kKJFeatures = 11;
 cudaError_t launch_kj_targets(const WakeCase *cases, const KJCase *kc, int ncases, int max_st,
                               const int *step, const double *ll, double4 *tp, BBox *bb,
                               cudaStream_t s);
-cudaError_t launch_kj_update(const WakeCase *cases, const KJCase *kc, int ncases, int max_st,
-                             const int *step, const double *uindb, const double *bxn,
-                             const double *byn, const double *bzn, const double *vblade,
-                             const double *chord, const int *foil, const int *foil_off,
-                             const double *aoa_t, const double *cl_t, const double *cd_t,
-                             double relax, double *bound, const int *converged,
-                             unsigned long long *res_max, int *diverged, double *cl_out,
-                             double *cd_out, double *aoa_out, cudaStream_t s);
+// kj_solve: the whole iteration of every case (kj_kernels.cu). vec_* / mat_*: the
+// working vectors and matrix rows of a CTA in doubles (strides: the largest
+// case's), in shared memory or in a global scratch of stride doubles per CTA,
+// kj_cluster() CTAs a case; without either the matrix is formed term by term.
+constexpr long long kKJSmemBytes = 200 * 1024;
+struct KJSolveArgs {
+  const WakeCase *cases;
+  const KJCase *kc;
+  const int *step;
+  const double4 *tp;
+  const double *dom, *trail_prev, *rc_s, *rc_t, *u_fix;
+  const double *bxn, *byn, *bzn, *vblade, *chord;
+  const int *foil, *foil_off;
+  const double *aoa_t, *cl_t, *cd_t;
+  double relax, tol;
+  int maxiter, model;
+  double d, n, co;
+  double *bound, *uindb, *uindb_conv, *cl_out, *cd_out, *aoa_out;
+  int *iters, *converged, *diverged, *it_max;
+  double *res_last;
+  int vec_smem, mat_smem;
+  long long vec_stride, mat_stride;
+  double *vec_scratch, *mat_scratch;
+};
+long long kj_vec_doubles(int ns, int nb);
+long long kj_mat_doubles(int ns, int nb);
+int kj_cluster();
+cudaError_t launch_kj_solve(const KJSolveArgs &a, int ncases, cudaStream_t s);
+cudaError_t launch_kj_finish(const WakeCase *cases, const KJCase *kc, int ncases, int max_st,
+                             const int *iters, const int *converged, const int *it_max,
+                             const double *uindb_conv, double *uindb, cudaStream_t s);
 cudaError_t launch_kj_features(const WakeCase *cases, const KJCase *kc, int ncases, int max_st,
                                const int *step, const double *bound, const double *bound_last,
                                const double *bound_last2,
@@ -63,17 +86,6 @@ cudaError_t launch_kj_loads(const WakeCase *cases, const KJCase *kc, int ncases,
                             const double *cd, const double *aoa, const double *st_tw,
                             const double *chord, const double *st_rr, const double *st_dr,
                             const double *rpm, const double *pitch, double *dl, double *out,
-                            cudaStream_t s);
-// Clears a graph WHILE condition at a step before WakeCase::kj_from.
-cudaError_t launch_kj_gate_cond(const WakeCase *cases, const int *step,
-                                cudaGraphConditionalHandle h, cudaStream_t s);
-// kj_check that also sets a graph WHILE condition (see kj_kernels.cu).
-cudaError_t launch_kj_check_cond(int ncases, double tol, int *converged, int *iters,
-                                 unsigned long long *res_max, double *res_last, int *active,
-                                 int *it_ctr, int maxiter, cudaGraphConditionalHandle h,
-                                 cudaStream_t s);
-cudaError_t launch_kj_check(int ncases, double tol, int *converged, int *iters,
-                            unsigned long long *res_max, double *res_last, int *active,
                             cudaStream_t s);
 
 }  // namespace winds

@@ -42,7 +42,6 @@ struct winds_wake_batch {
   long long nodes = 0, shed_n = 0, trail_n = 0, bound_n = 0, fil_pad = 0, kin_n = 0, wind_n = 0;
   long long ser_n = 0;
   long long max_nodes = 0, max_cols = 0, max_fil = 0, max_slots = 0;
-  int max_nb = 0;  // most blades of a case
   long long interactions = 0;  // per step of the last winds_wake_step call
   int launches = 0;
   int pcc_from = 0, kj_from = 0;  // first step of the corrector / the iteration (startup)
@@ -69,10 +68,9 @@ struct winds_wake_batch {
   std::vector<KJCase> kjc;
   long long n_ll = 0, frames_n = 0, stations_n = 0;
   int max_st = 0;
-  long long max_bound_cols = 0;  // largest nb (2 ns + nst): the loop's repack
   DevBuf kjc_d, ll, bxn, byn, bzn, vblade, chord, foil, foil_off, aoa_t, cl_t, cd_t;
   DevBuf tp_ll, perm_ll, uindb, kj_groups, kj_tiles, kj_items, kj_order, kj_part;
-  DevBuf conv, iters, res_max, res_last, active, diverged, cl_o, cd_o, aoa_o;
+  DevBuf conv, iters, res_last, diverged, cl_o, cd_o, aoa_o;
   int kj_ntiles = 0, kj_nitems = 0, kj_grid = 0, kj_tile_cap = 0, kj_T = 2, kj_KF = 64;
   long long kj_evals = 0;
   // bound-circulation MLP start value
@@ -84,18 +82,19 @@ struct winds_wake_batch {
   DevBuf st_stall;  // per station: AoA (deg) of its table's lowest and highest Cl
   winds_mlp *mlp = nullptr;
   MlpWork mw;
-  cudaGraphExec_t exec_pre = nullptr, exec_kj = nullptr, exec_post = nullptr;
-  cudaGraph_t g_pre = nullptr, g_kj = nullptr, g_post = nullptr;
-  // whole step with the iteration as a conditional WHILE node (no host round trip)
+  // whole step, lifting-line iteration included
   cudaGraphExec_t exec_step = nullptr;
   cudaGraph_t g_step = nullptr;
-  cudaStream_t body_stream = nullptr;
-  bool cond_ok = true;  // false after a failed build: host loop instead
   int step_launches = 0;
   DevBuf kj_it;         // iterations run in the current step
+  DevBuf uind_fix, uindb_conv, kj_vec, kj_mat;
+  long long kj_vec_stride = 0, kj_mat_stride = 0;
+  bool kj_vec_smem = true, kj_mat_smem = true;
 };
 
 namespace {
+
+constexpr long long kKJMatBytes = 2LL << 30;
 
 template <class T>
 T *P(DevBuf &b) {
@@ -361,80 +360,9 @@ cudaError_t enqueue_step(winds_wake_batch *b, int &launches) {
   return e;
 }
 
-// One Kutta-Joukowski iteration of every active case: Γ from the bound
-// iterate, filaments with the step's cores, induced velocity at the lifting
-// lines, station update and per-case convergence.
-cudaError_t enqueue_kj_iter(winds_wake_batch *b, int &launches, cudaStream_t s,
-                            const cudaGraphConditionalHandle *cond = nullptr) {
-  const WakeCase *cd = P<const WakeCase>(b->cases_d);
-  const KJCase *kd = P<const KJCase>(b->kjc_d);
-  PackedFilaments pf{P<float4>(b->pk),
-                     P<double4>(b->ra), P<double4>(b->rb)};
-  BBox *bb = P<BBox>(b->bbox);
-  // Γ of the bound iterate: columns 0-1 follow it (the others come from the
-  // previous step); only those are recomputed and repacked (enqueue_kj_begin
-  // did every column and every filament with the step's positions and cores)
-  const int *step = P<const int>(b->step_d);
-  cudaError_t e = launch_wake_bookkeep(cd, b->ncases, 2LL * b->max_nb, step, 0,
-                                       P<const double>(b->bound), P<const double>(b->trail_prev),
-                                       P<double>(b->shed_cur), P<double>(b->trail_cur), s, 2);
-  if (e == cudaSuccess)
-    e = launch_wake_filaments_bound_cols(cd, b->ncases, b->max_bound_cols, step,
-                                         P<const double>(b->dom), P<const double>(b->shed_cur),
-                                         P<const double>(b->trail_cur), P<const double>(b->rc_s),
-                                         P<const double>(b->rc_t), b->model, b->dcut, pf, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(b->ctr.p, 0, sizeof(unsigned), s);
-  F32cArgs a;
-  a.pk = pf.pk;
-  a.ra = pf.ra;
-  a.rb = pf.rb;
-  a.tp = P<const double4>(b->tp_ll);
-  a.live = P<const GroupLive>(b->live_kj);
-  a.groups = P<const Group>(b->kj_groups);
-  a.tiles = P<const Tile>(b->kj_tiles);
-  a.items = P<const Item>(b->kj_items);
-  a.order = P<const int>(b->kj_order);
-  a.n_items = b->kj_nitems;
-  a.tile_cap = b->kj_tile_cap;
-  a.part = P<double>(b->kj_part);
-  a.work_ctr = P<unsigned>(b->ctr);
-  a.err = P<unsigned>(b->err);
-  a.near_ctr = P<unsigned long long>(b->nearctr);
-  a.bbox = bb;
-  a.model = b->model;
-  a.d = b->dcut;
-  a.n = b->nidx;
-  a.co = b->prm.co;
-  a.wait_limit_ns = default_wait_limit_ns();
-  if (e == cudaSuccess)
-    e = b->prec == WINDS_PREC_F64 || b->kjp.ll_fp64 ? launch_f64(a, b->kj_grid, s)
-                                  : launch_f32c(a, b->model, b->kj_T, b->kj_KF, b->kj_grid, s);
-  if (e == cudaSuccess)
-    e = launch_reduce(P<const Tile>(b->kj_tiles), b->kj_ntiles, P<const Group>(b->kj_groups),
-                      P<const double>(b->kj_part), P<const int>(b->perm_ll), b->kj_tile_cap, s,
-                      P<const Item>(b->kj_items), P<const GroupLive>(b->live_kj));
-  if (e == cudaSuccess)
-    e = launch_kj_update(cd, kd, b->ncases, b->max_st, P<const int>(b->step_d),
-                         P<const double>(b->uindb), P<const double>(b->bxn), P<const double>(b->byn),
-                         P<const double>(b->bzn), P<const double>(b->vblade),
-                         P<const double>(b->chord), P<const int>(b->foil), P<const int>(b->foil_off),
-                         P<const double>(b->aoa_t), P<const double>(b->cl_t), P<const double>(b->cd_t),
-                         b->kjp.relax, P<double>(b->bound), P<const int>(b->conv),
-                         P<unsigned long long>(b->res_max), P<int>(b->diverged), P<double>(b->cl_o),
-                         P<double>(b->cd_o), P<double>(b->aoa_o), s);
-  if (e == cudaSuccess)
-    e = cond ? launch_kj_check_cond(b->ncases, b->kjp.tol, P<int>(b->conv), P<int>(b->iters),
-                                    P<unsigned long long>(b->res_max), P<double>(b->res_last),
-                                    P<int>(b->active), P<int>(b->kj_it), b->kjp.maxiter, *cond, s)
-             : launch_kj_check(b->ncases, b->kjp.tol, P<int>(b->conv), P<int>(b->iters),
-                               P<unsigned long long>(b->res_max), P<double>(b->res_last),
-                               P<int>(b->active), s);
-  launches = 8;
-  return e;
-}
-
-// Lifting-line targets and the per-step reset of the iteration state.
-cudaError_t enqueue_kj_begin(winds_wake_batch *b) {
+// The lifting line: its targets, features and start value, the induced velocity
+// of the filaments that do not follow the bound iterate, and the iteration.
+cudaError_t enqueue_kj(winds_wake_batch *b, int &launches) {
   cudaStream_t s = b->stream;
   cudaError_t e = launch_bbox_init(P<BBox>(b->bbox), s);
   // the step's live filaments; every lifting-line point is a target
@@ -445,7 +373,7 @@ cudaError_t enqueue_kj_begin(winds_wake_batch *b) {
     e = launch_kj_targets(P<const WakeCase>(b->cases_d), P<const KJCase>(b->kjc_d), b->ncases,
                           b->max_st, P<const int>(b->step_d), P<const double>(b->ll),
                           P<double4>(b->tp_ll), P<BBox>(b->bbox), s);
-  for (DevBuf *x : {&b->conv, &b->iters, &b->diverged, &b->res_max})
+  for (DevBuf *x : {&b->conv, &b->iters, &b->diverged})
     if (e == cudaSuccess) e = cudaMemsetAsync(x->p, 0, b->ncases * 8, s);
   if (e == cudaSuccess) e = cudaMemsetAsync(b->kj_it.p, 0, sizeof(int), s);
   const WakeCase *cd = P<const WakeCase>(b->cases_d);
@@ -484,129 +412,116 @@ cudaError_t enqueue_kj_begin(winds_wake_batch *b) {
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(b->guess.p, b->bound.p, b->bound_n * sizeof(double),
                         cudaMemcpyDeviceToDevice, s);
-  // every filament at the step's positions with the step's cores held fixed
-  // (as kj() does), Γ from the start value; the iterations repack only the
-  // columns that follow the bound iterate
+  // every filament at the step's positions with the step's cores held fixed (as
+  // kj() does); Γ of the columns that do not follow the bound iterate is the
+  // bookkeeping's of this step
+  PackedFilaments pf{P<float4>(b->pk), P<double4>(b->ra), P<double4>(b->rb)};
   if (e == cudaSuccess)
-    e = launch_wake_bookkeep(cd, b->ncases, b->max_cols, P<const int>(b->step_d), 0,
-                             P<const double>(b->bound), P<const double>(b->trail_prev),
-                             P<double>(b->shed_cur), P<double>(b->trail_cur), s);
-  if (e == cudaSuccess) {
-    PackedFilaments pf{P<float4>(b->pk), P<double4>(b->ra), P<double4>(b->rb)};
     e = launch_wake_filaments(cd, b->ncases, b->max_fil, P<const int>(b->step_d), 0,
                               P<const double>(b->ser), P<const double>(b->dom),
-                              P<const double>(b->shed_cur),
-                              P<const double>(b->trail_cur), nullptr, nullptr, 0, 0, nullptr,
-                              nullptr, nullptr, nullptr, P<const double>(b->rc_s),
-                              P<const double>(b->rc_t), b->model, b->dcut, pf, P<BBox>(b->bbox), s);
-  }
+                              P<const double>(b->shed_cur), P<const double>(b->trail_cur), nullptr,
+                              nullptr, 0, 0, nullptr, nullptr, nullptr, nullptr,
+                              P<const double>(b->rc_s), P<const double>(b->rc_t), b->model,
+                              b->dcut, pf, P<BBox>(b->bbox), s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(b->ctr.p, 0, sizeof(unsigned), s);
+  F32cArgs a;
+  a.pk = pf.pk;
+  a.ra = pf.ra;
+  a.rb = pf.rb;
+  a.tp = P<const double4>(b->tp_ll);
+  a.live = P<const GroupLive>(b->live_kj);
+  a.groups = P<const Group>(b->kj_groups);
+  a.tiles = P<const Tile>(b->kj_tiles);
+  a.items = P<const Item>(b->kj_items);
+  a.order = P<const int>(b->kj_order);
+  a.n_items = b->kj_nitems;
+  a.tile_cap = b->kj_tile_cap;
+  a.part = P<double>(b->kj_part);
+  a.work_ctr = P<unsigned>(b->ctr);
+  a.err = P<unsigned>(b->err);
+  a.near_ctr = P<unsigned long long>(b->nearctr);
+  a.bbox = P<BBox>(b->bbox);
+  a.model = b->model;
+  a.d = b->dcut;
+  a.n = b->nidx;
+  a.co = b->prm.co;
+  a.wait_limit_ns = default_wait_limit_ns();
+  if (e == cudaSuccess)
+    e = b->prec == WINDS_PREC_F64 || b->kjp.ll_fp64
+            ? launch_f64(a, b->kj_grid, s)
+            : launch_f32c(a, b->model, b->kj_T, b->kj_KF, b->kj_grid, s);
+  if (e == cudaSuccess)
+    e = launch_reduce(P<const Tile>(b->kj_tiles), b->kj_ntiles, P<const Group>(b->kj_groups),
+                      P<const double>(b->kj_part), P<const int>(b->perm_ll), b->kj_tile_cap, s,
+                      P<const Item>(b->kj_items), P<const GroupLive>(b->live_kj));
+  KJSolveArgs q;
+  std::memset(&q, 0, sizeof(q));
+  q.cases = cd, q.kc = kd, q.step = P<const int>(b->step_d);
+  q.tp = P<const double4>(b->tp_ll);
+  q.dom = P<const double>(b->dom), q.trail_prev = P<const double>(b->trail_prev);
+  q.rc_s = P<const double>(b->rc_s), q.rc_t = P<const double>(b->rc_t);
+  q.u_fix = P<const double>(b->uind_fix);
+  q.bxn = P<const double>(b->bxn), q.byn = P<const double>(b->byn), q.bzn = P<const double>(b->bzn);
+  q.vblade = P<const double>(b->vblade), q.chord = P<const double>(b->chord);
+  q.foil = P<const int>(b->foil), q.foil_off = P<const int>(b->foil_off);
+  q.aoa_t = P<const double>(b->aoa_t), q.cl_t = P<const double>(b->cl_t);
+  q.cd_t = P<const double>(b->cd_t);
+  q.relax = b->kjp.relax, q.tol = b->kjp.tol, q.maxiter = b->kjp.maxiter;
+  q.model = b->model, q.d = b->dcut, q.n = b->nidx, q.co = b->prm.co;
+  q.bound = P<double>(b->bound), q.uindb = P<double>(b->uindb);
+  q.uindb_conv = P<double>(b->uindb_conv);
+  q.cl_out = P<double>(b->cl_o), q.cd_out = P<double>(b->cd_o), q.aoa_out = P<double>(b->aoa_o);
+  q.iters = P<int>(b->iters), q.converged = P<int>(b->conv), q.diverged = P<int>(b->diverged);
+  q.it_max = P<int>(b->kj_it), q.res_last = P<double>(b->res_last);
+  q.vec_smem = b->kj_vec_smem, q.mat_smem = b->kj_mat_smem;
+  q.vec_stride = b->kj_vec_stride, q.mat_stride = b->kj_mat_stride;
+  q.vec_scratch = P<double>(b->kj_vec), q.mat_scratch = P<double>(b->kj_mat);
+  if (e == cudaSuccess) e = launch_kj_solve(q, b->ncases, s);
+  if (e == cudaSuccess)
+    e = launch_kj_finish(cd, kd, b->ncases, b->max_st, q.iters, q.converged, q.it_max,
+                         q.uindb_conv, q.uindb, s);
+  launches += 8 + (b->mlp_inputs ? 1 : 0);
   return e;
 }
 
 int kj_step_errors(winds_wake_batch *b);
 
-// One step as one graph: the part before the iteration, the lifting-line set-up,
-// a conditional WHILE node whose body is one iteration (kj_check_cond ends it),
-// then the commit. Built once, replayed every step.
+// One step as one graph: the part before the iteration, the lifting line, the
+// commit. Built once, replayed every step.
 int build_step_graph(winds_wake_batch *b) {
   cudaStream_t s = b->stream;
-  cudaError_t e = cudaSuccess;
-  if (!b->body_stream) e = cudaStreamCreateWithFlags(&b->body_stream, cudaStreamNonBlocking);
   int l1 = 0, l2 = 0, l3 = 0;
-  cudaGraph_t g = nullptr;
-  bool capturing = false;
-  if (e == cudaSuccess) e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
-  capturing = e == cudaSuccess;
-  if (e == cudaSuccess) e = enqueue_pre(b, l1);
-  if (e == cudaSuccess) e = enqueue_kj_begin(b);
-  cudaGraphConditionalHandle h = 0;
-  cudaGraphNode_t node = nullptr;
-  if (e == cudaSuccess) {
-    cudaStreamCaptureStatus st;
-    const cudaGraphNode_t *deps = nullptr;
-    size_t ndeps = 0;
-    e = cudaStreamGetCaptureInfo(s, &st, nullptr, &g, &deps, &ndeps);
-    if (e == cudaSuccess) e = cudaGraphConditionalHandleCreate(&h, g, 1, cudaGraphCondAssignDefault);
-    // no iteration at a step before the start-up's first (the condition is
-    // reset to 1 at every launch of the graph)
-    if (e == cudaSuccess && b->kj_from > 0) {
-      e = launch_kj_gate_cond(P<const WakeCase>(b->cases_d), P<const int>(b->step_d), h, s);
-      if (e == cudaSuccess) e = cudaStreamGetCaptureInfo(s, &st, nullptr, &g, &deps, &ndeps);
-      ++l1;
-    }
-    // zero-filled storage: the parameter union has no usable default constructor
-    union NodeParams {
-      cudaGraphNodeParams p;
-      unsigned char raw[sizeof(cudaGraphNodeParams)];
-      NodeParams() { std::memset(raw, 0, sizeof(raw)); }
-      ~NodeParams() {}
-    } np;
-    cudaGraphNodeParams &cp = np.p;
-    cp.type = cudaGraphNodeTypeConditional;
-    cp.conditional.handle = h;
-    cp.conditional.type = cudaGraphCondTypeWhile;
-    cp.conditional.size = 1;
-    if (e == cudaSuccess) e = cudaGraphAddNode(&node, g, deps, ndeps, &cp);
-    if (e == cudaSuccess)
-      e = cudaStreamUpdateCaptureDependencies(s, &node, 1, cudaStreamSetCaptureDependencies);
-    if (e == cudaSuccess) {
-      cudaGraph_t body = cp.conditional.phGraph_out[0];
-      e = cudaStreamBeginCaptureToGraph(b->body_stream, body, nullptr, nullptr, 0,
-                                        cudaStreamCaptureModeThreadLocal);
-      if (e == cudaSuccess) {
-        cudaError_t e2 = enqueue_kj_iter(b, l2, b->body_stream, &h);
-        e = cudaStreamEndCapture(b->body_stream, &body);
-        if (e2 != cudaSuccess) e = e2;
-      }
-    }
-  }
+  cudaError_t e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
+  if (e != cudaSuccess) return cuda_fail(e, "step capture");
+  e = enqueue_pre(b, l1);
+  if (e == cudaSuccess) e = enqueue_kj(b, l2);
   if (e == cudaSuccess) e = enqueue_post(b, l3);
-  if (capturing) {
-    cudaGraph_t done = nullptr;
-    cudaError_t e2 = cudaStreamEndCapture(s, &done);
-    if (e == cudaSuccess) e = e2;
-    g = done;
-  }
+  cudaGraph_t g = nullptr;
+  const cudaError_t e2 = cudaStreamEndCapture(s, &g);
+  if (e == cudaSuccess) e = e2;
   if (e == cudaSuccess) e = cudaGraphInstantiate(&b->exec_step, g, 0);
   if (e != cudaSuccess) {
     if (g) cudaGraphDestroy(g);
     b->exec_step = nullptr;
-    b->g_step = nullptr;
     cudaGetLastError();
-    return cuda_fail(e, "step graph with conditional iteration");
+    return cuda_fail(e, "step graph");
   }
   b->g_step = g;
   b->step_launches = l1 + l2 + l3;
   return WINDS_BS_OK;
 }
 
-int run_kj(winds_wake_batch *b, bool use_graph) {
-  if (b->steps_done < b->kj_from) {  // the start-up's first step has no iteration
-    b->kj_evals = 0;
-    return WINDS_BS_OK;
-  }
-  cudaError_t e = enqueue_kj_begin(b);
-  if (e != cudaSuccess) return cuda_fail(e, "kj begin");
-  if (use_graph && !b->exec_kj) {
-    int l = 0;
-    e = cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal);
-    cudaError_t e2 = e == cudaSuccess ? enqueue_kj_iter(b, l, b->stream) : e;
-    e = cudaStreamEndCapture(b->stream, &b->g_kj);
-    if (e2 != cudaSuccess) e = e2;
-    if (e == cudaSuccess) e = cudaGraphInstantiate(&b->exec_kj, b->g_kj, 0);
-    if (e != cudaSuccess) return cuda_fail(e, "kj capture");
-  }
+// The lifting line of one step launched directly; errors before the commit.
+int run_kj(winds_wake_batch *b, int &launches) {
   b->kj_evals = 0;
-  int active = 1;
-  for (int it = 0; it < b->kjp.maxiter && active; ++it) {
-    int l = 0;
-    e = use_graph ? cudaGraphLaunch(b->exec_kj, b->stream) : enqueue_kj_iter(b, l, b->stream);
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(&active, b->active.p, sizeof(int), cudaMemcpyDeviceToHost, b->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
-    if (e != cudaSuccess) return cuda_fail(e, "kj iteration");
-    ++b->kj_evals;
-  }
+  if (b->steps_done < b->kj_from) return WINDS_BS_OK;  // the start-up's first step has none
+  cudaError_t e = enqueue_kj(b, launches);
+  int it = 0;
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(&it, b->kj_it.p, sizeof(int), cudaMemcpyDeviceToHost, b->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
+  if (e != cudaSuccess) return cuda_fail(e, "kj iteration");
+  b->kj_evals = it;
   return kj_step_errors(b);
 }
 
@@ -728,7 +643,6 @@ int winds_wake_create(const winds_wake_case *cases, int ncases, const winds_wake
     wnd += 3LL * h.nsteps;
     b->max_nodes = std::max(b->max_nodes, nn);
     b->max_cols = std::max<long long>(b->max_cols, (long long)h.na * h.nb);
-    b->max_nb = std::max(b->max_nb, h.nb);
     b->max_fil = std::max(b->max_fil, c.fil_pad);
     b->max_slots = std::max(b->max_slots, nn);
     b->min_nsteps = k == 0 ? h.nsteps : std::min<long long>(b->min_nsteps, h.nsteps);
@@ -926,11 +840,12 @@ static int step_impl(winds_wake_batch *b, int nsteps, int use_graph) {
     if (rc) return rc;
   }
   cudaError_t e = cudaSuccess;
-  if (b->kj && use_graph && b->cond_ok) {
+  if (b->kj && use_graph) {
     // the whole step, iteration included, as one graph: one round trip per step
-    if (!b->exec_step && build_step_graph(b) != WINDS_BS_OK) b->cond_ok = false;
-  }
-  if (b->kj && use_graph && b->exec_step) {
+    if (!b->exec_step) {
+      int rc = build_step_graph(b);
+      if (rc) return rc;
+    }
     b->launches = b->step_launches;
     cudaEventRecord(b->ev0, b->stream);
     for (int k = 0; k < nsteps; ++k) {
@@ -952,33 +867,17 @@ static int step_impl(winds_wake_batch *b, int nsteps, int use_graph) {
     return e == cudaSuccess ? WINDS_BS_OK : cuda_fail(e, "wake step sync");
   }
   if (b->kj) {
-    // pre-commit part, the iteration (host loop on a device convergence flag), commit
+    // pre-commit part, the iteration, commit
     for (int k = 0; k < nsteps; ++k) {
-      if (use_graph && !b->exec_pre) {
-        int l1 = 0, l2 = 0;
-        e = cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal);
-        cudaError_t e2 = e == cudaSuccess ? enqueue_pre(b, l1) : e;
-        e = cudaStreamEndCapture(b->stream, &b->g_pre);
-        if (e2 != cudaSuccess) e = e2;
-        if (e == cudaSuccess) e = cudaGraphInstantiate(&b->exec_pre, b->g_pre, 0);
-        if (e == cudaSuccess) e = cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal);
-        e2 = e == cudaSuccess ? enqueue_post(b, l2) : e;
-        if (e == cudaSuccess) e = cudaStreamEndCapture(b->stream, &b->g_post);
-        if (e2 != cudaSuccess) e = e2;
-        if (e == cudaSuccess) e = cudaGraphInstantiate(&b->exec_post, b->g_post, 0);
-        b->launches = l1 + l2;
-        if (e != cudaSuccess) return cuda_fail(e, "wake step capture");
-      }
       if (k == 0) cudaEventRecord(b->ev0, b->stream);
-      int l = 0;
-      e = use_graph ? cudaGraphLaunch(b->exec_pre, b->stream) : enqueue_pre(b, l);
+      int l = 0, l2 = 0;
+      e = enqueue_pre(b, l);
       if (e != cudaSuccess) return cuda_fail(e, "wake step");
-      int rc = run_kj(b, use_graph != 0);
+      int rc = run_kj(b, l);
       if (!rc) rc = device_error_word(b);
       if (rc) return rc;
-      int l2 = 0;
-      e = use_graph ? cudaGraphLaunch(b->exec_post, b->stream) : enqueue_post(b, l2);
-      if (!use_graph) b->launches = l + l2;
+      e = enqueue_post(b, l2);
+      b->launches = l + l2;
       if (e != cudaSuccess) return cuda_fail(e, "wake step commit");
     }
     b->timed_steps = nsteps;
@@ -1074,20 +973,17 @@ int winds_wake_set_kj(winds_wake_batch *b, const winds_kj_case *kj, const winds_
   cudaSetDevice(b->dev);
   cudaStreamSynchronize(b->stream);
   // graphs captured for an earlier attachment describe other buffers
-  for (cudaGraphExec_t *x : {&b->exec_pre, &b->exec_kj, &b->exec_post, &b->exec_step})
-    if (*x) cudaGraphExecDestroy(*x), *x = nullptr;
-  for (cudaGraph_t *x : {&b->g_pre, &b->g_kj, &b->g_post, &b->g_step})
-    if (*x) cudaGraphDestroy(*x), *x = nullptr;
+  if (b->exec_step) cudaGraphExecDestroy(b->exec_step), b->exec_step = nullptr;
+  if (b->g_step) cudaGraphDestroy(b->g_step), b->g_step = nullptr;
   cudaStream_t s = b->stream;
   b->kjp = *prm;
   b->kjc.clear();
-  long long fr = 0, tt = 0, st = 0, tab = 0, az = 0, rp = 0;
+  long long fr = 0, tt = 0, st = 0, tab = 0, az = 0, rp = 0, vecs = 0, mats = 0;
   bool all_inputs = true, have_twist = true, all_loads = true, any_pitch = false;
   std::vector<int> foil_off, foils, lift;
   std::vector<double2> stall;
   std::vector<double> aoa, cl, cd, chord;
   b->max_st = 0;
-  b->max_bound_cols = 0;
   for (int k = 0; k < b->ncases; ++k) {
     const WakeCase &c = b->cases[k];
     const winds_kj_case &h = kj[k];
@@ -1152,11 +1048,23 @@ int winds_wake_set_kj(winds_wake_batch *b, const winds_kj_case *kj, const winds_
     tt += (long long)ns * c.nb;
     st += ns;
     b->max_st = std::max(b->max_st, ns * c.nb);
-    b->max_bound_cols = std::max<long long>(b->max_bound_cols, (long long)c.nb * (2 * ns + c.nst));
+    vecs = std::max(vecs, kj_vec_doubles(ns, c.nb));
+    mats = std::max(mats, kj_mat_doubles(ns, c.nb));
     b->kjc.push_back(q);
   }
   b->frames_n = fr, b->n_ll = tt, b->stations_n = st;
   int rc;
+  // kj_solve's vectors and matrix rows: shared memory where the largest case's
+  // fit, else a scratch; a matrix beyond kKJMatBytes is formed term by term
+  const long long ctas = (long long)b->ncases * kj_cluster();
+  b->kj_vec_stride = vecs, b->kj_mat_stride = mats;
+  b->kj_vec_smem = vecs * 8 <= kKJSmemBytes;
+  b->kj_mat_smem = b->kj_vec_smem && (vecs + mats) * 8 <= kKJSmemBytes;
+  if (!b->kj_vec_smem && (rc = b->kj_vec.ensure(ctas * vecs * 8, s))) return rc;
+  if (b->kj_mat_smem || ctas * mats * 8 > kKJMatBytes)
+    b->kj_mat.release();
+  else if ((rc = b->kj_mat.ensure(ctas * mats * 8, s)))
+    return rc;
   for (DevBuf *x : {&b->ll, &b->bxn, &b->byn, &b->bzn, &b->vblade})
     if ((rc = x->ensure(fr * sizeof(double), s))) return rc;
   if ((rc = b->kjc_d.ensure(b->ncases * sizeof(KJCase), s)) ||
@@ -1166,15 +1074,17 @@ int winds_wake_set_kj(winds_wake_batch *b, const winds_kj_case *kj, const winds_
       (rc = b->foil_off.ensure(foil_off.size() * sizeof(int), s)) ||
       (rc = b->aoa_t.ensure(tab * sizeof(double), s)) || (rc = b->cl_t.ensure(tab * sizeof(double), s)) ||
       (rc = b->cd_t.ensure(tab * sizeof(double), s)) || (rc = b->tp_ll.ensure(tt * sizeof(double4), s)) ||
-      (rc = b->perm_ll.ensure(tt * sizeof(int), s)) || (rc = b->uindb.ensure(tt * 3 * sizeof(double), s)))
+      (rc = b->perm_ll.ensure(tt * sizeof(int), s)) || (rc = b->uindb.ensure(tt * 3 * sizeof(double), s)) ||
+      (rc = b->uind_fix.ensure(tt * 3 * sizeof(double), s)) ||
+      (rc = b->uindb_conv.ensure(tt * 3 * sizeof(double), s)))
     return rc;
-  for (DevBuf *x : {&b->conv, &b->iters, &b->diverged, &b->res_max, &b->res_last, &b->active})
+  for (DevBuf *x : {&b->conv, &b->iters, &b->diverged, &b->res_last})
     if ((rc = x->ensure(std::max(b->ncases, 1) * 8 + 8, s))) return rc;
   if ((rc = b->kj_it.ensure(16, s))) return rc;
   for (DevBuf *x : {&b->cl_o, &b->cd_o, &b->aoa_o, &b->guess, &b->bound_last, &b->bound_last2})
     if ((rc = x->ensure(b->bound_n * sizeof(double), s))) return rc;
   // defined values before any iteration (a step without one reads them)
-  for (DevBuf *x : {&b->conv, &b->iters, &b->diverged, &b->res_max, &b->res_last, &b->active})
+  for (DevBuf *x : {&b->conv, &b->iters, &b->diverged, &b->res_last})
     if (cudaError_t e0 = cudaMemset(x->p, 0, std::max(b->ncases, 1) * 8 + 8); e0 != cudaSuccess)
       return cuda_fail(e0, "lifting-line counters");
   for (DevBuf *x : {&b->cl_o, &b->cd_o, &b->aoa_o})
@@ -1272,7 +1182,7 @@ int winds_wake_set_kj(winds_wake_batch *b, const winds_kj_case *kj, const winds_
   for (int k = 0; k < b->ncases; ++k) {
     const WakeCase &c = b->cases[k];
     GroupSpec g;
-    g.out = P<double>(b->uindb) + 3 * b->kjc[k].t_off;
+    g.out = P<double>(b->uind_fix) + 3 * b->kjc[k].t_off;
     g.t_begin = b->kjc[k].t_off;
     g.t_count = (long long)(c.nst - 1) * c.nb;
     g.ns_p = c.nst - 1;
@@ -1412,11 +1322,9 @@ void winds_wake_destroy(winds_wake_batch *b) {
   if (b->stream) cudaStreamSynchronize(b->stream);
   if (b->exec) cudaGraphExecDestroy(b->exec);
   if (b->graph) cudaGraphDestroy(b->graph);
-  for (cudaGraphExec_t x : {b->exec_pre, b->exec_kj, b->exec_post, b->exec_step})
-    if (x) cudaGraphExecDestroy(x);
-  for (cudaGraph_t x : {b->g_pre, b->g_kj, b->g_post, b->g_step})
-    if (x) cudaGraphDestroy(x);
-  if (b->body_stream) cudaStreamDestroy(b->body_stream);
+  if (b->exec_step) cudaGraphExecDestroy(b->exec_step);
+  if (b->g_step) cudaGraphDestroy(b->g_step);
+  for (DevBuf *x : {&b->uind_fix, &b->uindb_conv, &b->kj_vec, &b->kj_mat}) x->release();
   b->kj_it.release();
   b->st_lift.release();
   b->st_stall.release();
@@ -1424,7 +1332,7 @@ void winds_wake_destroy(winds_wake_batch *b) {
                     &b->foil_off, &b->aoa_t, &b->cl_t, &b->cd_t, &b->tp_ll, &b->perm_ll, &b->uindb,
                     &b->kj_groups, &b->kj_tiles, &b->kj_items, &b->kj_order, &b->kj_part,
                     &b->conv, &b->iters,
-                    &b->res_max, &b->res_last, &b->active, &b->diverged, &b->cl_o, &b->cd_o,
+                    &b->res_last, &b->diverged, &b->cl_o, &b->cd_o,
                     &b->aoa_o, &b->st_r, &b->st_c, &b->st_tw, &b->azim, &b->guess, &b->feat,
                     &b->bound_last, &b->bound_last2, &b->st_rr, &b->st_dr, &b->rpm, &b->pitch, &b->dl,
                     &b->loads_out})

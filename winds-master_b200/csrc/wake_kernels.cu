@@ -83,17 +83,14 @@ __device__ __forceinline__ double trail_col(const WakeCase &c, const double *bou
 // The step's live columns na_l = live_cols(c, *step + step_add): trailing
 // columns 1..na_l-2 come from the previous step's columns 0..na_l-3 (all of
 // them while the wake grows; at capacity the oldest is dropped).
-// cols > 0: only columns j < cols (the Kutta-Joukowski loop's bound-dependent
-// columns); the same arithmetic per column as the full pass.
 __global__ void wake_bookkeep(const WakeCase *cases, const int *step, int step_add,
                               const double *bound, const double *trail_prev, double *shed,
-                              double *trail, int cols) {
+                              double *trail) {
   const WakeCase c = cases[blockIdx.y];
   const int u = blockIdx.x * blockDim.x + threadIdx.x;  // (column j, blade b)
   const int na_l = live_cols(c, *step + step_add);
-  const int nc = cols > 0 && cols < na_l ? cols : na_l;
-  if (u >= nc * c.nb) return;
-  const int j = u % nc, b = u / nc;
+  if (u >= na_l * c.nb) return;
+  const int j = u % na_l, b = u / na_l;
   const int ns = c.nst - 1, m = na_l - 1;  // m live trailing columns
   if (j < m) {
 #pragma unroll 8
@@ -183,6 +180,8 @@ __global__ void wake_filaments(const WakeCase *cases, const int *step, int step_
     double rc;
     if (rc_in) {  // cores held fixed (the Kutta-Joukowski loop keeps the step's vcore)
       rc = rc_in[slot];
+      // the filaments that follow the bound iterate are kj_solve's
+      if (j < (f < nsh ? 2 : 1)) g = 0.0;
     } else {
       const double dx = x2 - x1, dy = y2 - y1, dz = z2 - z1;
       const double L = sqrt(dx * dx + dy * dy + dz * dz);  // |L| (FilamentLength.m:43)
@@ -204,57 +203,6 @@ __global__ void wake_filaments(const WakeCase *cases, const int *step, int step_
     pack_inert(c.fil_off + f, pf.pk, pf.ra, pf.rb);
   }
   bbox_accumulate(lo, hi, bb->fmin, bb->fmax);
-}
-
-// Repacks only the filaments whose circulation follows the bound iterate of
-// the Kutta-Joukowski loop -- shed columns 0 and 1 and trailing column 0 (the
-// bookkeeping's other columns come from the previous step) -- with the step's
-// positions and held cores; the other records stay as the full pack before
-// the loop wrote them. Same arithmetic and packed numbering (over the step's
-// live columns) as wake_filaments, so the records are identical to a full
-// repack. Needs at least two live columns (every step has them).
-__global__ void wake_filaments_bound_cols(const WakeCase *cases, const int *step,
-                                          const double *dom, const double *shed,
-                                          const double *trail, const double *rc_in_s,
-                                          const double *rc_in_t, int model, double dcut,
-                                          PackedFilaments pf) {
-  const WakeCase c = cases[blockIdx.y];
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const int ns = c.nst - 1;
-  const int n_shed = c.nb * 2 * ns;
-  if (t >= n_shed + c.nb * c.nst) return;
-  const int na_l = live_cols(c, *step);
-  int i, j, b;
-  double x1, y1, z1, x2, y2, z2, g, rc;
-  long long f;
-  if (t < n_shed) {  // shed column j in {0, 1}: dom(i) -> dom(i+1)
-    b = t / (2 * ns);
-    const int r = t - b * 2 * ns;
-    j = r / ns;
-    i = r - j * ns;
-    f = i + (long long)ns * (j + (long long)na_l * b);
-    const long long slot = c.shed_off + i + (long long)ns * (j + (long long)c.na * b);
-    x1 = node_comp(dom, c, i, 0, j, b), y1 = node_comp(dom, c, i, 1, j, b);
-    z1 = node_comp(dom, c, i, 2, j, b);
-    x2 = node_comp(dom, c, i + 1, 0, j, b), y2 = node_comp(dom, c, i + 1, 1, j, b);
-    z2 = node_comp(dom, c, i + 1, 2, j, b);
-    g = shed[slot];
-    rc = rc_in_s[slot];
-  } else {  // trailing column 0: dom(:, 1) -> dom(:, 0)
-    const int u = t - n_shed;
-    b = u / c.nst;
-    i = u - b * c.nst;
-    const long long slot = c.trail_off + i + (long long)c.nst * ((long long)(c.na - 1) * b);
-    f = (long long)ns * na_l * c.nb + (na_l - 1) * ((long long)i + (long long)c.nst * b);
-    x1 = node_comp(dom, c, i, 0, 1, b), y1 = node_comp(dom, c, i, 1, 1, b);
-    z1 = node_comp(dom, c, i, 2, 1, b);
-    x2 = node_comp(dom, c, i, 0, 0, b), y2 = node_comp(dom, c, i, 1, 0, b);
-    z2 = node_comp(dom, c, i, 2, 0, b);
-    g = trail[slot];
-    rc = rc_in_t[slot];
-  }
-  pack_filament(c.fil_off + f, x1, y1, z1, x2, y2, z2, g, rc, t < n_shed,
-                t < n_shed ? i == 0 : true, model, dcut, pf.pk, pf.ra, pf.rb);
 }
 
 // One thread per node slot of the case: nodes of the live columns of step
@@ -425,20 +373,9 @@ static dim3 case_grid(long long max_per_case, int ncases, int bs) {
 cudaError_t launch_wake_bookkeep(const WakeCase *cases, int ncases, long long max_cols,
                                  const int *step, int step_add, const double *bound,
                                  const double *trail_prev, double *shed, double *trail,
-                                 cudaStream_t s, int cols) {
+                                 cudaStream_t s) {
   wake_bookkeep<<<case_grid(max_cols, ncases, 128), 128, 0, s>>>(cases, step, step_add, bound,
-                                                                  trail_prev, shed, trail, cols);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_wake_filaments_bound_cols(const WakeCase *cases, int ncases, long long per_case,
-                                             const int *step, const double *dom,
-                                             const double *shed, const double *trail,
-                                             const double *rc_in_s, const double *rc_in_t,
-                                             int model, double dcut, const PackedFilaments &pf,
-                                             cudaStream_t s) {
-  wake_filaments_bound_cols<<<case_grid(per_case, ncases, 128), 128, 0, s>>>(
-      cases, step, dom, shed, trail, rc_in_s, rc_in_t, model, dcut, pf);
+                                                                  trail_prev, shed, trail);
   return cudaGetLastError();
 }
 

@@ -24,20 +24,13 @@ enum WakeLiveMode : int {
 
 // Kernels that depend on the wake's live columns read the step counter
 // (*step, plus step_add for the pcc prediction of the next step).
-// cols > 0: columns j < cols only (max_cols then nb * cols at most).
 cudaError_t launch_wake_bookkeep(const WakeCase *cases, int ncases, long long max_cols,
                                  const int *step, int step_add, const double *bound,
                                  const double *trail_prev, double *shed, double *trail,
-                                 cudaStream_t s, int cols = 0);
-// The Kutta-Joukowski loop's repack: shed columns 0-1 and trailing column 0
-// only; per_case is the largest nb * (2 (nst - 1) + nst) of the batch.
-cudaError_t launch_wake_filaments_bound_cols(const WakeCase *cases, int ncases, long long per_case,
-                                             const int *step, const double *dom,
-                                             const double *shed, const double *trail,
-                                             const double *rc_in_s, const double *rc_in_t,
-                                             int model, double dcut, const PackedFilaments &pf,
-                                             cudaStream_t s);
-// ser: per-step time and initial core radius (WakeCase::ser_off).
+                                 cudaStream_t s);
+// ser: per-step time and initial core radius (WakeCase::ser_off). With rc_in (the
+// lifting line's evaluation, cores held) shed columns 0-1 and trailing column 0
+// get no circulation: they are kj_solve's.
 cudaError_t launch_wake_filaments(const WakeCase *cases, int ncases, long long max_fil_pad,
                                   const int *step, int step_add, const double *ser,
                                   const double *dom, const double *shed, const double *trail,
