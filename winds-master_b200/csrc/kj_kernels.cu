@@ -41,18 +41,18 @@ __global__ void kj_targets(const WakeCase *cases, const KJCase *kc, const int *s
 // MATLAB interp1(x, y, xi) of two tables: linear, NaN outside [x(1), x(end)].
 __device__ void interp1(const double *x, const double *y, const double *z, int n, double xi,
                         double &yi, double &zi) {
-  if (!(xi >= x[0] && xi <= x[n - 1])) {
+  if (!(xi >= __ldg(x) && xi <= __ldg(x + n - 1))) {
     yi = zi = NAN;
     return;
   }
   int lo = 0, hi = n - 1;
   while (hi - lo > 1) {
     const int mid = (lo + hi) >> 1;
-    if (x[mid] <= xi) lo = mid; else hi = mid;
+    if (__ldg(x + mid) <= xi) lo = mid; else hi = mid;
   }
-  const double t = (xi - x[lo]) / (x[hi] - x[lo]);
-  yi = y[lo] + t * (y[hi] - y[lo]);
-  zi = z[lo] + t * (z[hi] - z[lo]);
+  const double t = (xi - __ldg(x + lo)) / (__ldg(x + hi) - __ldg(x + lo));
+  yi = __ldg(y + lo) + t * (__ldg(y + hi) - __ldg(y + lo));
+  zi = __ldg(z + lo) + t * (__ldg(z + hi) - __ldg(z + lo));
 }
 
 // ---------------------------------------------------------------- kj_solve
@@ -71,10 +71,12 @@ __device__ void interp1(const double *x, const double *y, const double *z, int n
 // (16 points x 363 filaments x 24 B on 41 nodes; beyond the limit the rows go to
 // the global scratch, and with no scratch each term is formed again in each
 // iteration), and every iteration a warp per point sums its row, updates its
-// station and sends the new circulation to all CTAs of the cluster. One cluster
-// barrier per iteration; each CTA then forms all own circulations by itself.
-// Latency bounds it: the barrier, the span sums and the station update are
-// chains. Every loop ends after maxiter iterations.
+// station and sends the new circulation to all CTAs of the cluster, each of which
+// then forms all own circulations by itself. The values travel as asynchronous
+// stores that complete on an mbarrier of the receiver: with a cluster barrier
+// instead, 4300 of an iteration's 10000 cycles went into it. Latency bounds the
+// rest: the span sums, the row sums and the station update are chains. Every
+// loop ends after maxiter iterations, every wait within the time limit.
 namespace cg = cooperative_groups;
 constexpr int kCluster = 8;
 constexpr int kSolveThreads = 512;
@@ -113,44 +115,74 @@ __device__ __forceinline__ OwnFilament own_filament(const WakeCase &c, const dou
   return o;
 }
 
-// Station (i, b) of the case with induced velocity u: writes cl, cd, aoa and
-// returns the updated circulation; the residual's bits in *res (0, and the
-// circulation unchanged, where Cl is NaN).
-__device__ double station_update(const KJSolveArgs &a, const WakeCase &c, const KJCase &k, int ci,
-                                 int s, int i, int b, const double u[3], double bound,
-                                 unsigned long long *res) {
-  const int ns = c.nst - 1;
+// What a station's update reads besides the velocity, gathered once per step:
+// the frame (9), vblade (3), |vblade| chord / 2 and the fixed velocity (3); and
+// what its last update gave: the velocity (3), cl, cd and aoa, kept here until
+// the end (a store to global memory would hold up every cluster barrier).
+constexpr int kStation = 22;
+__device__ __forceinline__ void load_station(const KJSolveArgs &a, const WakeCase &c,
+                                             const KJCase &k, int s, int t, double *st) {
+  const int ns = c.nst - 1, b = t / ns, i = t - b * ns;
   const long long fo = k.frame_off + i + (long long)ns * (3 * (s + (long long)c.nsteps * b));
-  double rot[3];
   const double *fr[3] = {a.bxn, a.byn, a.bzn};
+  const double *fix = a.u_fix + 3 * k.t_off + i + (long long)ns * 3 * b;
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+#pragma unroll
+    for (int r = 0; r < 3; ++r) st[3 * q + r] = fr[q][fo + r * ns];
+    st[9 + q] = a.vblade[fo + q * ns];
+    st[13 + q] = fix[q * ns];
+  }
+  st[12] = 0.5 * sqrt(st[9] * st[9] + st[10] * st[10] + st[11] * st[11]) *
+           a.chord[k.station_off + i];
+}
+
+// A station's update with induced velocity u; returns the updated circulation,
+// the residual's bits in *res (0, and the circulation unchanged, where Cl is
+// NaN).
+__device__ __forceinline__ double station_update(const KJSolveArgs &a, double *st, int ci, int o0,
+                                                 int o1, const double u[3], double bound,
+                                                 unsigned long long *res) {
+  double rot[3];
 #pragma unroll
   for (int q = 0; q < 3; ++q)
-    rot[q] = fr[q][fo] * u[0] + fr[q][fo + ns] * u[1] + fr[q][fo + 2 * ns] * u[2];
-  const double vb0 = a.vblade[fo], vb1 = a.vblade[fo + ns], vb2 = a.vblade[fo + 2 * ns];
-  const double tu = vb0 + rot[0], tv = vb1 + rot[1];
-  const double Vinf = sqrt(vb0 * vb0 + vb1 * vb1 + vb2 * vb2);
+    rot[q] = st[3 * q] * u[0] + st[3 * q + 1] * u[1] + st[3 * q + 2] * u[2];
+  const double tu = st[9] + rot[0], tv = st[10] + rot[1];
   const double aoa = atan2(-tv, tu) * (180.0 / kPi);
-  const int f = a.foil[k.station_off + i];
-  const int o0 = a.foil_off[k.foil_base + f], o1 = a.foil_off[k.foil_base + f + 1];
   double cl, cd;
   interp1(a.aoa_t + o0, a.cl_t + o0, a.cd_t + o0, o1 - o0, aoa, cl, cd);
-  const long long q = c.bound_off + i + (long long)ns * b;  // station slot of the case
-  a.cl_out[q] = cl;
-  a.cd_out[q] = cd;
-  a.aoa_out[q] = aoa;
+  st[16] = u[0], st[17] = u[1], st[18] = u[2];
+  st[19] = cl, st[20] = cd, st[21] = aoa;
   *res = 0ull;
   if (isnan(cl)) {
     atomicOr(&a.diverged[ci], 1);
     return bound;
   }
-  const double gamma = 0.5 * Vinf * a.chord[k.station_off + i] * cl;
+  const double gamma = st[12] * cl;
   const double dg = gamma - bound;
   *res = (unsigned long long)__double_as_longlong(fabs(dg / (fabs(gamma) + 1.0)));
   return bound + a.relax * dg;
 }
 
+// Address in CTA `rank` of the cluster of the shared-memory address p is here.
+__device__ __forceinline__ uint32_t cluster_address(const void *p, int rank) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(p)), "r"(rank));
+  return r;
+}
+// (g, r) to 16 bytes of another CTA's shared memory, completing on its mbarrier.
+__device__ __forceinline__ void send_pair(uint32_t dst, uint32_t bar, double g,
+                                          unsigned long long r) {
+  asm volatile(
+      "st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.b64 [%0], {%1, %2}, [%3];" ::"r"(
+          dst),
+      "l"((unsigned long long)__double_as_longlong(g)), "l"(r), "r"(bar)
+      : "memory");
+}
+
 __global__ void __launch_bounds__(kSolveThreads) kj_solve(const KJSolveArgs a) {
   extern __shared__ __align__(16) double kj_smem[];
+  __shared__ uint64_t arrived[2];
   cg::cluster_group cl = cg::this_cluster();
   const int ci = blockIdx.x / kCluster, rank = blockIdx.x % kCluster;
   const WakeCase c = a.cases[ci];
@@ -163,13 +195,11 @@ __global__ void __launch_bounds__(kSolveThreads) kj_solve(const KJSolveArgs a) {
   const int cnt = max(0, min(per, nt - t0));
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // shared or (vectors too long for it) global working vectors: the bound
-  // iterate and the residuals of all points, twice; the own circulations; the
-  // part of shed column 1 that stays
+  // iterate and the residual (its bits) of every point, twice; the own circulations; the
+  // part of shed column 1 that stays; this CTA's stations (load_station)
   double *vec = a.vec_smem ? kj_smem : a.vec_scratch + ((long long)ci * kCluster + rank) * a.vec_stride;
-  double *sB[2] = {vec, vec + nt};
-  unsigned long long *sR[2] = {reinterpret_cast<unsigned long long *>(vec + 2 * nt),
-                               reinterpret_cast<unsigned long long *>(vec + 3 * nt)};
-  double *sG = vec + 4 * nt, *sC = sG + own;
+  double2 *sB[2] = {reinterpret_cast<double2 *>(vec), reinterpret_cast<double2 *>(vec + 2 * nt)};
+  double *sG = vec + 4 * nt, *sC = sG + own, *sS = sC + nt;
   double *mat = a.mat_smem      ? kj_smem + (a.vec_smem ? a.vec_stride : 0)
                 : a.mat_scratch ? a.mat_scratch + ((long long)ci * kCluster + rank) * a.mat_stride
                                 : nullptr;
@@ -192,7 +222,14 @@ __global__ void __launch_bounds__(kSolveThreads) kj_solve(const KJSolveArgs a) {
 #pragma unroll
       for (int q = 0; q < 3; ++q) mat[(long long)(3 * tt + q) * own + f] = u[q];
     }
-  for (int t = tid; t < nt; t += kSolveThreads) sB[0][t] = a.bound[c.bound_off + t];
+  for (int t = tid; t < nt; t += kSolveThreads) sB[0][t].x = a.bound[c.bound_off + t];
+  if (tid == 0) {
+    mbar_init(&arrived[0], 1);
+    mbar_init(&arrived[1], 1);
+    fence_mbar_init();
+  }
+  for (int tt = tid; tt < cnt; tt += kSolveThreads)
+    load_station(a, c, k, s, t0 + tt, sS + kStation * tt);
   // shed(:, 1) = C_1 - C_0 (WInDS.m:139-140): C_1, of the previous step's
   // trailing column 0, stays; summed as wake_bookkeep does
   const int m = live_cols(c, s) - 1;
@@ -207,22 +244,34 @@ __global__ void __launch_bounds__(kSolveThreads) kj_solve(const KJSolveArgs a) {
   cl.sync();
   // the own circulations of iterate B; a non-finite one adds nothing, as its
   // terms are zeroed in the direct sum (BiotSavart.m:111)
-  const auto circulation = [&](const double *B) {
+  const auto circulation = [&](const double2 *B) {
     const auto put = [&](int f, double g) { sG[f] = isfinite(g) ? g : 0.0; };
     for (int t = tid; t < c.nb * c.nst; t += kSolveThreads) {
       const int b = t / c.nst, i = t - b * c.nst;
-      const double hi = i < ns ? B[i + ns * b] : 0.0, lo = i > 0 ? B[i - 1 + ns * b] : 0.0;
+      const double hi = i < ns ? B[i + ns * b].x : 0.0, lo = i > 0 ? B[i - 1 + ns * b].x : 0.0;
       put(n_shed + t, hi - lo);
       if (i < ns) put(2 * ns * b + i, hi);
     }
     if (lane == 0)  // one warp per blade: the span sums are chains
       for (int b = warp; b < c.nb; b += kSolveWarps) {
         double cum = 0.0, lo = 0.0;
-        for (int i = 0; i < ns; ++i) {
-          const double hi = B[i + ns * b];
-          cum += hi - lo;
-          lo = hi;
-          put(2 * ns * b + ns + i, sC[i + ns * b] - cum);
+        for (int i0 = 0; i0 < ns; i0 += 8) {
+          double h[8], g[8];
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {
+            const int i = min(i0 + q, ns - 1) + ns * b;
+            h[q] = B[i].x;
+            g[q] = sC[i];
+          }
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {
+            cum += h[q] - lo;
+            lo = h[q];
+            g[q] -= cum;
+          }
+#pragma unroll
+          for (int q = 0; q < 8; ++q)
+            if (i0 + q < ns) put(2 * ns * b + ns + i0 + q, g[q]);
         }
       }
     __syncthreads();
@@ -232,6 +281,7 @@ __global__ void __launch_bounds__(kSolveThreads) kj_solve(const KJSolveArgs a) {
     double v[3] = {0.0, 0.0, 0.0};
     if (mat) {
       const double *r = mat + (long long)3 * tt * own;
+#pragma unroll 4
       for (int f = lane; f < own; f += 32) {
         const double g = sG[f];
         v[0] = fma(r[f], g, v[0]);
@@ -247,20 +297,19 @@ __global__ void __launch_bounds__(kSolveThreads) kj_solve(const KJSolveArgs a) {
         for (int q = 0; q < 3; ++q) v[q] = fma(w[q], g, v[q]);
       }
     }
-    const int t = t0 + tt, b = t / ns, i = t - b * ns;
-    const double *fix = a.u_fix + 3 * k.t_off + i + (long long)ns * 3 * b;
 #pragma unroll
-    for (int q = 0; q < 3; ++q) {
+    for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_xor_sync(0xffffffffu, v[q], o);
-      u[q] = fix[q * ns] + v[q];
-    }
+      for (int q = 0; q < 3; ++q) v[q] += __shfl_xor_sync(0xffffffffu, v[q], o);
+#pragma unroll
+    for (int q = 0; q < 3; ++q) u[q] = sS[kStation * tt + 13 + q] + v[q];
   };
   int it = 0;
   bool done = false;
   double res = 0.0;
   while (it < a.maxiter && !done) {
     const int cur = it & 1, nxt = cur ^ 1;
+    if (a.vec_smem && tid == 0) mbar_arrive_expect_tx(&arrived[nxt], 16u * (unsigned)nt);
     circulation(sB[cur]);
     for (int tt = warp; tt < cnt; tt += kSolveWarps) {
       double u[3];
@@ -269,34 +318,49 @@ __global__ void __launch_bounds__(kSolveThreads) kj_solve(const KJSolveArgs a) {
       double g = 0.0;
       unsigned long long r = 0ull;
       if (lane == 0) {
-        g = station_update(a, c, k, ci, s, i, b, u, sB[cur][t], &r);
-        double *o = a.uindb + 3 * k.t_off + i + (long long)ns * 3 * b;  // [ns,3,nb] of this case
-#pragma unroll
-        for (int q = 0; q < 3; ++q) o[q * ns] = u[q];
+        const int fo = k.foil_base + __ldg(a.foil + k.station_off + i);
+        g = station_update(a, sS + kStation * tt, ci, __ldg(a.foil_off + fo),
+                           __ldg(a.foil_off + fo + 1), u, sB[cur][t].x, &r);
       }
       g = __shfl_sync(0xffffffffu, g, 0);
       r = __shfl_sync(0xffffffffu, r, 0);
       if (lane < kCluster) {
-        if (a.vec_smem) {
-          *cl.map_shared_rank(sB[nxt] + t, lane) = g;
-          *cl.map_shared_rank(sR[nxt] + t, lane) = r;
-        } else {
-          const long long o = ((long long)lane - rank) * a.vec_stride;
-          sB[nxt][o + t] = g;
-          sR[nxt][o + t] = r;
-        }
+        // a buffer is written again only after every CTA sent what it formed
+        // from it, two iterations on
+        if (a.vec_smem)
+          send_pair(cluster_address(sB[nxt] + t, lane), cluster_address(&arrived[nxt], lane), g, r);
+        else
+          reinterpret_cast<double2 *>(reinterpret_cast<double *>(sB[nxt]) +
+                                      ((long long)lane - rank) * a.vec_stride)[t] =
+              make_double2(g, __longlong_as_double((long long)r));
       }
     }
-    cl.sync();
+    if (a.vec_smem) {
+      // iteration it fills buffer nxt for the (it / 2)-th time
+      const bool ok = mbar_wait_bounded(&arrived[nxt], (unsigned)(it >> 1) & 1u, a.err, a.wait_limit_ns);
+      if (!__syncthreads_and(ok)) break;
+    } else {
+      cl.sync();
+    }
     unsigned long long r = 0ull;  // largest residual: the bits of non-negative doubles order them
-    for (int t = lane; t < nt; t += 32) r = max(r, sR[nxt][t]);
+    for (int t = lane; t < nt; t += 32) r = max(r, (unsigned long long)__double_as_longlong(sB[nxt][t].y));
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) r = max(r, __shfl_xor_sync(0xffffffffu, r, o));
     res = __longlong_as_double((long long)r);
     done = res <= a.tol;
     ++it;
   }
-  for (int t = t0 + tid; t < t0 + cnt; t += kSolveThreads) a.bound[c.bound_off + t] = sB[it & 1][t];
+  for (int tt = tid; tt < cnt; tt += kSolveThreads) {
+    const int t = t0 + tt, b = t / ns, i = t - b * ns;
+    const double *st = sS + kStation * tt;
+    double *o = a.uindb + 3 * k.t_off + i + (long long)ns * 3 * b;  // [ns,3,nb] of this case
+#pragma unroll
+    for (int q = 0; q < 3; ++q) o[q * ns] = st[16 + q];
+    a.cl_out[c.bound_off + t] = st[19];
+    a.cd_out[c.bound_off + t] = st[20];
+    a.aoa_out[c.bound_off + t] = st[21];
+    a.bound[c.bound_off + t] = sB[it & 1][t].x;
+  }
   if (done) {
     // the velocities of the converged circulation, for kj_finish
     circulation(sB[it & 1]);
@@ -477,7 +541,9 @@ cudaError_t launch_kj_targets(const WakeCase *cases, const KJCase *kc, int ncase
 // Doubles of a CTA's working vectors and matrix rows for a case of ns stations
 // and nb blades.
 long long kj_vec_doubles(int ns, int nb) {
-  return 4LL * ns * nb + (long long)nb * (3 * ns + 1) + (long long)ns * nb;
+  const long long n = 5LL * ns * nb + (long long)nb * (3 * ns + 1) +
+                      (long long)kStation * ((ns * nb + kCluster - 1) / kCluster);
+  return (n + 1) / 2 * 2;  // 16-byte strides
 }
 long long kj_mat_doubles(int ns, int nb) {
   return (long long)(ns * nb + kCluster - 1) / kCluster * 3 * nb * (3 * ns + 1);

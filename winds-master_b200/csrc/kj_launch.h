@@ -54,6 +54,8 @@ struct KJSolveArgs {
   int vec_smem, mat_smem;
   long long vec_stride, mat_stride;
   double *vec_scratch, *mat_scratch;
+  unsigned *err;
+  unsigned long long wait_limit_ns;
 };
 long long kj_vec_doubles(int ns, int nb);
 long long kj_mat_doubles(int ns, int nb);

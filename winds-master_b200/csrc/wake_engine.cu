@@ -476,6 +476,7 @@ cudaError_t enqueue_kj(winds_wake_batch *b, int &launches) {
   q.vec_smem = b->kj_vec_smem, q.mat_smem = b->kj_mat_smem;
   q.vec_stride = b->kj_vec_stride, q.mat_stride = b->kj_mat_stride;
   q.vec_scratch = P<double>(b->kj_vec), q.mat_scratch = P<double>(b->kj_mat);
+  q.err = P<unsigned>(b->err), q.wait_limit_ns = default_wait_limit_ns();
   if (e == cudaSuccess) e = launch_kj_solve(q, b->ncases, s);
   if (e == cudaSuccess)
     e = launch_kj_finish(cd, kd, b->ncases, b->max_st, q.iters, q.converged, q.it_max,
