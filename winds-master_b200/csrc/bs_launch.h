@@ -12,8 +12,8 @@ struct PackedFilaments {
   double4 *ra, *rb;
 };
 
-// Filament ranges of work items are multiples of this (a multiple of every
-// FP32 tile size and of the FP64 stage).
+// Filament ranges of groups are multiples of this (a multiple of every FP32 tile
+// size and of the FP64 stage).
 constexpr int kFilamentPad = 128;
 
 bool f32c_config_supported(int T, int KF);
@@ -22,6 +22,8 @@ bool f32c_config_supported(int T, int KF);
 // grid counts workers.
 int f32c_targets(int T);  // targets per lane that a choice of T runs with
 int f32c_tile(int T);
+int f32c_quantum(int KF);  // filaments of an item: a multiple of this
+int f32c_warps();          // workers per CTA
 int f64_threads();
 int f64_tile();
 int f32c_occupancy(int model, int T, int KF);

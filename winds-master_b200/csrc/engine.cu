@@ -291,6 +291,18 @@ int upload_plan(Context *c, const Plan &pl, cudaStream_t s) {
   return WINDS_BS_OK;
 }
 
+// Workers (FP32c: warps, else blocks) of a launch with n_items items: at most the
+// resident ones and, beyond one CTA per SM, the same number of CTAs on every
+// SM. The queue hands the items out, so a smaller even grid ends earlier than a
+// larger one that leaves some SMs a CTA more (3.2k targets x 6.1k filaments: 600
+// CTAs of one item a warp put five on 8 SMs and four on the others).
+int worker_grid(long long n_items, long long resident, int sms, bool f32c) {
+  const int per = f32c ? f32c_warps() : 1;
+  long long ctas = (std::min(n_items, resident) + per - 1) / per;
+  if (ctas > sms) ctas = ctas / sms * sms;
+  return (int)std::max<long long>(1, ctas * per);
+}
+
 // ------------------------------------------------------------- packing
 // chain: order each family along the index with more links between neighbours
 // (bs_pack_filaments), else in input order.
@@ -427,7 +439,7 @@ int run_direct_sum(Context *c, const std::vector<GroupSpec> &gs, int model, doub
     if (!f32c_config_supported(ch.T, ch.KF)) return fail(WINDS_BS_ERR_ARG, "bad tile choice");
     tile_cap = f32c_tile(ch.T);
     resident = f32c_occupancy(model, ch.T, ch.KF) * c->num_sms;
-    quantum = kFilamentPad;
+    quantum = f32c_quantum(ch.KF);
   }
   // sequential: one chunk per tile, so every target sums its filaments in order
   const double waves = sequential ? 0.0 : ch.waves;
@@ -483,7 +495,7 @@ int run_direct_sum(Context *c, const std::vector<GroupSpec> &gs, int model, doub
   // near-singular pairs are counted per evaluation
   if (e == cudaSuccess) e = cudaMemsetAsync(c->nearctr.p, 0, 2 * sizeof(unsigned long long), s);
   if (e != cudaSuccess) return cuda_fail(e, "work counter reset");
-  const int grid = (int)std::max<long long>(1, std::min<long long>(a.n_items, resident));
+  const int grid = worker_grid(a.n_items, resident, c->num_sms, precision != WINDS_PREC_F64);
   if (time_main) cudaEventRecord(c->ev_main0, s);
   if (precision == WINDS_PREC_F64)
     e = launch_f64(a, grid, s);

@@ -161,7 +161,7 @@ extern "C" int winds_bs_eval_device_noalloc(const winds_bs_family *fams, int nfa
   } else {
     tile_cap = f32c_tile(ch.T);
     resident = f32c_occupancy(model, ch.T, ch.KF) * sms;
-    quantum = kFilamentPad;
+    quantum = f32c_quantum(ch.KF);
   }
   const int n_tiles = (int)((nt + tile_cap - 1) / tile_cap);
   const long long max_items =
@@ -257,7 +257,7 @@ extern "C" int winds_bs_eval_device_noalloc(const winds_bs_family *fams, int nfa
   a.n = n;
   a.co = prm->co;
   a.wait_limit_ns = default_wait_limit_ns();
-  const int grid = std::max(1, std::min(n_items, resident));
+  const int grid = worker_grid(n_items, resident, sms, prec != WINDS_PREC_F64);
   e = prec == WINDS_PREC_F64 ? launch_f64(a, grid, s) : launch_f32c(a, model, ch.T, ch.KF, grid, s);
   if (e == cudaSuccess) e = launch_reduce(tiles, n_tiles, groups, part, perm, tile_cap, s);
   if (e != cudaSuccess) return cuda_fail(e, "noalloc direct-sum launch");

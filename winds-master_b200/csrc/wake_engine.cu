@@ -167,13 +167,13 @@ int build_plans(winds_wake_batch *b) {
   } else {
     b->tile_cap = f32c_tile(b->ch.T);
     resident = f32c_occupancy(b->model, b->ch.T, b->ch.KF) * sms;
-    quantum = kFilamentPad;
+    quantum = f32c_quantum(b->ch.KF);
   }
   Plan pl;
   build_plan(pl, gs, b->tile_cap, resident, b->ch.waves, quantum);
   b->n_tiles = (int)pl.tiles.size();
   b->n_items = (int)pl.items.size();
-  b->grid = std::max(1, std::min(b->n_items, resident));
+  b->grid = worker_grid(b->n_items, resident, sms, b->prec != WINDS_PREC_F64);
   std::vector<Group> gp = pl.groups;
   for (size_t k = 0; k < gp.size(); ++k) gp[k].out = P<double>(b->uind_pred) + b->cases[k].node_off * 3;
   int rc;
@@ -1202,13 +1202,14 @@ int winds_wake_set_kj(winds_wake_batch *b, const winds_kj_case *kj, const winds_
   } else {
     b->kj_tile_cap = f32c_tile(b->kj_T);
     resident = f32c_occupancy(b->model, b->kj_T, b->kj_KF) * sms;
-    quantum = kFilamentPad;
+    quantum = f32c_quantum(b->kj_KF);
   }
   Plan pl;
   build_plan(pl, gs, b->kj_tile_cap, resident, 4.0, quantum);
   b->kj_ntiles = (int)pl.tiles.size();
   b->kj_nitems = (int)pl.items.size();
-  b->kj_grid = std::max(1, std::min(b->kj_nitems, resident));
+  b->kj_grid = worker_grid(b->kj_nitems, resident, sms,
+                           !(b->prec == WINDS_PREC_F64 || b->kjp.ll_fp64));
   if ((rc = b->kj_groups.ensure(pl.groups.size() * sizeof(Group), s)) ||
       (rc = b->kj_tiles.ensure(pl.tiles.size() * sizeof(Tile), s)) ||
       (rc = b->kj_items.ensure(pl.items.size() * sizeof(Item), s)) ||
