@@ -369,4 +369,14 @@ __device__ __forceinline__ void pair64(const double4 A, const double4 B, double 
   uz = fma(ub, cz, uz);
 }
 
+// What an evaluation starts from: an empty bounding box and the work queue at its
+// start (one block of at least 32 threads).
+__device__ __forceinline__ void begin_evaluation(BBox *bb, unsigned *ctr) {
+  if (threadIdx.x < 3) {
+    bb->tmin[threadIdx.x] = bb->fmin[threadIdx.x] = float_key(FLT_MAX);
+    bb->tmax[threadIdx.x] = bb->fmax[threadIdx.x] = float_key(-FLT_MAX);
+  }
+  if (threadIdx.x == 3) *ctr = 0u;
+}
+
 }  // namespace winds

@@ -24,6 +24,7 @@
 //   bs_length          filament lengths (core/FilamentLength.m:27-44)
 #include "bs_device.cuh"
 #include "bs_launch.h"
+#include "bs_sort.cuh"
 #include "bs_types.h"
 
 #include <cfloat>
@@ -33,13 +34,11 @@
 namespace winds {
 
 // --------------------------------------------------------------- packing
-__global__ void bs_bbox_init(BBox *bb) {
-  if (threadIdx.x == 0) {
-    for (int c = 0; c < 3; ++c) {
-      bb->tmin[c] = bb->fmin[c] = float_key(FLT_MAX);
-      bb->tmax[c] = bb->fmax[c] = float_key(-FLT_MAX);
-    }
-  }
+__global__ void bs_begin(BBox *bb, unsigned *ctr, unsigned long long *near,
+                         unsigned long long *cnt) {
+  begin_evaluation(bb, ctr);
+  if (threadIdx.x < 2) near[threadIdx.x] = 0ull;
+  if (threadIdx.x < 2 * kPackFams) cnt[threadIdx.x] = 0ull;
 }
 
 // WInDS's filaments meet at the wake's nodes: the shed call's F2(i) is its
@@ -59,64 +58,64 @@ __device__ __forceinline__ bool same_point(const double *__restrict__ F2, long l
   return F2[b2] == F1[b1] && F2[b2 + d0] == F1[b1 + d0] && F2[b2 + 2 * d0] == F1[b1 + 2 * d0];
 }
 
-__global__ void bs_chain_count(const double *__restrict__ F1, const double *__restrict__ F2,
-                               long long d0, long long d2, long long nf,
-                               unsigned long long *cnt) {
-  const long long f = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+// Up to kPackFams families per launch, each with its run of blocks.
+__global__ void bs_chain_count(const PackArgs a) {
+  int k = 0;
+  while (k + 1 < a.nfam && (int)blockIdx.x >= a.fam[k + 1].block0) ++k;
+  const PackArgs::Fam &m = a.fam[k];
+  const long long f = (long long)(blockIdx.x - m.block0) * blockDim.x + threadIdx.x;
   bool s = false, t = false;
-  if (f < nf) {
-    const long long jb = f / d0, i = f - jb * d0, j = jb % d2;
+  if (f < m.nf) {
+    const long long d0 = m.d0, jb = f / d0, i = f - jb * d0, j = jb % m.d2;
     const long long b = i + d0 * 3 * jb;
-    if (i + 1 < d0) s = same_point(F2, b, F1, b + 1, d0);   // F2(i) == F1(i+1)
-    if (j >= 1) t = same_point(F2, b, F1, b - 3 * d0, d0);  // F2(:,:,j) == F1(:,:,j-1)
+    if (i + 1 < d0) s = same_point(m.F2, b, m.F1, b + 1, d0);   // F2(i) == F1(i+1)
+    if (j >= 1) t = same_point(m.F2, b, m.F1, b - 3 * d0, d0);  // F2(:,:,j) == F1(:,:,j-1)
   }
   const unsigned ns = __popc(__ballot_sync(0xffffffffu, s));
   const unsigned nt = __popc(__ballot_sync(0xffffffffu, t));
   if ((threadIdx.x & 31) == 0) {
-    if (ns) atomicAdd(cnt, (unsigned long long)ns);
-    if (nt) atomicAdd(cnt + 1, (unsigned long long)nt);
+    if (ns) atomicAdd(m.cnt, (unsigned long long)ns);
+    if (nt) atomicAdd(m.cnt + 1, (unsigned long long)nt);
   }
 }
 
-// One thread per filament of the family, in input order; its record goes to
-// slot off + f, or (cnt given and cnt[1] > cnt[0]) to its place along the third
-// index.
-__global__ void bs_pack_filaments(const double *__restrict__ F1, const double *__restrict__ F2,
-                                  const double *__restrict__ gam, const double *__restrict__ rc,
-                                  long long d0, long long d2, long long nf, long long off,
-                                  const unsigned long long *__restrict__ cnt, int model,
-                                  double dcut, float4 *pk, double4 *ra, double4 *rb, BBox *bb) {
-  const long long f = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+// One thread per filament of a family, in input order; its record goes to slot
+// off + f, or (cnt given and cnt[1] > cnt[0]) to its place along the third
+// index. The blocks past the families fill [pad_from, pad_to) with inert
+// filaments: far away, zero length, zero circulation.
+__global__ void bs_pack_filaments(const PackArgs a) {
   float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
-  if (f < nf) {
-    const bool along3 = cnt && cnt[1] > cnt[0];
-    const long long jb = f / d0, i = f - jb * d0;
+  if ((int)blockIdx.x >= a.pad_block0) {
+    const long long f =
+        a.pad_from + (long long)(blockIdx.x - a.pad_block0) * blockDim.x + threadIdx.x;
+    if (f < a.pad_to) pack_inert(f, a.pk, a.ra, a.rb);
+    return;
+  }
+  int k = 0;
+  while (k + 1 < a.nfam && (int)blockIdx.x >= a.fam[k + 1].block0) ++k;
+  const PackArgs::Fam &m = a.fam[k];
+  const long long f = (long long)(blockIdx.x - m.block0) * blockDim.x + threadIdx.x;
+  if (f < m.nf) {
+    const bool along3 = m.cnt && m.cnt[1] > m.cnt[0];
+    const long long d0 = m.d0, jb = f / d0, i = f - jb * d0;
     const long long b = i + d0 * 3 * jb;
-    const double x1 = F1[b], y1 = F1[b + d0], z1 = F1[b + 2 * d0];
-    const double x2 = F2[b], y2 = F2[b + d0], z2 = F2[b + 2 * d0];
-    long long slot = off + f;
+    const double x1 = m.F1[b], y1 = m.F1[b + d0], z1 = m.F1[b + 2 * d0];
+    const double x2 = m.F2[b], y2 = m.F2[b + d0], z2 = m.F2[b + 2 * d0];
+    long long slot = m.off + f;
     bool head;
     if (along3) {
-      const long long bl = jb / d2, j = jb - bl * d2;
-      slot = off + j + d2 * (i + d0 * bl);
-      head = !(j >= 1 && same_point(F2, b, F1, b - 3 * d0, d0));
+      const long long bl = jb / m.d2, j = jb - bl * m.d2;
+      slot = m.off + j + m.d2 * (i + d0 * bl);
+      head = !(j >= 1 && same_point(m.F2, b, m.F1, b - 3 * d0, d0));
     } else {
-      head = !(i >= 1 && same_point(F2, b - 1, F1, b, d0));
+      head = !(i >= 1 && same_point(m.F2, b - 1, m.F1, b, d0));
     }
-    pack_filament(slot, x1, y1, z1, x2, y2, z2, gam[f], rc[f], !along3, head, model, dcut, pk, ra,
-                  rb);
+    pack_filament(slot, x1, y1, z1, x2, y2, z2, m.gam[f], m.rc[f], !along3, head, a.model, a.dcut,
+                  a.pk, a.ra, a.rb);
     lo[0] = (float)fmin(x1, x2), lo[1] = (float)fmin(y1, y2), lo[2] = (float)fmin(z1, z2);
     hi[0] = (float)fmax(x1, x2), hi[1] = (float)fmax(y1, y2), hi[2] = (float)fmax(z1, z2);
   }
-  bbox_accumulate(lo, hi, bb->fmin, bb->fmax);
-}
-
-// Inert filaments filling [from, to): far away, zero length, zero circulation.
-__global__ void bs_pad_filaments(long long from, long long to, float4 *pk, double4 *ra,
-                                 double4 *rb) {
-  const long long f = from + (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= to) return;
-  pack_inert(f, pk, ra, rb);
+  bbox_accumulate(lo, hi, a.bb->fmin, a.bb->fmax);
 }
 
 __global__ void bs_pack_targets(const double *__restrict__ P, long long ns, long long np,
@@ -136,69 +135,22 @@ __global__ void bs_pack_targets(const double *__restrict__ P, long long ns, long
   bbox_accumulate(lo, hi, bb->tmin, bb->tmax);
 }
 
-// Spreads the low 10 bits of v so that they occupy every third bit.
-__device__ __forceinline__ unsigned long long spread3(unsigned v) {
-  unsigned long long x = v & 0x3ffu;
-  x = (x | (x << 16)) & 0x30000ffull;
-  x = (x | (x << 8)) & 0x300f00full;
-  x = (x | (x << 4)) & 0x30c30c3ull;
-  x = (x | (x << 2)) & 0x9249249ull;
-  return x;
-}
-
-// Distance along a 3-D Hilbert curve of 10 bits a coordinate (Skilling's
-// transpose algorithm, "Programming the Hilbert curve", AIP Conf. Proc. 707,
-// 2004). Consecutive targets on it are neighbours in space without exception,
-// where a Morton code jumps at every power of two: on the large wake the
-// radius of 96 consecutive targets is 9.1 m (median; largest 34 m) instead of
-// 10.1 m (82 m).
-__device__ __forceinline__ unsigned long long hilbert30(unsigned x, unsigned y, unsigned z) {
-  unsigned X[3] = {x, y, z};
-#pragma unroll
-  for (unsigned Q = 512u; Q > 1u; Q >>= 1) {
-    const unsigned m = Q - 1u;
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      if (X[c] & Q) {
-        X[0] ^= m;
-      } else {
-        const unsigned t = (X[0] ^ X[c]) & m;
-        X[0] ^= t;
-        X[c] ^= t;
-      }
-    }
-  }
-  X[1] ^= X[0];
-  X[2] ^= X[1];
-  unsigned t = 0;
-#pragma unroll
-  for (unsigned Q = 512u; Q > 1u; Q >>= 1)
-    if (X[2] & Q) t ^= Q - 1u;
-  return spread3(X[0] ^ t) << 2 | spread3(X[1] ^ t) << 1 | spread3(X[2] ^ t);
-}
-
 // Sort key of a target: group id above the 30-bit Hilbert position in the
-// targets' bounding box (bit 31: the target is unused).
+// targets' bounding box (bit 30: the target is unused, and sorts after every
+// live target of its group).
+template <class KEY>
 __global__ void bs_target_keys(const double4 *__restrict__ tp, const int *__restrict__ tgroup,
-                               long long n, const BBox *bb, unsigned long long *keys, int *vals) {
+                               long long n, const BBox *bb, KEY *keys, int *vals) {
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
   const double4 p = tp[t];
   const double q[3] = {p.x, p.y, p.z};
-  unsigned cell[3];
-  for (int c = 0; c < 3; ++c) {
-    const double lo = key_float(bb->tmin[c]), hi = key_float(bb->tmax[c]);
-    const double w = hi > lo ? hi - lo : 1.0;
-    double u = (q[c] - lo) / w * 1023.999;
-    if (!(u >= 0.0)) u = 0.0;  // also catches NaN
-    if (u > 1023.0) u = 1023.0;
-    cell[c] = (unsigned)u;
-  }
-  unsigned long long code = hilbert30(cell[0], cell[1], cell[2]);
-  // a target marked unused (w != 0: past a growing wake's live columns) sorts
-  // after every live target of its group
-  if (p.w != 0.0) code |= 1ull << 31;
-  keys[t] = ((unsigned long long)(unsigned)tgroup[t] << 32) | code;
+  const float lo[3] = {key_float(bb->tmin[0]), key_float(bb->tmin[1]), key_float(bb->tmin[2])};
+  const float hi[3] = {key_float(bb->tmax[0]), key_float(bb->tmax[1]), key_float(bb->tmax[2])};
+  KEY code = hilbert_key(q, lo, hi);
+  if (p.w != 0.0) code |= (KEY)1 << 30;
+  if (sizeof(KEY) == 8) code |= (KEY)(unsigned)tgroup[t] << 31;
+  keys[t] = code;
   vals[t] = (int)t;
 }
 
@@ -1084,13 +1036,20 @@ __global__ void __launch_bounds__(kF64Threads) bs_f64(const F32cArgs a) {
 }
 
 // --------------------------------------------------------------- reduce
-// With a live table, only the live targets of a tile are written, from the
+// A block sums 32 consecutive targets of a tile: each warp a run of the tile's
+// items in order, lanes the targets, then the warps' sums in order. (One thread
+// per target, all items in one chain of loads, took 30 us on the 3.1k-target
+// wake; spread over eight warps 12.) With a live table, only the live targets of a tile are written, from the
 // items before the group's live filament end (a tile's items cover increasing
-// filament ranges, so those come first).
-__global__ void bs_reduce(const Tile *__restrict__ tiles, const Group *__restrict__ groups,
-                          const double *__restrict__ part, const int *__restrict__ perm,
-                          int tile_cap, const Item *__restrict__ items,
-                          const GroupLive *__restrict__ live) {
+// filament ranges, so those come first). The last kernel of an evaluation: it
+// leaves the work queue at its start.
+constexpr int kReduceWarps = 8;
+__global__ void __launch_bounds__(32 * kReduceWarps)
+    bs_reduce(const Tile *__restrict__ tiles, const Group *__restrict__ groups,
+              const double *__restrict__ part, const int *__restrict__ perm, int tile_cap,
+              const Item *__restrict__ items, const GroupLive *__restrict__ live, unsigned *ctr) {
+  __shared__ double s_sum[kReduceWarps][3][32];
+  if (blockIdx.x + blockIdx.y == 0 && threadIdx.x == 0) *ctr = 0u;
   Tile tl = tiles[blockIdx.x];
   const Group g = groups[tl.group];
   if (live) {
@@ -1098,32 +1057,37 @@ __global__ void bs_reduce(const Tile *__restrict__ tiles, const Group *__restric
     const long long tn = gl.t_end - tl.t_begin;
     if (tn <= 0) return;
     if (tn < tl.t_count) tl.t_count = (int)tn;
-    int k = 0;
-    while (k < tl.n_items && items[tl.first_item + k].f_begin < gl.f_end) ++k;
-    tl.n_items = k;
+    int lo = 0, hi = tl.n_items;  // the first item at or past the live end
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      if (items[tl.first_item + mid].f_begin < gl.f_end) lo = mid + 1; else hi = mid;
+    }
+    tl.n_items = lo;
   }
-  for (int l = threadIdx.x; l < tl.t_count; l += blockDim.x) {
-    double s0 = 0.0, s1 = 0.0, s2 = 0.0;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int l = 32 * blockIdx.y + lane;
+  if (32 * (int)blockIdx.y >= tl.t_count) return;
+  double s0 = 0.0, s1 = 0.0, s2 = 0.0;
+  if (l < tl.t_count) {
+    const int k0 = tl.n_items * warp / kReduceWarps, k1 = tl.n_items * (warp + 1) / kReduceWarps;
+    const double *p = part + (size_t)(tl.first_item + k0) * 3 * tile_cap + l;
 #pragma unroll 4
-    for (int k = 0; k < tl.n_items; ++k) {
-      const double *p = part + (size_t)(tl.first_item + k) * 3 * tile_cap;
-      s0 += p[l];
-      s1 += p[tile_cap + l];
-      s2 += p[2 * tile_cap + l];
-    }
-    const long long local = (long long)perm[tl.t_begin + l] - g.t_begin;
-    const long long j = local / g.ns_p, i = local - j * g.ns_p;
-    double *o = g.out + i + 3 * g.ns_p * j;
-    if (g.accumulate) {
-      o[0] += s0;
-      o[g.ns_p] += s1;
-      o[2 * g.ns_p] += s2;
-    } else {
-      o[0] = s0;
-      o[g.ns_p] = s1;
-      o[2 * g.ns_p] = s2;
+    for (int k = k0; k < k1; ++k, p += 3 * (size_t)tile_cap) {
+      s0 += p[0];
+      s1 += p[tile_cap];
+      s2 += p[2 * tile_cap];
     }
   }
+  s_sum[warp][0][lane] = s0, s_sum[warp][1][lane] = s1, s_sum[warp][2][lane] = s2;
+  __syncthreads();
+  if (warp >= 3 || l >= tl.t_count) return;
+  double s = 0.0;  // warp c: component c
+#pragma unroll
+  for (int w = 0; w < kReduceWarps; ++w) s += s_sum[w][warp][lane];
+  const long long local = (long long)perm[tl.t_begin + l] - g.t_begin;
+  const long long j = local / g.ns_p, i = local - j * g.ns_p;
+  double *o = g.out + i + 3 * g.ns_p * j + warp * g.ns_p;
+  *o = g.accumulate ? *o + s : s;
 }
 
 // --------------------------------------------------------------- lengths
@@ -1258,37 +1222,60 @@ cudaError_t launch_f64(const F32cArgs &a, int grid, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_bbox_init(BBox *bb, cudaStream_t s) {
-  bs_bbox_init<<<1, 32, 0, s>>>(bb);
+cudaError_t launch_begin(BBox *bb, unsigned *ctr, unsigned long long *near, unsigned long long *cnt,
+                         cudaStream_t s) {
+  bs_begin<<<1, 32, 0, s>>>(bb, ctr, near, cnt);
   return cudaGetLastError();
 }
 
-cudaError_t launch_pack_filaments(const double *F1, const double *F2, const double *gam,
-                                  const double *rc, const long long d[4], long long off,
-                                  unsigned long long *cnt, int model, double dcut,
-                                  const PackedFilaments &pf, BBox *bb, cudaStream_t s) {
-  const long long nf = d[0] * d[2] * d[3];
-  if (nf <= 0) return cudaSuccess;
+cudaError_t launch_pack_families(const winds_bs_family *fams, int nfam, unsigned long long *cnt,
+                                 long long pad_to, int model, double dcut,
+                                 const PackedFilaments &pf, BBox *bb, cudaStream_t s,
+                                 int *launches) {
   const int bs = 256;
-  const unsigned grid = (unsigned)((nf + bs - 1) / bs);
-  cudaError_t e;
-  if (cnt) {
-    if ((e = cudaMemsetAsync(cnt, 0, 2 * sizeof(unsigned long long), s)) != cudaSuccess) return e;
-    bs_chain_count<<<grid, bs, 0, s>>>(F1, F2, d[0], d[2], nf, cnt);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  }
-  bs_pack_filaments<<<grid, bs, 0, s>>>(F1, F2, gam, rc, d[0], d[2], nf, off, cnt, model, dcut,
-                                        pf.pk, pf.ra, pf.rb, bb);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_pad_filaments(long long from, long long to, const PackedFilaments &pf,
-                                 cudaStream_t s) {
-  if (to <= from) return cudaSuccess;
-  const int bs = 256;
-  const long long grid = (to - from + bs - 1) / bs;
-  bs_pad_filaments<<<(unsigned)grid, bs, 0, s>>>(from, to, pf.pk, pf.ra, pf.rb);
-  return cudaGetLastError();
+  long long off = 0;
+  int k = 0;
+  bool first = true;
+  do {
+    PackArgs a;
+    a.nfam = 0;
+    long long blocks = 0;
+    for (; k < nfam && a.nfam < kPackFams; ++k) {
+      const winds_bs_family &m = fams[k];
+      const long long nf = m.dims[0] * m.dims[2] * m.dims[3];
+      if (nf <= 0) continue;
+      PackArgs::Fam &f = a.fam[a.nfam];
+      f.F1 = m.F1, f.F2 = m.F2, f.gam = m.gamma, f.rc = m.rc;
+      f.d0 = m.dims[0], f.d2 = m.dims[2], f.nf = nf, f.off = off;
+      f.cnt = cnt ? cnt + 2 * a.nfam : nullptr;
+      ++a.nfam;
+      f.block0 = (int)blocks;
+      blocks += (nf + bs - 1) / bs;
+      off += nf;
+    }
+    a.model = model, a.dcut = dcut;
+    a.pk = pf.pk, a.ra = pf.ra, a.rb = pf.rb, a.bb = bb;
+    a.pad_block0 = (int)blocks;
+    a.pad_from = off;
+    a.pad_to = k >= nfam ? pad_to : off;
+    if (cnt && blocks > 0) {
+      if (!first) {
+        const cudaError_t e = cudaMemsetAsync(cnt, 0, 2 * kPackFams * sizeof(*cnt), s);
+        if (e != cudaSuccess) return e;
+      }
+      first = false;
+      bs_chain_count<<<(unsigned)blocks, bs, 0, s>>>(a);
+      if (launches) ++*launches;
+    }
+    const long long total = blocks + (a.pad_to - a.pad_from + bs - 1) / bs;
+    if (total > 0) {
+      bs_pack_filaments<<<(unsigned)total, bs, 0, s>>>(a);
+      if (launches) ++*launches;
+    }
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+  } while (k < nfam);
+  return cudaSuccess;
 }
 
 cudaError_t launch_pack_targets(const double *P, long long ns, long long np, long long off,
@@ -1300,13 +1287,6 @@ cudaError_t launch_pack_targets(const double *P, long long ns, long long np, lon
   return cudaGetLastError();
 }
 
-cudaError_t launch_target_keys(const double4 *tp, const int *tgroup, long long n, const BBox *bb,
-                               unsigned long long *keys, int *vals, cudaStream_t s) {
-  if (n <= 0) return cudaSuccess;
-  bs_target_keys<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(tp, tgroup, n, bb, keys, vals);
-  return cudaGetLastError();
-}
-
 cudaError_t launch_gather_targets(const double4 *src, const int *perm, long long n, double4 *dst,
                                   cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
@@ -1314,21 +1294,68 @@ cudaError_t launch_gather_targets(const double4 *src, const int *perm, long long
   return cudaGetLastError();
 }
 
-// Sorts (key, value) pairs with CUB's radix sort; temp == nullptr queries the
-// scratch size into *temp_bytes.
-cudaError_t sort_target_keys(void *temp, size_t *temp_bytes, const unsigned long long *kin,
-                             unsigned long long *kout, const int *vin, int *vout, long long n,
-                             cudaStream_t s) {
-  return cub::DeviceRadixSort::SortPairs(temp, *temp_bytes, kin, kout, vin, vout, (int)n, 0, 64, s);
+// The device-wide sort: 31-bit keys for one group, the group id above them for
+// more, and only these bits sorted (one group: four passes of the library's
+// radix sort, where all 64 bits took eight).
+static int group_bits(int groups) {
+  int b = 0;
+  while ((1ll << b) < groups) ++b;
+  return b;
+}
+
+cudaError_t sort_targets_bytes(long long n, int groups, size_t *bytes) {
+  *bytes = 0;
+  if (groups == 1)
+    return cub::DeviceRadixSort::SortPairs(nullptr, *bytes, (const unsigned *)nullptr,
+                                           (unsigned *)nullptr, (const int *)nullptr,
+                                           (int *)nullptr, (int)n, 0, 31, (cudaStream_t)0);
+  return cub::DeviceRadixSort::SortPairs(nullptr, *bytes, (const unsigned long long *)nullptr,
+                                         (unsigned long long *)nullptr, (const int *)nullptr,
+                                         (int *)nullptr, (int)n, 0, 31 + group_bits(groups),
+                                         (cudaStream_t)0);
+}
+
+cudaError_t launch_sort_targets(const TargetBufs &b, long long n, int groups, const BBox *bb,
+                                cudaStream_t s) {
+  if (n <= 0) return cudaSuccess;
+  const unsigned grid = (unsigned)((n + 255) / 256);
+  size_t bytes = b.sort_bytes;
+  cudaError_t e;
+  if (groups == 1) {
+    unsigned *k0 = reinterpret_cast<unsigned *>(b.keys), *k1 = k0 + n;
+    bs_target_keys<<<grid, 256, 0, s>>>(b.tp_raw, b.tgroup, n, bb, k0, b.vals);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    e = cub::DeviceRadixSort::SortPairs(b.sort_tmp, bytes, (const unsigned *)k0, k1,
+                                        (const int *)b.vals, b.perm, (int)n, 0, 31, s);
+  } else {
+    unsigned long long *k0 = b.keys, *k1 = k0 + n;
+    bs_target_keys<<<grid, 256, 0, s>>>(b.tp_raw, b.tgroup, n, bb, k0, b.vals);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    e = cub::DeviceRadixSort::SortPairs(b.sort_tmp, bytes, (const unsigned long long *)k0, k1,
+                                        (const int *)b.vals, b.perm, (int)n, 0,
+                                        31 + group_bits(groups), s);
+  }
+  return e != cudaSuccess ? e : launch_gather_targets(b.tp_raw, b.perm, n, b.tp, s);
+}
+
+cudaError_t launch_matlab_targets(const double *P, long long ns, long long n, const TargetBufs &b,
+                                  BBox *bb, cudaStream_t s) {
+  if (n <= 0) return cudaSuccess;
+  if (n <= kBlockSortMax) {
+    MatlabTargets src{P, ns, (int)n};
+    return launch_block_sort(src, 1, n, b.tp, b.perm, bb, s);
+  }
+  cudaError_t e = launch_pack_targets(P, ns, n, 0, 0, b.tp_raw, b.tgroup, bb, s);
+  return e != cudaSuccess ? e : launch_sort_targets(b, n, 1, bb, s);
 }
 
 cudaError_t launch_reduce(const Tile *tiles, int n_tiles, const Group *groups, const double *part,
-                          const int *perm, int tile_cap, cudaStream_t s, const Item *items,
-                          const GroupLive *live) {
+                          const int *perm, int tile_cap, unsigned *ctr, cudaStream_t s,
+                          const Item *items, const GroupLive *live) {
   if (n_tiles <= 0) return cudaSuccess;
   if (live && !items) return cudaErrorInvalidValue;
-  const int bs = tile_cap >= 256 ? 256 : (tile_cap + 31) / 32 * 32;  // one thread per target
-  bs_reduce<<<n_tiles, bs, 0, s>>>(tiles, groups, part, perm, tile_cap, items, live);
+  const dim3 grid((unsigned)n_tiles, (unsigned)(tile_cap + 31) / 32);
+  bs_reduce<<<grid, 32 * kReduceWarps, 0, s>>>(tiles, groups, part, perm, tile_cap, items, live, ctr);
   return cudaGetLastError();
 }
 

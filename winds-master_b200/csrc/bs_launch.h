@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include "bs_types.h"
+#include "winds_bs.h"
 
 namespace winds {
 
@@ -30,29 +31,42 @@ int f32c_occupancy(int model, int T, int KF);
 int f64_occupancy();
 unsigned long long default_wait_limit_ns();
 
-cudaError_t launch_bbox_init(BBox *bb, cudaStream_t s);
-// Packs a [d0,3,d2,d3] family from slot off on, in input order or (cnt: 2 device
-// words of scratch) in the order with more links between neighbours.
-cudaError_t launch_pack_filaments(const double *F1, const double *F2, const double *gam,
-                                  const double *rc, const long long d[4], long long off,
-                                  unsigned long long *cnt, int model, double dcut,
-                                  const PackedFilaments &pf, BBox *bb, cudaStream_t s);
-cudaError_t launch_pad_filaments(long long from, long long to, const PackedFilaments &pf,
-                                 cudaStream_t s);
-cudaError_t launch_pack_targets(const double *P, long long ns, long long np, long long off,
-                                int group, double4 *tp, int *tgroup, BBox *bb, cudaStream_t s);
-cudaError_t launch_target_keys(const double4 *tp, const int *tgroup, long long n, const BBox *bb,
-                               unsigned long long *keys, int *vals, cudaStream_t s);
-cudaError_t launch_gather_targets(const double4 *src, const int *perm, long long n, double4 *dst,
-                                  cudaStream_t s);
-cudaError_t sort_target_keys(void *temp, size_t *temp_bytes, const unsigned long long *kin,
-                             unsigned long long *kout, const int *vin, int *vout, long long n,
-                             cudaStream_t s);
+// First kernel of an evaluation: empty bounding box, work queue at its start,
+// near (2 words) and cnt (2 kPackFams words) zero.
+cudaError_t launch_begin(BBox *bb, unsigned *ctr, unsigned long long *near, unsigned long long *cnt,
+                         cudaStream_t s);
+// Packs the families (device arrays) one after the other, in input order or
+// (cnt: as launch_begin leaves it) each in the order with more links between
+// neighbours, then inert filaments up to pad_to. Adds to *launches.
+cudaError_t launch_pack_families(const winds_bs_family *fams, int nfam, unsigned long long *cnt,
+                                 long long pad_to, int model, double dcut,
+                                 const PackedFilaments &pf, BBox *bb, cudaStream_t s,
+                                 int *launches);
+// Targets sorted by (group, place on a Hilbert curve). Groups of at most
+// kBlockSortMax targets are sorted by one CTA each (bs_sort.cuh) and need tp and
+// perm only; the device-wide sort needs the rest (keys: 2 n words of 32 bits for one
+// group, of 64 for more).
+constexpr long long kBlockSortMax = 16384;
+struct TargetBufs {
+  double4 *tp, *tp_raw;
+  int *tgroup, *vals, *perm;
+  unsigned long long *keys;
+  void *sort_tmp;
+  size_t sort_bytes;
+};
+cudaError_t launch_matlab_targets(const double *P, long long ns, long long n, const TargetBufs &b,
+                                  BBox *bb, cudaStream_t s);
+// Device-wide sort of n targets already in tp_raw / tgroup (groups of them), and
+// the scratch bytes it needs.
+cudaError_t launch_sort_targets(const TargetBufs &b, long long n, int groups, const BBox *bb,
+                                cudaStream_t s);
+cudaError_t sort_targets_bytes(long long n, int groups, size_t *bytes);
 cudaError_t launch_f32c(const F32cArgs &a, int model, int T, int KF, int grid, cudaStream_t s);
 cudaError_t launch_f64(const F32cArgs &a, int grid, cudaStream_t s);
-// live (with the plan's items): only each group's live part (GroupLive).
+// live (with the plan's items): only each group's live part (GroupLive). Leaves
+// the work queue's counter ctr at its start.
 cudaError_t launch_reduce(const Tile *tiles, int n_tiles, const Group *groups, const double *part,
-                          const int *perm, int tile_cap, cudaStream_t s,
+                          const int *perm, int tile_cap, unsigned *ctr, cudaStream_t s,
                           const Item *items = nullptr, const GroupLive *live = nullptr);
 cudaError_t launch_ffma_peak(float *out, int blocks, int iters, cudaStream_t s);
 cudaError_t launch_wait_selftest(unsigned *err, unsigned long long limit_ns, cudaStream_t s);

@@ -77,6 +77,23 @@ struct BBox {           // ordered-int keys of float bounds (see float_key)
   int fmin[3], fmax[3]; // filament endpoints
 };
 
+constexpr int kPackFams = 4;
+struct PackArgs {       // bs_chain_count, bs_pack_filaments
+  struct Fam {
+    const double *F1, *F2, *gam, *rc;
+    long long d0, d2, nf, off;
+    unsigned long long *cnt;
+    int block0;
+  } fam[kPackFams];
+  int nfam, model;
+  long long pad_from, pad_to;
+  int pad_block0;
+  double dcut;
+  float4 *pk;
+  double4 *ra, *rb;
+  BBox *bb;
+};
+
 struct F32cArgs {
   const float4 *pk;  // records, 4 float4 per filament
   const double4 *ra, *rb;

@@ -307,70 +307,45 @@ int worker_grid(long long n_items, long long resident, int sms, bool f32c) {
 // chain: order each family along the index with more links between neighbours
 // (bs_pack_filaments), else in input order.
 int pack_inputs(Context *c, const winds_bs_family *fams, int nfam,
-                const std::vector<TargetSpec> &tsets, int model, double dcut, cudaStream_t s,
+                const TargetSpec &tset, int model, double dcut, cudaStream_t s,
                 long long *nf_real, long long *nf_pad, long long *nt_total, bool chain) {
   long long nf = 0;
   for (int k = 0; k < nfam; ++k) nf += fams[k].dims[0] * fams[k].dims[2] * fams[k].dims[3];
   const long long nfp = std::max<long long>(round_up(nf, kFilamentPad), kFilamentPad);
-  long long nt = 0;
-  for (const TargetSpec &t : tsets) nt += t.count;
+  const long long nt = tset.count;
   int rc;
+  const long long n1 = std::max<long long>(nt, 1);
   if ((rc = c->pk.ensure(nfp * 4 * sizeof(float4), s)) ||
       (rc = c->ra.ensure(nfp * sizeof(double4), s)) ||
       (rc = c->rb.ensure(nfp * sizeof(double4), s)) ||
-      (rc = c->tp.ensure(std::max<long long>(nt, 1) * sizeof(double4), s)) ||
-      (rc = c->tp_raw.ensure(std::max<long long>(nt, 1) * sizeof(double4), s)) ||
-      (rc = c->tgroup.ensure(std::max<long long>(nt, 1) * sizeof(int), s)) ||
-      (rc = c->keys.ensure(std::max<long long>(nt, 1) * 2 * sizeof(unsigned long long), s)) ||
-      (rc = c->vals.ensure(std::max<long long>(nt, 1) * sizeof(int), s)) ||
-      (rc = c->perm.ensure(std::max<long long>(nt, 1) * sizeof(int), s)))
+      (rc = c->tp.ensure(n1 * sizeof(double4), s)) || (rc = c->perm.ensure(n1 * sizeof(int), s)) ||
+      (rc = c->chaincnt.ensure(2 * kPackFams * sizeof(unsigned long long), s)))
     return rc;
-  if ((rc = c->chaincnt.ensure(std::max(nfam, 1) * 2 * sizeof(unsigned long long), s)))
-    return rc;
-  size_t sort_bytes = 0;
-  if (sort_target_keys(nullptr, &sort_bytes, nullptr, nullptr, nullptr, nullptr, nt, s) !=
-      cudaSuccess)
-    return fail(WINDS_BS_ERR_CUDA, "target sort size query failed");
-  if ((rc = c->sort_tmp.ensure(sort_bytes + 256, s))) return rc;
+  TargetBufs tb{};
+  if (nt > kBlockSortMax) {
+    if (sort_targets_bytes(nt, 1, &tb.sort_bytes) != cudaSuccess)
+      return fail(WINDS_BS_ERR_CUDA, "target sort size query failed");
+    if ((rc = c->tp_raw.ensure(n1 * sizeof(double4), s)) ||
+        (rc = c->tgroup.ensure(n1 * sizeof(int), s)) ||
+        (rc = c->keys.ensure(n1 * 2 * sizeof(unsigned), s)) ||
+        (rc = c->vals.ensure(n1 * sizeof(int), s)) ||
+        (rc = c->sort_tmp.ensure(tb.sort_bytes + 256, s)))
+      return rc;
+  }
+  tb.tp = (double4 *)c->tp.p, tb.tp_raw = (double4 *)c->tp_raw.p;
+  tb.tgroup = (int *)c->tgroup.p, tb.vals = (int *)c->vals.p, tb.perm = (int *)c->perm.p;
+  tb.keys = (unsigned long long *)c->keys.p, tb.sort_tmp = c->sort_tmp.p;
   PackedFilaments pf{(float4 *)c->pk.p, (double4 *)c->ra.p, (double4 *)c->rb.p};
-  cudaError_t e = launch_bbox_init((BBox *)c->bbox.p, s);
+  BBox *bb = (BBox *)c->bbox.p;
+  unsigned long long *cnt = (unsigned long long *)c->chaincnt.p;
+  cudaError_t e = launch_begin(bb, (unsigned *)c->ctr.p, (unsigned long long *)c->nearctr.p, cnt, s);
   c->launches += 1;
   c->chained = chain;
-  long long off = 0;
-  for (int k = 0; k < nfam && e == cudaSuccess; ++k) {
-    const long long *d = fams[k].dims;
-    const long long n = d[0] * d[2] * d[3];
-    e = launch_pack_filaments(fams[k].F1, fams[k].F2, fams[k].gamma, fams[k].rc, d, off,
-                              chain ? (unsigned long long *)c->chaincnt.p + 2 * k : nullptr, model,
-                              dcut, pf, (BBox *)c->bbox.p, s);
-    c->launches += n > 0 ? (chain ? 2 : 1) : 0;
-    off += n;
-  }
-  if (e == cudaSuccess) {
-    e = launch_pad_filaments(nf, nfp, pf, s);
-    c->launches += nfp > nf;
-  }
-  long long toff = 0;
-  int gid = 0;
-  for (const TargetSpec &t : tsets) {
-    if (e != cudaSuccess) break;
-    e = launch_pack_targets(t.P, t.ns, t.count, toff, gid++, (double4 *)c->tp_raw.p,
-                            (int *)c->tgroup.p, (BBox *)c->bbox.p, s);
-    c->launches += t.count > 0;
-    toff += t.count;
-  }
-  // Sort targets by (set, Hilbert position) so each thread's targets lie close together.
-  unsigned long long *k0 = (unsigned long long *)c->keys.p, *k1 = k0 + std::max<long long>(nt, 1);
   if (e == cudaSuccess)
-    e = launch_target_keys((const double4 *)c->tp_raw.p, (const int *)c->tgroup.p, nt,
-                           (const BBox *)c->bbox.p, k0, (int *)c->vals.p, s);
-  if (e == cudaSuccess && nt > 0)
-    e = sort_target_keys(c->sort_tmp.p, &sort_bytes, k0, k1, (const int *)c->vals.p,
-                         (int *)c->perm.p, nt, s);
-  if (e == cudaSuccess)
-    e = launch_gather_targets((const double4 *)c->tp_raw.p, (const int *)c->perm.p, nt,
-                              (double4 *)c->tp.p, s);
-  c->launches += nt > 0 ? 5 : 0;  // keys, 3 radix-sort passes (library), gather (approx.)
+    e = launch_pack_families(fams, nfam, chain ? cnt : nullptr, nfp, model, dcut, pf, bb, s,
+                             &c->launches);
+  if (e == cudaSuccess) e = launch_matlab_targets(tset.P, tset.ns, nt, tb, bb, s);
+  c->launches += nt <= 0 ? 0 : (nt <= kBlockSortMax ? 1 : 9);  // 9: with the library's passes
   if (e != cudaSuccess) return cuda_fail(e, "pack kernels");
   *nf_real = nf;
   *nf_pad = nfp;
@@ -491,10 +466,7 @@ int run_direct_sum(Context *c, const std::vector<GroupSpec> &gs, int model, doub
   a.n = n;
   a.co = co;
   a.wait_limit_ns = default_wait_limit_ns();
-  cudaError_t e = cudaMemsetAsync(c->ctr.p, 0, sizeof(unsigned), s);
-  // near-singular pairs are counted per evaluation
-  if (e == cudaSuccess) e = cudaMemsetAsync(c->nearctr.p, 0, 2 * sizeof(unsigned long long), s);
-  if (e != cudaSuccess) return cuda_fail(e, "work counter reset");
+  cudaError_t e;
   const int grid = worker_grid(a.n_items, resident, c->num_sms, precision != WINDS_PREC_F64);
   if (time_main) cudaEventRecord(c->ev_main0, s);
   if (precision == WINDS_PREC_F64)
@@ -506,7 +478,8 @@ int run_direct_sum(Context *c, const std::vector<GroupSpec> &gs, int model, doub
   c->timed = time_main;
   if (e != cudaSuccess) return cuda_fail(e, "direct-sum launch");
   e = launch_reduce((const Tile *)c->tiles.p, (int)pl.tiles.size(), (const Group *)c->groups.p,
-                    (const double *)c->part.p, (const int *)c->perm.p, tile_cap, s);
+                    (const double *)c->part.p, (const int *)c->perm.p, tile_cap,
+                    (unsigned *)c->ctr.p, s);
   c->launches += 1;
   if (e != cudaSuccess) return cuda_fail(e, "reduce launch");
   return WINDS_BS_OK;
@@ -552,34 +525,27 @@ int resolve_model(const winds_bs_params *prm, int *model, double *dcut, double *
   return WINDS_BS_OK;
 }
 
-// Packs the inputs in one layout and describes one group per target set.
-static int pack_groups(Context *c, const winds_bs_family *fams, int nfam,
-                       const std::vector<TargetSpec> &tsets, int model, double dcut,
-                       cudaStream_t s, bool chain, std::vector<GroupSpec> *gs, long long *nf,
-                       long long *nt) {
+// Packs the inputs in one layout and describes the targets' group.
+static int pack_groups(Context *c, const winds_bs_family *fams, int nfam, const TargetSpec &t,
+                       int model, double dcut, cudaStream_t s, bool chain,
+                       std::vector<GroupSpec> *gs, long long *nf, long long *nt) {
   long long nfp;
   int rc;
-  if ((rc = pack_inputs(c, fams, nfam, tsets, model, dcut, s, nf, &nfp, nt, chain))) return rc;
-  gs->clear();
-  long long toff = 0;
-  for (const TargetSpec &t : tsets) {
-    GroupSpec g;
-    g.out = t.out;
-    g.t_begin = toff;
-    g.t_count = t.count;
-    g.ns_p = t.ns;
-    g.f_begin = 0;
-    g.f_end = (int)nfp;
-    g.accumulate = t.accumulate;
-    gs->push_back(g);
-    toff += t.count;
-  }
+  if ((rc = pack_inputs(c, fams, nfam, t, model, dcut, s, nf, &nfp, nt, chain))) return rc;
+  GroupSpec g;
+  g.out = t.out;
+  g.t_begin = 0;
+  g.t_count = t.count;
+  g.ns_p = t.ns;
+  g.f_begin = 0;
+  g.f_end = (int)nfp;
+  g.accumulate = t.accumulate;
+  gs->assign(1, g);
   return WINDS_BS_OK;
 }
 
-int eval_device(Context *c, const winds_bs_family *fams, int nfam,
-                const std::vector<TargetSpec> &tsets, const winds_bs_params *prm,
-                cudaStream_t s, bool sequential) {
+int eval_device(Context *c, const winds_bs_family *fams, int nfam, const TargetSpec &tset,
+                const winds_bs_params *prm, cudaStream_t s, bool sequential) {
   int model, prec, rc;
   double dcut, n;
   if ((rc = resolve_model(prm, &model, &dcut, &n, &prec))) return rc;
@@ -588,7 +554,7 @@ int eval_device(Context *c, const winds_bs_family *fams, int nfam,
   c->launches = 0;
   long long nf = 0, nt = 0;
   for (int k = 0; k < nfam; ++k) nf += fams[k].dims[0] * fams[k].dims[2] * fams[k].dims[3];
-  for (const TargetSpec &t : tsets) nt += t.count;
+  nt = tset.count;
   // The FP64 path (and the sequential mode that reproduces the reference's
   // order) runs on the input order. FP32c runs on the layout its tuned choice
   // names; the autotuner times both layouts, each with every tiling.
@@ -600,7 +566,7 @@ int eval_device(Context *c, const winds_bs_family *fams, int nfam,
     for (int layout = 0; layout < 2; ++layout) {
       TuneChoice tc;
       float ms = 1e30f;
-      if ((rc = pack_groups(c, fams, nfam, tsets, model, dcut, s, layout == 1, &gs, &nf, &nt)) ||
+      if ((rc = pack_groups(c, fams, nfam, tset, model, dcut, s, layout == 1, &gs, &nf, &nt)) ||
           (rc = autotune(c, gs, model, dcut, n, prm->co, &tc, &ms)))
         return rc;
       tc.chain = layout == 1;
@@ -608,14 +574,19 @@ int eval_device(Context *c, const winds_bs_family *fams, int nfam,
     }
     store_tune(model, nt, nf, ch, true);
   }
-  if ((rc = pack_groups(c, fams, nfam, tsets, model, dcut, s, fast && ch.chain, &gs, &nf, &nt)))
+  if ((rc = pack_groups(c, fams, nfam, tset, model, dcut, s, fast && ch.chain, &gs, &nf, &nt)))
     return rc;
   if (nt == 0) return WINDS_BS_OK;
   return run_direct_sum(c, gs, model, dcut, n, prm->co, prec, sequential, ch, s, true);
 }
 
-// Times each candidate (T, KF, waves) twice after a warm-up on the inputs as
-// packed and returns the fastest with its time.
+// Repeats an autotuner times a candidate for after a warm-up of ms: as many in a
+// row as 300 us hold, 1 to 16. (Runs of 60 us timed one by one differ by 4 us, more
+// than the candidates do.)
+int tune_repeats(float ms) { return std::max(1, std::min(16, (int)(0.3f / std::max(ms, 1e-3f)))); }
+
+// Times each candidate (T, KF, waves) on the inputs as packed and returns the
+// fastest with its time.
 int autotune(Context *c, const std::vector<GroupSpec> &gs, int model, double dcut, double n,
              double co, TuneChoice *best, float *best_ms_out) {
   // T = 8 (supported, settable) is left out: its target balls are too wide
@@ -628,40 +599,38 @@ int autotune(Context *c, const std::vector<GroupSpec> &gs, int model, double dcu
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
-  for (int T : Ts) {
+  int rc = WINDS_BS_OK;
+  for (int T : Ts)
     for (int KF : KFs)
       for (double w : Ws) {
         TuneChoice ch;
         ch.T = T;
         ch.KF = KF;
         ch.waves = w;
-        int rc = run_direct_sum(c, gs, model, dcut, n, co, WINDS_PREC_F32C, false, ch, c->stream,
-                                false);
-        if (rc) return rc;
-        float ms = 1e30f;
-        for (int rep = 0; rep < 2; ++rep) {  // the faster of two timed runs
+        float ms = 0.f;
+        // the candidate's plan, then a warm-up, then the timed runs
+        for (int pass = 0; pass < 3 && !rc; ++pass) {
+          const int reps = pass < 2 ? 1 : tune_repeats(ms);
           cudaEventRecord(e0, c->stream);
-          rc = run_direct_sum(c, gs, model, dcut, n, co, WINDS_PREC_F32C, false, ch, c->stream,
-                              false);
-          if (rc) return rc;
+          for (int k = 0; k < reps && !rc; ++k)
+            rc = run_direct_sum(c, gs, model, dcut, n, co, WINDS_PREC_F32C, false, ch, c->stream,
+                                false);
           cudaEventRecord(e1, c->stream);
-          cudaError_t e = cudaEventSynchronize(e1);
-          if (e != cudaSuccess) return cuda_fail(e, "autotune");
-          float t = 0.f;
-          cudaEventElapsedTime(&t, e0, e1);
-          ms = std::min(ms, t);
+          const cudaError_t e = cudaEventSynchronize(e1);
+          if (!rc && e != cudaSuccess) rc = cuda_fail(e, "autotune");
+          cudaEventElapsedTime(&ms, e0, e1);
+          ms /= (float)reps;
         }
-        if (ms < best_ms) {
+        if (!rc && ms < best_ms) {
           best_ms = ms;
           bc = ch;
         }
       }
-  }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   *best = bc;
   *best_ms_out = best_ms;
-  return WINDS_BS_OK;
+  return rc;
 }
 
 int check_device_error(Context *c, cudaStream_t s) {
@@ -711,7 +680,7 @@ int winds_bs_set_device(int device) {
 }
 
 static int targets_from(const double *P, const long long pdims[4], double *uind,
-                        std::vector<TargetSpec> *ts) {
+                        TargetSpec *ts) {
   if (!pdims) return fail(WINDS_BS_ERR_ARG, "null P dims");
   if (pdims[1] != 3 || pdims[0] < 0 || pdims[2] < 0 || pdims[3] < 0)
     return fail(WINDS_BS_ERR_ARG, "P must be [n,3,m,k] (got [%lld,%lld,%lld,%lld])", pdims[0],
@@ -723,7 +692,7 @@ static int targets_from(const double *P, const long long pdims[4], double *uind,
   t.out = uind;
   t.accumulate = 0;
   if (t.count > 0 && (!P || !uind)) return fail(WINDS_BS_ERR_ARG, "null P or uind");
-  ts->push_back(t);
+  *ts = t;
   return WINDS_BS_OK;
 }
 
@@ -734,13 +703,13 @@ int winds_bs_eval_device(const winds_bs_family *fams, int nfam, const double *P,
   int rc;
   Context *c = get_context(&rc);
   if (!c) return rc;
-  std::vector<TargetSpec> ts;
+  TargetSpec ts;
   if ((rc = targets_from(P, pdims, uind, &ts))) return rc;
   cudaStream_t s = stream ? (cudaStream_t)stream : c->stream;
   const bool seq = prm && (prm->flags & WINDS_BS_FLAG_SEQUENTIAL);
-  if (nfam == 0 || ts[0].count == 0) {
-    if (ts[0].count > 0) {
-      cudaError_t e = cudaMemsetAsync(uind, 0, ts[0].count * 3 * sizeof(double), s);
+  if (nfam == 0 || ts.count == 0) {
+    if (ts.count > 0) {
+      cudaError_t e = cudaMemsetAsync(uind, 0, ts.count * 3 * sizeof(double), s);
       if (e != cudaSuccess) return cuda_fail(e, "zero output");
     }
     return WINDS_BS_OK;
@@ -754,9 +723,9 @@ int winds_bs_eval_host(const winds_bs_family *fams, int nfam, const double *P,
   int rc;
   Context *c = get_context(&rc);
   if (!c) return rc;
-  std::vector<TargetSpec> ts;
+  TargetSpec ts;
   if ((rc = targets_from(P, pdims, uind, &ts))) return rc;
-  const long long np = ts[0].count;
+  const long long np = ts.count;
   cudaStream_t s = c->stream;
   if (np == 0) return WINDS_BS_OK;
   for (int k = 0; k < nfam; ++k)
@@ -796,9 +765,9 @@ int winds_bs_eval_host(const winds_bs_family *fams, int nfam, const double *P,
     base += 8 * n;
   }
   if (e != cudaSuccess) return cuda_fail(e, "host to device copy");
-  std::vector<TargetSpec> dts = ts;
-  dts[0].P = (const double *)c->in_P.p;
-  dts[0].out = (double *)c->out_u.p;
+  TargetSpec dts = ts;
+  dts.P = (const double *)c->in_P.p;
+  dts.out = (double *)c->out_u.p;
   const bool seq = prm && (prm->flags & WINDS_BS_FLAG_SEQUENTIAL);
   if (nfam == 0) {
     e = cudaMemsetAsync(c->out_u.p, 0, np * 3 * sizeof(double), s);

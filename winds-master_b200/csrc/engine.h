@@ -94,12 +94,12 @@ TuneChoice default_choice(long long nt);
 // the evaluation entry points (eval = true: their choice includes the stream
 // layout) and the callers that pack their own unchained stream.
 bool lookup_tune(int model, long long nt, long long nf, TuneChoice *out, bool eval = false);
+int tune_repeats(float ms);
 void store_tune(int model, long long nt, long long nf, const TuneChoice &ch, bool eval = false);
 int cuda_fail(cudaError_t e, const char *what);
 Context *get_context(int *rc);
-int eval_device(Context *c, const winds_bs_family *fams, int nfam,
-                const std::vector<TargetSpec> &tsets, const winds_bs_params *prm, cudaStream_t s,
-                bool sequential);
+int eval_device(Context *c, const winds_bs_family *fams, int nfam, const TargetSpec &tset,
+                const winds_bs_params *prm, cudaStream_t s, bool sequential);
 int autotune(Context *c, const std::vector<GroupSpec> &gs, int model, double dcut, double n,
              double co, TuneChoice *best, float *best_ms);
 int check_device_error(Context *c, cudaStream_t s);

@@ -21,8 +21,14 @@
 
 namespace winds {
 
+// Also the state an iteration starts from: none done, none converged.
 __global__ void kj_targets(const WakeCase *cases, const KJCase *kc, const int *step,
-                           const double *ll, double4 *tp, BBox *bb) {
+                           const double *ll, double4 *tp, BBox *bb, int *iters, int *converged,
+                           int *diverged, int *it_max) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    iters[blockIdx.y] = converged[blockIdx.y] = diverged[blockIdx.y] = 0;
+    if (blockIdx.y == 0) *it_max = 0;
+  }
   const WakeCase c = cases[blockIdx.y];
   const KJCase k = kc[blockIdx.y];
   const int ns = c.nst - 1;
@@ -188,12 +194,14 @@ __global__ void __launch_bounds__(kSolveThreads) kj_solve(const KJSolveArgs a) {
   const WakeCase c = a.cases[ci];
   const KJCase k = a.kc[ci];
   const int s = *a.step;
-  if (s < c.kj_from) return;  // the start-up's first step has no iteration
   const int ns = c.nst - 1, nt = ns * c.nb, n_shed = c.nb * 2 * ns, own = n_shed + c.nb * c.nst;
   const int per = (nt + kCluster - 1) / kCluster;
   const int t0 = rank * per;
   const int cnt = max(0, min(per, nt - t0));
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  for (int tt = tid; tt < cnt; tt += kSolveThreads)  // the start value, kept for the caller
+    a.guess[c.bound_off + t0 + tt] = a.bound[c.bound_off + t0 + tt];
+  if (s < c.kj_from) return;  // the start-up's first step has no iteration
   // shared or (vectors too long for it) global working vectors: the bound
   // iterate and the residual (its bits) of every point, twice; the own circulations; the
   // part of shed column 1 that stays; this CTA's stations (load_station)
@@ -401,10 +409,10 @@ __global__ void kj_finish(const WakeCase *cases, const KJCase *kc, const int *it
 // (uindb, zero before the first step): vblade + [bxn; byn; bzn] uindb, the
 // velocity the first iteration of kj() would see (core/KuttaJoukowski.m:241-249).
 // The history: bound (the last converged value), bound_last and bound_last2
-// (the two before it; equal to bound before there were any).
+// (the two before it; equal to bound before there were any), which move one step
+// on here for the next step's change features.
 __global__ void kj_features(const WakeCase *cases, const KJCase *kc, const int *step,
-                            const double *bound, const double *bound_last,
-                            const double *bound_last2,
+                            const double *bound, double *bound_last, double *bound_last2,
                             const double *vblade, const double *bxn,
                             const double *byn, const double *bzn, const double *uindb,
                             const double *st_r, const double *st_c, const double *st_tw,
@@ -431,9 +439,12 @@ __global__ void kj_features(const WakeCase *cases, const KJCase *kc, const int *
     f[5 + a] = (float)(vblade[fo + a * ns] +
                        (fr[a][fo] * u[0] + fr[a][fo + ns] * u[ns] + fr[a][fo + 2 * ns] * u[2 * ns]));
   const long long q = c.bound_off + i + (long long)ns * b;
-  f[8] = (float)bound[q];
-  f[9] = (float)(bound[q] - bound_last[q]);
-  f[10] = (float)(bound_last[q] - bound_last2[q]);
+  const double g0 = bound[q], g1 = bound_last[q], g2 = bound_last2[q];
+  f[8] = (float)g0;
+  f[9] = (float)(g0 - g1);
+  f[10] = (float)(g1 - g2);
+  bound_last[q] = g0;
+  bound_last2[q] = g1;
 }
 
 // bound = base + out_scale * y, base Gamma_prev or, with *base != 0, its
@@ -532,9 +543,10 @@ __global__ void kj_sum_loads(const WakeCase *cases, const KJCase *kc, int ncases
 }
 
 cudaError_t launch_kj_targets(const WakeCase *cases, const KJCase *kc, int ncases, int max_st,
-                              const int *step, const double *ll, double4 *tp, BBox *bb,
-                              cudaStream_t s) {
-  kj_targets<<<dim3((max_st + 127) / 128, ncases), 128, 0, s>>>(cases, kc, step, ll, tp, bb);
+                              const int *step, const double *ll, double4 *tp, BBox *bb, int *iters,
+                              int *converged, int *diverged, int *it_max, cudaStream_t s) {
+  kj_targets<<<dim3((max_st + 127) / 128, ncases), 128, 0, s>>>(cases, kc, step, ll, tp, bb, iters,
+                                                                converged, diverged, it_max);
   return cudaGetLastError();
 }
 
@@ -579,8 +591,8 @@ cudaError_t launch_kj_finish(const WakeCase *cases, const KJCase *kc, int ncases
 }
 
 cudaError_t launch_kj_features(const WakeCase *cases, const KJCase *kc, int ncases, int max_st,
-                               const int *step, const double *bound, const double *bound_last,
-                               const double *bound_last2, const double *vblade,
+                               const int *step, const double *bound, double *bound_last,
+                               double *bound_last2, const double *vblade,
                                const double *bxn, const double *byn, const double *bzn,
                                const double *uindb, const double *st_r,
                                const double *st_c, const double *st_tw, const double *azim,

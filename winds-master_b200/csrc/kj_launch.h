@@ -29,8 +29,8 @@ struct KJCase {
 constexpr int kKJFeatures = 11;
 
 cudaError_t launch_kj_targets(const WakeCase *cases, const KJCase *kc, int ncases, int max_st,
-                              const int *step, const double *ll, double4 *tp, BBox *bb,
-                              cudaStream_t s);
+                              const int *step, const double *ll, double4 *tp, BBox *bb, int *iters,
+                              int *converged, int *diverged, int *it_max, cudaStream_t s);
 // kj_solve: the whole iteration of every case (kj_kernels.cu). vec_* / mat_*: the
 // working vectors and matrix rows of a CTA in doubles (strides: the largest
 // case's), in shared memory or in a global scratch of stride doubles per CTA,
@@ -48,7 +48,7 @@ struct KJSolveArgs {
   double relax, tol;
   int maxiter, model;
   double d, n, co;
-  double *bound, *uindb, *uindb_conv, *cl_out, *cd_out, *aoa_out;
+  double *bound, *guess, *uindb, *uindb_conv, *cl_out, *cd_out, *aoa_out;
   int *iters, *converged, *diverged, *it_max;
   double *res_last;
   int vec_smem, mat_smem;
@@ -65,8 +65,8 @@ cudaError_t launch_kj_finish(const WakeCase *cases, const KJCase *kc, int ncases
                              const int *iters, const int *converged, const int *it_max,
                              const double *uindb_conv, double *uindb, cudaStream_t s);
 cudaError_t launch_kj_features(const WakeCase *cases, const KJCase *kc, int ncases, int max_st,
-                               const int *step, const double *bound, const double *bound_last,
-                               const double *bound_last2,
+                               const int *step, const double *bound, double *bound_last,
+                               double *bound_last2,
                                const double *vblade, const double *bxn, const double *byn,
                                const double *bzn, const double *uindb, const double *st_r,
                                const double *st_c, const double *st_tw, const double *azim,

@@ -55,11 +55,13 @@ int scratch_address(unsigned char **out) {
 
 // One target set: tile j holds targets [j*tile_cap, ...), item i is tile
 // i / n_chunks against filament chunk i % n_chunks.
-__global__ void bs_noalloc_plan(Group *groups, Tile *tiles, Item *items, double *out,
+// It also clears the error word.
+__global__ void bs_noalloc_plan(Group *groups, Tile *tiles, Item *items, unsigned *err, double *out,
                                 long long nt, long long ns_p, int nf_pad, int tile_cap,
                                 int chunk, int n_chunks, int n_tiles) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i == 0) {
+    *err = 0u;
     Group g;
     g.out = out;
     g.t_begin = 0;
@@ -179,8 +181,7 @@ extern "C" int winds_bs_eval_device_noalloc(const winds_bs_family *fams, int nfa
 
   // ---- carve the scratch array
   size_t sort_bytes = 0;
-  if (sort_target_keys(nullptr, &sort_bytes, nullptr, nullptr, nullptr, nullptr, nt, s) !=
-      cudaSuccess)
+  if (nt > kBlockSortMax && sort_targets_bytes(nt, 1, &sort_bytes) != cudaSuccess)
     return fail(WINDS_BS_ERR_CUDA, "target sort size query failed");
   Carve cv{base};
   BBox *bbox = cv.take<BBox>(1);
@@ -188,15 +189,17 @@ extern "C" int winds_bs_eval_device_noalloc(const winds_bs_family *fams, int nfa
   unsigned *err = cv.take<unsigned>(4);
   unsigned long long *nearc = cv.take<unsigned long long>(2);  // near, core-free pairs
   PackedFilaments pf{cv.take<float4>(nfp * 4), cv.take<double4>(nfp), cv.take<double4>(nfp)};
-  unsigned long long *chaincnt = cv.take<unsigned long long>(2);
-  double4 *tp = cv.take<double4>(nt);
-  double4 *tp_raw = cv.take<double4>(nt);
-  int *tgroup = cv.take<int>(nt);
-  int *vals = cv.take<int>(nt);
-  int *perm = cv.take<int>(nt);
-  unsigned long long *k0 = cv.take<unsigned long long>(nt);
-  unsigned long long *k1 = cv.take<unsigned long long>(nt);
-  void *sort_tmp = cv.take<unsigned char>(sort_bytes);
+  unsigned long long *chaincnt = cv.take<unsigned long long>(2 * kPackFams);
+  TargetBufs tb{};
+  const long long nd = nt > kBlockSortMax ? nt : 0;  // targets of the device-wide sort
+  tb.tp = cv.take<double4>(nt);
+  tb.tp_raw = cv.take<double4>(nd);
+  tb.tgroup = cv.take<int>(nd);
+  tb.vals = cv.take<int>(nd);
+  tb.perm = cv.take<int>(nt);
+  tb.keys = cv.take<unsigned long long>(nd);  // one group: two 32-bit keys each
+  tb.sort_tmp = cv.take<unsigned char>(sort_bytes);
+  tb.sort_bytes = sort_bytes;
   Group *groups = cv.take<Group>(1);
   Tile *tiles = cv.take<Tile>(n_tiles);
   Item *items = cv.take<Item>(n_items);
@@ -205,34 +208,17 @@ extern "C" int winds_bs_eval_device_noalloc(const winds_bs_family *fams, int nfa
     return fail(WINDS_BS_ERR_ARG, "noalloc scratch too small: need %zu of %zu bytes", cv.off,
                 kNoallocBytes);
 
-  // ---- state carried over from the previous call: clear what starts at zero
-  if ((e = cudaMemsetAsync(ctr, 0, 4 * sizeof(unsigned), s)) != cudaSuccess ||
-      (e = cudaMemsetAsync(err, 0, 4 * sizeof(unsigned), s)) != cudaSuccess ||
-      (e = cudaMemsetAsync(nearc, 0, 2 * sizeof(unsigned long long), s)) != cudaSuccess)
-    return cuda_fail(e, "scratch reset");
-
-  // ---- pack (the same kernels as winds_bs_eval_device)
-  e = launch_bbox_init(bbox, s);
-  long long off = 0;
-  for (int k = 0; k < nfam && e == cudaSuccess; ++k) {
-    const long long *d = fams[k].dims;
-    const long long m = d[0] * d[2] * d[3];
-    e = launch_pack_filaments(fams[k].F1, fams[k].F2, fams[k].gamma, fams[k].rc, d, off,
-                              prec == WINDS_PREC_F32C ? chaincnt : nullptr, model, dcut, pf, bbox,
-                              s);
-    off += m;
-  }
-  if (e == cudaSuccess) e = launch_pad_filaments(nf, nfp, pf, s);
-  if (e == cudaSuccess) e = launch_pack_targets(P, pdims[0], nt, 0, 0, tp_raw, tgroup, bbox, s);
-  if (e == cudaSuccess) e = launch_target_keys(tp_raw, tgroup, nt, bbox, k0, vals, s);
-  if (e == cudaSuccess) e = sort_target_keys(sort_tmp, &sort_bytes, k0, k1, vals, perm, nt, s);
-  if (e == cudaSuccess) e = launch_gather_targets(tp_raw, perm, nt, tp, s);
-  if (e == cudaSuccess) {
-    const int grid = (n_items + 255) / 256;
-    bs_noalloc_plan<<<grid, 256, 0, s>>>(groups, tiles, items, uind, nt, pdims[0], (int)nfp,
-                                         tile_cap, (int)chunk, n_chunks, n_tiles);
-    e = cudaGetLastError();
-  }
+  // ---- plan, state carried over from the previous call, and packing (the same
+  // kernels as winds_bs_eval_device)
+  bs_noalloc_plan<<<(n_items + 255) / 256, 256, 0, s>>>(groups, tiles, items, err, uind, nt,
+                                                        pdims[0], (int)nfp, tile_cap, (int)chunk,
+                                                        n_chunks, n_tiles);
+  e = cudaGetLastError();
+  if (e == cudaSuccess) e = launch_begin(bbox, ctr, nearc, chaincnt, s);
+  if (e == cudaSuccess)
+    e = launch_pack_families(fams, nfam, prec == WINDS_PREC_F32C ? chaincnt : nullptr, nfp,
+                             model, dcut, pf, bbox, s, nullptr);
+  if (e == cudaSuccess) e = launch_matlab_targets(P, pdims[0], nt, tb, bbox, s);
   if (e != cudaSuccess) return cuda_fail(e, "noalloc pack/plan kernels");
 
   // ---- direct sum and reduction
@@ -240,7 +226,7 @@ extern "C" int winds_bs_eval_device_noalloc(const winds_bs_family *fams, int nfa
   a.pk = pf.pk;
   a.ra = pf.ra;
   a.rb = pf.rb;
-  a.tp = tp;
+  a.tp = tb.tp;
   a.groups = groups;
   a.tiles = tiles;
   a.items = items;
@@ -259,7 +245,7 @@ extern "C" int winds_bs_eval_device_noalloc(const winds_bs_family *fams, int nfa
   a.wait_limit_ns = default_wait_limit_ns();
   const int grid = worker_grid(n_items, resident, sms, prec != WINDS_PREC_F64);
   e = prec == WINDS_PREC_F64 ? launch_f64(a, grid, s) : launch_f32c(a, model, ch.T, ch.KF, grid, s);
-  if (e == cudaSuccess) e = launch_reduce(tiles, n_tiles, groups, part, perm, tile_cap, s);
+  if (e == cudaSuccess) e = launch_reduce(tiles, n_tiles, groups, part, tb.perm, tile_cap, ctr, s);
   if (e != cudaSuccess) return cuda_fail(e, "noalloc direct-sum launch");
 
   // ---- synchronous: report a device-side timeout recorded in the error word,

@@ -129,17 +129,19 @@ int alloc_all(winds_wake_batch *b) {
   const long long nf = b->fil_pad, nt = std::max<long long>(b->nodes, 1);
   if ((rc = b->pk.ensure(nf * 4 * sizeof(float4), s)) ||
       (rc = b->ra.ensure(nf * sizeof(double4), s)) || (rc = b->rb.ensure(nf * sizeof(double4), s)) ||
-      (rc = b->tp.ensure(nt * sizeof(double4), s)) ||
-      (rc = b->tp_raw.ensure(nt * sizeof(double4), s)) ||
-      (rc = b->tgroup.ensure(nt * sizeof(int), s)) ||
-      (rc = b->keys.ensure(nt * 2 * sizeof(unsigned long long), s)) ||
-      (rc = b->vals.ensure(nt * sizeof(int), s)) || (rc = b->perm.ensure(nt * sizeof(int), s)) ||
+      (rc = b->tp.ensure(nt * sizeof(double4), s)) || (rc = b->perm.ensure(nt * sizeof(int), s)) ||
       (rc = b->bbox.ensure(sizeof(BBox), s)) || (rc = b->ctr.ensure(64, s)) ||
       (rc = b->err.ensure(64, s)) || (rc = b->nearctr.ensure(64, s)))
     return rc;
-  if (sort_target_keys(nullptr, &b->sort_bytes, nullptr, nullptr, nullptr, nullptr, b->nodes, s) !=
-      cudaSuccess)
-    return fail(WINDS_BS_ERR_CUDA, "target sort size query failed");
+  if (b->max_nodes > kBlockSortMax) {
+    if (sort_targets_bytes(b->nodes, b->ncases, &b->sort_bytes) != cudaSuccess)
+      return fail(WINDS_BS_ERR_CUDA, "target sort size query failed");
+    if ((rc = b->tp_raw.ensure(nt * sizeof(double4), s)) ||
+        (rc = b->tgroup.ensure(nt * sizeof(int), s)) ||
+        (rc = b->keys.ensure(nt * (b->ncases == 1 ? 1 : 2) * sizeof(unsigned long long), s)) ||
+        (rc = b->vals.ensure(nt * sizeof(int), s)))
+      return rc;
+  }
   return b->sort_tmp.ensure(b->sort_bytes + 256, s);
 }
 
@@ -214,26 +216,16 @@ cudaError_t enqueue_eval(winds_wake_batch *b, const double *dom, const double *s
                      P<double4>(b->ra), P<double4>(b->rb)};
   BBox *bb = P<BBox>(b->bbox);
   GroupLive *live = P<GroupLive>(live_mode == kLivePredicted ? b->live_pred : b->live_main);
-  cudaError_t e = launch_bbox_init(bb, s);
-  if (e == cudaSuccess) e = launch_wake_live(cd, b->ncases, step, step_add, live_mode, live, s);
+  cudaError_t e = launch_wake_live(cd, b->ncases, step, step_add, live_mode, live, bb,
+                                   P<unsigned>(b->ctr), s);
   if (e == cudaSuccess)
     e = launch_wake_filaments(cd, b->ncases, b->max_fil, step, step_add, P<const double>(b->ser),
                               dom, shed, trail, lold_s, lold_t, have_old, b->prm.stretch, lnew_s,
                               lnew_t, rc_s, rc_t, nullptr, nullptr, b->model, b->dcut, pf, bb, s);
+  TargetBufs tb{P<double4>(b->tp),  P<double4>(b->tp_raw), P<int>(b->tgroup), P<int>(b->vals),
+                P<int>(b->perm),    P<unsigned long long>(b->keys), b->sort_tmp.p, b->sort_bytes};
   if (e == cudaSuccess)
-    e = launch_wake_targets(cd, b->ncases, b->max_nodes, step, step_add, dom,
-                            P<double4>(b->tp_raw), P<int>(b->tgroup), bb, s);
-  unsigned long long *k0 = P<unsigned long long>(b->keys), *k1 = k0 + std::max<long long>(b->nodes, 1);
-  if (e == cudaSuccess)
-    e = launch_target_keys(P<const double4>(b->tp_raw), P<const int>(b->tgroup), b->nodes, bb, k0,
-                           P<int>(b->vals), s);
-  if (e == cudaSuccess)
-    e = sort_target_keys(b->sort_tmp.p, &b->sort_bytes, k0, k1, P<const int>(b->vals),
-                         P<int>(b->perm), b->nodes, s);
-  if (e == cudaSuccess)
-    e = launch_gather_targets(P<const double4>(b->tp_raw), P<const int>(b->perm), b->nodes,
-                              P<double4>(b->tp), s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(b->ctr.p, 0, sizeof(unsigned), s);
+    e = launch_wake_targets(cd, b->ncases, b->max_nodes, b->nodes, step, step_add, dom, tb, bb, s);
   F32cArgs a;
   a.pk = pf.pk;
   a.ra = pf.ra;
@@ -261,9 +253,10 @@ cudaError_t enqueue_eval(winds_wake_batch *b, const double *dom, const double *s
                                   : launch_f32c(a, b->model, b->ch.T, b->ch.KF, b->grid, s);
   if (e == cudaSuccess)
     e = launch_reduce(P<const Tile>(b->tiles), b->n_tiles, P<const Group>(groups),
-                      P<const double>(b->part), P<const int>(b->perm), b->tile_cap, s,
-                      P<const Item>(b->items), live);
-  launches += 13;  // bbox, live, filaments, targets, keys, sort (4), gather, memset, sum, reduce
+                      P<const double>(b->part), P<const int>(b->perm), b->tile_cap,
+                      P<unsigned>(b->ctr), s, P<const Item>(b->items), live);
+  // live, filaments, targets, sum, reduce; the device-wide sort adds 8
+  launches += b->max_nodes <= kBlockSortMax ? 5 : 13;
   return e;
 }
 
@@ -364,36 +357,26 @@ cudaError_t enqueue_step(winds_wake_batch *b, int &launches) {
 // of the filaments that do not follow the bound iterate, and the iteration.
 cudaError_t enqueue_kj(winds_wake_batch *b, int &launches) {
   cudaStream_t s = b->stream;
-  cudaError_t e = launch_bbox_init(P<BBox>(b->bbox), s);
   // the step's live filaments; every lifting-line point is a target
-  if (e == cudaSuccess)
-    e = launch_wake_live(P<const WakeCase>(b->cases_d), b->ncases, P<const int>(b->step_d), 0,
-                         kLiveAll, P<GroupLive>(b->live_kj), s);
+  cudaError_t e = launch_wake_live(P<const WakeCase>(b->cases_d), b->ncases, P<const int>(b->step_d),
+                                   0, kLiveAll, P<GroupLive>(b->live_kj), P<BBox>(b->bbox),
+                                   P<unsigned>(b->ctr), s);
   if (e == cudaSuccess)
     e = launch_kj_targets(P<const WakeCase>(b->cases_d), P<const KJCase>(b->kjc_d), b->ncases,
                           b->max_st, P<const int>(b->step_d), P<const double>(b->ll),
-                          P<double4>(b->tp_ll), P<BBox>(b->bbox), s);
-  for (DevBuf *x : {&b->conv, &b->iters, &b->diverged})
-    if (e == cudaSuccess) e = cudaMemsetAsync(x->p, 0, b->ncases * 8, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(b->kj_it.p, 0, sizeof(int), s);
+                          P<double4>(b->tp_ll), P<BBox>(b->bbox), P<int>(b->iters),
+                          P<int>(b->conv), P<int>(b->diverged), P<int>(b->kj_it), s);
   const WakeCase *cd = P<const WakeCase>(b->cases_d);
   const KJCase *kd = P<const KJCase>(b->kjc_d);
   if (e == cudaSuccess && b->mlp_inputs)
     e = launch_kj_features(cd, kd, b->ncases, b->max_st, P<const int>(b->step_d),
-                           P<const double>(b->bound), P<const double>(b->bound_last),
-                           P<const double>(b->bound_last2), P<const double>(b->vblade),
+                           P<const double>(b->bound), P<double>(b->bound_last),
+                           P<double>(b->bound_last2), P<const double>(b->vblade),
                            P<const double>(b->bxn), P<const double>(b->byn),
                            P<const double>(b->bzn), P<const double>(b->uindb),
                            P<const double>(b->st_r), P<const double>(b->st_c),
                            P<const double>(b->st_tw), P<const double>(b->azim), P<float>(b->feat),
                            s);
-  // the history one step on, for the next step's change features
-  if (e == cudaSuccess && b->mlp_inputs)
-    e = cudaMemcpyAsync(b->bound_last2.p, b->bound_last.p, b->bound_n * sizeof(double),
-                        cudaMemcpyDeviceToDevice, s);
-  if (e == cudaSuccess && b->mlp_inputs)
-    e = cudaMemcpyAsync(b->bound_last.p, b->bound.p, b->bound_n * sizeof(double),
-                        cudaMemcpyDeviceToDevice, s);
   if (e == cudaSuccess && b->mlp) {
     // start value Gamma_prev + out_scale * network(features)
     e = launch_mlp_prep(P<float>(b->feat), b->n_ll, kKJFeatures, mlp_shift_dev(b->mlp),
@@ -409,9 +392,6 @@ cudaError_t enqueue_kj(winds_wake_batch *b, int &launches) {
                                 P<const float>(b->feat), mlp_base_dev(b->mlp), P<double>(b->bound),
                                 s);
   }
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(b->guess.p, b->bound.p, b->bound_n * sizeof(double),
-                        cudaMemcpyDeviceToDevice, s);
   // every filament at the step's positions with the step's cores held fixed (as
   // kj() does); Γ of the columns that do not follow the bound iterate is the
   // bookkeeping's of this step
@@ -423,7 +403,6 @@ cudaError_t enqueue_kj(winds_wake_batch *b, int &launches) {
                               nullptr, 0, 0, nullptr, nullptr, nullptr, nullptr,
                               P<const double>(b->rc_s), P<const double>(b->rc_t), b->model,
                               b->dcut, pf, P<BBox>(b->bbox), s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(b->ctr.p, 0, sizeof(unsigned), s);
   F32cArgs a;
   a.pk = pf.pk;
   a.ra = pf.ra;
@@ -452,8 +431,9 @@ cudaError_t enqueue_kj(winds_wake_batch *b, int &launches) {
             : launch_f32c(a, b->model, b->kj_T, b->kj_KF, b->kj_grid, s);
   if (e == cudaSuccess)
     e = launch_reduce(P<const Tile>(b->kj_tiles), b->kj_ntiles, P<const Group>(b->kj_groups),
-                      P<const double>(b->kj_part), P<const int>(b->perm_ll), b->kj_tile_cap, s,
-                      P<const Item>(b->kj_items), P<const GroupLive>(b->live_kj));
+                      P<const double>(b->kj_part), P<const int>(b->perm_ll), b->kj_tile_cap,
+                      P<unsigned>(b->ctr), s, P<const Item>(b->kj_items),
+                      P<const GroupLive>(b->live_kj));
   KJSolveArgs q;
   std::memset(&q, 0, sizeof(q));
   q.cases = cd, q.kc = kd, q.step = P<const int>(b->step_d);
@@ -468,7 +448,7 @@ cudaError_t enqueue_kj(winds_wake_batch *b, int &launches) {
   q.cd_t = P<const double>(b->cd_t);
   q.relax = b->kjp.relax, q.tol = b->kjp.tol, q.maxiter = b->kjp.maxiter;
   q.model = b->model, q.d = b->dcut, q.n = b->nidx, q.co = b->prm.co;
-  q.bound = P<double>(b->bound), q.uindb = P<double>(b->uindb);
+  q.bound = P<double>(b->bound), q.guess = P<double>(b->guess), q.uindb = P<double>(b->uindb);
   q.uindb_conv = P<double>(b->uindb_conv);
   q.cl_out = P<double>(b->cl_o), q.cd_out = P<double>(b->cd_o), q.aoa_out = P<double>(b->aoa_o);
   q.iters = P<int>(b->iters), q.converged = P<int>(b->conv), q.diverged = P<int>(b->diverged);
@@ -481,7 +461,7 @@ cudaError_t enqueue_kj(winds_wake_batch *b, int &launches) {
   if (e == cudaSuccess)
     e = launch_kj_finish(cd, kd, b->ncases, b->max_st, q.iters, q.converged, q.it_max,
                          q.uindb_conv, q.uindb, s);
-  launches += 8 + (b->mlp_inputs ? 1 : 0);
+  launches += 7 + (b->mlp_inputs ? 1 : 0);
   return e;
 }
 
@@ -755,6 +735,8 @@ static int autotune_batch(winds_wake_batch *b) {
   if (!c) return rc;
   b->tuned = true;
   if (!c->autotune) return build_plans(b);
+  // another batch of this size may have been timed since this one was made
+  if (lookup_tune(b->model, b->nodes, b->fil_pad, &b->ch)) return build_plans(b);
   cudaStream_t s = b->stream;
   cudaError_t e = launch_wake_bookkeep(P<const WakeCase>(b->cases_d), b->ncases, b->max_cols,
                                        P<const int>(b->step_d), 0, P<const double>(b->bound),
@@ -772,17 +754,20 @@ static int autotune_batch(winds_wake_batch *b) {
         b->ch.T = T, b->ch.KF = KF, b->ch.waves = w;
         if ((rc = build_plans(b))) break;
         float ms = 0.f;
-        for (int rep = 0; rep < 2 && e == cudaSuccess; ++rep) {  // warm-up, then timed
+        for (int pass = 0; pass < 2 && e == cudaSuccess; ++pass) {  // warm-up, then timed
           int l = 0;
+          const int reps = pass == 0 ? 1 : tune_repeats(ms);
           cudaEventRecord(e0, s);
-          e = enqueue_eval(b, P<const double>(b->dom), P<const double>(b->shed_cur),
-                           P<const double>(b->trail_cur), 0, P<const double>(b->len_old_s),
-                           P<const double>(b->len_old_t), 1, P<double>(b->len_s),
-                           P<double>(b->len_t), P<double>(b->rc_s), P<double>(b->rc_t),
-                           b->groups_main, l);
+          for (int k = 0; k < reps && e == cudaSuccess; ++k)
+            e = enqueue_eval(b, P<const double>(b->dom), P<const double>(b->shed_cur),
+                             P<const double>(b->trail_cur), 0, P<const double>(b->len_old_s),
+                             P<const double>(b->len_old_t), 1, P<double>(b->len_s),
+                             P<double>(b->len_t), P<double>(b->rc_s), P<double>(b->rc_t),
+                             b->groups_main, l);
           cudaEventRecord(e1, s);
           if (e == cudaSuccess) e = cudaEventSynchronize(e1);
           cudaEventElapsedTime(&ms, e0, e1);
+          ms /= (float)reps;
         }
         if (e != cudaSuccess) break;
         if (ms < best_ms) best_ms = ms, best = b->ch;

@@ -20,6 +20,7 @@
 // connected filaments that the direct sum follows), so the live ones are the
 // first of the case's range.
 #include "bs_device.cuh"
+#include "bs_sort.cuh"
 #include "wake_launch.h"
 #include "wake_types.h"
 
@@ -346,8 +347,11 @@ __global__ void wake_commit(const WakeCase *cases, int *step, double *dom, const
 // filament pad; as targets (mode kLiveNodes) the nodes of that step's live
 // columns, (kLivePredicted) the same but none before the pcc corrector starts
 // (pcc.m:40), (kLiveAll) every target of the group (lifting-line points).
+// The first kernel of an evaluation: block 0 also empties the bounding box and
+// puts the work queue at its start.
 __global__ void wake_live(const WakeCase *cases, int ncases, const int *step, int step_add,
-                          int mode, GroupLive *live) {
+                          int mode, GroupLive *live, BBox *bb, unsigned *ctr) {
+  if (blockIdx.x == 0) begin_evaluation(bb, ctr);
   const int ci = blockIdx.x * blockDim.x + threadIdx.x;
   if (ci >= ncases) return;
   const WakeCase c = cases[ci];
@@ -393,12 +397,35 @@ cudaError_t launch_wake_filaments(const WakeCase *cases, int ncases, long long m
   return cudaGetLastError();
 }
 
+// The nodes of one case per group (bs_sort_targets): as wake_targets.
+struct WakeTargets {
+  const WakeCase *cases;
+  const int *step;
+  int step_add;
+  const double *dom;
+  __device__ int count(int g) const { return cases[g].nst * cases[g].na * cases[g].nb; }
+  __device__ long long offset(int g) const { return cases[g].node_off; }
+  __device__ bool load(int g, int t, double p[3]) const {
+    const int nst = cases[g].nst, na = cases[g].na;
+    const int jk = t / nst, i = t - jk * nst;
+    if (jk % na >= live_cols(cases[g], *step + step_add)) return false;
+    const double *q = dom + cases[g].node_off * 3 + i + nst * 3 * (long long)jk;
+    p[0] = q[0], p[1] = q[nst], p[2] = q[2 * nst];
+    return true;
+  }
+};
+
 cudaError_t launch_wake_targets(const WakeCase *cases, int ncases, long long max_nodes,
-                                const int *step, int step_add, const double *dom, double4 *tp,
-                                int *tgroup, BBox *bb, cudaStream_t s) {
-  wake_targets<<<case_grid(max_nodes, ncases, 256), 256, 0, s>>>(cases, step, step_add, dom, tp,
-                                                                  tgroup, bb);
-  return cudaGetLastError();
+                                long long nodes, const int *step, int step_add, const double *dom,
+                                const TargetBufs &b, BBox *bb, cudaStream_t s) {
+  if (max_nodes <= kBlockSortMax) {
+    WakeTargets src{cases, step, step_add, dom};
+    return launch_block_sort(src, ncases, max_nodes, b.tp, b.perm, bb, s);
+  }
+  wake_targets<<<case_grid(max_nodes, ncases, 256), 256, 0, s>>>(cases, step, step_add, dom,
+                                                                  b.tp_raw, b.tgroup, bb);
+  const cudaError_t e = cudaGetLastError();
+  return e != cudaSuccess ? e : launch_sort_targets(b, nodes, ncases, bb, s);
 }
 
 cudaError_t launch_wake_convect(const WakeCase *cases, int ncases, long long max_nodes,
@@ -425,8 +452,8 @@ cudaError_t launch_wake_commit(const WakeCase *cases, int ncases, long long max_
 }
 
 cudaError_t launch_wake_live(const WakeCase *cases, int ncases, const int *step, int step_add,
-                             int mode, GroupLive *live, cudaStream_t s) {
-  wake_live<<<(ncases + 127) / 128, 128, 0, s>>>(cases, ncases, step, step_add, mode, live);
+                             int mode, GroupLive *live, BBox *bb, unsigned *ctr, cudaStream_t s) {
+  wake_live<<<(ncases + 127) / 128, 128, 0, s>>>(cases, ncases, step, step_add, mode, live, bb, ctr);
   return cudaGetLastError();
 }
 

@@ -39,12 +39,15 @@ cudaError_t launch_wake_filaments(const WakeCase *cases, int ncases, long long m
                                   double *rc_t, const double *rc_in_s, const double *rc_in_t,
                                   int model, double dcut, const PackedFilaments &pf, BBox *bb,
                                   cudaStream_t s);
+// The nodes of every case sorted for the direct sum (max_nodes: the largest
+// case's, nodes: all).
 cudaError_t launch_wake_targets(const WakeCase *cases, int ncases, long long max_nodes,
-                                const int *step, int step_add, const double *dom, double4 *tp,
-                                int *tgroup, BBox *bb, cudaStream_t s);
-// live[case] for one evaluation of step *step + step_add (WakeLiveMode).
+                                long long nodes, const int *step, int step_add, const double *dom,
+                                const TargetBufs &b, BBox *bb, cudaStream_t s);
+// live[case] for one evaluation of step *step + step_add (WakeLiveMode); the
+// evaluation's first kernel (empties bb, puts the work queue's ctr at its start).
 cudaError_t launch_wake_live(const WakeCase *cases, int ncases, const int *step, int step_add,
-                             int mode, GroupLive *live, cudaStream_t s);
+                             int mode, GroupLive *live, BBox *bb, unsigned *ctr, cudaStream_t s);
 cudaError_t launch_wake_convect(const WakeCase *cases, int ncases, long long max_nodes,
                                 const int *step, int mode, const double *dom, const double *uind,
                                 const double *carry, const double *pred, const double *uind_pred,
