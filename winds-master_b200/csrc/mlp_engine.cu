@@ -68,6 +68,14 @@ int ksplit_for(long long n) {
   return (int)ks;
 }
 
+// Host to device on the model's stream: a plain cudaMemcpy from pageable memory
+// may return before the data is on the device, and kernels on a non-blocking
+// stream do not wait for it. src outlives the copy's staging, as the callers
+// synchronise before they let go of it.
+cudaError_t upload(void *dst, const void *src, size_t bytes, cudaStream_t s) {
+  return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s);
+}
+
 MlpGemmArgs gemm_args(const winds_mlp *m) {
   MlpGemmArgs g;
   std::memset(&g, 0, sizeof(g));
@@ -298,15 +306,14 @@ int winds_mlp_create(const winds_mlp_config *cfg, winds_mlp **out) {
   std::normal_distribution<double> nd5(0.0, 1.0 / std::sqrt((double)W));
   for (int j = 0; j < W; ++j) th[kOffW5 + j] = (float)nd5(gen);
   for (int i = 0; i < 16; ++i) m->h_shift[i] = 0.f, m->h_scale[i] = 1.f;
-  e = cudaMemcpy(m->theta.p, th.data(), kNParam * 4, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(m->shift.p, m->h_shift, 64, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(m->scale.p, m->h_scale, 64, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess)
-    e = cudaMemcpy(P<float>(m->scale) + 16, &m->out_scale, 4, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemset(P<float>(m->scale) + 17, 0, 4);  // base 0
-  if (e == cudaSuccess) e = cudaMemset(m->mom.p, 0, kNParam * 4);
-  if (e == cudaSuccess) e = cudaMemset(m->vel.p, 0, kNParam * 4);
-  if (e == cudaSuccess) e = cudaMemset(m->err.p, 0, 16);
+  e = upload(m->theta.p, th.data(), kNParam * 4, s);
+  if (e == cudaSuccess) e = upload(m->shift.p, m->h_shift, 64, s);
+  if (e == cudaSuccess) e = upload(m->scale.p, m->h_scale, 64, s);
+  if (e == cudaSuccess) e = upload(P<float>(m->scale) + 16, &m->out_scale, 4, s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(P<float>(m->scale) + 17, 0, 4, s);  // base 0
+  if (e == cudaSuccess) e = cudaMemsetAsync(m->mom.p, 0, kNParam * 4, s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(m->vel.p, 0, kNParam * 4, s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(m->err.p, 0, 16, s);
   if (e == cudaSuccess) e = launch_mlp_to_bf16(P<float>(m->theta), P<__nv_bfloat16>(m->theta_bf), kNParam, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) {
@@ -334,7 +341,7 @@ int winds_mlp_set_params(winds_mlp *m, const float *theta) {
   std::vector<float> th(theta, theta + kNParam);
   for (int o = 0; o < W; ++o)  // padded inputs of layer 1 stay zero
     for (int i = m->n_in; i < kMlpInPad; ++i) th[kOffW[0] + (long long)o * kMlpInPad + i] = 0.f;
-  cudaError_t e = cudaMemcpy(m->theta.p, th.data(), kNParam * 4, cudaMemcpyHostToDevice);
+  cudaError_t e = upload(m->theta.p, th.data(), kNParam * 4, m->stream);
   if (e == cudaSuccess)
     e = launch_mlp_to_bf16(P<float>(m->theta), P<__nv_bfloat16>(m->theta_bf), kNParam, m->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(m->mom.p, 0, kNParam * 4, m->stream);
@@ -354,9 +361,10 @@ int winds_mlp_set_scaling(winds_mlp *m, const float *shift, const float *scale, 
   }
   m->out_scale = out_scale;
   cudaStreamSynchronize(m->stream);
-  cudaError_t e = cudaMemcpy(m->shift.p, m->h_shift, 64, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(m->scale.p, m->h_scale, 64, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(P<float>(m->scale) + 16, &out_scale, 4, cudaMemcpyHostToDevice);
+  cudaError_t e = upload(m->shift.p, m->h_shift, 64, m->stream);
+  if (e == cudaSuccess) e = upload(m->scale.p, m->h_scale, 64, m->stream);
+  if (e == cudaSuccess) e = upload(P<float>(m->scale) + 16, &out_scale, 4, m->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(m->stream);
   return e == cudaSuccess ? WINDS_BS_OK : cuda_fail(e, "mlp scaling");
 }
 
@@ -366,7 +374,8 @@ int winds_mlp_set_base(winds_mlp *m, int base) {
   cudaSetDevice(m->dev);
   cudaStreamSynchronize(m->stream);
   const float f = (float)base;
-  cudaError_t e = cudaMemcpy(P<float>(m->scale) + 17, &f, 4, cudaMemcpyHostToDevice);
+  cudaError_t e = upload(P<float>(m->scale) + 17, &f, 4, m->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(m->stream);
   if (e != cudaSuccess) return cuda_fail(e, "mlp base");
   m->base = base;
   return WINDS_BS_OK;
@@ -451,7 +460,7 @@ int winds_mlp_train_host(winds_mlp *m, const float *x, const float *t, long long
   float total_ms = 0.f;
   for (int ep = 0; ep < p->epochs; ++ep) {
     std::shuffle(perm.begin(), perm.end(), gen);
-    e = cudaMemcpy(m->idx.p, perm.data(), n * 4, cudaMemcpyHostToDevice);
+    e = upload(m->idx.p, perm.data(), n * 4, s);
     if (e != cudaSuccess) return cuda_fail(e, "mlp shuffle upload");
     cudaEventRecord(m->e0, s);
     for (long long b = 0; b < nbatch; ++b) {

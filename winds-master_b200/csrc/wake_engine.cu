@@ -197,7 +197,9 @@ int build_plans(winds_wake_batch *b) {
       (e = cudaMemcpy(b->items.p, pl.items.data(), pl.items.size() * sizeof(Item),
                       cudaMemcpyHostToDevice)) != cudaSuccess ||
       (e = cudaMemcpy(b->order.p, pl.order.data(), pl.order.size() * sizeof(int),
-                      cudaMemcpyHostToDevice)) != cudaSuccess)
+                      cudaMemcpyHostToDevice)) != cudaSuccess ||
+      // the batch's stream does not wait for copies from pageable memory
+      (e = cudaStreamSynchronize(cudaStreamLegacy)) != cudaSuccess)
     return cuda_fail(e, "wake plan upload");
   return WINDS_BS_OK;
 }
@@ -694,6 +696,8 @@ int winds_wake_create(const winds_wake_case *cases, int ncases, const winds_wake
   // no previous lengths yet: copying the initial lengths makes the first strain zero
   if (e == cudaSuccess) e = cudaMemset(b->step_d.p, 0, 4 * sizeof(int));
   if (e == cudaSuccess) e = cudaMemset(b->err.p, 0, 64);
+  // the batch's stream does not wait for copies from pageable memory or memsets
+  if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
   if (e != cudaSuccess) {
     winds_wake_destroy(b);
     return cuda_fail(e, "wake upload");
@@ -712,7 +716,7 @@ int winds_wake_create(const winds_wake_case *cases, int ncases, const winds_wake
                         P<double>(b->len_old_t), nullptr, nullptr, b->groups_pred, l);
     if (e2 == cudaSuccess) e2 = cudaStreamSynchronize(b->stream);
     // that evaluation wrote the predicted-induction buffer: no carry at step 0
-    if (e2 == cudaSuccess) e2 = cudaMemset(b->uind_pred.p, 0, n3);
+    if (e2 == cudaSuccess) e2 = cudaMemsetAsync(b->uind_pred.p, 0, n3, b->stream);
     if (e2 != cudaSuccess) {
       winds_wake_destroy(b);
       return cuda_fail(e2, "wake initial lengths");
@@ -1204,7 +1208,8 @@ int winds_wake_set_kj(winds_wake_batch *b, const winds_kj_case *kj, const winds_
   if ((e = cudaMemcpy(b->kj_groups.p, pl.groups.data(), pl.groups.size() * sizeof(Group), cudaMemcpyHostToDevice)) != cudaSuccess ||
       (e = cudaMemcpy(b->kj_tiles.p, pl.tiles.data(), pl.tiles.size() * sizeof(Tile), cudaMemcpyHostToDevice)) != cudaSuccess ||
       (e = cudaMemcpy(b->kj_items.p, pl.items.data(), pl.items.size() * sizeof(Item), cudaMemcpyHostToDevice)) != cudaSuccess ||
-      (e = cudaMemcpy(b->kj_order.p, pl.order.data(), pl.order.size() * sizeof(int), cudaMemcpyHostToDevice)) != cudaSuccess)
+      (e = cudaMemcpy(b->kj_order.p, pl.order.data(), pl.order.size() * sizeof(int), cudaMemcpyHostToDevice)) != cudaSuccess ||
+      (e = cudaStreamSynchronize(cudaStreamLegacy)) != cudaSuccess)
     return cuda_fail(e, "lifting-line plan upload");
   // graphs captured without the iteration must be rebuilt
   if (b->exec) {
