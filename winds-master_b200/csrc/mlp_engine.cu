@@ -1,14 +1,10 @@
 // mlp_engine.cu -- host side of the bound-circulation MLP: parameters,
 // forward / backward launch sequences, Adam training, C ABI (winds_mlp.h).
 //
-// One training step on a batch of n rows (15 launches):
-//   forward   4 x GEMM (bias + GELU epilogue, pre-activations kept), head
-//   backward  head (loss, dz4 and the output-layer partial sums), then for
-//             layers 4, 3, 2: weight-gradient GEMM (split over rows) and
-//             input-gradient GEMM (GELU' epilogue with bias-gradient column
-//             sums); layer 1: weight-gradient GEMM; one reduction of every
-//             partial sum in a fixed order (deterministic)
-//   update    Adam on the FP32 master vector, BF16 copy for the GEMMs
+// One training step on a batch of n rows is two launches: mlp_net (forward and
+// backward of every 128 rows, gradients summed per CTA) and mlp_update (the
+// CTAs' gradients summed in order, which keeps the result deterministic, and
+// Adam on the FP32 master vector with its BF16 copy). Inference is one.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -22,10 +18,11 @@
 struct winds_mlp {
   int dev = 0;
   int n_in = 0;
+  int sms = 0;
   cudaStream_t stream = nullptr;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
-  winds::DevBuf theta, theta_bf, grad, mom, vel, shift, scale, err, jobs, loss, lossbuf, idx;
-  winds::DevBuf Xall, Tall, xall_raw;
+  winds::DevBuf theta, theta_bf, grad, mom, vel, shift, scale, err, loss, lossbuf, idx;
+  winds::DevBuf Xall, Tall;
   float out_scale = 1.f;
   int base = 0;  // start value the output is added to (winds_mlp_set_base)
   float h_shift[16], h_scale[16];
@@ -39,15 +36,8 @@ namespace winds {
 namespace {
 
 constexpr int W = kMlpWidth;
-constexpr int kHeadRows = 64;  // rows per block of the head's backward kernel
-
-// Offsets in the parameter vector.
-constexpr long long kOffW[4] = {0, 2176, 18688, 35200};
-constexpr long long kOffB[4] = {2048, 18560, 35072, 51584};
-constexpr long long kOffW5 = 51712;
-constexpr long long kOffB5 = 51840;
-constexpr long long kNParam = 51841;
-constexpr int kInK[4] = {kMlpInPad, W, W, W};  // input width of each GEMM layer
+constexpr long long kNParam = kMlpNParam;
+constexpr int kInK[4] = {kMlpInPad, W, W, W};  // input width of each layer
 
 template <class T>
 T *P(DevBuf &b) {
@@ -60,14 +50,6 @@ const T *P(const DevBuf &b) {
 
 long long cdiv(long long a, long long b) { return (a + b - 1) / b; }
 
-int ksplit_for(long long n) {
-  const long long chunks = cdiv(n, 64);
-  long long ks = chunks / 4;
-  if (ks < 1) ks = 1;
-  if (ks > 256) ks = 256;
-  return (int)ks;
-}
-
 // Host to device on the model's stream: a plain cudaMemcpy from pageable memory
 // may return before the data is on the device, and kernels on a non-blocking
 // stream do not wait for it. src outlives the copy's staging, as the callers
@@ -76,9 +58,16 @@ cudaError_t upload(void *dst, const void *src, size_t bytes, cudaStream_t s) {
   return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s);
 }
 
-MlpGemmArgs gemm_args(const winds_mlp *m) {
-  MlpGemmArgs g;
+MlpNetArgs net_args(const winds_mlp *m, const float *x, long long n) {
+  MlpNetArgs g;
   std::memset(&g, 0, sizeof(g));
+  g.x = x;
+  g.shift = static_cast<const float *>(m->shift.p);
+  g.scale = static_cast<const float *>(m->scale.p);
+  g.n_in = m->n_in;
+  g.n = n;
+  g.theta = static_cast<const float *>(m->theta.p);
+  g.wbf = static_cast<const __nv_bfloat16 *>(m->theta_bf.p);
   g.err = static_cast<unsigned *>(m->err.p);
   g.wait_limit_ns = default_wait_limit_ns();
   return g;
@@ -96,164 +85,70 @@ int check_err(winds_mlp *m) {
   return WINDS_BS_OK;
 }
 
-// Backward pass of the rows the last forward (with train) ran on, targets t:
-// gradient into m->grad, 0.5 * mean squared error into m->loss.
-int mlp_backward(winds_mlp *m, const __nv_bfloat16 *X, const float *t, long long n, MlpWork &w,
-                 cudaStream_t s) {
-  const float *theta = P<float>(m->theta);
-  const __nv_bfloat16 *wbf = P<__nv_bfloat16>(m->theta_bf);
-  const int nb_head = (int)cdiv(n, kHeadRows);
-  const int nb_rows = (int)cdiv(n, 128);
-  const int ks = ksplit_for(n);
-  cudaError_t e = launch_mlp_head_bwd(P<float>(w.y), t, P<float>(w.Z[3]), P<__nv_bfloat16>(w.A[3]),
-                                      theta + kOffW5, n, (float)(1.0 / (double)n),
-                                      P<__nv_bfloat16>(w.dZa), P<float>(w.dw5p),
-                                      P<float>(w.part_b[3]), P<float>(w.db5p), P<float>(w.lossp),
-                                      kHeadRows, s);
-  __nv_bfloat16 *dz = P<__nv_bfloat16>(w.dZa), *dz_next = P<__nv_bfloat16>(w.dZb);
-  for (int L = 3; L >= 0 && e == cudaSuccess; --L) {
-    // weight gradient: dW_L[out][in] = sum_rows dz[row][out] * a_{L-1}[row][in]
-    MlpGemmArgs g = gemm_args(m);
-    g.A = dz;
-    g.lda = W;
-    g.a_mn = 1;
-    g.B = L > 0 ? P<__nv_bfloat16>(w.A[L - 1]) : X;
-    g.ldb = kInK[L];
-    g.b_mn = 1;
-    g.M = W;
-    g.K = n;
-    g.out_f32 = P<float>(w.part_w[L]);
-    g.ldo = kInK[L];
-    e = launch_mlp_gemm(g, kInK[L], kEpiPartial, ks, s);
-    if (L == 0 || e != cudaSuccess) break;
-    // input gradient through GELU: dz_{L-1} = (dz W_L) * gelu'(z_{L-1})
-    MlpGemmArgs h = gemm_args(m);
-    h.A = dz;
-    h.lda = W;
-    h.a_mn = 0;
-    h.B = wbf + kOffW[L];
-    h.ldb = W;
-    h.b_mn = 1;
-    h.M = n;
-    h.K = W;
-    h.z_in = P<float>(w.Z[L - 1]);
-    h.dz_out = dz_next;
-    h.colsum_part = P<float>(w.part_b[L - 1]);
-    h.ldo = W;
-    e = launch_mlp_gemm(h, W, kEpiGeluBwd, 1, s);
-    std::swap(dz, dz_next);
-  }
-  if (e != cudaSuccess) return cuda_fail(e, "mlp backward");
-  float *grad = P<float>(m->grad);
-  std::vector<MlpReduceJob> jobs;
-  for (int L = 0; L < 4; ++L) {
-    jobs.push_back({P<float>(w.part_w[L]), ks, W * kInK[L], grad + kOffW[L], 1.f});
-    jobs.push_back({P<float>(w.part_b[L]), L == 3 ? nb_head : nb_rows, W, grad + kOffB[L], 1.f});
-  }
-  jobs.push_back({P<float>(w.dw5p), nb_head, W, grad + kOffW5, 1.f});
-  jobs.push_back({P<float>(w.db5p), nb_head, 1, grad + kOffB5, 1.f});
-  jobs.push_back({P<float>(w.lossp), nb_head, 1, P<float>(m->loss), (float)(0.5 / (double)n)});
-  e = cudaMemcpyAsync(m->jobs.p, jobs.data(), jobs.size() * sizeof(MlpReduceJob),
-                      cudaMemcpyHostToDevice, s);
-  if (e == cudaSuccess) e = launch_mlp_reduce(P<MlpReduceJob>(m->jobs), (int)jobs.size(), W * W, s);
-  // the host vector must outlive the (pageable, staged) copy
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  return e == cudaSuccess ? WINDS_BS_OK : cuda_fail(e, "mlp gradient reduction");
+// Gradient of the rows x (those of idx, when given) with targets t, in parts for
+// launch_mlp_update(u) to sum, which puts 0.5 * mean squared error in loss.
+int gradient(winds_mlp *m, const float *x, const float *t, const int *idx, long long n, float *loss,
+             MlpUpdateArgs *u, cudaStream_t s) {
+  MlpNetArgs g = net_args(m, x, n);
+  g.t = t;
+  g.idx = idx;
+  g.inv_n = (float)(1.0 / (double)n);
+  const int tiles = mlp_tiles(n);
+  g.part_w = P<float>(m->w.part);
+  g.part_b = g.part_w + (tiles + 1) / 2 * kMlpPartW;
+  g.part_h = g.part_b + tiles * 3LL * W;
+  std::memset(u, 0, sizeof(*u));
+  u->part_w = g.part_w, u->part_b = g.part_b, u->part_h = g.part_h;
+  u->tiles = tiles;
+  u->loss = loss;
+  u->loss_scale = (float)(0.5 / (double)n);
+  const cudaError_t e = launch_mlp_gradient(g, s);
+  return e == cudaSuccess ? WINDS_BS_OK : cuda_fail(e, "mlp gradient");
 }
 
-int adam_step(winds_mlp *m, const winds_mlp_train_params &p, cudaStream_t s) {
-  ++m->adam_t;
-  const double c1 = 1.0 - std::pow((double)p.beta1, (double)m->adam_t);
-  const double c2 = 1.0 - std::pow((double)p.beta2, (double)m->adam_t);
-  cudaError_t e = launch_mlp_adam(P<float>(m->theta), P<__nv_bfloat16>(m->theta_bf),
-                                  P<float>(m->grad), P<float>(m->mom), P<float>(m->vel), kNParam,
-                                  p.lr, p.beta1, p.beta2, p.eps, p.weight_decay, (float)c1,
-                                  (float)c2, s);
-  return e == cudaSuccess ? WINDS_BS_OK : cuda_fail(e, "mlp adam");
-}
-
-int upload_inputs(winds_mlp *m, const float *x, long long n, MlpWork &w, cudaStream_t s) {
-  cudaError_t e = cudaMemcpyAsync(w.xraw.p, x, (size_t)n * m->n_in * sizeof(float),
-                                  cudaMemcpyHostToDevice, s);
-  if (e == cudaSuccess)
-    e = launch_mlp_prep(P<float>(w.xraw), n, m->n_in, P<float>(m->shift), P<float>(m->scale),
-                        P<__nv_bfloat16>(w.X), s);
+int upload_inputs(winds_mlp *m, const float *x, long long n, cudaStream_t s) {
+  const cudaError_t e = upload(m->w.xraw.p, x, (size_t)n * m->n_in * sizeof(float), s);
   return e == cudaSuccess ? WINDS_BS_OK : cuda_fail(e, "mlp input upload");
+}
+
+int adam_step(winds_mlp *m, const winds_mlp_train_params &p, MlpUpdateArgs u, cudaStream_t s) {
+  ++m->adam_t;
+  u.theta = P<float>(m->theta);
+  u.theta_bf = P<__nv_bfloat16>(m->theta_bf);
+  u.m = P<float>(m->mom);
+  u.v = P<float>(m->vel);
+  u.lr = p.lr, u.b1 = p.beta1, u.b2 = p.beta2, u.eps = p.eps, u.wd = p.weight_decay;
+  u.c1 = (float)(1.0 - std::pow((double)p.beta1, (double)m->adam_t));
+  u.c2 = (float)(1.0 - std::pow((double)p.beta2, (double)m->adam_t));
+  const cudaError_t e = launch_mlp_update(u, s);
+  return e == cudaSuccess ? WINDS_BS_OK : cuda_fail(e, "mlp adam");
 }
 
 }  // namespace
 
-int MlpWork::ensure(long long n, bool tr, cudaStream_t s) {
-  if (n <= cap && (train || !tr)) return WINDS_BS_OK;
-  const long long c = n > cap ? n : cap;
-  const bool t2 = tr || train;
+int MlpWork::ensure_parts(long long n, cudaStream_t s) {
+  const long long tiles = mlp_tiles(n);
+  return part.ensure(((tiles + 1) / 2 * kMlpPartW + tiles * (3 * W + 2 * kMlpPartHead)) * sizeof(float), s);
+}
+
+int MlpWork::ensure(long long n, bool train, cudaStream_t s) {
   int rc;
-  if ((rc = X.ensure(c * kMlpInPad * 2, s)) || (rc = t.ensure(c * 4, s)) ||
-      (rc = y.ensure(c * 4, s)) || (rc = xraw.ensure(c * 16 * 4, s)))
+  if ((rc = t.ensure(n * 4, s)) || (rc = y.ensure(n * 4, s)) || (rc = xraw.ensure(n * 16 * 4, s)))
     return rc;
-  for (int L = 0; L < 4; ++L) {
-    if ((rc = A[L].ensure(c * W * 2, s))) return rc;
-    if (t2 && (rc = Z[L].ensure(c * W * 4, s))) return rc;
-  }
-  if (t2) {
-    const int ks = ksplit_for(c);
-    const long long nbh = cdiv(c, kHeadRows), nbr = cdiv(c, 128);
-    if ((rc = dZa.ensure(c * W * 2, s)) || (rc = dZb.ensure(c * W * 2, s)) ||
-        (rc = dw5p.ensure(nbh * W * 4, s)) || (rc = db5p.ensure(nbh * 4, s)) ||
-        (rc = lossp.ensure(nbh * 4, s)))
-      return rc;
-    for (int L = 0; L < 4; ++L) {
-      if ((rc = part_w[L].ensure((size_t)ks * W * kInK[L] * 4, s))) return rc;
-      if ((rc = part_b[L].ensure((size_t)(L == 3 ? nbh : nbr) * W * 4, s))) return rc;
-    }
-  }
-  cap = c;
-  train = t2;
-  return WINDS_BS_OK;
+  return train ? ensure_parts(n, s) : WINDS_BS_OK;
 }
 
 void MlpWork::release() {
-  for (DevBuf *b : {&X, &t, &y, &dZa, &dZb, &dw5p, &db5p, &lossp, &xraw}) b->release();
-  for (int L = 0; L < 4; ++L) {
-    Z[L].release();
-    A[L].release();
-    part_w[L].release();
-    part_b[L].release();
-  }
-  cap = 0;
-  train = false;
+  for (DevBuf *b : {&t, &y, &xraw, &part}) b->release();
 }
 
-int mlp_forward(const winds_mlp *m, const __nv_bfloat16 *X, long long n, MlpWork &w, float *y,
-                cudaStream_t s) {
-  if (n <= 0) return WINDS_BS_OK;
-  const float *theta = static_cast<const float *>(m->theta.p);
-  const __nv_bfloat16 *wbf = static_cast<const __nv_bfloat16 *>(m->theta_bf.p);
-  cudaError_t e = cudaSuccess;
-  for (int L = 0; L < 4 && e == cudaSuccess; ++L) {
-    MlpGemmArgs g = gemm_args(m);
-    g.A = L == 0 ? X : P<__nv_bfloat16>(w.A[L - 1]);
-    g.lda = kInK[L];
-    g.a_mn = 0;
-    g.B = wbf + kOffW[L];
-    g.ldb = kInK[L];
-    g.b_mn = 0;
-    g.M = n;
-    g.K = kInK[L];
-    g.bias = theta + kOffB[L];
-    g.z_out = w.train ? P<float>(w.Z[L]) : nullptr;
-    g.a_out = P<__nv_bfloat16>(w.A[L]);
-    g.ldo = W;
-    e = launch_mlp_gemm(g, W, kEpiBiasGelu, 1, s);
-  }
-  if (e == cudaSuccess)
-    e = launch_mlp_head_fwd(P<__nv_bfloat16>(w.A[3]), n, theta + kOffW5, theta + kOffB5, y, s);
+int mlp_forward(const winds_mlp *m, const float *x, long long n, float *y, cudaStream_t s) {
+  MlpNetArgs g = net_args(m, x, n);
+  g.y = y;
+  const cudaError_t e = launch_mlp_forward(g, m->sms, s);
   return e == cudaSuccess ? WINDS_BS_OK : cuda_fail(e, "mlp forward");
 }
 
-const float *mlp_shift_dev(const winds_mlp *m) { return static_cast<const float *>(m->shift.p); }
-const float *mlp_scale_dev(const winds_mlp *m) { return static_cast<const float *>(m->scale.p); }
-float mlp_out_scale(const winds_mlp *m) { return m->out_scale; }
 // out_scale and the base flag on the device (after the 16 input scales), read
 // when a captured step replays
 const float *mlp_out_scale_dev(const winds_mlp *m) { return static_cast<const float *>(m->scale.p) + 16; }
@@ -278,6 +173,7 @@ int winds_mlp_create(const winds_mlp_config *cfg, winds_mlp **out) {
   cudaGetDevice(&m->dev);
   m->n_in = cfg->n_in;
   cudaError_t e = cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&m->sms, cudaDevAttrMultiProcessorCount, m->dev);
   if (e == cudaSuccess) e = cudaEventCreate(&m->e0);
   if (e == cudaSuccess) e = cudaEventCreate(&m->e1);
   if (e != cudaSuccess) {
@@ -290,7 +186,7 @@ int winds_mlp_create(const winds_mlp_config *cfg, winds_mlp **out) {
       (rc = m->grad.ensure(kNParam * 4, s)) || (rc = m->mom.ensure(kNParam * 4, s)) ||
       (rc = m->vel.ensure(kNParam * 4, s)) || (rc = m->shift.ensure(64, s)) ||
       (rc = m->scale.ensure(128, s)) || (rc = m->err.ensure(16, s)) ||
-      (rc = m->jobs.ensure(32 * sizeof(MlpReduceJob), s)) || (rc = m->loss.ensure(16, s))) {
+      (rc = m->loss.ensure(16, s))) {
     winds_mlp_destroy(m);
     return rc;
   }
@@ -301,10 +197,10 @@ int winds_mlp_create(const winds_mlp_config *cfg, winds_mlp **out) {
     const int fan = L == 0 ? cfg->n_in : W;
     std::normal_distribution<double> nd01(0.0, 1.0 / std::sqrt((double)fan));
     for (int o = 0; o < W; ++o)
-      for (int i = 0; i < fan; ++i) th[kOffW[L] + (long long)o * kInK[L] + i] = (float)nd01(gen);
+      for (int i = 0; i < fan; ++i) th[mlp_off_w(L) + (long long)o * kInK[L] + i] = (float)nd01(gen);
   }
   std::normal_distribution<double> nd5(0.0, 1.0 / std::sqrt((double)W));
-  for (int j = 0; j < W; ++j) th[kOffW5 + j] = (float)nd5(gen);
+  for (int j = 0; j < W; ++j) th[kMlpOffW5 + j] = (float)nd5(gen);
   for (int i = 0; i < 16; ++i) m->h_shift[i] = 0.f, m->h_scale[i] = 1.f;
   e = upload(m->theta.p, th.data(), kNParam * 4, s);
   if (e == cudaSuccess) e = upload(m->shift.p, m->h_shift, 64, s);
@@ -340,7 +236,7 @@ int winds_mlp_set_params(winds_mlp *m, const float *theta) {
   cudaStreamSynchronize(m->stream);
   std::vector<float> th(theta, theta + kNParam);
   for (int o = 0; o < W; ++o)  // padded inputs of layer 1 stay zero
-    for (int i = m->n_in; i < kMlpInPad; ++i) th[kOffW[0] + (long long)o * kMlpInPad + i] = 0.f;
+    for (int i = m->n_in; i < kMlpInPad; ++i) th[mlp_off_w(0) + (long long)o * kMlpInPad + i] = 0.f;
   cudaError_t e = upload(m->theta.p, th.data(), kNParam * 4, m->stream);
   if (e == cudaSuccess)
     e = launch_mlp_to_bf16(P<float>(m->theta), P<__nv_bfloat16>(m->theta_bf), kNParam, m->stream);
@@ -402,8 +298,8 @@ int winds_mlp_forward_host(winds_mlp *m, const float *x, long long n, float *y) 
   for (long long r0 = 0; r0 < n; r0 += chunk) {
     const long long k = n - r0 < chunk ? n - r0 : chunk;
     int rc = m->w.ensure(k, false, s);
-    if (!rc) rc = upload_inputs(m, x + r0 * m->n_in, k, m->w, s);
-    if (!rc) rc = mlp_forward(m, P<__nv_bfloat16>(m->w.X), k, m->w, P<float>(m->w.y), s);
+    if (!rc) rc = upload_inputs(m, x + r0 * m->n_in, k, s);
+    if (!rc) rc = mlp_forward(m, P<float>(m->w.xraw), k, P<float>(m->w.y), s);
     if (rc) return rc;
     cudaError_t e = cudaMemcpyAsync(y + r0, m->w.y.p, k * 4, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
@@ -418,15 +314,20 @@ int winds_mlp_loss_grad_host(winds_mlp *m, const float *x, const float *t, long 
   cudaSetDevice(m->dev);
   cudaStream_t s = m->stream;
   int rc = m->w.ensure(n, true, s);
-  if (!rc) rc = upload_inputs(m, x, n, m->w, s);
+  if (!rc) rc = upload_inputs(m, x, n, s);
   if (rc) return rc;
-  cudaError_t e = cudaMemcpyAsync(m->w.t.p, t, n * 4, cudaMemcpyHostToDevice, s);
+  cudaError_t e = upload(m->w.t.p, t, n * 4, s);
   if (e != cudaSuccess) return cuda_fail(e, "mlp targets");
-  if ((rc = mlp_forward(m, P<__nv_bfloat16>(m->w.X), n, m->w, P<float>(m->w.y), s))) return rc;
-  if ((rc = mlp_backward(m, P<__nv_bfloat16>(m->w.X), P<float>(m->w.t), n, m->w, s))) return rc;
+  MlpUpdateArgs u;
+  if ((rc = gradient(m, P<float>(m->w.xraw), P<float>(m->w.t), nullptr, n, P<float>(m->loss), &u, s)))
+    return rc;
+  u.grad = P<float>(m->grad);
   float l = 0.f;
-  e = cudaMemcpy(&l, m->loss.p, 4, cudaMemcpyDeviceToHost);
-  if (e == cudaSuccess && grad) e = cudaMemcpy(grad, m->grad.p, kNParam * 4, cudaMemcpyDeviceToHost);
+  e = launch_mlp_update(u, s);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&l, m->loss.p, 4, cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess && grad)
+    e = cudaMemcpyAsync(grad, m->grad.p, kNParam * 4, cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return cuda_fail(e, "mlp gradient read");
   if (loss) *loss = l;
   return check_err(m);
@@ -441,16 +342,12 @@ int winds_mlp_train_host(winds_mlp *m, const float *x, const float *t, long long
   const long long B = p->batch < n ? p->batch : n;
   const long long nbatch = cdiv(n, B);
   int rc;
-  if ((rc = m->xall_raw.ensure(n * m->n_in * 4, s)) || (rc = m->Xall.ensure(n * kMlpInPad * 2, s)) ||
-      (rc = m->Tall.ensure(n * 4, s)) || (rc = m->idx.ensure(n * 4, s)) ||
-      (rc = m->lossbuf.ensure(nbatch * 4, s)) || (rc = m->w.ensure(B, true, s)))
+  if ((rc = m->Xall.ensure(n * m->n_in * 4, s)) || (rc = m->Tall.ensure(n * 4, s)) ||
+      (rc = m->idx.ensure(n * 4, s)) || (rc = m->lossbuf.ensure(nbatch * 4, s)) ||
+      (rc = m->w.ensure_parts(B, s)))
     return rc;
-  cudaError_t e = cudaMemcpyAsync(m->xall_raw.p, x, n * m->n_in * 4, cudaMemcpyHostToDevice, s);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(m->Tall.p, t, n * 4, cudaMemcpyHostToDevice, s);
-  if (e == cudaSuccess)
-    e = launch_mlp_prep(P<float>(m->xall_raw), n, m->n_in, P<float>(m->shift), P<float>(m->scale),
-                        P<__nv_bfloat16>(m->Xall), s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  cudaError_t e = upload(m->Xall.p, x, n * m->n_in * 4, s);
+  if (e == cudaSuccess) e = upload(m->Tall.p, t, n * 4, s);
   if (e != cudaSuccess) return cuda_fail(e, "mlp training upload");
   std::vector<int> perm(n);
   for (long long i = 0; i < n; ++i) perm[i] = (int)i;
@@ -465,14 +362,11 @@ int winds_mlp_train_host(winds_mlp *m, const float *x, const float *t, long long
     cudaEventRecord(m->e0, s);
     for (long long b = 0; b < nbatch; ++b) {
       const long long r0 = b * B, nb = n - r0 < B ? n - r0 : B;
-      e = launch_mlp_gather(P<__nv_bfloat16>(m->Xall), P<float>(m->Tall), P<int>(m->idx) + r0, nb,
-                            P<__nv_bfloat16>(m->w.X), P<float>(m->w.t), s);
-      if (e != cudaSuccess) return cuda_fail(e, "mlp gather");
-      if ((rc = mlp_forward(m, P<__nv_bfloat16>(m->w.X), nb, m->w, P<float>(m->w.y), s))) return rc;
-      if ((rc = mlp_backward(m, P<__nv_bfloat16>(m->w.X), P<float>(m->w.t), nb, m->w, s))) return rc;
-      e = cudaMemcpyAsync(P<float>(m->lossbuf) + b, m->loss.p, 4, cudaMemcpyDeviceToDevice, s);
-      if (e != cudaSuccess) return cuda_fail(e, "mlp loss copy");
-      if ((rc = adam_step(m, *p, s))) return rc;
+      MlpUpdateArgs u;
+      if ((rc = gradient(m, P<float>(m->Xall), P<float>(m->Tall), P<int>(m->idx) + r0, nb,
+                         P<float>(m->lossbuf) + b, &u, s)) ||
+          (rc = adam_step(m, *p, u, s)))
+        return rc;
       ++m->train_steps;
     }
     cudaEventRecord(m->e1, s);
@@ -509,8 +403,7 @@ void winds_mlp_destroy(winds_mlp *m) {
   if (m->stream) cudaStreamSynchronize(m->stream);
   m->w.release();
   for (DevBuf *b : {&m->theta, &m->theta_bf, &m->grad, &m->mom, &m->vel, &m->shift, &m->scale,
-                    &m->err, &m->jobs, &m->loss, &m->lossbuf, &m->idx, &m->Xall, &m->Tall,
-                    &m->xall_raw})
+                    &m->err, &m->loss, &m->lossbuf, &m->idx, &m->Xall, &m->Tall})
     b->release();
   if (m->e0) cudaEventDestroy(m->e0);
   if (m->e1) cudaEventDestroy(m->e1);

@@ -11,24 +11,18 @@
 
 namespace winds {
 
-// Activations and partial sums for up to `cap` rows.
+// Rows and the parts of a gradient.
 struct MlpWork {
-  long long cap = 0;
-  bool train = false;
-  DevBuf X, t, y, Z[4], A[4], dZa, dZb, part_w[4], part_b[4], dw5p, db5p, lossp, xraw;
+  DevBuf t, y, xraw, part;
   int ensure(long long n, bool train, cudaStream_t s);
+  int ensure_parts(long long n, cudaStream_t s);
   void release();
 };
 
-// Runs the forward pass on rows X (BF16 [n][16], standardised) into y [n];
-// with w.train the pre-activations are kept for a backward pass.
-int mlp_forward(const winds_mlp *m, const __nv_bfloat16 *X, long long n, MlpWork &w, float *y,
-                cudaStream_t s);
+// y [n] = network on the raw rows x [n][n_in] (one launch).
+int mlp_forward(const winds_mlp *m, const float *x, long long n, float *y, cudaStream_t s);
 
-// Device copies of the input standardisation and the output scale.
-const float *mlp_shift_dev(const winds_mlp *m);
-const float *mlp_scale_dev(const winds_mlp *m);
-float mlp_out_scale(const winds_mlp *m);
+// Device copies of the output scale and the base flag.
 const float *mlp_out_scale_dev(const winds_mlp *m);
 const float *mlp_base_dev(const winds_mlp *m);
 int mlp_n_in(const winds_mlp *m);

@@ -81,7 +81,7 @@ struct winds_wake_batch {
   DevBuf st_lift;   // per station: 1 when its airfoil table has lift (start value applies)
   DevBuf st_stall;  // per station: AoA (deg) of its table's lowest and highest Cl
   winds_mlp *mlp = nullptr;
-  MlpWork mw;
+  DevBuf mlp_y;
   // whole step, lifting-line iteration included
   cudaGraphExec_t exec_step = nullptr;
   cudaGraph_t g_step = nullptr;
@@ -381,15 +381,12 @@ cudaError_t enqueue_kj(winds_wake_batch *b, int &launches) {
                            s);
   if (e == cudaSuccess && b->mlp) {
     // start value Gamma_prev + out_scale * network(features)
-    e = launch_mlp_prep(P<float>(b->feat), b->n_ll, kKJFeatures, mlp_shift_dev(b->mlp),
-                        mlp_scale_dev(b->mlp), P<__nv_bfloat16>(b->mw.X), s);
-    if (e == cudaSuccess &&
-        mlp_forward(b->mlp, P<__nv_bfloat16>(b->mw.X), b->n_ll, b->mw, P<float>(b->mw.y), s))
+    if (mlp_forward(b->mlp, P<float>(b->feat), b->n_ll, P<float>(b->mlp_y), s))
       e = cudaErrorLaunchFailure;
     if (e == cudaSuccess)
       e = launch_kj_apply_guess(cd, kd, b->ncases, b->max_st, P<const int>(b->step_d),
                                 P<const int>(b->st_lift), P<const double2>(b->st_stall),
-                                P<const double>(b->aoa_o), P<const float>(b->mw.y),
+                                P<const double>(b->aoa_o), P<const float>(b->mlp_y),
                                 mlp_out_scale_dev(b->mlp),
                                 P<const float>(b->feat), mlp_base_dev(b->mlp), P<double>(b->bound),
                                 s);
@@ -1238,7 +1235,7 @@ int winds_wake_set_mlp(winds_wake_batch *b, winds_mlp *m) {
                 kKJFeatures);
   if (mlp_device(m) != b->dev) return fail(WINDS_BS_ERR_ARG, "MLP and batch on different devices");
   cudaSetDevice(b->dev);
-  int rc = b->mw.ensure(std::max<long long>(b->n_ll, 1), false, b->stream);
+  int rc = b->mlp_y.ensure(std::max<long long>(b->n_ll, 1) * sizeof(float), b->stream);
   if (rc) return rc;
   b->mlp = m;
   return WINDS_BS_OK;
@@ -1329,7 +1326,7 @@ void winds_wake_destroy(winds_wake_batch *b) {
                     &b->bound_last, &b->bound_last2, &b->st_rr, &b->st_dr, &b->rpm, &b->pitch, &b->dl,
                     &b->loads_out})
     x->release();
-  b->mw.release();
+  b->mlp_y.release();
   for (DevBuf *x : {&b->cases_d, &b->step_d, &b->dom, &b->dom_pred, &b->dom_new, &b->vel, &b->h1,
                     &b->h2, &b->h3, &b->uind, &b->uind_pred, &b->bound, &b->trail_prev,
                     &b->shed_cur, &b->trail_cur, &b->shed_next, &b->trail_next, &b->rc_s,
