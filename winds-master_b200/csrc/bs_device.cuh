@@ -369,6 +369,78 @@ __device__ __forceinline__ void pair64(const double4 A, const double4 B, double 
   uz = fma(ub, cz, uz);
 }
 
+// 1/sqrt(x) and 1/x to FP64 roundoff for x well inside the normal range: the
+// hardware's approximation and one third-order step, y (1 + e/2 + 3e^2/8) with
+// e = 1 - x y^2 and y (1 + e + e^2) with e = 1 - x y (Householder's method).
+__device__ __forceinline__ double rsqrt64(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-(x * y), y, 1.0);
+  return fma(y * e, fma(e, 0.375, 0.5), y);
+}
+__device__ __forceinline__ double rcp64(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-x, y, 1.0);
+  return fma(y, fma(e, e, e), y);
+}
+
+// High words of positive doubles order as the doubles do.
+constexpr int kHiMin = (1023 - 480) << 20, kHiMax = (1023 + 480) << 20;    // 2^-480, 2^480
+constexpr int kHiMin2 = (1023 - 960) << 20, kHiMax2 = (1023 + 960) << 20;  // 2^-960, 2^960
+
+// High word of the reach's square; a negative reach drops every pair.
+__device__ __forceinline__ int reach_hi(double co) {
+  return co < 0.0 ? -1 : __double2hiint(co * co);
+}
+
+// The term of ref_pair times 4 pi in 48 (Vatistas; cut-off 43) FP64 operations, for
+// sums of all pairs. C: L = x2 - x1 and (Vatistas) (rc L^2)^2 or (cut-off) d L^2;
+// axis_hi: axis_limit(L^2). False, with u unchanged, for what ref_pair does
+// instead: scales far from one, the reach's edge, a point on a filament's end, and
+// where ref_pair's differences cancel, so that both agree there too: 1 + cos of the
+// angle between the ends below 2^-8 (next to the segment) and, with the Vatistas
+// core, a sine below 2^-4 or so of the angle to the filament's line.
+constexpr int kHiE = (1023 - 8) << 20;
+__device__ __forceinline__ int axis_limit(double L2) {
+  return __double2hiint(L2) - (8 << 20);
+}
+template <int MODEL>
+__device__ __forceinline__ bool pair64_short(const double4 A, const double4 B, const double4 C,
+                                             int axis_hi, double px, double py, double pz, int co_hi,
+                                             double &ux, double &uy, double &uz) {
+  const double ax = px - A.x, ay = py - A.y, az = pz - A.z;
+  const double bx = px - B.x, by = py - B.y, bz = pz - B.z;
+  const double r1s = fma(ax, ax, fma(ay, ay, az * az));
+  const double r2s = fma(bx, bx, fma(by, by, bz * bz));
+  const double dot = fma(ax, bx, fma(ay, by, az * bz));
+  const double cx = fma(C.y, az, -(C.z * ay)), cy = fma(C.z, ax, -(C.x * az)),
+               cz = fma(C.x, ay, -(C.y * ax));
+  const int h1 = __double2hiint(r1s), h2 = __double2hiint(r2s), hmin = min(h1, h2);
+  const double i1 = rsqrt64(r1s), i2 = rsqrt64(r2s), gg = i1 * i2, e = fma(dot, gg, 1.0);
+  double ub;
+  bool hard = __double2hiint(e) < kHiE || hmin < kHiMin || max(h1, h2) > kHiMax || hmin == co_hi;
+  int hq;
+  if (MODEL == kCoreCutoff) {
+    const double q = fma(C.w, gg * gg, e);
+    hq = __double2hiint(q);
+    ub = (i1 + i2) * gg * rcp64(q);
+  } else {
+    const double c2 = fma(cx, cx, fma(cy, cy, cz * cz)), q = fma(c2, c2, C.w);
+    hq = __double2hiint(q);
+    hard = hard || __double2hiint(c2) - h1 < axis_hi - (1023 << 20);
+    ub = (i1 + i2) * (c2 * gg) * rsqrt64(q * (e * e));
+  }
+  ub *= A.w;
+  if (hard || hq < kHiMin2 || hq > kHiMax2 || (__double2hiint(ub) & 0x7ff00000) == 0x7ff00000)
+    return false;
+  if (hmin > co_hi) return true;
+  ux = fma(ub, cx, ux);
+  uy = fma(ub, cy, uy);
+  uz = fma(ub, cz, uz);
+  return true;
+}
+
 // What an evaluation starts from: an empty bounding box and the work queue at its
 // start (one block of at least 32 threads).
 __device__ __forceinline__ void begin_evaluation(BBox *bb, unsigned *ctr) {

@@ -982,10 +982,28 @@ __global__ void __launch_bounds__(kThreads, MinBlocks<T>::value) bs_f32c(const F
 
 // ------------------------------------------------------- FP64 direct sum
 constexpr int kF64Threads = 128;
-constexpr int kF64Tile = 128;  // filaments per shared-memory stage
+constexpr int kF64Tile = 64;  // filaments per shared-memory stage
 
+// A thread per target, filaments through shared memory. FORM kF64Ref: ref_pair's
+// terms added in order, what a sequential evaluation promises and a general
+// Vatistas index needs; otherwise the short form of the core model, with ref_pair
+// for the pairs that it leaves. Bound by the FP64 units (69% of their cycles, 56
+// operations a pair, where ref_pair's three roots and four divisions make some
+// 150): 12.5k targets x 24.7k filaments take 1.46 ms, 3.03 with ref_pair
+// throughout (cut-off core 1.11, 1.86). Two targets a thread take 1.76 ms, 40
+// registers less 1.48.
+enum F64Form : int { kF64Ref = 0, kF64Vatistas = 1, kF64Cutoff = 2 };
+static F64Form f64_form(int model, double n, bool sequential) {
+  if (sequential || (model != kCoreCutoff && n != 2.0)) return kF64Ref;
+  return model == kCoreCutoff ? kF64Cutoff : kF64Vatistas;
+}
+
+template <int FORM>
 __global__ void __launch_bounds__(kF64Threads) bs_f64(const F32cArgs a) {
-  __shared__ double4 sA[2][kF64Tile], sB[2][kF64Tile];
+  constexpr bool kShort = FORM != kF64Ref;
+  constexpr int kModel = FORM == kF64Cutoff ? kCoreCutoff : kCoreVatistas;
+  __shared__ double4 sA[2][kF64Tile], sB[2][kF64Tile], sC[kShort ? 2 : 1][kShort ? kF64Tile : 1];
+  __shared__ int sD[kShort ? 2 : 1][kShort ? kF64Tile : 1];
   __shared__ int s_item;
   const int tid = threadIdx.x;
   RefParams rp;
@@ -993,6 +1011,19 @@ __global__ void __launch_bounds__(kF64Threads) bs_f64(const F32cArgs a) {
   rp.d = a.d;
   rp.n = a.n;
   rp.co = a.co;
+  const int co_hi = reach_hi(a.co);
+  const auto stage = [&](int b, const double4 A, const double4 B) {
+    sA[b][tid] = A;
+    sB[b][tid] = B;
+    if constexpr (kShort) {
+      const double x = B.x - A.x, y = B.y - A.y, z = B.z - A.z, L2 = fma(x, x, fma(y, y, z * z));
+      double w = FORM == kF64Cutoff ? a.d * L2 : B.w * L2;
+      if (FORM == kF64Vatistas) w *= w;
+      if (!isfinite(A.w)) w = NAN;  // such a filament adds nothing: left to ref_pair
+      sC[b][tid] = make_double4(x, y, z, w);
+      sD[b][tid] = axis_limit(L2);
+    }
+  };
   while (true) {
     if (tid == 0) s_item = (int)atomicAdd(a.work_ctr, 1u);
     __syncthreads();
@@ -1003,34 +1034,37 @@ __global__ void __launch_bounds__(kF64Threads) bs_f64(const F32cArgs a) {
     Item it = a.items[item_id];
     Tile tl = a.tiles[it.tile];
     if (a.live && !clip_live(a.live, it, tl)) continue;  // uniform over the block
-    int l = tid < tl.t_count ? tid : tl.t_count - 1;
-    const double4 p = a.tp[tl.t_begin + l];
-    double ux = 0.0, uy = 0.0, uz = 0.0;
+    const double4 p = a.tp[tl.t_begin + (tid < tl.t_count ? tid : tl.t_count - 1)];
+    double u[3] = {0.0, 0.0, 0.0}, v[3] = {0.0, 0.0, 0.0};
     const int ntiles = (it.f_end - it.f_begin) / kF64Tile;
-    // stage 0
-    sA[0][tid] = a.ra[it.f_begin + tid];
-    sB[0][tid] = a.rb[it.f_begin + tid];
+    if (tid < kF64Tile) stage(0, a.ra[it.f_begin + tid], a.rb[it.f_begin + tid]);
     __syncthreads();
     for (int i = 0; i < ntiles; ++i) {
       const int b = i & 1;
       double4 nA, nB;
-      const bool more = i + 1 < ntiles;
+      const bool more = i + 1 < ntiles && tid < kF64Tile;
       if (more) {
         nA = a.ra[it.f_begin + (i + 1) * kF64Tile + tid];
         nB = a.rb[it.f_begin + (i + 1) * kF64Tile + tid];
       }
-      for (int k = 0; k < kF64Tile; ++k) ref_pair(sA[b][k], sB[b][k], p.x, p.y, p.z, rp, ux, uy, uz);
-      if (more) {
-        sA[b ^ 1][tid] = nA;
-        sB[b ^ 1][tid] = nB;
+#pragma unroll 1
+      for (int k = 0; k < kF64Tile; ++k) {
+        const double4 A = sA[b][k], B = sB[b][k];
+        if constexpr (kShort) {
+          if (!pair64_short<kModel>(A, B, sC[b][k], sD[b][k], p.x, p.y, p.z, co_hi, v[0], v[1], v[2]))
+            ref_pair<false>(A, B, p.x, p.y, p.z, rp, u[0], u[1], u[2]);
+        } else {
+          ref_pair(A, B, p.x, p.y, p.z, rp, u[0], u[1], u[2]);
+        }
       }
+      if (more) stage(b ^ 1, nA, nB);
       __syncthreads();
     }
     if (tid < tl.t_count) {
-      double *part = a.part + (size_t)item_id * 3 * a.tile_cap;
-      part[tid] = ux;
-      part[a.tile_cap + tid] = uy;
-      part[2 * a.tile_cap + tid] = uz;
+      double *part = a.part + (size_t)item_id * 3 * a.tile_cap + tid;
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+        part[c * a.tile_cap] = kShort ? fma(v[c], 1.0 / k4Pi, u[c]) : u[c];
     }
   }
 }
@@ -1210,16 +1244,25 @@ int f32c_occupancy(int model, int T, int KF) {
   return 1;
 }
 
-int f64_occupancy() {
-  int n = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, bs_f64, kF64Threads, 0) != cudaSuccess)
-    return 1;
-  return n > 0 ? n : 1;
+static const void *f64_kernel(int model, double n, bool sequential) {
+  const F64Form f = f64_form(model, n, sequential);
+  return f == kF64Ref      ? (const void *)bs_f64<kF64Ref>
+         : f == kF64Cutoff ? (const void *)bs_f64<kF64Cutoff>
+                           : (const void *)bs_f64<kF64Vatistas>;
 }
 
-cudaError_t launch_f64(const F32cArgs &a, int grid, cudaStream_t s) {
-  bs_f64<<<grid, kF64Threads, 0, s>>>(a);
-  return cudaGetLastError();
+int f64_occupancy(int model, double n, bool sequential) {
+  int k = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, f64_kernel(model, n, sequential), kF64Threads,
+                                                    0) != cudaSuccess)
+    return 1;
+  return k > 0 ? k : 1;
+}
+
+cudaError_t launch_f64(const F32cArgs &a, bool sequential, int grid, cudaStream_t s) {
+  void *args[] = {const_cast<F32cArgs *>(&a)};
+  return cudaLaunchKernel(f64_kernel(a.model, a.n, sequential), dim3((unsigned)grid),
+                          dim3(kF64Threads), args, 0, s);
 }
 
 cudaError_t launch_begin(BBox *bb, unsigned *ctr, unsigned long long *near, unsigned long long *cnt,

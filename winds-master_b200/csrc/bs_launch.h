@@ -28,7 +28,7 @@ int f32c_warps();          // workers per CTA
 int f64_threads();
 int f64_tile();
 int f32c_occupancy(int model, int T, int KF);
-int f64_occupancy();
+int f64_occupancy(int model, double n, bool sequential);
 unsigned long long default_wait_limit_ns();
 
 // First kernel of an evaluation: empty bounding box, work queue at its start,
@@ -62,7 +62,8 @@ cudaError_t launch_sort_targets(const TargetBufs &b, long long n, int groups, co
                                 cudaStream_t s);
 cudaError_t sort_targets_bytes(long long n, int groups, size_t *bytes);
 cudaError_t launch_f32c(const F32cArgs &a, int model, int T, int KF, int grid, cudaStream_t s);
-cudaError_t launch_f64(const F32cArgs &a, int grid, cudaStream_t s);
+// sequential: every target's terms in the filaments' order, as ref_pair has them.
+cudaError_t launch_f64(const F32cArgs &a, bool sequential, int grid, cudaStream_t s);
 // live (with the plan's items): only each group's live part (GroupLive). Leaves
 // the work queue's counter ctr at its start.
 cudaError_t launch_reduce(const Tile *tiles, int n_tiles, const Group *groups, const double *part,

@@ -408,7 +408,7 @@ int run_direct_sum(Context *c, const std::vector<GroupSpec> &gs, int model, doub
   int tile_cap, resident, quantum;
   if (precision == WINDS_PREC_F64) {
     tile_cap = f64_threads();
-    resident = f64_occupancy() * c->num_sms;
+    resident = f64_occupancy(model, n, sequential) * c->num_sms;
     quantum = f64_tile();
   } else {
     if (!f32c_config_supported(ch.T, ch.KF)) return fail(WINDS_BS_ERR_ARG, "bad tile choice");
@@ -470,7 +470,7 @@ int run_direct_sum(Context *c, const std::vector<GroupSpec> &gs, int model, doub
   const int grid = worker_grid(a.n_items, resident, c->num_sms, precision != WINDS_PREC_F64);
   if (time_main) cudaEventRecord(c->ev_main0, s);
   if (precision == WINDS_PREC_F64)
-    e = launch_f64(a, grid, s);
+    e = launch_f64(a, sequential, grid, s);
   else
     e = launch_f32c(a, model, ch.T, ch.KF, grid, s);
   if (time_main) cudaEventRecord(c->ev_main1, s);

@@ -158,7 +158,7 @@ extern "C" int winds_bs_eval_device_noalloc(const winds_bs_family *fams, int nfa
   int tile_cap, resident, quantum;
   if (prec == WINDS_PREC_F64) {
     tile_cap = f64_threads();
-    resident = f64_occupancy() * sms;
+    resident = f64_occupancy(model, n, false) * sms;
     quantum = f64_tile();
   } else {
     tile_cap = f32c_tile(ch.T);
@@ -244,7 +244,7 @@ extern "C" int winds_bs_eval_device_noalloc(const winds_bs_family *fams, int nfa
   a.co = prm->co;
   a.wait_limit_ns = default_wait_limit_ns();
   const int grid = worker_grid(n_items, resident, sms, prec != WINDS_PREC_F64);
-  e = prec == WINDS_PREC_F64 ? launch_f64(a, grid, s) : launch_f32c(a, model, ch.T, ch.KF, grid, s);
+  e = prec == WINDS_PREC_F64 ? launch_f64(a, false, grid, s) : launch_f32c(a, model, ch.T, ch.KF, grid, s);
   if (e == cudaSuccess) e = launch_reduce(tiles, n_tiles, groups, part, tb.perm, tile_cap, ctr, s);
   if (e != cudaSuccess) return cuda_fail(e, "noalloc direct-sum launch");
 

@@ -164,7 +164,7 @@ int build_plans(winds_wake_batch *b) {
   int resident, quantum;
   if (b->prec == WINDS_PREC_F64) {
     b->tile_cap = f64_threads();
-    resident = f64_occupancy() * sms;
+    resident = f64_occupancy(b->model, b->nidx, false) * sms;
     quantum = f64_tile();
   } else {
     b->tile_cap = f32c_tile(b->ch.T);
@@ -251,7 +251,7 @@ cudaError_t enqueue_eval(winds_wake_batch *b, const double *dom, const double *s
   a.wait_limit_ns = default_wait_limit_ns();
   a.live = live;
   if (e == cudaSuccess)
-    e = b->prec == WINDS_PREC_F64 ? launch_f64(a, b->grid, s)
+    e = b->prec == WINDS_PREC_F64 ? launch_f64(a, false, b->grid, s)
                                   : launch_f32c(a, b->model, b->ch.T, b->ch.KF, b->grid, s);
   if (e == cudaSuccess)
     e = launch_reduce(P<const Tile>(b->tiles), b->n_tiles, P<const Group>(groups),
@@ -426,7 +426,7 @@ cudaError_t enqueue_kj(winds_wake_batch *b, int &launches) {
   a.wait_limit_ns = default_wait_limit_ns();
   if (e == cudaSuccess)
     e = b->prec == WINDS_PREC_F64 || b->kjp.ll_fp64
-            ? launch_f64(a, b->kj_grid, s)
+            ? launch_f64(a, false, b->kj_grid, s)
             : launch_f32c(a, b->model, b->kj_T, b->kj_KF, b->kj_grid, s);
   if (e == cudaSuccess)
     e = launch_reduce(P<const Tile>(b->kj_tiles), b->kj_ntiles, P<const Group>(b->kj_groups),
@@ -1183,7 +1183,7 @@ int winds_wake_set_kj(winds_wake_batch *b, const winds_kj_case *kj, const winds_
   int resident, quantum;
   if (b->prec == WINDS_PREC_F64 || b->kjp.ll_fp64) {
     b->kj_tile_cap = f64_threads();
-    resident = f64_occupancy() * sms;
+    resident = f64_occupancy(b->model, b->nidx, false) * sms;
     quantum = f64_tile();
   } else {
     b->kj_tile_cap = f32c_tile(b->kj_T);
