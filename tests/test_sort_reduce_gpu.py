@@ -1,5 +1,5 @@
-"""The evaluation's target sort (one CTA per group up to 16384 targets, the device-wide sort above)
-and the reduction by eight warps, at the sizes where they change.
+"""The evaluation's target sort (by counting up to 3.6e8 comparisons, 18973 targets of one group, the
+device-wide sort above) and the reduction by eight warps, at the sizes where they change.
 
 Filaments and targets are apart, so that a term's rounding is a few 1e-16 and a sum of 200 of them
 stays below 1e-13 of the sum of magnitudes: FP64 has to be within 1e-12 of the largest velocity of
@@ -20,7 +20,8 @@ def _family(rng, dims):
             np.asfortranarray(rng.uniform(0.01, 0.02, g)))
 
 
-@pytest.mark.parametrize("nt", [1, 33, 2048, 2049, 4097, 8192, 8193, 16384, 16385, 20001])
+@pytest.mark.parametrize("nt", [1, 33, 2048, 2049, 4097, 8192, 8193, 16384, 16385, 20001, 127, 128, 129, 18973,
+                                18974])
 def test_sorted_evaluation(wb, oracle, nt):
     """Seven families (two packing launches; one is empty), a ragged target count."""
     rng = np.random.default_rng(nt)
@@ -38,7 +39,7 @@ def test_sorted_evaluation(wb, oracle, nt):
 
 @pytest.mark.parametrize("nst,steps", [(9, 20), (17, 60), (33, 80), (41, 120)])
 def test_one_cta_and_device_wide_sort_agree(wb, synth, nst, steps):
-    """A case alone (its nodes sorted by one CTA) and beside one of 17k nodes (all sorted together)."""
+    """A case alone (its nodes sorted by counting) and beside one of 17k nodes (all sorted together)."""
     import importlib
     wake = importlib.import_module("winds-master_b200.wake")
     case = lambda n, s: synth.make_wake_case(synth.RotorCase(nst=n, nsteps=s), nsteps=3)  # noqa: E731

@@ -4,12 +4,12 @@
 //
 // Kernels
 //   bs_chain_count,    MATLAB-layout F1/F2/gamma/rc -> 64-byte records (+ FP64
-//   bs_pack_filaments  copies), the device-side replacement of the host crunch_f
+//   bs_pack  copies), the device-side replacement of the host crunch_f
 //                      / crunch_rg packing (BiotSavartMex.cu:316-357), in input
 //                      order or laid out along the wake's lines of filaments
 //                      (x2 of a record = x1 of the one before, but for marked
 //                      heads where a line starts or the input has no link)
-//   bs_pack_targets    MATLAB-layout P -> double4 targets (crunch_p, :361-379)
+//                      and MATLAB-layout P -> double4 targets (crunch_p, :361-379)
 //   bs_f32c            persistent FP32 direct sum on independent warp workers:
 //                      each warp stages its filament tiles into its own shared
 //                      memory by bulk copies (cp.async.bulk + mbarrier), keeps
@@ -28,6 +28,7 @@
 #include "bs_types.h"
 
 #include <cfloat>
+#include <type_traits>
 
 #include <cub/device/device_radix_sort.cuh>
 
@@ -82,9 +83,22 @@ __global__ void bs_chain_count(const PackArgs a) {
 // One thread per filament of a family, in input order; its record goes to slot
 // off + f, or (cnt given and cnt[1] > cnt[0]) to its place along the third
 // index. The blocks past the families fill [pad_from, pad_to) with inert
-// filaments: far away, zero length, zero circulation.
-__global__ void bs_pack_filaments(const PackArgs a) {
+// filaments (far away, zero length, zero circulation), those past them pack the
+// targets of a MATLAB array P [ns, 3, ...].
+__global__ void bs_pack(const PackArgs a) {
   float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
+  if ((int)blockIdx.x >= a.tgt_block0) {
+    const long long t = (long long)(blockIdx.x - a.tgt_block0) * blockDim.x + threadIdx.x;
+    if (t < a.nt) {
+      const long long j = t / a.ns, b = t - j * a.ns + a.ns * 3 * j;
+      const double x = a.P[b], y = a.P[b + a.ns], z = a.P[b + 2 * a.ns];
+      a.tp_raw[t] = make_double4(x, y, z, 0.0);
+      if (a.tgroup) a.tgroup[t] = 0;
+      lo[0] = hi[0] = (float)x, lo[1] = hi[1] = (float)y, lo[2] = hi[2] = (float)z;
+    }
+    bbox_accumulate(lo, hi, a.bb->tmin, a.bb->tmax);
+    return;
+  }
   if ((int)blockIdx.x >= a.pad_block0) {
     const long long f =
         a.pad_from + (long long)(blockIdx.x - a.pad_block0) * blockDim.x + threadIdx.x;
@@ -118,26 +132,9 @@ __global__ void bs_pack_filaments(const PackArgs a) {
   bbox_accumulate(lo, hi, a.bb->fmin, a.bb->fmax);
 }
 
-__global__ void bs_pack_targets(const double *__restrict__ P, long long ns, long long np,
-                                long long off, int group, double4 *tp, int *tgroup, BBox *bb) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
-  if (t < np) {
-    const long long j = t / ns, i = t - j * ns;
-    const long long b = i + ns * 3 * j;
-    const double x = P[b], y = P[b + ns], z = P[b + 2 * ns];
-    tp[off + t] = make_double4(x, y, z, 0.0);
-    tgroup[off + t] = group;
-    lo[0] = hi[0] = (float)x;
-    lo[1] = hi[1] = (float)y;
-    lo[2] = hi[2] = (float)z;
-  }
-  bbox_accumulate(lo, hi, bb->tmin, bb->tmax);
-}
-
 // Sort key of a target: group id above the 30-bit Hilbert position in the
 // targets' bounding box (bit 30: the target is unused, and sorts after every
-// live target of its group).
+// live target of its group); for counting, the position's leading 24 bits.
 template <class KEY>
 __global__ void bs_target_keys(const double4 *__restrict__ tp, const int *__restrict__ tgroup,
                                long long n, const BBox *bb, KEY *keys, int *vals) {
@@ -147,11 +144,16 @@ __global__ void bs_target_keys(const double4 *__restrict__ tp, const int *__rest
   const double q[3] = {p.x, p.y, p.z};
   const float lo[3] = {key_float(bb->tmin[0]), key_float(bb->tmin[1]), key_float(bb->tmin[2])};
   const float hi[3] = {key_float(bb->tmax[0]), key_float(bb->tmax[1]), key_float(bb->tmax[2])};
-  KEY code = hilbert_key(q, lo, hi);
-  if (p.w != 0.0) code |= (KEY)1 << 30;
-  if (sizeof(KEY) == 8) code |= (KEY)(unsigned)tgroup[t] << 31;
-  keys[t] = code;
-  vals[t] = (int)t;
+  const unsigned h = hilbert_key(q, lo, hi);
+  if constexpr (sizeof(KEY) == 4 && !std::is_integral<KEY>::value) {
+    keys[t] = p.w != 0.0 ? 16777216.f : (float)(h >> 6);  // 8 bits a coordinate
+  } else {
+    KEY code = h;
+    if (p.w != 0.0) code |= (KEY)1 << 30;
+    if (sizeof(KEY) == 8) code |= (KEY)(unsigned)tgroup[t] << 31;
+    keys[t] = code;
+    vals[t] = (int)t;
+  }
 }
 
 __global__ void bs_gather_targets(const double4 *__restrict__ src, const int *__restrict__ perm,
@@ -1271,10 +1273,10 @@ cudaError_t launch_begin(BBox *bb, unsigned *ctr, unsigned long long *near, unsi
   return cudaGetLastError();
 }
 
-cudaError_t launch_pack_families(const winds_bs_family *fams, int nfam, unsigned long long *cnt,
-                                 long long pad_to, int model, double dcut,
-                                 const PackedFilaments &pf, BBox *bb, cudaStream_t s,
-                                 int *launches) {
+cudaError_t launch_pack(const winds_bs_family *fams, int nfam, unsigned long long *cnt,
+                        long long pad_to, int model, double dcut, const PackedFilaments &pf,
+                        const double *P, long long ns, long long nt, const TargetBufs &tb, BBox *bb,
+                        cudaStream_t s, int *launches) {
   const int bs = 256;
   long long off = 0;
   int k = 0;
@@ -1296,11 +1298,14 @@ cudaError_t launch_pack_families(const winds_bs_family *fams, int nfam, unsigned
       blocks += (nf + bs - 1) / bs;
       off += nf;
     }
+    const bool last = k >= nfam;
     a.model = model, a.dcut = dcut;
     a.pk = pf.pk, a.ra = pf.ra, a.rb = pf.rb, a.bb = bb;
+    a.P = P, a.ns = ns, a.nt = last ? nt : 0;
+    a.tp_raw = tb.tp_raw, a.tgroup = tb.tgroup;
     a.pad_block0 = (int)blocks;
     a.pad_from = off;
-    a.pad_to = k >= nfam ? pad_to : off;
+    a.pad_to = last ? pad_to : off;
     if (cnt && blocks > 0) {
       if (!first) {
         const cudaError_t e = cudaMemsetAsync(cnt, 0, 2 * kPackFams * sizeof(*cnt), s);
@@ -1310,24 +1315,17 @@ cudaError_t launch_pack_families(const winds_bs_family *fams, int nfam, unsigned
       bs_chain_count<<<(unsigned)blocks, bs, 0, s>>>(a);
       if (launches) ++*launches;
     }
-    const long long total = blocks + (a.pad_to - a.pad_from + bs - 1) / bs;
-    if (total > 0) {
-      bs_pack_filaments<<<(unsigned)total, bs, 0, s>>>(a);
+    blocks += (a.pad_to - a.pad_from + bs - 1) / bs;
+    a.tgt_block0 = (int)blocks;
+    blocks += (a.nt + bs - 1) / bs;
+    if (blocks > 0) {
+      bs_pack<<<(unsigned)blocks, bs, 0, s>>>(a);
       if (launches) ++*launches;
     }
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   } while (k < nfam);
   return cudaSuccess;
-}
-
-cudaError_t launch_pack_targets(const double *P, long long ns, long long np, long long off,
-                                int group, double4 *tp, int *tgroup, BBox *bb, cudaStream_t s) {
-  if (np <= 0) return cudaSuccess;
-  const int bs = 256;
-  const long long grid = (np + bs - 1) / bs;
-  bs_pack_targets<<<(unsigned)grid, bs, 0, s>>>(P, ns, np, off, group, tp, tgroup, bb);
-  return cudaGetLastError();
 }
 
 cudaError_t launch_gather_targets(const double4 *src, const int *perm, long long n, double4 *dst,
@@ -1381,15 +1379,15 @@ cudaError_t launch_sort_targets(const TargetBufs &b, long long n, int groups, co
   return e != cudaSuccess ? e : launch_gather_targets(b.tp_raw, b.perm, n, b.tp, s);
 }
 
-cudaError_t launch_matlab_targets(const double *P, long long ns, long long n, const TargetBufs &b,
-                                  BBox *bb, cudaStream_t s) {
-  if (n <= 0) return cudaSuccess;
-  if (n <= kBlockSortMax) {
-    MatlabTargets src{P, ns, (int)n};
-    return launch_block_sort(src, 1, n, b.tp, b.perm, bb, s);
-  }
-  cudaError_t e = launch_pack_targets(P, ns, n, 0, 0, b.tp_raw, b.tgroup, bb, s);
-  return e != cudaSuccess ? e : launch_sort_targets(b, n, 1, bb, s);
+cudaError_t launch_target_keys(const double4 *tp, long long n, const BBox *bb, float *keys,
+                               cudaStream_t s) {
+  bs_target_keys<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(tp, (const int *)nullptr, n, bb, keys,
+                                                             (int *)nullptr);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_order_targets(long long n, const TargetBufs &b, const BBox *bb, cudaStream_t s) {
+  return launch_order_targets(OneGroup{(int)n}, 1, n, n, b, bb, s);
 }
 
 cudaError_t launch_reduce(const Tile *tiles, int n_tiles, const Group *groups, const double *part,

@@ -35,18 +35,9 @@ unsigned long long default_wait_limit_ns();
 // near (2 words) and cnt (2 kPackFams words) zero.
 cudaError_t launch_begin(BBox *bb, unsigned *ctr, unsigned long long *near, unsigned long long *cnt,
                          cudaStream_t s);
-// Packs the families (device arrays) one after the other, in input order or
-// (cnt: as launch_begin leaves it) each in the order with more links between
-// neighbours, then inert filaments up to pad_to. Adds to *launches.
-cudaError_t launch_pack_families(const winds_bs_family *fams, int nfam, unsigned long long *cnt,
-                                 long long pad_to, int model, double dcut,
-                                 const PackedFilaments &pf, BBox *bb, cudaStream_t s,
-                                 int *launches);
-// Targets sorted by (group, place on a Hilbert curve). Groups of at most
-// kBlockSortMax targets are sorted by one CTA each (bs_sort.cuh) and need tp and
-// perm only; the device-wide sort needs the rest (keys: 2 n words of 32 bits for one
-// group, of 64 for more).
-constexpr long long kBlockSortMax = 16384;
+// Targets sorted by (group, place on a Hilbert curve), from tp_raw. Counting
+// needs tp, perm, tp_raw and one 32-bit key a target; the device-wide sort needs the
+// rest too (keys: two words of 32 bits for one group, of 64 for more).
 struct TargetBufs {
   double4 *tp, *tp_raw;
   int *tgroup, *vals, *perm;
@@ -54,8 +45,27 @@ struct TargetBufs {
   void *sort_tmp;
   size_t sort_bytes;
 };
-cudaError_t launch_matlab_targets(const double *P, long long ns, long long n, const TargetBufs &b,
-                                  BBox *bb, cudaStream_t s);
+// Counting compares each target with its group's others: 3.2k targets take 6 us, 16k
+// 28 and 22k 65, against 66 us and more launches for the device-wide sort of 31-bit
+// keys; past 148 blocks of 128 targets some SMs have two. (One CTA per group with a
+// radix sort in shared memory: 31 us on 3.2k, 121 on 16k.) More groups share the
+// same units, so the line is their sum of squares.
+constexpr long long kCountingMax = 360ll * 1000 * 1000;
+inline bool sort_by_counting(long long groups, long long max_n) {
+  return max_n <= 65536 && groups * max_n * max_n <= kCountingMax;
+}
+// Packs the families (device arrays) one after the other, in input order or
+// (cnt: as launch_begin leaves it) each in the order with more links between
+// neighbours, then inert filaments up to pad_to, and the nt targets P [ns,3,...]
+// into tb.tp_raw. Adds to *launches.
+cudaError_t launch_pack(const winds_bs_family *fams, int nfam, unsigned long long *cnt,
+                        long long pad_to, int model, double dcut, const PackedFilaments &pf,
+                        const double *P, long long ns, long long nt, const TargetBufs &tb, BBox *bb,
+                        cudaStream_t s, int *launches);
+cudaError_t launch_target_keys(const double4 *tp, long long n, const BBox *bb, float *keys,
+                               cudaStream_t s);
+// The n targets of one group in order.
+cudaError_t launch_order_targets(long long n, const TargetBufs &b, const BBox *bb, cudaStream_t s);
 // Device-wide sort of n targets already in tp_raw / tgroup (groups of them), and
 // the scratch bytes it needs.
 cudaError_t launch_sort_targets(const TargetBufs &b, long long n, int groups, const BBox *bb,

@@ -1,19 +1,11 @@
-// bs_sort.cuh -- targets of one group sorted along a Hilbert curve by one CTA:
-// bounding box, keys, radix sort and gather in a single launch. For groups of
-// up to kBlockSortMax targets; larger ones take the device-wide radix sort
-// (launch_sort_targets). On 3.1k targets one launch of 31 us takes the place of
-// 13, whose eight passes over 64-bit keys alone took 72 us.
+// bs_sort.cuh -- targets of each group ordered along a Hilbert curve by counting:
+// a target's place is the number of keys below its own.
 #pragma once
 
-#include <cub/block/block_radix_sort.cuh>
-
 #include "bs_device.cuh"
+#include "bs_launch.h"
 
 namespace winds {
-
-constexpr int kSortThreads = 1024;
-constexpr int kSortBits = 5;   // radix digit: 25-bit keys take five passes
-constexpr int kKeyBits = 25;   // 8 bits a coordinate, and bit 24: the target is unused
 
 // Spreads the low 10 bits of v so that they occupy every third bit.
 __device__ __forceinline__ unsigned spread3(unsigned v) {
@@ -71,106 +63,107 @@ __device__ __forceinline__ unsigned hilbert_key(const double p[3], const float l
   return hilbert30(cell[0], cell[1], cell[2]);
 }
 
-// Targets of a MATLAB array P [ns, 3, ...]; one group.
-struct MatlabTargets {
-  const double *P;
-  long long ns;
+// The one group of an evaluation's targets.
+struct OneGroup {
   int n;
   __device__ int count(int) const { return n; }
   __device__ long long offset(int) const { return 0; }
-  __device__ bool load(int, int t, double p[3]) const {
-    const long long j = t / ns, b = t - j * ns + ns * 3 * j;
-    p[0] = P[b], p[1] = P[b + ns], p[2] = P[b + 2 * ns];
-    return true;
-  }
 };
 
-template <int ITEMS>
-using TargetSort = cub::BlockRadixSort<unsigned, kSortThreads, ITEMS, int, kSortBits>;
-
-// One CTA per group of SRC. tp: the sorted targets (w = 1 and the origin for
-// unused ones, which come last); perm: their places in the input order.
-template <int ITEMS, class SRC>
-__global__ void __launch_bounds__(kSortThreads) bs_sort_targets(const SRC src, double4 *tp,
-                                                                int *perm, BBox *bb) {
-  extern __shared__ __align__(16) unsigned char sort_smem[];
-  auto &temp = *reinterpret_cast<typename TargetSort<ITEMS>::TempStorage *>(sort_smem);
-  __shared__ float s_lo[3][32], s_hi[3][32];
-  const int g = blockIdx.x, n = src.count(g), tid = threadIdx.x;
-  const long long off = src.offset(g);
-  float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
-  for (int t = tid; t < n; t += kSortThreads) {
-    double p[3];
-    if (src.load(g, t, p))
+// A block places 32 R targets of a group, R a lane; each of its warps counts a run
+// of the group's keys, read by the warp into shared memory and from there four at a
+// time. Keys are whole numbers below 2^25 as floats, so that a comparison is a
+// saturated difference, at the full rate of the FP32 units where an integer
+// comparison has half: 16k targets take 28 us (as integers 41), 3.2k 6
+// (11.4). R: enough blocks for the SMs before fewer reads of the keys.
+constexpr int kRankWarps = 16;
+template <int R, class GROUPS>
+__global__ void __launch_bounds__(32 * kRankWarps)
+    bs_rank_targets(const GROUPS gr, const float *__restrict__ keys,
+                    const double4 *__restrict__ tp_raw, double4 *tp, int *perm) {
+  extern __shared__ float4 s_key[];  // a run of `run` keys per warp
+  __shared__ float s_cnt[kRankWarps][32 * R];
+  const int g = blockIdx.y, n = gr.count(g), i0 = blockIdx.x * 32 * R;
+  if (i0 >= n) return;
+  const long long off = gr.offset(g);
+  const float *key = keys + off;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int run = ((n + kRankWarps - 1) / kRankWarps + 3) / 4, j0 = 4 * run * warp;  // run: of four
+  const float inf = __int_as_float(0x7f800000);
+  float *mine = reinterpret_cast<float *>(s_key + run * warp);
+  for (int j = lane; j < 4 * run; j += 32) mine[j] = j0 + j < n ? key[j0 + j] : inf;
+  float k[R], c[R];
 #pragma unroll
-      for (int c = 0; c < 3; ++c) lo[c] = fminf(lo[c], (float)p[c]), hi[c] = fmaxf(hi[c], (float)p[c]);
+  for (int q = 0; q < R; ++q) {
+    const int i = i0 + 32 * q + lane;
+    k[q] = i < n ? key[i] : 0.f;
+    c[q] = 0.f;
   }
+  __syncwarp();
+  // keys before the block come first where equal, those after it do not
+  const float4 *x = s_key + run * warp;
+  const int lo = min(max((i0 - j0) / 4, 0), run), hi = min(max((i0 - j0) / 4 + 8 * R, 0), run);
+  const auto count = [&](int f, int t, float add) {
+#pragma unroll 4
+    for (int j = f; j < t; ++j) {
+      const float4 v = x[j];
 #pragma unroll
-  for (int c = 0; c < 3; ++c) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      lo[c] = fminf(lo[c], __shfl_xor_sync(0xffffffffu, lo[c], o));
-      hi[c] = fmaxf(hi[c], __shfl_xor_sync(0xffffffffu, hi[c], o));
+      for (int q = 0; q < R; ++q) {
+        const float y = k[q] + add;
+        c[q] += (__saturatef(y - v.x) + __saturatef(y - v.y)) +
+                (__saturatef(y - v.z) + __saturatef(y - v.w));
+      }
     }
-    if ((tid & 31) == 0) s_lo[c][tid >> 5] = lo[c], s_hi[c][tid >> 5] = hi[c];
+  };
+  count(0, lo, 1.f);
+  count(hi, run, 0.f);
+  for (int j = lo; j < hi; ++j) {
+    const float4 v = x[j];
+    const float w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int q = 0; q < R; ++q)
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        c[q] += __saturatef(k[q] + (j0 + 4 * j + e < i0 + 32 * q + lane ? 1.f : 0.f) - w[e]);
   }
+#pragma unroll
+  for (int q = 0; q < R; ++q) s_cnt[warp][32 * q + lane] = c[q];
   __syncthreads();
+  const int i = i0 + (int)threadIdx.x;
+  if (threadIdx.x >= 32 * R || i >= n) return;
+  float r = 0.f;
 #pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    lo[c] = s_lo[c][tid & 31], hi[c] = s_hi[c][tid & 31];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      lo[c] = fminf(lo[c], __shfl_xor_sync(0xffffffffu, lo[c], o));
-      hi[c] = fmaxf(hi[c], __shfl_xor_sync(0xffffffffu, hi[c], o));
-    }
-    if (tid == c && lo[c] != FLT_MAX) atomicMin(&bb->tmin[c], float_key(lo[c]));
-    if (tid == c && hi[c] != -FLT_MAX) atomicMax(&bb->tmax[c], float_key(hi[c]));
-  }
-  unsigned key[ITEMS];
-  int val[ITEMS];
-#pragma unroll
-  for (int k = 0; k < ITEMS; ++k) {
-    const int t = tid * ITEMS + k;
-    val[k] = t;
-    key[k] = (1u << kKeyBits) - 1u;  // past the end: after the last target, as the sort is stable
-    if (t < n) {
-      double p[3];
-      const bool used = src.load(g, t, p);
-      key[k] = used ? hilbert_key(p, lo, hi) >> 6 : 1u << (kKeyBits - 1);
-    }
-  }
-  TargetSort<ITEMS>(temp).SortBlockedToStriped(key, val, 0, kKeyBits);
-#pragma unroll
-  for (int k = 0; k < ITEMS; ++k) {
-    const int r = k * kSortThreads + tid;
-    if (r < n) {
-      double p[3];
-      const bool used = src.load(g, val[k], p);
-      tp[off + r] = used ? make_double4(p[0], p[1], p[2], 0.0) : make_double4(0.0, 0.0, 0.0, 1.0);
-      perm[off + r] = (int)(off + val[k]);
-    }
-  }
+  for (int w = 0; w < kRankWarps; ++w) r += s_cnt[w][threadIdx.x];
+  tp[off + (int)r] = tp_raw[off + i];
+  perm[off + (int)r] = (int)(off + i);
 }
 
-template <int ITEMS, class SRC>
-cudaError_t launch_block_sort_t(const SRC &src, int groups, double4 *tp, int *perm, BBox *bb,
+template <int R, class GROUPS>
+cudaError_t launch_rank_targets(const GROUPS &gr, int groups, long long max_n, const TargetBufs &b,
                                 cudaStream_t s) {
-  const int smem = (int)sizeof(typename TargetSort<ITEMS>::TempStorage);
-  cudaError_t e = cudaFuncSetAttribute(bs_sort_targets<ITEMS, SRC>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  const int run = ((int)((max_n + kRankWarps - 1) / kRankWarps) + 3) / 4;
+  const int smem = run * kRankWarps * (int)sizeof(float4);
+  const cudaError_t e = cudaFuncSetAttribute(bs_rank_targets<R, GROUPS>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
-  bs_sort_targets<ITEMS, SRC><<<groups, kSortThreads, smem, s>>>(src, tp, perm, bb);
+  const dim3 grid((unsigned)((max_n + 32 * R - 1) / (32 * R)), (unsigned)groups);
+  bs_rank_targets<R><<<grid, 32 * kRankWarps, smem, s>>>(
+      gr, reinterpret_cast<const float *>(b.keys), b.tp_raw, b.tp, b.perm);
   return cudaGetLastError();
 }
 
-// max_n: the largest group, at most kBlockSortMax.
-template <class SRC>
-cudaError_t launch_block_sort(const SRC &src, int groups, long long max_n, double4 *tp, int *perm,
-                              BBox *bb, cudaStream_t s) {
-  if (max_n <= 2 * kSortThreads) return launch_block_sort_t<2>(src, groups, tp, perm, bb, s);
-  if (max_n <= 4 * kSortThreads) return launch_block_sort_t<4>(src, groups, tp, perm, bb, s);
-  if (max_n <= 8 * kSortThreads) return launch_block_sort_t<8>(src, groups, tp, perm, bb, s);
-  return launch_block_sort_t<16>(src, groups, tp, perm, bb, s);
+// n targets in tp_raw (tgroup: their groups; not read by the counting sort).
+template <class GROUPS>
+cudaError_t launch_order_targets(const GROUPS &gr, int groups, long long max_n, long long n,
+                                 const TargetBufs &b, const BBox *bb, cudaStream_t s) {
+  if (n <= 0) return cudaSuccess;
+  if (!sort_by_counting(groups, max_n)) return launch_sort_targets(b, n, groups, bb, s);
+  const cudaError_t e = launch_target_keys(b.tp_raw, n, bb, reinterpret_cast<float *>(b.keys), s);
+  if (e != cudaSuccess) return e;
+  const long long warps = groups * ((max_n + 31) / 32);
+  if (warps <= 148) return launch_rank_targets<1>(gr, groups, max_n, b, s);
+  if (warps <= 2 * 148) return launch_rank_targets<2>(gr, groups, max_n, b, s);
+  return launch_rank_targets<4>(gr, groups, max_n, b, s);
 }
 
 }  // namespace winds

@@ -78,7 +78,7 @@ struct BBox {           // ordered-int keys of float bounds (see float_key)
 };
 
 constexpr int kPackFams = 4;
-struct PackArgs {       // bs_chain_count, bs_pack_filaments
+struct PackArgs {       // bs_chain_count, bs_pack
   struct Fam {
     const double *F1, *F2, *gam, *rc;
     long long d0, d2, nf, off;
@@ -87,7 +87,11 @@ struct PackArgs {       // bs_chain_count, bs_pack_filaments
   } fam[kPackFams];
   int nfam, model;
   long long pad_from, pad_to;
-  int pad_block0;
+  int pad_block0, tgt_block0;
+  const double *P;
+  long long ns, nt;
+  double4 *tp_raw;
+  int *tgroup;
   double dcut;
   float4 *pk;
   double4 *ra, *rb;

@@ -305,7 +305,7 @@ int worker_grid(long long n_items, long long resident, int sms, bool f32c) {
 
 // ------------------------------------------------------------- packing
 // chain: order each family along the index with more links between neighbours
-// (bs_pack_filaments), else in input order.
+// (bs_pack), else in input order.
 int pack_inputs(Context *c, const winds_bs_family *fams, int nfam,
                 const TargetSpec &tset, int model, double dcut, cudaStream_t s,
                 long long *nf_real, long long *nf_pad, long long *nt_total, bool chain) {
@@ -322,18 +322,19 @@ int pack_inputs(Context *c, const winds_bs_family *fams, int nfam,
       (rc = c->chaincnt.ensure(2 * kPackFams * sizeof(unsigned long long), s)))
     return rc;
   TargetBufs tb{};
-  if (nt > kBlockSortMax) {
+  const bool counting = sort_by_counting(1, nt);
+  if ((rc = c->tp_raw.ensure(n1 * sizeof(double4), s)) ||
+      (rc = c->keys.ensure(n1 * (counting ? 1 : 2) * sizeof(unsigned), s)))
+    return rc;
+  if (!counting) {
     if (sort_targets_bytes(nt, 1, &tb.sort_bytes) != cudaSuccess)
       return fail(WINDS_BS_ERR_CUDA, "target sort size query failed");
-    if ((rc = c->tp_raw.ensure(n1 * sizeof(double4), s)) ||
-        (rc = c->tgroup.ensure(n1 * sizeof(int), s)) ||
-        (rc = c->keys.ensure(n1 * 2 * sizeof(unsigned), s)) ||
-        (rc = c->vals.ensure(n1 * sizeof(int), s)) ||
+    if ((rc = c->tgroup.ensure(n1 * sizeof(int), s)) || (rc = c->vals.ensure(n1 * sizeof(int), s)) ||
         (rc = c->sort_tmp.ensure(tb.sort_bytes + 256, s)))
       return rc;
   }
   tb.tp = (double4 *)c->tp.p, tb.tp_raw = (double4 *)c->tp_raw.p;
-  tb.tgroup = (int *)c->tgroup.p, tb.vals = (int *)c->vals.p, tb.perm = (int *)c->perm.p;
+  tb.tgroup = counting ? nullptr : (int *)c->tgroup.p, tb.vals = (int *)c->vals.p, tb.perm = (int *)c->perm.p;
   tb.keys = (unsigned long long *)c->keys.p, tb.sort_tmp = c->sort_tmp.p;
   PackedFilaments pf{(float4 *)c->pk.p, (double4 *)c->ra.p, (double4 *)c->rb.p};
   BBox *bb = (BBox *)c->bbox.p;
@@ -342,10 +343,10 @@ int pack_inputs(Context *c, const winds_bs_family *fams, int nfam,
   c->launches += 1;
   c->chained = chain;
   if (e == cudaSuccess)
-    e = launch_pack_families(fams, nfam, chain ? cnt : nullptr, nfp, model, dcut, pf, bb, s,
-                             &c->launches);
-  if (e == cudaSuccess) e = launch_matlab_targets(tset.P, tset.ns, nt, tb, bb, s);
-  c->launches += nt <= 0 ? 0 : (nt <= kBlockSortMax ? 1 : 9);  // 9: with the library's passes
+    e = launch_pack(fams, nfam, chain ? cnt : nullptr, nfp, model, dcut, pf, tset.P, tset.ns, nt, tb,
+                    bb, s, &c->launches);
+  if (e == cudaSuccess) e = launch_order_targets(nt, tb, bb, s);
+  c->launches += nt <= 0 ? 0 : (counting ? 2 : 8);  // 8: with the library's passes
   if (e != cudaSuccess) return cuda_fail(e, "pack kernels");
   *nf_real = nf;
   *nf_pad = nfp;

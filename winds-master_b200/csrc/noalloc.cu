@@ -181,7 +181,8 @@ extern "C" int winds_bs_eval_device_noalloc(const winds_bs_family *fams, int nfa
 
   // ---- carve the scratch array
   size_t sort_bytes = 0;
-  if (nt > kBlockSortMax && sort_targets_bytes(nt, 1, &sort_bytes) != cudaSuccess)
+  const bool counting = sort_by_counting(1, nt);
+  if (!counting && sort_targets_bytes(nt, 1, &sort_bytes) != cudaSuccess)
     return fail(WINDS_BS_ERR_CUDA, "target sort size query failed");
   Carve cv{base};
   BBox *bbox = cv.take<BBox>(1);
@@ -191,13 +192,13 @@ extern "C" int winds_bs_eval_device_noalloc(const winds_bs_family *fams, int nfa
   PackedFilaments pf{cv.take<float4>(nfp * 4), cv.take<double4>(nfp), cv.take<double4>(nfp)};
   unsigned long long *chaincnt = cv.take<unsigned long long>(2 * kPackFams);
   TargetBufs tb{};
-  const long long nd = nt > kBlockSortMax ? nt : 0;  // targets of the device-wide sort
+  const long long nd = counting ? 0 : nt;  // targets of the device-wide sort
   tb.tp = cv.take<double4>(nt);
-  tb.tp_raw = cv.take<double4>(nd);
-  tb.tgroup = cv.take<int>(nd);
+  tb.tp_raw = cv.take<double4>(nt);
+  tb.tgroup = nd ? cv.take<int>(nd) : nullptr;
   tb.vals = cv.take<int>(nd);
   tb.perm = cv.take<int>(nt);
-  tb.keys = cv.take<unsigned long long>(nd);  // one group: two 32-bit keys each
+  tb.keys = reinterpret_cast<unsigned long long *>(cv.take<unsigned>(nt + nd));
   tb.sort_tmp = cv.take<unsigned char>(sort_bytes);
   tb.sort_bytes = sort_bytes;
   Group *groups = cv.take<Group>(1);
@@ -216,9 +217,9 @@ extern "C" int winds_bs_eval_device_noalloc(const winds_bs_family *fams, int nfa
   e = cudaGetLastError();
   if (e == cudaSuccess) e = launch_begin(bbox, ctr, nearc, chaincnt, s);
   if (e == cudaSuccess)
-    e = launch_pack_families(fams, nfam, prec == WINDS_PREC_F32C ? chaincnt : nullptr, nfp,
-                             model, dcut, pf, bbox, s, nullptr);
-  if (e == cudaSuccess) e = launch_matlab_targets(P, pdims[0], nt, tb, bbox, s);
+    e = launch_pack(fams, nfam, prec == WINDS_PREC_F32C ? chaincnt : nullptr, nfp, model, dcut, pf, P,
+                    pdims[0], nt, tb, bbox, s, nullptr);
+  if (e == cudaSuccess) e = launch_order_targets(nt, tb, bbox, s);
   if (e != cudaSuccess) return cuda_fail(e, "noalloc pack/plan kernels");
 
   // ---- direct sum and reduction

@@ -133,15 +133,14 @@ int alloc_all(winds_wake_batch *b) {
       (rc = b->bbox.ensure(sizeof(BBox), s)) || (rc = b->ctr.ensure(64, s)) ||
       (rc = b->err.ensure(64, s)) || (rc = b->nearctr.ensure(64, s)))
     return rc;
-  if (b->max_nodes > kBlockSortMax) {
-    if (sort_targets_bytes(b->nodes, b->ncases, &b->sort_bytes) != cudaSuccess)
-      return fail(WINDS_BS_ERR_CUDA, "target sort size query failed");
-    if ((rc = b->tp_raw.ensure(nt * sizeof(double4), s)) ||
-        (rc = b->tgroup.ensure(nt * sizeof(int), s)) ||
-        (rc = b->keys.ensure(nt * (b->ncases == 1 ? 1 : 2) * sizeof(unsigned long long), s)) ||
-        (rc = b->vals.ensure(nt * sizeof(int), s)))
-      return rc;
-  }
+  const bool counting = sort_by_counting(b->ncases, b->max_nodes);
+  const size_t key = counting ? sizeof(unsigned) : (b->ncases == 1 ? 2 : 4) * sizeof(unsigned);
+  if ((rc = b->tp_raw.ensure(nt * sizeof(double4), s)) || (rc = b->keys.ensure(nt * key, s))) return rc;
+  if (counting) return WINDS_BS_OK;
+  if (sort_targets_bytes(b->nodes, b->ncases, &b->sort_bytes) != cudaSuccess)
+    return fail(WINDS_BS_ERR_CUDA, "target sort size query failed");
+  if ((rc = b->tgroup.ensure(nt * sizeof(int), s)) || (rc = b->vals.ensure(nt * sizeof(int), s)))
+    return rc;
   return b->sort_tmp.ensure(b->sort_bytes + 256, s);
 }
 
@@ -257,8 +256,8 @@ cudaError_t enqueue_eval(winds_wake_batch *b, const double *dom, const double *s
     e = launch_reduce(P<const Tile>(b->tiles), b->n_tiles, P<const Group>(groups),
                       P<const double>(b->part), P<const int>(b->perm), b->tile_cap,
                       P<unsigned>(b->ctr), s, P<const Item>(b->items), live);
-  // live, filaments, targets, sum, reduce; the device-wide sort adds 8
-  launches += b->max_nodes <= kBlockSortMax ? 5 : 13;
+  // live, filaments, targets, keys, order, sum, reduce; the device-wide sort adds 6
+  launches += sort_by_counting(b->ncases, b->max_nodes) ? 7 : 13;
   return e;
 }
 

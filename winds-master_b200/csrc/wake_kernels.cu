@@ -217,7 +217,7 @@ __global__ void wake_targets(const WakeCase *cases, const int *step, int step_ad
   float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
   if (t < n) {
     const int ti = (int)t, jk = ti / c.nst, i = ti - jk * c.nst;
-    tgroup[c.node_off + t] = (int)blockIdx.y;
+    if (tgroup) tgroup[c.node_off + t] = (int)blockIdx.y;
     if (jk % c.na < live_cols(c, *step + step_add)) {
       const long long base = c.node_off * 3 + i + c.nst * 3 * (long long)jk;
       const double x = dom[base], y = dom[base + c.nst], z = dom[base + 2 * c.nst];
@@ -397,35 +397,22 @@ cudaError_t launch_wake_filaments(const WakeCase *cases, int ncases, long long m
   return cudaGetLastError();
 }
 
-// The nodes of one case per group (bs_sort_targets): as wake_targets.
-struct WakeTargets {
+// The nodes of a case are a group.
+struct WakeGroups {
   const WakeCase *cases;
-  const int *step;
-  int step_add;
-  const double *dom;
   __device__ int count(int g) const { return cases[g].nst * cases[g].na * cases[g].nb; }
   __device__ long long offset(int g) const { return cases[g].node_off; }
-  __device__ bool load(int g, int t, double p[3]) const {
-    const int nst = cases[g].nst, na = cases[g].na;
-    const int jk = t / nst, i = t - jk * nst;
-    if (jk % na >= live_cols(cases[g], *step + step_add)) return false;
-    const double *q = dom + cases[g].node_off * 3 + i + nst * 3 * (long long)jk;
-    p[0] = q[0], p[1] = q[nst], p[2] = q[2 * nst];
-    return true;
-  }
 };
 
 cudaError_t launch_wake_targets(const WakeCase *cases, int ncases, long long max_nodes,
                                 long long nodes, const int *step, int step_add, const double *dom,
                                 const TargetBufs &b, BBox *bb, cudaStream_t s) {
-  if (max_nodes <= kBlockSortMax) {
-    WakeTargets src{cases, step, step_add, dom};
-    return launch_block_sort(src, ncases, max_nodes, b.tp, b.perm, bb, s);
-  }
   wake_targets<<<case_grid(max_nodes, ncases, 256), 256, 0, s>>>(cases, step, step_add, dom,
                                                                   b.tp_raw, b.tgroup, bb);
   const cudaError_t e = cudaGetLastError();
-  return e != cudaSuccess ? e : launch_sort_targets(b, nodes, ncases, bb, s);
+  return e != cudaSuccess
+             ? e
+             : launch_order_targets(WakeGroups{cases}, ncases, max_nodes, nodes, b, bb, s);
 }
 
 cudaError_t launch_wake_convect(const WakeCase *cases, int ncases, long long max_nodes,
