@@ -22,6 +22,7 @@
 
 #include "bs_launch.h"
 #include "engine.h"
+#include "host_stage.h"
 #include "winds_bs.h"
 
 namespace winds {
@@ -166,7 +167,7 @@ void shutdown_all() {
                       &c->tgroup, &c->keys, &c->vals, &c->perm, &c->sort_tmp, &c->groups,
                       &c->tiles, &c->items, &c->order, &c->part, &c->bbox, &c->ctr, &c->err,
                       &c->nearctr, &c->chaincnt,
-                      &c->in_P, &c->in_F, &c->out_u})
+                      &c->in_F, &c->out_u})
       b->release();
     c->htab.release();
     c->hstat.release();
@@ -634,20 +635,21 @@ int autotune(Context *c, const std::vector<GroupSpec> &gs, int model, double dcu
   return rc;
 }
 
+// The error word v of the device, cleared there when it is set.
+static int report_error_word(Context *c, unsigned v) {
+  if (!v) return WINDS_BS_OK;
+  cudaMemset(c->err.p, 0, sizeof(unsigned));
+  if (v & kErrWaitTimeout)
+    return fail(WINDS_BS_ERR_TIMEOUT, "a bounded device wait ran out (error word 0x%x)", v);
+  return fail(WINDS_BS_ERR_CUDA, "device reported error word 0x%x", v);
+}
+
 int check_device_error(Context *c, cudaStream_t s) {
   cudaError_t e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return cuda_fail(e, "stream synchronize");
   unsigned *h = static_cast<unsigned *>(c->hstat.p);
   e = cudaMemcpy(h, c->err.p, sizeof(unsigned), cudaMemcpyDeviceToHost);
-  if (e != cudaSuccess) return cuda_fail(e, "error word read");
-  if (*h) {
-    const unsigned v = *h;
-    cudaMemset(c->err.p, 0, sizeof(unsigned));
-    if (v & kErrWaitTimeout)
-      return fail(WINDS_BS_ERR_TIMEOUT, "a bounded device wait ran out (error word 0x%x)", v);
-    return fail(WINDS_BS_ERR_CUDA, "device reported error word 0x%x", v);
-  }
-  return WINDS_BS_OK;
+  return e != cudaSuccess ? cuda_fail(e, "error word read") : report_error_word(c, *h);
 }
 
 }  // namespace winds
@@ -737,37 +739,32 @@ int winds_bs_eval_host(const winds_bs_family *fams, int nfam, const double *P,
     const long long n = fams[k].dims[0] * fams[k].dims[2] * fams[k].dims[3];
     fbytes += (size_t)n * 8 * sizeof(double);
   }
-  if ((rc = c->in_P.ensure(np * 3 * sizeof(double), s)) || (rc = c->in_F.ensure(fbytes + 64, s)) ||
+  if ((rc = c->in_F.ensure(np * 3 * sizeof(double) + fbytes + 64, s)) ||
       (rc = c->out_u.ensure(np * 3 * sizeof(double), s)))
     return rc;
-  cudaError_t e = cudaMemcpyAsync(c->in_P.p, P, np * 3 * sizeof(double), cudaMemcpyHostToDevice, s);
+  StageLease stage;
   std::vector<winds_bs_family> dev(nfam);
+  std::vector<HostSpan> in;
   double *base = (double *)c->in_F.p;
-  for (int k = 0; k < nfam && e == cudaSuccess; ++k) {
+  const auto put = [&](const double *p, long long n) {
+    double *d = base;
+    in.push_back(HostSpan{const_cast<double *>(p), d, (size_t)n * sizeof(double)});
+    base += n;
+    return d;
+  };
+  const double *dP = put(P, 3 * np);
+  for (int k = 0; k < nfam; ++k) {
     const long long n = fams[k].dims[0] * fams[k].dims[2] * fams[k].dims[3];
     dev[k] = fams[k];
-    dev[k].F1 = base;
-    dev[k].F2 = base + 3 * n;
-    dev[k].gamma = base + 6 * n;
-    dev[k].rc = base + 7 * n;
-    if (n > 0) {
-      e = cudaMemcpyAsync((void *)dev[k].F1, fams[k].F1, 3 * n * sizeof(double),
-                          cudaMemcpyHostToDevice, s);
-      if (e == cudaSuccess)
-        e = cudaMemcpyAsync((void *)dev[k].F2, fams[k].F2, 3 * n * sizeof(double),
-                            cudaMemcpyHostToDevice, s);
-      if (e == cudaSuccess)
-        e = cudaMemcpyAsync((void *)dev[k].gamma, fams[k].gamma, n * sizeof(double),
-                            cudaMemcpyHostToDevice, s);
-      if (e == cudaSuccess)
-        e = cudaMemcpyAsync((void *)dev[k].rc, fams[k].rc, n * sizeof(double),
-                            cudaMemcpyHostToDevice, s);
-    }
-    base += 8 * n;
+    dev[k].F1 = put(fams[k].F1, 3 * n);
+    dev[k].F2 = put(fams[k].F2, 3 * n);
+    dev[k].gamma = put(fams[k].gamma, n);
+    dev[k].rc = put(fams[k].rc, n);
   }
+  cudaError_t e = stage.upload(in.data(), (int)in.size(), s);
   if (e != cudaSuccess) return cuda_fail(e, "host to device copy");
   TargetSpec dts = ts;
-  dts.P = (const double *)c->in_P.p;
+  dts.P = dP;
   dts.out = (double *)c->out_u.p;
   const bool seq = prm && (prm->flags & WINDS_BS_FLAG_SEQUENTIAL);
   if (nfam == 0) {
@@ -776,9 +773,10 @@ int winds_bs_eval_host(const winds_bs_family *fams, int nfam, const double *P,
   } else if ((rc = eval_device(c, dev.data(), nfam, dts, prm, s, seq))) {
     return rc;
   }
-  e = cudaMemcpyAsync(uind, c->out_u.p, np * 3 * sizeof(double), cudaMemcpyDeviceToHost, s);
-  if (e != cudaSuccess) return cuda_fail(e, "device to host copy");
-  return check_device_error(c, s);
+  unsigned word = 0;
+  const HostSpan out[] = {{uind, c->out_u.p, np * 3 * sizeof(double)}, {&word, c->err.p, sizeof(word)}};
+  e = stage.download(out, 2, s);
+  return e != cudaSuccess ? cuda_fail(e, "device to host copy") : report_error_word(c, word);
 }
 
 int winds_bs_length_device(const double *F1, const double *F2, const long long dims[4], double *L,
@@ -927,6 +925,9 @@ int winds_bs_selftest_wait_timeout(unsigned long long limit_ns) {
   return check_device_error(c, c->stream);
 }
 
-void winds_bs_shutdown(void) { shutdown_all(); }
+void winds_bs_shutdown(void) {
+  release_stages();
+  shutdown_all();
+}
 
 }  // extern "C"

@@ -70,7 +70,7 @@ struct Context {
   DevBuf chaincnt;
   bool chained = false;  // the packed filaments are a chained stream
   // device copies of host inputs/outputs (host API)
-  DevBuf in_P, in_F, out_u;
+  DevBuf in_F, out_u;
   HostBuf htab, hstat;
   Plan plan;
   // what the uploaded plan was built from: a call with the same groups and

@@ -19,6 +19,7 @@
 
 #include "bs_device.cuh"
 #include "engine.h"
+#include "host_stage.h"
 #include "winds_kin.h"
 
 namespace winds {
@@ -231,15 +232,19 @@ extern "C" int winds_kinematics(const winds_kin_rotor *r, winds_kin_out *out) {
   const long long in_n = nt * (1 + nb + 1 + 6 + 3) + 3 * nst + 3 * ns + nb;
   const long long trail_n = nst * 3 * nt * nb, st_n = ns * 3 * nt * nb;
   const long long out_n = 3 * nt + 3 * trail_n + 3 * st_n + 3 * trail_n + 5 * st_n;
-  double *blk = nullptr;
-  cudaError_t e = cudaMalloc(&blk, (size_t)(in_n + out_n) * sizeof(double));
-  if (e != cudaSuccess) return cuda_fail(e, "kinematics buffers");
-  std::vector<double> h;
-  h.reserve((size_t)in_n);
+  StageLease stage;
+  if (stage.error() != cudaSuccess) return cuda_fail(stage.error(), "kinematics stage");
+  const cudaStream_t s = stage.stream();
+  if (const int rc = stage.scratch().ensure((size_t)(in_n + out_n) * sizeof(double), s)) return rc;
+  double *blk = (double *)stage.scratch().p;
+  HostSpan in[13];
+  int nin = 0;
+  double *next = blk;
   auto put = [&](const double *p, long long n) {
-    const long long off = (long long)h.size();
-    h.insert(h.end(), p, p + n);
-    return blk + off;
+    double *d = next;
+    in[nin++] = HostSpan{const_cast<double *>(p), d, (size_t)n * sizeof(double)};
+    next += n;
+    return d;
   };
   KinDev k;
   k.nt = r->nt, k.nb = r->nb, k.nst = r->nst, k.ns = r->ns;
@@ -269,31 +274,26 @@ extern "C" int winds_kinematics(const winds_kin_rotor *r, winds_kin_out *out) {
   k.bxt = take(trail_n), k.byt = take(trail_n), k.bzt = take(trail_n);
   k.bxn = take(st_n), k.byn = take(st_n), k.bzn = take(st_n), k.vbound = take(st_n),
   k.vblade = take(st_n);
-  e = cudaMemcpy(blk, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice);
+  cudaError_t e = stage.upload(in, nin, s);
   const long long threads = (nst + ns) * nt * nb;
   if (e == cudaSuccess) {
-    kin_hub<<<(unsigned)((nt + 127) / 128), 128>>>(k);
-    kin_points<<<(unsigned)((threads + 127) / 128), 128>>>(k);
-    kin_frames<<<(unsigned)((threads + 127) / 128), 128>>>(k);
+    kin_hub<<<(unsigned)((nt + 127) / 128), 128, 0, s>>>(k);
+    kin_points<<<(unsigned)((threads + 127) / 128), 128, 0, s>>>(k);
+    kin_frames<<<(unsigned)((threads + 127) / 128), 128, 0, s>>>(k);
     e = cudaGetLastError();
   }
-  if (e == cudaSuccess) e = cudaDeviceSynchronize();
-  struct Copy {
-    double *dst;
-    const double *src;
-    long long n;
+  const auto span = [](double *host, double *dev, long long n) {
+    return HostSpan{host, dev, host ? (size_t)n * sizeof(double) : 0};
   };
-  const Copy copies[] = {{out->hub, k.hub, 3 * nt},         {out->lead, k.lead, trail_n},
-                         {out->quarter, k.quarter, trail_n}, {out->trail, k.trail, trail_n},
-                         {out->bound, k.bound, st_n},        {out->colloc, k.colloc, st_n},
-                         {out->end, k.end, st_n},            {out->bxt, k.bxt, trail_n},
-                         {out->byt, k.byt, trail_n},         {out->bzt, k.bzt, trail_n},
-                         {out->bxn, k.bxn, st_n},            {out->byn, k.byn, st_n},
-                         {out->bzn, k.bzn, st_n},            {out->vbound, k.vbound, st_n},
-                         {out->vblade, k.vblade, st_n}};
-  for (const Copy &c : copies)
-    if (e == cudaSuccess && c.dst)
-      e = cudaMemcpy(c.dst, c.src, (size_t)c.n * sizeof(double), cudaMemcpyDeviceToHost);
-  cudaFree(blk);
+  const HostSpan copies[] = {
+      span(out->hub, k.hub, 3 * nt),         span(out->lead, k.lead, trail_n),
+      span(out->quarter, k.quarter, trail_n), span(out->trail, k.trail, trail_n),
+      span(out->bound, k.bound, st_n),       span(out->colloc, k.colloc, st_n),
+      span(out->end, k.end, st_n),           span(out->bxt, k.bxt, trail_n),
+      span(out->byt, k.byt, trail_n),        span(out->bzt, k.bzt, trail_n),
+      span(out->bxn, k.bxn, st_n),           span(out->byn, k.byn, st_n),
+      span(out->bzn, k.bzn, st_n),           span(out->vbound, k.vbound, st_n),
+      span(out->vblade, k.vblade, st_n)};
+  if (e == cudaSuccess) e = stage.download(copies, 15, s);
   return e == cudaSuccess ? WINDS_BS_OK : cuda_fail(e, "kinematics");
 }

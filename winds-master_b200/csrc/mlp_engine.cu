@@ -12,6 +12,7 @@
 #include <vector>
 
 #include "bs_launch.h"
+#include "host_stage.h"
 #include "mlp_engine.h"
 #include "mlp_launch.h"
 
@@ -294,15 +295,25 @@ int winds_mlp_forward_host(winds_mlp *m, const float *x, long long n, float *y) 
   if (n == 0) return WINDS_BS_OK;
   cudaSetDevice(m->dev);
   cudaStream_t s = m->stream;
-  const long long chunk = 1 << 16;
-  for (long long r0 = 0; r0 < n; r0 += chunk) {
-    const long long k = n - r0 < chunk ? n - r0 : chunk;
-    int rc = m->w.ensure(k, false, s);
-    if (!rc) rc = upload_inputs(m, x + r0 * m->n_in, k, s);
-    if (!rc) rc = mlp_forward(m, P<float>(m->w.xraw), k, P<float>(m->w.y), s);
-    if (rc) return rc;
-    cudaError_t e = cudaMemcpyAsync(y + r0, m->w.y.p, k * 4, cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  // rows go up in pieces while the network runs on those before; results come
+  // back together, up to 4M rows at a time
+  const long long chunk = 1 << 15, most = 1 << 22;
+  StageLease stage;
+  int rc;
+  if ((rc = m->w.ensure(std::min(n, chunk), false, s)) || (rc = m->w.y.ensure(std::min(n, most) * 4, s)))
+    return rc;
+  for (long long y0 = 0; y0 < n; y0 += most) {
+    const long long ny = std::min(most, n - y0);
+    for (long long r0 = 0; r0 < ny; r0 += chunk) {
+      const long long k = std::min(chunk, ny - r0);
+      const HostSpan in = {const_cast<float *>(x + (y0 + r0) * m->n_in), m->w.xraw.p,
+                           (size_t)k * m->n_in * sizeof(float)};
+      const cudaError_t e = stage.upload(&in, 1, s);
+      if (e != cudaSuccess) return cuda_fail(e, "mlp input upload");
+      if ((rc = mlp_forward(m, P<float>(m->w.xraw), k, P<float>(m->w.y) + r0, s))) return rc;
+    }
+    const HostSpan out = {y + y0, m->w.y.p, (size_t)ny * 4};
+    const cudaError_t e = stage.download(&out, 1, s);
     if (e != cudaSuccess) return cuda_fail(e, "mlp forward");
   }
   return check_err(m);
@@ -346,8 +357,10 @@ int winds_mlp_train_host(winds_mlp *m, const float *x, const float *t, long long
       (rc = m->idx.ensure(n * 4, s)) || (rc = m->lossbuf.ensure(nbatch * 4, s)) ||
       (rc = m->w.ensure_parts(B, s)))
     return rc;
-  cudaError_t e = upload(m->Xall.p, x, n * m->n_in * 4, s);
-  if (e == cudaSuccess) e = upload(m->Tall.p, t, n * 4, s);
+  StageLease stage;
+  const HostSpan in[] = {{const_cast<float *>(x), m->Xall.p, (size_t)n * m->n_in * 4},
+                         {const_cast<float *>(t), m->Tall.p, (size_t)n * 4}};
+  cudaError_t e = stage.upload(in, 2, s);
   if (e != cudaSuccess) return cuda_fail(e, "mlp training upload");
   std::vector<int> perm(n);
   for (long long i = 0; i < n; ++i) perm[i] = (int)i;

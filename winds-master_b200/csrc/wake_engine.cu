@@ -20,6 +20,7 @@
 
 #include "bs_launch.h"
 #include "engine.h"
+#include "host_stage.h"
 #include "kj_launch.h"
 #include "mlp_engine.h"
 #include "mlp_launch.h"
@@ -463,7 +464,6 @@ cudaError_t enqueue_kj(winds_wake_batch *b, int &launches) {
   return e;
 }
 
-int kj_step_errors(winds_wake_batch *b);
 
 // One step as one graph: the part before the iteration, the lifting line, the
 // commit. Built once, replayed every step.
@@ -490,38 +490,41 @@ int build_step_graph(winds_wake_batch *b) {
   return WINDS_BS_OK;
 }
 
+// An error word of the direct sum's or the network's kernels, cleared where it is set.
+int report_word(unsigned word, unsigned *dev, const char *whose) {
+  if (!word) return WINDS_BS_OK;
+  cudaMemset(dev, 0, sizeof(unsigned));
+  if (word & kErrWaitTimeout)
+    return fail(WINDS_BS_ERR_TIMEOUT, "a bounded wait of %s ran out (error word 0x%x)", whose, word);
+  return fail(WINDS_BS_ERR_CUDA, "%s reported error word 0x%x", whose, word);
+}
+
+// After the work enqueued for a step's iteration, in one read: its iteration count,
+// NaN Cl anywhere, an error word.
+int kj_step_errors(winds_wake_batch *b) {
+  std::vector<int> div(b->ncases);
+  unsigned word = 0, net = 0;
+  int it = 0;
+  const HostSpan v[] = {{div.data(), b->diverged.p, b->ncases * sizeof(int)},
+                        {&word, b->err.p, sizeof(word)},
+                        {&it, b->kj_it.p, sizeof(it)},
+                        {&net, b->mlp ? mlp_err_word(b->mlp) : nullptr, b->mlp ? sizeof(net) : 0}};
+  StageLease stage;
+  const cudaError_t e = stage.download(v, 4, b->stream);
+  if (e != cudaSuccess) return cuda_fail(e, "wake step");
+  for (int k = 0; k < b->ncases; ++k)
+    if (div[k]) return fail(WINDS_BS_ERR_DIVERGED, "case %d: Diverging soln!!! (Cl is NaN)", k);
+  b->kj_evals = it;
+  if (int rc = report_word(net, b->mlp ? mlp_err_word(b->mlp) : nullptr, "the network")) return rc;
+  return report_word(word, P<unsigned>(b->err), "the device");
+}
+
 // The lifting line of one step launched directly; errors before the commit.
 int run_kj(winds_wake_batch *b, int &launches) {
   b->kj_evals = 0;
   if (b->steps_done < b->kj_from) return WINDS_BS_OK;  // the start-up's first step has none
-  cudaError_t e = enqueue_kj(b, launches);
-  int it = 0;
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(&it, b->kj_it.p, sizeof(int), cudaMemcpyDeviceToHost, b->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
-  if (e != cudaSuccess) return cuda_fail(e, "kj iteration");
-  b->kj_evals = it;
-  return kj_step_errors(b);
-}
-
-// After a step's iteration: NaN Cl anywhere, or an error word of the network.
-int kj_step_errors(winds_wake_batch *b) {
-  std::vector<int> div(b->ncases);
-  cudaError_t e = cudaMemcpy(div.data(), b->diverged.p, b->ncases * sizeof(int), cudaMemcpyDeviceToHost);
-  if (e != cudaSuccess) return cuda_fail(e, "kj flags");
-  for (int k = 0; k < b->ncases; ++k)
-    if (div[k]) return fail(WINDS_BS_ERR_DIVERGED, "case %d: Diverging soln!!! (Cl is NaN)", k);
-  if (b->mlp) {
-    unsigned word = 0;
-    e = cudaMemcpy(&word, mlp_err_word(b->mlp), sizeof(word), cudaMemcpyDeviceToHost);
-    if (e != cudaSuccess) return cuda_fail(e, "mlp error word");
-    if (word) {
-      cudaMemset(mlp_err_word(b->mlp), 0, sizeof(unsigned));
-      return fail(word & kErrWaitTimeout ? WINDS_BS_ERR_TIMEOUT : WINDS_BS_ERR_CUDA,
-                  "mlp kernels reported error word 0x%x", word);
-    }
-  }
-  return WINDS_BS_OK;
+  const cudaError_t e = enqueue_kj(b, launches);
+  return e == cudaSuccess ? kj_step_errors(b) : cuda_fail(e, "kj iteration");
 }
 
 // Interactions of step s over all cases and evaluations (the live columns'
@@ -785,14 +788,9 @@ static int autotune_batch(winds_wake_batch *b) {
 // Error word of the direct-sum kernels (bounded waits that ran out).
 static int device_error_word(winds_wake_batch *b) {
   unsigned word = 0;
-  cudaError_t e = cudaMemcpy(&word, b->err.p, sizeof(word), cudaMemcpyDeviceToHost);
-  if (e != cudaSuccess) return cuda_fail(e, "error word read");
-  if (word) {
-    cudaMemset(b->err.p, 0, sizeof(unsigned));
-    return fail(word & kErrWaitTimeout ? WINDS_BS_ERR_TIMEOUT : WINDS_BS_ERR_CUDA,
-                "device reported error word 0x%x", word);
-  }
-  return WINDS_BS_OK;
+  const cudaError_t e = cudaMemcpy(&word, b->err.p, sizeof(word), cudaMemcpyDeviceToHost);
+  return e != cudaSuccess ? cuda_fail(e, "error word read")
+                          : report_word(word, P<unsigned>(b->err), "the device");
 }
 
 static int step_impl(winds_wake_batch *b, int nsteps, int use_graph);
@@ -836,16 +834,9 @@ static int step_impl(winds_wake_batch *b, int nsteps, int use_graph) {
     cudaEventRecord(b->ev0, b->stream);
     for (int k = 0; k < nsteps; ++k) {
       e = cudaGraphLaunch(b->exec_step, b->stream);
-      if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
       if (e != cudaSuccess) return cuda_fail(e, "wake step");
-      int rc = kj_step_errors(b);
-      if (!rc) rc = device_error_word(b);
-      if (rc) return rc;
+      if (const int rc = kj_step_errors(b)) return rc;
       ++b->steps_done;
-      int it = 0;
-      if ((e = cudaMemcpy(&it, b->kj_it.p, sizeof(int), cudaMemcpyDeviceToHost)) != cudaSuccess)
-        return cuda_fail(e, "iteration count");
-      b->kj_evals = it;
     }
     cudaEventRecord(b->ev1, b->stream);
     b->timed_steps = nsteps;
@@ -907,22 +898,21 @@ int winds_wake_get_state(winds_wake_batch *b, int icase, double *dom, double *bo
                          double *trail, double *rc_shed, double *rc_trail, double *uind) {
   if (!b || icase < 0 || icase >= b->ncases) return fail(WINDS_BS_ERR_ARG, "bad case index");
   cudaSetDevice(b->dev);
-  cudaStreamSynchronize(b->stream);
   const WakeCase &c = b->cases[icase];
   const size_t nn = (size_t)c.nst * c.na * c.nb, ns = (size_t)(c.nst - 1) * c.na * c.nb,
                nt = (size_t)c.nst * (c.na - 1) * c.nb, nbd = (size_t)(c.nst - 1) * c.nb;
-  cudaError_t e = cudaSuccess;
-  auto get = [&](double *dst, DevBuf &src, long long off, size_t n) {
-    if (dst && e == cudaSuccess)
-      e = cudaMemcpy(dst, P<double>(src) + off, n * sizeof(double), cudaMemcpyDeviceToHost);
+  auto span = [](double *dst, DevBuf &src, long long off, size_t n) {
+    return HostSpan{dst, P<double>(src) + off, dst ? n * sizeof(double) : 0};
   };
-  get(dom, b->dom, c.node_off * 3, nn * 3);
-  get(bound, b->bound, c.bound_off, nbd);
-  get(shed, b->shed_cur, c.shed_off, ns);
-  get(trail, b->trail_cur, c.trail_off, nt);
-  get(rc_shed, b->rc_s, c.shed_off, ns);
-  get(rc_trail, b->rc_t, c.trail_off, nt);
-  get(uind, b->uind, c.node_off * 3, nn * 3);
+  const HostSpan v[] = {span(dom, b->dom, c.node_off * 3, nn * 3),
+                        span(bound, b->bound, c.bound_off, nbd),
+                        span(shed, b->shed_cur, c.shed_off, ns),
+                        span(trail, b->trail_cur, c.trail_off, nt),
+                        span(rc_shed, b->rc_s, c.shed_off, ns),
+                        span(rc_trail, b->rc_t, c.trail_off, nt),
+                        span(uind, b->uind, c.node_off * 3, nn * 3)};
+  StageLease stage;
+  const cudaError_t e = stage.download(v, 7, b->stream);
   return e == cudaSuccess ? WINDS_BS_OK : cuda_fail(e, "wake state read");
 }
 
