@@ -595,7 +595,8 @@ int autotune(Context *c, const std::vector<GroupSpec> &gs, int model, double dcu
   // (6 targets per lane 1.52 ms, 8 1.67 ms on the 60k-filament wake)
   const int Ts[3] = {2, 3, 4};
   const int KFs[2] = {32, 64};
-  const double Ws[3] = {16.0, 32.0, 64.0};
+  // more than 32 never was the fastest; 8 is on 30k targets (1.40 ms, 16: 1.45)
+  const double Ws[3] = {8.0, 16.0, 32.0};
   float best_ms = 1e30f;
   TuneChoice bc;
   cudaEvent_t e0, e1;
