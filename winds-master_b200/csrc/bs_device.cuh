@@ -442,6 +442,13 @@ __device__ __forceinline__ bool pair64_short(const double4 A, const double4 B, c
   return true;
 }
 
+// First statement of a kernel launched with launch_after: waits for the kernels
+// before it in the stream, all their writes included, and lets the next one's blocks
+// take their places (where they wait in turn).
+__device__ __forceinline__ void after_previous() {
+  asm volatile("griddepcontrol.wait;\n\tgriddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // What an evaluation starts from: an empty bounding box and the work queue at its
 // start (one block of at least 32 threads).
 __device__ __forceinline__ void begin_evaluation(BBox *bb, unsigned *ctr) {

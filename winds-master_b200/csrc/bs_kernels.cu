@@ -37,6 +37,7 @@ namespace winds {
 // --------------------------------------------------------------- packing
 __global__ void bs_begin(BBox *bb, unsigned *ctr, unsigned long long *near,
                          unsigned long long *cnt) {
+  after_previous();
   begin_evaluation(bb, ctr);
   if (threadIdx.x < 2) near[threadIdx.x] = 0ull;
   if (threadIdx.x < 2 * kPackFams) cnt[threadIdx.x] = 0ull;
@@ -61,6 +62,7 @@ __device__ __forceinline__ bool same_point(const double *__restrict__ F2, long l
 
 // Up to kPackFams families per launch, each with its run of blocks.
 __global__ void bs_chain_count(const PackArgs a) {
+  after_previous();
   int k = 0;
   while (k + 1 < a.nfam && (int)blockIdx.x >= a.fam[k + 1].block0) ++k;
   const PackArgs::Fam &m = a.fam[k];
@@ -86,6 +88,7 @@ __global__ void bs_chain_count(const PackArgs a) {
 // filaments (far away, zero length, zero circulation), those past them pack the
 // targets of a MATLAB array P [ns, 3, ...].
 __global__ void bs_pack(const PackArgs a) {
+  after_previous();
   float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
   if ((int)blockIdx.x >= a.tgt_block0) {
     const long long t = (long long)(blockIdx.x - a.tgt_block0) * blockDim.x + threadIdx.x;
@@ -138,6 +141,7 @@ __global__ void bs_pack(const PackArgs a) {
 template <class KEY>
 __global__ void bs_target_keys(const double4 *__restrict__ tp, const int *__restrict__ tgroup,
                                long long n, const BBox *bb, KEY *keys, int *vals) {
+  after_previous();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
   const double4 p = tp[t];
@@ -158,6 +162,7 @@ __global__ void bs_target_keys(const double4 *__restrict__ tp, const int *__rest
 
 __global__ void bs_gather_targets(const double4 *__restrict__ src, const int *__restrict__ perm,
                                   long long n, double4 *dst) {
+  after_previous();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t < n) dst[t] = src[perm[t]];
 }
@@ -864,6 +869,7 @@ struct MinBlocks {
 
 template <int T, int KF, int MODEL>
 __global__ void __launch_bounds__(kThreads, MinBlocks<T>::value) bs_f32c(const F32cArgs a) {
+  after_previous();
   static_assert(KF % 32 == 0 && KF <= 64, "one screen word per 32 filaments, a head bit per filament");
   static_assert(T % 2 == 0 && T <= 8, "targets go in pairs, near-singular bits eight to a filament");
   constexpr int S = StageSmem<KF>::kStages;
@@ -1002,6 +1008,7 @@ static F64Form f64_form(int model, double n, bool sequential) {
 
 template <int FORM>
 __global__ void __launch_bounds__(kF64Threads) bs_f64(const F32cArgs a) {
+  after_previous();
   constexpr bool kShort = FORM != kF64Ref;
   constexpr int kModel = FORM == kF64Cutoff ? kCoreCutoff : kCoreVatistas;
   __shared__ double4 sA[2][kF64Tile], sB[2][kF64Tile], sC[kShort ? 2 : 1][kShort ? kF64Tile : 1];
@@ -1084,6 +1091,7 @@ __global__ void __launch_bounds__(32 * kReduceWarps)
     bs_reduce(const Tile *__restrict__ tiles, const Group *__restrict__ groups,
               const double *__restrict__ part, const int *__restrict__ perm, int tile_cap,
               const Item *__restrict__ items, const GroupLive *__restrict__ live, unsigned *ctr) {
+  after_previous();
   __shared__ double s_sum[kReduceWarps][3][32];
   if (blockIdx.x + blockIdx.y == 0 && threadIdx.x == 0) *ctr = 0u;
   Tile tl = tiles[blockIdx.x];
@@ -1246,11 +1254,10 @@ int f32c_occupancy(int model, int T, int KF) {
   return 1;
 }
 
-static const void *f64_kernel(int model, double n, bool sequential) {
+using F64Kernel = void (*)(const F32cArgs);
+static F64Kernel f64_kernel(int model, double n, bool sequential) {
   const F64Form f = f64_form(model, n, sequential);
-  return f == kF64Ref      ? (const void *)bs_f64<kF64Ref>
-         : f == kF64Cutoff ? (const void *)bs_f64<kF64Cutoff>
-                           : (const void *)bs_f64<kF64Vatistas>;
+  return f == kF64Ref ? bs_f64<kF64Ref> : f == kF64Cutoff ? bs_f64<kF64Cutoff> : bs_f64<kF64Vatistas>;
 }
 
 int f64_occupancy(int model, double n, bool sequential) {
@@ -1262,14 +1269,13 @@ int f64_occupancy(int model, double n, bool sequential) {
 }
 
 cudaError_t launch_f64(const F32cArgs &a, bool sequential, int grid, cudaStream_t s) {
-  void *args[] = {const_cast<F32cArgs *>(&a)};
-  return cudaLaunchKernel(f64_kernel(a.model, a.n, sequential), dim3((unsigned)grid),
-                          dim3(kF64Threads), args, 0, s);
+  f64_kernel(a.model, a.n, sequential)<<<grid, kF64Threads, 0, s>>>(a);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_begin(BBox *bb, unsigned *ctr, unsigned long long *near, unsigned long long *cnt,
                          cudaStream_t s) {
-  bs_begin<<<1, 32, 0, s>>>(bb, ctr, near, cnt);
+  launch_after(bs_begin, 1, 32, 0, s, bb, ctr, near, cnt);
   return cudaGetLastError();
 }
 
@@ -1312,14 +1318,14 @@ cudaError_t launch_pack(const winds_bs_family *fams, int nfam, unsigned long lon
         if (e != cudaSuccess) return e;
       }
       first = false;
-      bs_chain_count<<<(unsigned)blocks, bs, 0, s>>>(a);
+      launch_after(bs_chain_count, (unsigned)blocks, bs, 0, s, a);
       if (launches) ++*launches;
     }
     blocks += (a.pad_to - a.pad_from + bs - 1) / bs;
     a.tgt_block0 = (int)blocks;
     blocks += (a.nt + bs - 1) / bs;
     if (blocks > 0) {
-      bs_pack<<<(unsigned)blocks, bs, 0, s>>>(a);
+      launch_after(bs_pack, (unsigned)blocks, bs, 0, s, a);
       if (launches) ++*launches;
     }
     const cudaError_t e = cudaGetLastError();
@@ -1331,7 +1337,7 @@ cudaError_t launch_pack(const winds_bs_family *fams, int nfam, unsigned long lon
 cudaError_t launch_gather_targets(const double4 *src, const int *perm, long long n, double4 *dst,
                                   cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
-  bs_gather_targets<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(src, perm, n, dst);
+  launch_after(bs_gather_targets, (unsigned)((n + 255) / 256), 256, 0, s, src, perm, n, dst);
   return cudaGetLastError();
 }
 
@@ -1364,13 +1370,14 @@ cudaError_t launch_sort_targets(const TargetBufs &b, long long n, int groups, co
   cudaError_t e;
   if (groups == 1) {
     unsigned *k0 = reinterpret_cast<unsigned *>(b.keys), *k1 = k0 + n;
-    bs_target_keys<<<grid, 256, 0, s>>>(b.tp_raw, b.tgroup, n, bb, k0, b.vals);
+    launch_after(bs_target_keys<unsigned>, grid, 256, 0, s, b.tp_raw, b.tgroup, n, bb, k0, b.vals);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     e = cub::DeviceRadixSort::SortPairs(b.sort_tmp, bytes, (const unsigned *)k0, k1,
                                         (const int *)b.vals, b.perm, (int)n, 0, 31, s);
   } else {
     unsigned long long *k0 = b.keys, *k1 = k0 + n;
-    bs_target_keys<<<grid, 256, 0, s>>>(b.tp_raw, b.tgroup, n, bb, k0, b.vals);
+    launch_after(bs_target_keys<unsigned long long>, grid, 256, 0, s, b.tp_raw, b.tgroup, n, bb,
+                 k0, b.vals);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     e = cub::DeviceRadixSort::SortPairs(b.sort_tmp, bytes, (const unsigned long long *)k0, k1,
                                         (const int *)b.vals, b.perm, (int)n, 0,
@@ -1381,8 +1388,8 @@ cudaError_t launch_sort_targets(const TargetBufs &b, long long n, int groups, co
 
 cudaError_t launch_target_keys(const double4 *tp, long long n, const BBox *bb, float *keys,
                                cudaStream_t s) {
-  bs_target_keys<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(tp, (const int *)nullptr, n, bb, keys,
-                                                             (int *)nullptr);
+  launch_after(bs_target_keys<float>, (unsigned)((n + 255) / 256), 256, 0, s, tp,
+               (const int *)nullptr, n, bb, keys, (int *)nullptr);
   return cudaGetLastError();
 }
 
@@ -1396,7 +1403,8 @@ cudaError_t launch_reduce(const Tile *tiles, int n_tiles, const Group *groups, c
   if (n_tiles <= 0) return cudaSuccess;
   if (live && !items) return cudaErrorInvalidValue;
   const dim3 grid((unsigned)n_tiles, (unsigned)(tile_cap + 31) / 32);
-  bs_reduce<<<grid, 32 * kReduceWarps, 0, s>>>(tiles, groups, part, perm, tile_cap, items, live, ctr);
+  launch_after(bs_reduce, grid, 32 * kReduceWarps, 0, s, tiles, groups, part, perm, tile_cap,
+               items, live, ctr);
   return cudaGetLastError();
 }
 

@@ -3,10 +3,34 @@
 
 #include <cuda_runtime.h>
 
+#include <utility>
+
 #include "bs_types.h"
 #include "winds_bs.h"
 
 namespace winds {
+
+// Launches a kernel that begins with after_previous() so that its blocks may be set
+// up while the kernel before it in the stream still runs: an evaluation's seven
+// launches on 3.1k targets take 117 us instead of 126. Not for the direct sums, whose
+// workers are as many per SM: set up beside blocks of the kernel before they are
+// spread unevenly (7.6k targets 404 us instead of 325).
+template <class... P, class... A>
+cudaError_t launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                         A &&...args) {
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c = {};
+  c.gridDim = grid;
+  c.blockDim = block;
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  c.attrs = &at;
+  c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, kernel, std::forward<A>(args)...);
+}
+
 
 struct PackedFilaments {
   float4 *pk;  // records: 4 float4 per filament (layout in bs_types.h)

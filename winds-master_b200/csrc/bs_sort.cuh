@@ -81,6 +81,7 @@ template <int R, class GROUPS>
 __global__ void __launch_bounds__(32 * kRankWarps)
     bs_rank_targets(const GROUPS gr, const float *__restrict__ keys,
                     const double4 *__restrict__ tp_raw, double4 *tp, int *perm) {
+  after_previous();
   extern __shared__ float4 s_key[];  // a run of `run` keys per warp
   __shared__ float s_cnt[kRankWarps][32 * R];
   const int g = blockIdx.y, n = gr.count(g), i0 = blockIdx.x * 32 * R;
@@ -147,8 +148,8 @@ cudaError_t launch_rank_targets(const GROUPS &gr, int groups, long long max_n, c
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
   const dim3 grid((unsigned)((max_n + 32 * R - 1) / (32 * R)), (unsigned)groups);
-  bs_rank_targets<R><<<grid, 32 * kRankWarps, smem, s>>>(
-      gr, reinterpret_cast<const float *>(b.keys), b.tp_raw, b.tp, b.perm);
+  launch_after(bs_rank_targets<R, GROUPS>, grid, 32 * kRankWarps, smem, s, gr,
+               reinterpret_cast<const float *>(b.keys), b.tp_raw, b.tp, b.perm);
   return cudaGetLastError();
 }
 

@@ -16,6 +16,7 @@
 #include <cmath>
 
 #include "bs_device.cuh"
+#include "bs_launch.h"
 #include "kj_launch.h"
 #include "wake_types.h"
 
@@ -25,6 +26,7 @@ namespace winds {
 __global__ void kj_targets(const WakeCase *cases, const KJCase *kc, const int *step,
                            const double *ll, double4 *tp, BBox *bb, int *iters, int *converged,
                            int *diverged, int *it_max) {
+  after_previous();
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     iters[blockIdx.y] = converged[blockIdx.y] = diverged[blockIdx.y] = 0;
     if (blockIdx.y == 0) *it_max = 0;
@@ -187,6 +189,7 @@ __device__ __forceinline__ void send_pair(uint32_t dst, uint32_t bar, double g,
 }
 
 __global__ void __launch_bounds__(kSolveThreads) kj_solve(const KJSolveArgs a) {
+  after_previous();
   extern __shared__ __align__(16) double kj_smem[];
   __shared__ uint64_t arrived[2];
   cg::cluster_group cl = cg::this_cluster();
@@ -397,6 +400,7 @@ __global__ void __launch_bounds__(kSolveThreads) kj_solve(const KJSolveArgs a) {
 __global__ void kj_finish(const WakeCase *cases, const KJCase *kc, const int *iters,
                           const int *converged, const int *it_max, const double *uindb_conv,
                           double *uindb) {
+  after_previous();
   const int ci = blockIdx.y;
   const int n = 3 * (cases[ci].nst - 1) * cases[ci].nb;
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -417,6 +421,7 @@ __global__ void kj_features(const WakeCase *cases, const KJCase *kc, const int *
                             const double *byn, const double *bzn, const double *uindb,
                             const double *st_r, const double *st_c, const double *st_tw,
                             const double *azim, float *x) {
+  after_previous();
   const WakeCase c = cases[blockIdx.y];
   const KJCase k = kc[blockIdx.y];
   const int ns = c.nst - 1;
@@ -463,6 +468,7 @@ __global__ void kj_apply_guess(const WakeCase *cases, const KJCase *kc, const in
                                const int *st_lift, const double2 *st_stall,
                                const double *aoa_prev, const float *y, const float *out_scale,
                                const float *feat, const float *base, double *bound) {
+  after_previous();
   const WakeCase c = cases[blockIdx.y];
   const KJCase k = kc[blockIdx.y];
   const int ns = c.nst - 1;
@@ -488,6 +494,7 @@ __global__ void kj_dloads(const WakeCase *cases, const KJCase *kc, const int *st
                           const double *aoa, const double *st_tw, const double *chord,
                           const double *st_rr, const double *st_dr, const double *rpm,
                           const double *pitch, double *dl) {
+  after_previous();
   const WakeCase c = cases[blockIdx.y];
   const KJCase k = kc[blockIdx.y];
   const int ns = c.nst - 1;
@@ -527,6 +534,7 @@ __global__ void kj_dloads(const WakeCase *cases, const KJCase *kc, const int *st
 // Rotor totals, summed over stations and then blades as sum(sum(dT,1),4).
 __global__ void kj_sum_loads(const WakeCase *cases, const KJCase *kc, int ncases,
                              const double *dl, double *out) {
+  after_previous();
   const int ci = blockIdx.x * blockDim.x + threadIdx.x;
   if (ci >= ncases) return;
   const WakeCase c = cases[ci];
@@ -545,8 +553,8 @@ __global__ void kj_sum_loads(const WakeCase *cases, const KJCase *kc, int ncases
 cudaError_t launch_kj_targets(const WakeCase *cases, const KJCase *kc, int ncases, int max_st,
                               const int *step, const double *ll, double4 *tp, BBox *bb, int *iters,
                               int *converged, int *diverged, int *it_max, cudaStream_t s) {
-  kj_targets<<<dim3((max_st + 127) / 128, ncases), 128, 0, s>>>(cases, kc, step, ll, tp, bb, iters,
-                                                                converged, diverged, it_max);
+  launch_after(kj_targets, dim3((max_st + 127) / 128, ncases), 128, 0, s, cases, kc, step, ll, tp,
+               bb, iters, converged, diverged, it_max);
   return cudaGetLastError();
 }
 
@@ -573,20 +581,22 @@ cudaError_t launch_kj_solve(const KJSolveArgs &a, int ncases, cudaStream_t s) {
   cfg.blockDim = dim3(kSolveThreads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = kCluster;
   at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.numAttrs = 2;
   return cudaLaunchKernelEx(&cfg, kj_solve, a);
 }
 
 cudaError_t launch_kj_finish(const WakeCase *cases, const KJCase *kc, int ncases, int max_st,
                              const int *iters, const int *converged, const int *it_max,
                              const double *uindb_conv, double *uindb, cudaStream_t s) {
-  kj_finish<<<dim3((3 * max_st + 127) / 128, ncases), 128, 0, s>>>(cases, kc, iters, converged,
-                                                                   it_max, uindb_conv, uindb);
+  launch_after(kj_finish, dim3((3 * max_st + 127) / 128, ncases), 128, 0, s, cases, kc, iters,
+               converged, it_max, uindb_conv, uindb);
   return cudaGetLastError();
 }
 
@@ -597,9 +607,8 @@ cudaError_t launch_kj_features(const WakeCase *cases, const KJCase *kc, int ncas
                                const double *uindb, const double *st_r,
                                const double *st_c, const double *st_tw, const double *azim,
                                float *x, cudaStream_t s) {
-  kj_features<<<dim3((max_st + 127) / 128, ncases), 128, 0, s>>>(
-      cases, kc, step, bound, bound_last, bound_last2, vblade, bxn, byn, bzn, uindb, st_r, st_c,
-      st_tw, azim, x);
+  launch_after(kj_features, dim3((max_st + 127) / 128, ncases), 128, 0, s, cases, kc, step, bound,
+               bound_last, bound_last2, vblade, bxn, byn, bzn, uindb, st_r, st_c, st_tw, azim, x);
   return cudaGetLastError();
 }
 
@@ -608,8 +617,8 @@ cudaError_t launch_kj_apply_guess(const WakeCase *cases, const KJCase *kc, int n
                                   const double *aoa_prev, const float *y, const float *out_scale,
                                   const float *feat, const float *base, double *bound,
                                   cudaStream_t s) {
-  kj_apply_guess<<<dim3((max_st + 127) / 128, ncases), 128, 0, s>>>(
-      cases, kc, step, st_lift, st_stall, aoa_prev, y, out_scale, feat, base, bound);
+  launch_after(kj_apply_guess, dim3((max_st + 127) / 128, ncases), 128, 0, s, cases, kc, step,
+               st_lift, st_stall, aoa_prev, y, out_scale, feat, base, bound);
   return cudaGetLastError();
 }
 
@@ -619,11 +628,11 @@ cudaError_t launch_kj_loads(const WakeCase *cases, const KJCase *kc, int ncases,
                             const double *chord, const double *st_rr, const double *st_dr,
                             const double *rpm, const double *pitch, double *dl, double *out,
                             cudaStream_t s) {
-  kj_dloads<<<dim3((max_st + 127) / 128, ncases), 128, 0, s>>>(
-      cases, kc, step, vblade, cl, cd, aoa, st_tw, chord, st_rr, st_dr, rpm, pitch, dl);
+  launch_after(kj_dloads, dim3((max_st + 127) / 128, ncases), 128, 0, s, cases, kc, step, vblade,
+               cl, cd, aoa, st_tw, chord, st_rr, st_dr, rpm, pitch, dl);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  kj_sum_loads<<<(ncases + 127) / 128, 128, 0, s>>>(cases, kc, ncases, dl, out);
+  launch_after(kj_sum_loads, (ncases + 127) / 128, 128, 0, s, cases, kc, ncases, dl, out);
   return cudaGetLastError();
 }
 

@@ -28,6 +28,7 @@
 
 #include <algorithm>
 
+#include "bs_device.cuh"
 #include "bs_launch.h"
 #include "engine.h"
 #include "winds_bs.h"
@@ -59,6 +60,7 @@ int scratch_address(unsigned char **out) {
 __global__ void bs_noalloc_plan(Group *groups, Tile *tiles, Item *items, unsigned *err, double *out,
                                 long long nt, long long ns_p, int nf_pad, int tile_cap,
                                 int chunk, int n_chunks, int n_tiles) {
+  after_previous();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i == 0) {
     *err = 0u;
@@ -211,9 +213,8 @@ extern "C" int winds_bs_eval_device_noalloc(const winds_bs_family *fams, int nfa
 
   // ---- plan, state carried over from the previous call, and packing (the same
   // kernels as winds_bs_eval_device)
-  bs_noalloc_plan<<<(n_items + 255) / 256, 256, 0, s>>>(groups, tiles, items, err, uind, nt,
-                                                        pdims[0], (int)nfp, tile_cap, (int)chunk,
-                                                        n_chunks, n_tiles);
+  launch_after(bs_noalloc_plan, (n_items + 255) / 256, 256, 0, s, groups, tiles, items, err, uind,
+               nt, pdims[0], (int)nfp, tile_cap, (int)chunk, n_chunks, n_tiles);
   e = cudaGetLastError();
   if (e == cudaSuccess) e = launch_begin(bbox, ctr, nearc, chaincnt, s);
   if (e == cudaSuccess)

@@ -87,6 +87,7 @@ __device__ __forceinline__ double trail_col(const WakeCase &c, const double *bou
 __global__ void wake_bookkeep(const WakeCase *cases, const int *step, int step_add,
                               const double *bound, const double *trail_prev, double *shed,
                               double *trail) {
+  after_previous();
   const WakeCase c = cases[blockIdx.y];
   const int u = blockIdx.x * blockDim.x + threadIdx.x;  // (column j, blade b)
   const int na_l = live_cols(c, *step + step_add);
@@ -129,6 +130,7 @@ __global__ void wake_filaments(const WakeCase *cases, const int *step, int step_
                                double *len_t, double *rc_s, double *rc_t, const double *rc_in_s,
                                const double *rc_in_t, int model, double dcut, PackedFilaments pf,
                                BBox *bb) {
+  after_previous();
   const WakeCase c = cases[blockIdx.y];
   const long long f = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
@@ -211,6 +213,7 @@ __global__ void wake_filaments(const WakeCase *cases, const int *step, int step_
 // which sorts them after every live target of the case.
 __global__ void wake_targets(const WakeCase *cases, const int *step, int step_add,
                              const double *dom, double4 *tp, int *tgroup, BBox *bb) {
+  after_previous();
   const WakeCase c = cases[blockIdx.y];
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long n = (long long)c.nst * c.na * c.nb;
@@ -247,6 +250,7 @@ __global__ void wake_convect(const WakeCase *cases, const int *step, int mode, c
                              const double *uind_pred, double *vel, const double *h1,
                              const double *h2, const double *h3, const double *quarter,
                              const double *trailing, const double *wind, double *out) {
+  after_previous();
   const WakeCase c = cases[blockIdx.y];
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long n = (long long)c.nst * c.na * c.nb;
@@ -317,6 +321,7 @@ __global__ void wake_commit(const WakeCase *cases, int *step, double *dom, const
                             double *vel, double *h1, double *h2, double *h3, int keep_hist,
                             double *trail_prev, const double *trail_cur, double *len_old_s,
                             const double *len_s, double *len_old_t, const double *len_t) {
+  after_previous();
   const WakeCase c = cases[blockIdx.y];
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long nn = (long long)c.nst * c.na * c.nb;
@@ -351,6 +356,7 @@ __global__ void wake_commit(const WakeCase *cases, int *step, double *dom, const
 // puts the work queue at its start.
 __global__ void wake_live(const WakeCase *cases, int ncases, const int *step, int step_add,
                           int mode, GroupLive *live, BBox *bb, unsigned *ctr) {
+  after_previous();
   if (blockIdx.x == 0) begin_evaluation(bb, ctr);
   const int ci = blockIdx.x * blockDim.x + threadIdx.x;
   if (ci >= ncases) return;
@@ -378,8 +384,8 @@ cudaError_t launch_wake_bookkeep(const WakeCase *cases, int ncases, long long ma
                                  const int *step, int step_add, const double *bound,
                                  const double *trail_prev, double *shed, double *trail,
                                  cudaStream_t s) {
-  wake_bookkeep<<<case_grid(max_cols, ncases, 128), 128, 0, s>>>(cases, step, step_add, bound,
-                                                                  trail_prev, shed, trail);
+  launch_after(wake_bookkeep, case_grid(max_cols, ncases, 128), 128, 0, s, cases, step, step_add,
+               bound, trail_prev, shed, trail);
   return cudaGetLastError();
 }
 
@@ -391,9 +397,9 @@ cudaError_t launch_wake_filaments(const WakeCase *cases, int ncases, long long m
                                   double *rc_t, const double *rc_in_s, const double *rc_in_t,
                                   int model, double dcut, const PackedFilaments &pf, BBox *bb,
                                   cudaStream_t s) {
-  wake_filaments<<<case_grid(max_fil_pad, ncases, 256), 256, 0, s>>>(
-      cases, step, step_add, ser, dom, shed, trail, len_old_s, len_old_t, have_old, stretch,
-      len_s, len_t, rc_s, rc_t, rc_in_s, rc_in_t, model, dcut, pf, bb);
+  launch_after(wake_filaments, case_grid(max_fil_pad, ncases, 256), 256, 0, s, cases, step,
+               step_add, ser, dom, shed, trail, len_old_s, len_old_t, have_old, stretch, len_s,
+               len_t, rc_s, rc_t, rc_in_s, rc_in_t, model, dcut, pf, bb);
   return cudaGetLastError();
 }
 
@@ -407,8 +413,8 @@ struct WakeGroups {
 cudaError_t launch_wake_targets(const WakeCase *cases, int ncases, long long max_nodes,
                                 long long nodes, const int *step, int step_add, const double *dom,
                                 const TargetBufs &b, BBox *bb, cudaStream_t s) {
-  wake_targets<<<case_grid(max_nodes, ncases, 256), 256, 0, s>>>(cases, step, step_add, dom,
-                                                                  b.tp_raw, b.tgroup, bb);
+  launch_after(wake_targets, case_grid(max_nodes, ncases, 256), 256, 0, s, cases, step, step_add,
+               dom, b.tp_raw, b.tgroup, bb);
   const cudaError_t e = cudaGetLastError();
   return e != cudaSuccess
              ? e
@@ -421,9 +427,8 @@ cudaError_t launch_wake_convect(const WakeCase *cases, int ncases, long long max
                                 double *vel, const double *h1, const double *h2, const double *h3,
                                 const double *quarter, const double *trailing, const double *wind,
                                 double *out, cudaStream_t s) {
-  wake_convect<<<case_grid(max_nodes, ncases, 256), 256, 0, s>>>(
-      cases, step, mode, dom, uind, carry, pred, uind_pred, vel, h1, h2, h3, quarter, trailing,
-      wind, out);
+  launch_after(wake_convect, case_grid(max_nodes, ncases, 256), 256, 0, s, cases, step, mode, dom,
+               uind, carry, pred, uind_pred, vel, h1, h2, h3, quarter, trailing, wind, out);
   return cudaGetLastError();
 }
 
@@ -432,15 +437,16 @@ cudaError_t launch_wake_commit(const WakeCase *cases, int ncases, long long max_
                                double *h2, double *h3, int keep_hist, double *trail_prev,
                                const double *trail_cur, double *len_old_s, const double *len_s,
                                double *len_old_t, const double *len_t, cudaStream_t s) {
-  wake_commit<<<case_grid(max_slots, ncases, 256), 256, 0, s>>>(
-      cases, step, dom, dom_new, vel, h1, h2, h3, keep_hist, trail_prev, trail_cur, len_old_s,
-      len_s, len_old_t, len_t);
+  launch_after(wake_commit, case_grid(max_slots, ncases, 256), 256, 0, s, cases, step, dom,
+               dom_new, vel, h1, h2, h3, keep_hist, trail_prev, trail_cur, len_old_s, len_s,
+               len_old_t, len_t);
   return cudaGetLastError();
 }
 
 cudaError_t launch_wake_live(const WakeCase *cases, int ncases, const int *step, int step_add,
                              int mode, GroupLive *live, BBox *bb, unsigned *ctr, cudaStream_t s) {
-  wake_live<<<(ncases + 127) / 128, 128, 0, s>>>(cases, ncases, step, step_add, mode, live, bb, ctr);
+  launch_after(wake_live, (ncases + 127) / 128, 128, 0, s, cases, ncases, step, step_add, mode,
+               live, bb, ctr);
   return cudaGetLastError();
 }
 
