@@ -47,16 +47,22 @@ __global__ void kj_targets(const WakeCase *cases, const KJCase *kc, const int *s
 }
 
 // MATLAB interp1(x, y, xi) of two tables: linear, NaN outside [x(1), x(end)].
+// lo: the interval of the last call, where the search starts (from one iteration to
+// the next it seldom changes), and of this one.
 __device__ void interp1(const double *x, const double *y, const double *z, int n, double xi,
-                        double &yi, double &zi) {
+                        double &yi, double &zi, int &last) {
   if (!(xi >= __ldg(x) && xi <= __ldg(x + n - 1))) {
     yi = zi = NAN;
     return;
   }
-  int lo = 0, hi = n - 1;
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (__ldg(x + mid) <= xi) lo = mid; else hi = mid;
+  int lo = last, hi = lo + 1;
+  if (hi >= n || !(__ldg(x + lo) <= xi && xi < __ldg(x + hi))) {
+    lo = 0, hi = n - 1;
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (__ldg(x + mid) <= xi) lo = mid; else hi = mid;
+    }
+    last = lo;
   }
   const double t = (xi - __ldg(x + lo)) / (__ldg(x + hi) - __ldg(x + lo));
   yi = __ldg(y + lo) + t * (__ldg(y + hi) - __ldg(y + lo));
@@ -83,7 +89,9 @@ __device__ void interp1(const double *x, const double *y, const double *z, int n
 // then forms all own circulations by itself. The values travel as asynchronous
 // stores that complete on an mbarrier of the receiver: with a cluster barrier
 // instead, 4300 of an iteration's 10000 cycles went into it. Latency bounds the
-// rest: the span sums, the row sums and the station update are chains. Every
+// rest: the row sums, the station update and the stores' way are one chain of some
+// 5000 cycles (99 us for 30 iterations on 17 nodes; 124 with the span sums as a
+// chain, a search of the whole table and a butterfly for the residual). Every
 // loop ends after maxiter iterations, every wait within the time limit.
 namespace cg = cooperative_groups;
 constexpr int kCluster = 8;
@@ -127,7 +135,7 @@ __device__ __forceinline__ OwnFilament own_filament(const WakeCase &c, const dou
 // the frame (9), vblade (3), |vblade| chord / 2 and the fixed velocity (3); and
 // what its last update gave: the velocity (3), cl, cd and aoa, kept here until
 // the end (a store to global memory would hold up every cluster barrier).
-constexpr int kStation = 22;
+constexpr int kStation = 24;
 __device__ __forceinline__ void load_station(const KJSolveArgs &a, const WakeCase &c,
                                              const KJCase &k, int s, int t, double *st) {
   const int ns = c.nst - 1, b = t / ns, i = t - b * ns;
@@ -143,13 +151,16 @@ __device__ __forceinline__ void load_station(const KJSolveArgs &a, const WakeCas
   }
   st[12] = 0.5 * sqrt(st[9] * st[9] + st[10] * st[10] + st[11] * st[11]) *
            a.chord[k.station_off + i];
+  int *table = reinterpret_cast<int *>(st + 22);
+  const int fo2 = k.foil_base + a.foil[k.station_off + i];
+  table[0] = a.foil_off[fo2], table[1] = a.foil_off[fo2 + 1], table[2] = 0;
 }
 
 // A station's update with induced velocity u; returns the updated circulation,
 // the residual's bits in *res (0, and the circulation unchanged, where Cl is
 // NaN).
-__device__ __forceinline__ double station_update(const KJSolveArgs &a, double *st, int ci, int o0,
-                                                 int o1, const double u[3], double bound,
+__device__ __forceinline__ double station_update(const KJSolveArgs &a, double *st, int ci,
+                                                 const double u[3], double bound,
                                                  unsigned long long *res) {
   double rot[3];
 #pragma unroll
@@ -158,7 +169,9 @@ __device__ __forceinline__ double station_update(const KJSolveArgs &a, double *s
   const double tu = st[9] + rot[0], tv = st[10] + rot[1];
   const double aoa = atan2(-tv, tu) * (180.0 / kPi);
   double cl, cd;
-  interp1(a.aoa_t + o0, a.cl_t + o0, a.cd_t + o0, o1 - o0, aoa, cl, cd);
+  int *table = reinterpret_cast<int *>(st + 22);
+  const int o0 = table[0];
+  interp1(a.aoa_t + o0, a.cl_t + o0, a.cd_t + o0, table[1] - o0, aoa, cl, cd, table[2]);
   st[16] = u[0], st[17] = u[1], st[18] = u[2];
   st[19] = cl, st[20] = cd, st[21] = aoa;
   *res = 0ull;
@@ -257,34 +270,25 @@ __global__ void __launch_bounds__(kSolveThreads) kj_solve(const KJSolveArgs a) {
   // terms are zeroed in the direct sum (BiotSavart.m:111)
   const auto circulation = [&](const double2 *B) {
     const auto put = [&](int f, double g) { sG[f] = isfinite(g) ? g : 0.0; };
+    bool bad = false;
     for (int t = tid; t < c.nb * c.nst; t += kSolveThreads) {
       const int b = t / c.nst, i = t - b * c.nst;
       const double hi = i < ns ? B[i + ns * b].x : 0.0, lo = i > 0 ? B[i - 1 + ns * b].x : 0.0;
+      bad = bad || !isfinite(hi);
       put(n_shed + t, hi - lo);
-      if (i < ns) put(2 * ns * b + i, hi);
+      // shed column 1: C_1 - C_0, where C_0, a running sum of differences from the
+      // first station on, is hi itself (formed as a sum it took 1200 of 6700 cycles)
+      if (i < ns) put(2 * ns * b + i, hi), put(2 * ns * b + ns + i, sC[i + ns * b] - hi);
     }
-    if (lane == 0)  // one warp per blade: the span sums are chains
-      for (int b = warp; b < c.nb; b += kSolveWarps) {
-        double cum = 0.0, lo = 0.0;
-        for (int i0 = 0; i0 < ns; i0 += 8) {
-          double h[8], g[8];
-#pragma unroll
-          for (int q = 0; q < 8; ++q) {
-            const int i = min(i0 + q, ns - 1) + ns * b;
-            h[q] = B[i].x;
-            g[q] = sC[i];
-          }
-#pragma unroll
-          for (int q = 0; q < 8; ++q) {
-            cum += h[q] - lo;
-            lo = h[q];
-            g[q] -= cum;
-          }
-#pragma unroll
-          for (int q = 0; q < 8; ++q)
-            if (i0 + q < ns) put(2 * ns * b + ns + i0 + q, g[q]);
-        }
+    if (!__syncthreads_or(bad)) return;
+    // unless one is not finite, which the sum passes on to the stations after it
+    for (int b = tid; b < c.nb; b += kSolveThreads) {
+      double cum = 0.0;
+      for (int i = 0; i < ns; ++i) {
+        cum += B[i + ns * b].x - (i > 0 ? B[i - 1 + ns * b].x : 0.0);
+        put(2 * ns * b + ns + i, sC[i + ns * b] - cum);
       }
+    }
     __syncthreads();
   };
   // velocity at point tt of this CTA, in every lane of the warp
@@ -329,9 +333,7 @@ __global__ void __launch_bounds__(kSolveThreads) kj_solve(const KJSolveArgs a) {
       double g = 0.0;
       unsigned long long r = 0ull;
       if (lane == 0) {
-        const int fo = k.foil_base + __ldg(a.foil + k.station_off + i);
-        g = station_update(a, sS + kStation * tt, ci, __ldg(a.foil_off + fo),
-                           __ldg(a.foil_off + fo + 1), u, sB[cur][t].x, &r);
+        g = station_update(a, sS + kStation * tt, ci, u, sB[cur][t].x, &r);
       }
       g = __shfl_sync(0xffffffffu, g, 0);
       r = __shfl_sync(0xffffffffu, r, 0);
@@ -355,8 +357,9 @@ __global__ void __launch_bounds__(kSolveThreads) kj_solve(const KJSolveArgs a) {
     }
     unsigned long long r = 0ull;  // largest residual: the bits of non-negative doubles order them
     for (int t = lane; t < nt; t += 32) r = max(r, (unsigned long long)__double_as_longlong(sB[nxt][t].y));
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) r = max(r, __shfl_xor_sync(0xffffffffu, r, o));
+    const unsigned top = __reduce_max_sync(0xffffffffu, (unsigned)(r >> 32));
+    const unsigned low = __reduce_max_sync(0xffffffffu, (unsigned)(r >> 32) == top ? (unsigned)r : 0u);
+    r = (unsigned long long)top << 32 | low;
     res = __longlong_as_double((long long)r);
     done = res <= a.tol;
     ++it;
