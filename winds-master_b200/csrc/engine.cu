@@ -376,16 +376,17 @@ static int log2_bucket(long long n) {
   return b;
 }
 
-// Untuned tiling: more targets per lane spread a filament's loads and the
-// screen over more pairs, fewer keep the warp's ball of targets small. Measured
-// in input order or chained: 2 against 4 targets per lane 82 against 82 us on
-// 3.2k targets, 4 against 6 (T = 3) 1.51 against 1.52 ms on 30k targets and
-// 13.1 against 12.1 ms on 89k.
+// Untuned tiling: more targets per lane spread a filament's loads and the screen
+// over more pairs, fewer keep the warp's ball of targets small; more items balance
+// the workers better, fewer cost less around the sum. Evaluations on the chained
+// layout: 4 targets a lane against 2 117 and 135 us on 3.1k targets, 4 against 6
+// (T = 3) 509 and 536 us on 14k, 1588 and 1552 on 30k; 16 items a worker against 32
+// 513 and 553 us on 14k, 1570 and 1599 on 30k.
 TuneChoice default_choice(long long nt) {
   TuneChoice ch;
-  ch.T = nt >= 49152 ? 3 : (nt >= 2048 ? 4 : 2);
+  ch.T = nt >= 24576 ? 3 : (nt >= 2048 ? 4 : 2);
   ch.KF = 64;
-  ch.waves = 32.0;
+  ch.waves = 16.0;
   return ch;
 }
 

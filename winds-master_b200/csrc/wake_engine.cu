@@ -2,7 +2,7 @@
 //
 // One batch holds every case's state in shared device buffers. A step is a
 // fixed sequence of kernel launches on the batch's stream:
-//   bookkeeping -> [pack filaments + targets -> sort -> direct sum -> reduce]
+//   bookkeeping -> [pack filaments, targets -> order -> direct sum -> reduce]
 //   -> convect (fe/ab2/ab4, or pcc predictor) -> (pcc: bookkeeping for p+1
 //   -> [direct sum at the predicted nodes] -> corrector) -> commit.
 // All sizes are fixed at creation (each wake has a capacity of na columns),
