@@ -432,11 +432,11 @@ def batch_start_value(seed=12, n_train=48, n_val=8, steps=10, relax=0.3, tol=1e-
 def wake_kj_bench(rcases, cases, tol=1e-6, relax=0.3, maxiter=200, warm=3, timed=3, mlp=None):
     """The 64-case batch with the lifting line and rotor loads: every pcc step
     runs the Kutta-Joukowski fixed point to the same tolerance on every path.
-    Fast: FP32c, one CUDA graph per step (the iteration a conditional node),
+    Fast: FP32c, one CUDA graph per step (the iteration one of its launches),
     started from the previous step's circulation (the reference), from its
     extrapolation alone, and from the extrapolation plus the network (when
-    given). Host loop: the same FP32c batch with the host reading the
-    convergence flag every iteration. Plain: each case alone, FP64, eager.
+    given). Host loop: the same FP32c batch launched kernel by kernel, the
+    lifting line's flags read before the commit. Plain: each case alone, FP64, eager.
     ``warm`` untimed steps, then ``timed`` steps; iterations are summed over
     the timed steps and split by case subset: converged on both the fast and
     the plain path at every timed step, and the rest (stations past the
@@ -663,8 +663,8 @@ def e2e_run_bench(steps, ncases=16, ages=1440, seed=5, plain_cases=2):
             "power_history_W": f["P"].sum(1).round(1).tolist(),
             "mlp_training_s": round(train_s, 2), "mlp_base": mlp_base, "mlp_output_shrink": mlp_shrink,
             "mlp_validation": mlp_val, "mlp_bases_tried": mlp_tried,
-            "timing": "CUDA events around each step (fast paths: the lifting-line loop runs inside "
-            "the step's graph; plain path: the host waits on a per-iteration convergence flag, its "
+            "timing": "CUDA events around each step (fast paths: the lifting-line iteration is one "
+            "launch of the step's graph; plain path: launched kernel by kernel, its "
             f"time per step measured on {len(p['idx'])} of the {ncases} equal-size cases and scaled "
             "to all of them)"}
 

@@ -3,8 +3,9 @@
 // BiotSavart_sh kernels of cuda/source/BiotSavartMex.cu:131-193.
 //
 // Kernels
+//   bs_begin           counters and bounding box at the start of an evaluation
 //   bs_chain_count,    MATLAB-layout F1/F2/gamma/rc -> 64-byte records (+ FP64
-//   bs_pack  copies), the device-side replacement of the host crunch_f
+//   bs_pack            copies), the device-side replacement of the host crunch_f
 //                      / crunch_rg packing (BiotSavartMex.cu:316-357), in input
 //                      order or laid out along the wake's lines of filaments
 //                      (x2 of a record = x1 of the one before, but for marked
@@ -18,7 +19,9 @@
 //                      pairs in FP64 with all 32 lanes; each interaction
 //                      reuses the previous record's endpoint rsqrt, and groups
 //                      distant from the warp's targets run in an expanded form
-//   bs_f64             plain FP64 direct sum (the comparison GPU path)
+//   bs_target_keys     places on a Hilbert curve (the order: bs_sort.cuh)
+//   bs_f64             FP64 direct sum: short forms of the terms, or the reference's
+//                      sequence in order
 //   bs_reduce          deterministic sum of the per-chunk partials, written in
 //                      MATLAB layout (reassem_uind, :383-401)
 //   bs_length          filament lengths (core/FilamentLength.m:27-44)
@@ -1082,10 +1085,10 @@ __global__ void __launch_bounds__(kF64Threads) bs_f64(const F32cArgs a) {
 // A block sums 32 consecutive targets of a tile: each warp a run of the tile's
 // items in order, lanes the targets, then the warps' sums in order. (One thread
 // per target, all items in one chain of loads, took 30 us on the 3.1k-target
-// wake; spread over eight warps 12.) With a live table, only the live targets of a tile are written, from the
-// items before the group's live filament end (a tile's items cover increasing
-// filament ranges, so those come first). The last kernel of an evaluation: it
-// leaves the work queue at its start.
+// wake; spread over eight warps 12.) With a live table, only the live targets of a
+// tile are written, from the items before the group's live filament end (a tile's
+// items cover increasing filament ranges, so those come first). The last kernel of
+// an evaluation: it leaves the work queue at its start.
 constexpr int kReduceWarps = 8;
 __global__ void __launch_bounds__(32 * kReduceWarps)
     bs_reduce(const Tile *__restrict__ tiles, const Group *__restrict__ groups,
