@@ -247,7 +247,7 @@ __device__ __forceinline__ float column_sums(float (&v)[32]) {
 // threads on one tile, whose gelu' of three layers and accumulators take all 512
 // columns of tensor memory. As one launch per GEMM, with activations through
 // memory, 100k rows forward took 236 us of device time and a step on 4096 rows
-// 349 us; now 97 and 73 us.
+// 349 us; now 97 and 54 us (73 with the weight gradients' parts row by row).
 template <bool TRAIN>
 __global__ void __launch_bounds__(kNetThreads, 1) mlp_net(const MlpNetArgs g) {
   extern __shared__ __align__(1024) unsigned char net_smem[];
@@ -498,10 +498,11 @@ __global__ void __launch_bounds__(kNetThreads, 1) mlp_net(const MlpNetArgs g) {
       };
       put_dz(sm.w[0]);
       // Weight gradients of the pair's 256 rows are one chain of MMAs: the first
-      // CTA's accumulator goes through memory into the second's.
+      // CTA's accumulator goes through memory into the second's. In parts (but W1's)
+      // four columns of all rows lie together, so that a warp's rows are one run.
       float *pw = g.part_w + (long long)(blockIdx.x / 2) * kMlpPartW;
       const auto chain_in = [&](uint32_t acc, int L) {
-        const float *src = pw + (L == 0 ? row * kMlpInPad : mlp_part_w(L) + row * kMlpWidth + c0);
+        const float *src = pw + (L == 0 ? row * kMlpInPad : mlp_part_w(L) + c0 * kTileM + 4 * row);
         if (L == 0 && colg > 0) return;
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
@@ -509,24 +510,25 @@ __global__ void __launch_bounds__(kNetThreads, 1) mlp_net(const MlpNetArgs g) {
           float w[16];
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
-            const float4 u = __ldcg(reinterpret_cast<const float4 *>(src + 16 * c) + q);
+            const float4 u = __ldcg(reinterpret_cast<const float4 *>(
+                src + (L == 0 ? 4 * q : (16 * c + 4 * q) * kTileM)));
             w[4 * q] = u.x, w[4 * q + 1] = u.y, w[4 * q + 2] = u.z, w[4 * q + 3] = u.w;
           }
           tmem_st16(acc + lane_base + (L == 0 ? 0 : c0 + 16 * c), w);
         }
       };
       const auto chain_out = [&](uint32_t acc, int L) {
-        float *dst = pw + (L == 0 ? row * kMlpInPad : mlp_part_w(L) + row * kMlpWidth + c0);
+        float *dst = pw + (L == 0 ? row * kMlpInPad : mlp_part_w(L) + c0 * kTileM + 4 * row);
         if (L == 0 && colg > 0) return;
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
           if (L == 0 && c > 0) break;
           float w[16];
           tmem_ld16(acc + lane_base + (L == 0 ? 0 : c0 + 16 * c), w);
-          float4 *o = reinterpret_cast<float4 *>(dst + 16 * c);
 #pragma unroll
           for (int q = 0; q < 4; ++q)
-            o[q] = make_float4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
+            *reinterpret_cast<float4 *>(dst + (L == 0 ? 4 * q : (16 * c + 4 * q) * kTileM)) =
+                make_float4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
         }
       };
       const auto chain_wait = [&](int k) {  // second CTA: the first's k-th output is there
@@ -616,7 +618,7 @@ __global__ void __launch_bounds__(kNetThreads, 1) mlp_net(const MlpNetArgs g) {
 // c2 = 1 - b2^t and decoupled weight decay wd) or the gradient itself. The last
 // element is the loss.
 __global__ void mlp_update(const MlpUpdateArgs a) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i > kMlpLoss) return;
   const float *p;
   long long stride;
@@ -627,8 +629,11 @@ __global__ void mlp_update(const MlpUpdateArgs a) {
     const int L = i < mlp_off_w(1) ? 0 : 1 + (i - mlp_off_w(1)) / 16512;
     if (i >= mlp_off_b(L))  // of a tile
       p = a.part_b + L * kMlpWidth + (i - mlp_off_b(L)), stride = 3 * kMlpWidth, count = a.tiles;
-    else  // of a pair of tiles
-      p = a.part_w + mlp_part_w(L) + (i - mlp_off_w(L)), stride = kMlpPartW, count = (a.tiles + 1) / 2;
+    else {  // of a pair of tiles, four columns of all rows together (but for W1)
+      const int t = i - mlp_off_w(L);
+      p = a.part_w + mlp_part_w(L) + t, stride = kMlpPartW, count = (a.tiles + 1) / 2;
+      if (L > 0) i = mlp_off_w(L) + ((t >> 2) & 127) * kMlpWidth + (t >> 9) * 4 + (t & 3);
+    }
   }
   float s = 0.f;
 #pragma unroll 8
