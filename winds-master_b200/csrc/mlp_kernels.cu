@@ -24,6 +24,7 @@
 #include <cuda_bf16.h>
 
 #include "bs_device.cuh"
+#include "bs_launch.h"
 #include "mlp_launch.h"
 
 namespace winds {
@@ -250,6 +251,7 @@ __device__ __forceinline__ float column_sums(float (&v)[32]) {
 // 349 us; now 97 and 54 us (73 with the weight gradients' parts row by row).
 template <bool TRAIN>
 __global__ void __launch_bounds__(kNetThreads, 1) mlp_net(const MlpNetArgs g) {
+  after_previous();
   extern __shared__ __align__(1024) unsigned char net_smem[];
   using Smem = NetSmem<TRAIN>;
   Smem &sm = *reinterpret_cast<Smem *>(net_smem);
@@ -618,6 +620,7 @@ __global__ void __launch_bounds__(kNetThreads, 1) mlp_net(const MlpNetArgs g) {
 // c2 = 1 - b2^t and decoupled weight decay wd) or the gradient itself. The last
 // element is the loss.
 __global__ void mlp_update(const MlpUpdateArgs a) {
+  after_previous();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i > kMlpLoss) return;
   const float *p;
@@ -675,12 +678,14 @@ cudaError_t launch_net(const MlpNetArgs &g, int grid, cudaStream_t s) {
   c.blockDim = dim3(kNetThreads);
   c.dynamicSmemBytes = smem;
   c.stream = s;
-  cudaLaunchAttribute at;
-  at.id = cudaLaunchAttributeClusterDimension;
-  at.val.clusterDim.x = 2;
-  at.val.clusterDim.y = at.val.clusterDim.z = 1;
-  c.attrs = &at;
-  c.numAttrs = TRAIN ? 1 : 0;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = 2;
+  at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+  c.attrs = at;
+  c.numAttrs = TRAIN ? 2 : 1;
   return cudaLaunchKernelEx(&c, mlp_net<TRAIN>, g);
 }
 
@@ -700,8 +705,7 @@ cudaError_t launch_mlp_gradient(const MlpNetArgs &g, cudaStream_t s) {
 }
 
 cudaError_t launch_mlp_update(const MlpUpdateArgs &a, cudaStream_t s) {
-  mlp_update<<<blocks(kMlpLoss + 1, 128), 128, 0, s>>>(a);
-  return cudaGetLastError();
+  return launch_after(mlp_update, blocks(kMlpLoss + 1, 128), 128, 0, s, a);
 }
 
 cudaError_t launch_mlp_to_bf16(const float *theta, __nv_bfloat16 *theta_bf, long long n,
