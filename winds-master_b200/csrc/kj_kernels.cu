@@ -214,6 +214,11 @@ __global__ void __launch_bounds__(kSolveThreads) kj_solve(const KJSolveArgs a) {
   const int per = (nt + kCluster - 1) / kCluster;
   const int t0 = rank * per;
   const int cnt = max(0, min(per, nt - t0));
+  // CTAs of the exchange: those that own points (42 points leave the last none, as
+  // fewer than 8 leave several). Nobody would wait for another, so a buffer it still
+  // reads would be filled again; it goes on to the end. With the vectors in memory
+  // cluster barriers keep all CTAs in step.
+  const int parts = a.vec_smem ? (nt + per - 1) / per : kCluster;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   for (int tt = tid; tt < cnt; tt += kSolveThreads)  // the start value, kept for the caller
     a.guess[c.bound_off + t0 + tt] = a.bound[c.bound_off + t0 + tt];
@@ -322,7 +327,7 @@ __global__ void __launch_bounds__(kSolveThreads) kj_solve(const KJSolveArgs a) {
   int it = 0;
   bool done = false;
   double res = 0.0;
-  while (it < a.maxiter && !done) {
+  while (rank < parts && it < a.maxiter && !done) {
     const int cur = it & 1, nxt = cur ^ 1;
     if (a.vec_smem && tid == 0) mbar_arrive_expect_tx(&arrived[nxt], 16u * (unsigned)nt);
     circulation(sB[cur]);
@@ -337,9 +342,9 @@ __global__ void __launch_bounds__(kSolveThreads) kj_solve(const KJSolveArgs a) {
       }
       g = __shfl_sync(0xffffffffu, g, 0);
       r = __shfl_sync(0xffffffffu, r, 0);
-      if (lane < kCluster) {
-        // a buffer is written again only after every CTA sent what it formed
-        // from it, two iterations on
+      if (lane < parts) {
+        // a buffer is written again only after every CTA of the exchange sent what
+        // it formed from it, two iterations on
         if (a.vec_smem)
           send_pair(cluster_address(sB[nxt] + t, lane), cluster_address(&arrived[nxt], lane), g, r);
         else
