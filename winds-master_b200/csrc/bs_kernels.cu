@@ -833,10 +833,10 @@ __device__ __forceinline__ bool f32c_item(const F32cArgs &a, const Item &it, uns
         __syncwarp();
       }
     }
-    // Every lane is done with the stage (tile and near list): refill it with
-    // tile i + S. Lanes wrote to it (prepared records, near list): each orders
-    // its own accesses before the copy.
-    if (issued < ntiles) fence_proxy_async_smem();
+    // Every lane is done with the stage (tile and near list). Lanes wrote to it
+    // (prepared records, near list): each orders its own accesses before the copy
+    // that fills it next, tile i + S here or a tile of the warp's next item.
+    fence_proxy_async_smem();
     __syncwarp();
     if (lane == 0 && issued < ntiles) {
       issue_stage<KF>(a, stages + st * kB, &full[st], it.f_begin + issued * KF);
