@@ -210,8 +210,6 @@ struct StageSmem {
   static constexpr int kBytes = KF * 64;
   // two stages: a warp's tile takes ~5-50 us, a bulk copy ~2 us
   static constexpr int kStages = 2;
-  // tiles per Kahan fold: the FP32 partial sums span 64 filaments
-static constexpr int kFold = 64 / KF;
 };
 
 // Shared memory of one worker: its filament stages, the Kahan state of its
@@ -426,8 +424,9 @@ __device__ __forceinline__ void chain_start(const Fil &f, const float2 (&npx)[NP
 //   cut-off   every target is at least r from it with r^4 >= 2^24 d |L|^2, so
 //             the denominator's d |L|^2 gg^2 <= 2^-24 <= 2^-24 e (e >= 1 there).
 // Rounding: |x1 - P|^2 is formed from terms of at most |q|^2 + 2|q||p| + |p|^2
-// with |p| <= |q| / kDistantRatio. Error against FP64 over the wakes of 6k to
-// 175k filaments (2-norm, all targets): 4.3e-8 to 5.0e-8, as without this form.
+// with |p| <= |q| / kDistantRatio. The form is the more exact one: with it at three
+// radii the error against FP64 (2-norm, wakes of 3k to 175k filaments, steps of one to
+// eight rotors) is 2 to 15% larger, and the core left out or not makes no difference.
 constexpr float kDistantRatio = 1.5f;
 // squared distances for which no product of the form leaves FP32's range, and
 // |M|^2 |q|^2 for which the fourth power of the cross product does not
@@ -564,6 +563,28 @@ __device__ __forceinline__ bool f32c_item(const F32cArgs &a, const Item &it, uns
   float2 ax[NP], ay[NP], az[NP];
 #pragma unroll
   for (int p = 0; p < NP; ++p) ax[p] = ay[p] = az[p] = make_float2(0.f, 0.f);
+  // The FP32 sums' rounding, more than the terms', sets the error, and the chained order
+  // of a wake puts the large terms of a target next to one another. So a near sum spans
+  // eight filaments before it joins the others, and these join the Kahan state after
+  // each tile, and before its second half where both halves have near groups. Error
+  // against FP64 (2-norm) of a step of eight rotors: 4.7e-8 (Vatistas core) and 4.2e-8
+  // (cut-off) with one sum over 64 filaments, now 3.5e-8 and 3.2e-8 (without chains, in
+  // input order: 3.7e-8 and 3.3e-8). The sums take 1 to 4% longer for it: 11.8 -> 11.9
+  // ms on the large wake, 195 -> 203 us on 7.6k targets. (A second level of sums, over
+  // 32, or two sets for the distant form cost registers: up to 10%.)
+  const auto fold = [&] {
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+      const int sl = lane * T + 2 * p;
+      kahan_add(s_k[0 * 32 * T + sl], s_k[1 * 32 * T + sl], ax[p].x);
+      kahan_add(s_k[2 * 32 * T + sl], s_k[3 * 32 * T + sl], ay[p].x);
+      kahan_add(s_k[4 * 32 * T + sl], s_k[5 * 32 * T + sl], az[p].x);
+      kahan_add(s_k[0 * 32 * T + sl + 1], s_k[1 * 32 * T + sl + 1], ax[p].y);
+      kahan_add(s_k[2 * 32 * T + sl + 1], s_k[3 * 32 * T + sl + 1], ay[p].y);
+      kahan_add(s_k[4 * 32 * T + sl + 1], s_k[5 * 32 * T + sl + 1], az[p].y);
+      ax[p] = ay[p] = az[p] = make_float2(0.f, 0.f);
+    }
+  };
 
   int i = 0;
   for (; i < ntiles; ++i) {
@@ -726,10 +747,14 @@ __device__ __forceinline__ bool f32c_item(const F32cArgs &a, const Item &it, uns
                              -s_p[(2 * T + 2 * p + 1) * 32 + lane]);
         ti[p] = make_float2(0.f, 0.f);
       }
+      float2 gx[NP], gy[NP], gz[NP];  // over eight filaments
+#pragma unroll
+      for (int p = 0; p < NP; ++p) gx[p] = gy[p] = gz[p] = make_float2(0.f, 0.f);
       int last = -2;
 #pragma unroll 1
       for (unsigned gm = ~gdist & kGroups; gm; gm &= gm - 1u) {
         const int gr = __ffs(gm) - 1;
+        if (KF == 64 && gr >= 8 && last < 8 && last >= 0) fold();
         const unsigned hg = group_heads(gr) | (gr != last + 1 ? 1u : 0u);
         last = gr;
         const bool near_some = (careful >> gr) & 1u;
@@ -745,9 +770,18 @@ __device__ __forceinline__ bool f32c_item(const F32cArgs &a, const Item &it, uns
           unsigned m = 0;
 #pragma unroll
           for (int p = 0; p < NP; ++p)
-            interact<MODEL>(npx[p], npy[p], npz[p], f, Rn2, near_some, co2, co_on, ax[p], ay[p],
-                            az[p], m, 1u << (2 * p), 2u << (2 * p), ti[p]);
+            interact<MODEL>(npx[p], npy[p], npz[p], f, Rn2, near_some, co2, co_on, gx[p], gy[p],
+                            gz[p], m, 1u << (2 * p), 2u << (2 * p), ti[p]);
           nbits |= m << (kPer * j);
+        }
+        if ((gr & 1) || gm < (2u << gr)) {  // the second of a pair of groups, or the last
+#pragma unroll
+          for (int p = 0; p < NP; ++p) {
+            ax[p] = __fadd2_rn(ax[p], gx[p]);
+            ay[p] = __fadd2_rn(ay[p], gy[p]);
+            az[p] = __fadd2_rn(az[p], gz[p]);
+            gx[p] = gy[p] = gz[p] = make_float2(0.f, 0.f);
+          }
         }
         if (near_some) {
           s_nb[gr * 32 + lane] = (typename NearBits<T>::type)nbits;
@@ -756,20 +790,7 @@ __device__ __forceinline__ bool f32c_item(const F32cArgs &a, const Item &it, uns
       }
     }
     __syncwarp();
-    // Kahan-fold the partial sums into the per-target totals every 64 filaments.
-    if ((i + 1) % StageSmem<KF>::kFold == 0 || i + 1 == ntiles) {
-#pragma unroll
-      for (int p = 0; p < NP; ++p) {
-        const int sl = lane * T + 2 * p;
-        kahan_add(s_k[0 * 32 * T + sl], s_k[1 * 32 * T + sl], ax[p].x);
-        kahan_add(s_k[2 * 32 * T + sl], s_k[3 * 32 * T + sl], ay[p].x);
-        kahan_add(s_k[4 * 32 * T + sl], s_k[5 * 32 * T + sl], az[p].x);
-        kahan_add(s_k[0 * 32 * T + sl + 1], s_k[1 * 32 * T + sl + 1], ax[p].y);
-        kahan_add(s_k[2 * 32 * T + sl + 1], s_k[3 * 32 * T + sl + 1], ay[p].y);
-        kahan_add(s_k[4 * 32 * T + sl + 1], s_k[5 * 32 * T + sl + 1], az[p].y);
-        ax[p] = ay[p] = az[p] = make_float2(0.f, 0.f);
-      }
-    }
+    fold();
     // Near-singular pairs of this tile: the reference formula in FP64, added to
     // the owner's Kahan state as an exact hi + lo pair. In rounds, every lane
     // lists the next kList of its pairs in the consumed stage (its groups in
