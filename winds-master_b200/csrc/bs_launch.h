@@ -75,8 +75,12 @@ struct TargetBufs {
 // radix sort in shared memory: 31 us on 3.2k, 121 on 16k.) More groups share the
 // same units, so the line is their sum of squares.
 constexpr long long kCountingMax = 360ll * 1000 * 1000;
+constexpr long long kCountingTargets = 18973;  // most of one group
+static_assert(kCountingTargets * kCountingTargets <= kCountingMax &&
+                  (kCountingTargets + 1) * (kCountingTargets + 1) > kCountingMax,
+              "largest group that is counted");
 inline bool sort_by_counting(long long groups, long long max_n) {
-  return max_n <= 65536 && groups * max_n * max_n <= kCountingMax;
+  return max_n <= kCountingTargets && groups * max_n * max_n <= kCountingMax;
 }
 // Packs the families (device arrays) one after the other, in input order or
 // (cnt: as launch_begin leaves it) each in the order with more links between

@@ -139,14 +139,21 @@ __global__ void __launch_bounds__(32 * kRankWarps)
   perm[off + (int)r] = (int)(off + i);
 }
 
+// Shared memory of a block for groups of up to n targets.
+constexpr int rank_smem(long long n) {
+  return ((int)((n + kRankWarps - 1) / kRankWarps) + 3) / 4 * kRankWarps * (int)sizeof(float4);
+}
+
 template <int R, class GROUPS>
 cudaError_t launch_rank_targets(const GROUPS &gr, int groups, long long max_n, const TargetBufs &b,
                                 cudaStream_t s) {
-  const int run = ((int)((max_n + kRankWarps - 1) / kRankWarps) + 3) / 4;
-  const int smem = run * kRankWarps * (int)sizeof(float4);
-  const cudaError_t e = cudaFuncSetAttribute(bs_rank_targets<R, GROUPS>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  // The attribute is the function's, for all threads: always the largest group's size, so
+  // that no call can set less between another's setting and its launch.
+  const cudaError_t e =
+      cudaFuncSetAttribute(bs_rank_targets<R, GROUPS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           rank_smem(kCountingTargets));
   if (e != cudaSuccess) return e;
+  const int smem = rank_smem(max_n);
   const dim3 grid((unsigned)((max_n + 32 * R - 1) / (32 * R)), (unsigned)groups);
   launch_after(bs_rank_targets<R, GROUPS>, grid, 32 * kRankWarps, smem, s, gr,
                reinterpret_cast<const float *>(b.keys), b.tp_raw, b.tp, b.perm);
