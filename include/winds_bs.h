@@ -195,6 +195,12 @@ int winds_bs_fp32_peak(double *tflops);
  * when the timeout was detected and reported; the context stays usable. */
 int winds_bs_selftest_wait_timeout(unsigned long long limit_ns);
 
+/* Target-order self-test: the places of n targets P [n,3] of one group (host
+ * arrays, n up to 18973, the sizes ordered by counting), of which those with
+ * unused[t] != 0 come last as the unused slots of a growing wake do. perm[k] is
+ * the target at place k. */
+int winds_bs_selftest_order(const double *P, const int *unused, long long n, int *perm);
+
 /* Frees every device buffer, stream and event of every device context
  * (the mexAtExit hook of the MEX layer). */
 void winds_bs_shutdown(void);

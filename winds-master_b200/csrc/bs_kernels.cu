@@ -140,7 +140,8 @@ __global__ void bs_pack(const PackArgs a) {
 
 // Sort key of a target: group id above the 30-bit Hilbert position in the
 // targets' bounding box (bit 30: the target is unused, and sorts after every
-// live target of its group); for counting, the position's leading 24 bits.
+// live target of its group); for counting, the position's leading 24 bits, of which
+// the last value is the unused targets' (kUnusedKey, bs_sort.cuh).
 template <class KEY>
 __global__ void bs_target_keys(const double4 *__restrict__ tp, const int *__restrict__ tgroup,
                                long long n, const BBox *bb, KEY *keys, int *vals) {
@@ -153,7 +154,7 @@ __global__ void bs_target_keys(const double4 *__restrict__ tp, const int *__rest
   const float hi[3] = {key_float(bb->tmax[0]), key_float(bb->tmax[1]), key_float(bb->tmax[2])};
   const unsigned h = hilbert_key(q, lo, hi);
   if constexpr (sizeof(KEY) == 4 && !std::is_integral<KEY>::value) {
-    keys[t] = p.w != 0.0 ? 16777216.f : (float)(h >> 6);  // 8 bits a coordinate
+    keys[t] = p.w != 0.0 ? kUnusedKey : fminf((float)(h >> 6), kUnusedKey - 1.f);  // 8 bits a coordinate
   } else {
     KEY code = h;
     if (p.w != 0.0) code |= (KEY)1 << 30;

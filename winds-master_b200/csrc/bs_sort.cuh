@@ -72,11 +72,12 @@ struct OneGroup {
 
 // A block places 32 R targets of a group, R a lane; each of its warps counts a run
 // of the group's keys, read by the warp into shared memory and from there four at a
-// time. Keys are whole numbers below 2^25 as floats, so that a comparison is a
-// saturated difference, at the full rate of the FP32 units where an integer
+// time. Keys are whole numbers below 2^24 as floats, so that a key and one more are
+// exact (2^24 + 1 is no float) and a comparison is a saturated difference, at the full rate of the FP32 units where an integer
 // comparison has half: 16k targets take 28 us (as integers 41), 3.2k 6
 // (11.4). R: enough blocks for the SMs before fewer reads of the keys.
 constexpr int kRankWarps = 16;
+constexpr float kUnusedKey = 16777215.f;  // after every live target's
 template <int R, class GROUPS>
 __global__ void __launch_bounds__(32 * kRankWarps)
     bs_rank_targets(const GROUPS gr, const float *__restrict__ keys,

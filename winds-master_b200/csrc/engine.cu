@@ -927,6 +927,35 @@ int winds_bs_selftest_wait_timeout(unsigned long long limit_ns) {
   return check_device_error(c, c->stream);
 }
 
+int winds_bs_selftest_order(const double *P, const int *unused, long long n, int *perm) {
+  if (!P || !unused || !perm || n < 1 || !sort_by_counting(1, n))
+    return fail(WINDS_BS_ERR_ARG, "bad order self-test arguments");
+  int rc;
+  Context *c = get_context(&rc);
+  if (!c) return rc;
+  cudaStream_t s = c->stream;
+  if ((rc = c->in_F.ensure(n * 4 * sizeof(double), s))) return rc;
+  double *dP = (double *)c->in_F.p, *dw = dP + 3 * n;
+  std::vector<double> w(unused, unused + n);
+  cudaError_t e = cudaMemcpyAsync(dP, P, 3 * n * sizeof(double), cudaMemcpyHostToDevice, s);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(dw, w.data(), n * sizeof(double), cudaMemcpyHostToDevice, s);
+  if (e != cudaSuccess) return cuda_fail(e, "order self-test upload");
+  const TargetSpec ts = {dP, n, n, nullptr, 0};
+  long long nf, nfp, nt;
+  if ((rc = pack_inputs(c, nullptr, 0, ts, kCoreVatistas, 0.0, s, &nf, &nfp, &nt, false))) return rc;
+  TargetBufs tb{};
+  tb.tp = (double4 *)c->tp.p, tb.tp_raw = (double4 *)c->tp_raw.p;
+  tb.perm = (int *)c->perm.p, tb.keys = (unsigned long long *)c->keys.p;
+  e = cudaMemcpy2DAsync((double *)c->tp_raw.p + 3, sizeof(double4), dw, sizeof(double),
+                        sizeof(double), n, cudaMemcpyDeviceToDevice, s);
+  if (e == cudaSuccess) e = launch_order_targets(n, tb, (const BBox *)c->bbox.p, s);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(perm, tb.perm, n * sizeof(int), cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  return e == cudaSuccess ? WINDS_BS_OK : cuda_fail(e, "order self-test");
+}
+
 void winds_bs_shutdown(void) {
   release_stages();
   shutdown_all();
