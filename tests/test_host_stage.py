@@ -1,0 +1,49 @@
+"""The host transfers (csrc/host_stage.cu) against a fake of the CUDA runtime (host_stage_fake.cpp), on the
+CPU: whole copies, and no processor time while a transfer waits for the work before it."""
+from __future__ import annotations
+
+import ctypes as C
+import os
+import subprocess
+import time
+
+import numpy as np
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CSRC = os.path.join(ROOT, "winds-master_b200", "csrc")
+
+
+@pytest.fixture(scope="module")
+def stage(tmp_path_factory):
+    so = str(tmp_path_factory.mktemp("stage") / "stage.so")
+    subprocess.run(["g++", "-std=c++17", "-O2", "-shared", "-fPIC", "-I/usr/local/cuda/include",
+                    "-I" + os.path.join(ROOT, "include"), "-I" + CSRC, "-x", "c++",
+                    os.path.join(CSRC, "host_stage.cu"), os.path.join(ROOT, "tests", "host_stage_fake.cpp"),
+                    "-o", so, "-lpthread"], check=True, capture_output=True)
+    L = C.CDLL(so)
+    L.stage_download.argtypes = [C.c_void_p, C.c_void_p, C.c_size_t, C.c_int, C.c_int]
+    L.stage_upload.argtypes = [C.c_void_p, C.c_void_p, C.c_size_t, C.c_int]
+    yield L
+    L.stage_release()
+
+
+@pytest.mark.parametrize("mb", [0.001, 1.0, 1.5, 8.0, 40.0])
+def test_download_is_whole(stage, mb):
+    src = np.random.default_rng(0).integers(0, 255, int(mb * 2 ** 20), dtype=np.uint8)
+    dst = np.zeros_like(src)
+    assert stage.stage_download(dst.ctypes.data, src.ctypes.data, src.nbytes, 0, 0) == 0
+    np.testing.assert_array_equal(dst, src)
+
+
+def test_waiting_takes_no_processor_time(stage):
+    """Eight threads copy 16 MB out once the first chunk has landed, 0.5 s after the call. The copies take
+    some 10 ms of processor time; a tenth of the wait is far above that."""
+    src = np.ones(16 * 2 ** 20, dtype=np.uint8)
+    dst = np.zeros_like(src)
+    stage.stage_download(dst.ctypes.data, src.ctypes.data, src.nbytes, 0, 0)  # pages of both
+    cpu, wall = time.process_time(), time.perf_counter()
+    assert stage.stage_download(dst.ctypes.data, src.ctypes.data, src.nbytes, 500, 0) == 0
+    cpu, wall = time.process_time() - cpu, time.perf_counter() - wall
+    assert wall >= 0.5
+    assert cpu <= 0.1 * wall, (cpu, wall)

@@ -3,6 +3,8 @@
 
 #include <algorithm>
 #include <atomic>
+#include <chrono>
+#include <condition_variable>
 #include <cstring>
 #include <mutex>
 #include <new>
@@ -47,6 +49,7 @@ std::vector<StageLease::Stage *> g_free;
 
 constexpr size_t kChunk = 1u << 20;
 constexpr size_t kSmallUpload = 1u << 20;
+constexpr std::chrono::microseconds kSpin{200};
 
 // A part of a span within one chunk of the staging memory.
 struct Piece {
@@ -156,7 +159,10 @@ cudaError_t StageLease::download(const HostSpan *v, int n, cudaStream_t s) {
   if (err_ != cudaSuccess) return err_;
   std::vector<Piece> pieces;
   // up to kMaxPinned bytes of pieces: a DMA per chunk and run of device memory, then
-  // the threads copy each chunk once its event has passed
+  // the threads copy each chunk once its event has passed. They start before it has,
+  // beside the work that the first DMA waits for: kSpin long they look for themselves,
+  // as long as the kinematics of a run take (waking eight threads takes 0.3 ms of its
+  // 0.9), then they sleep, so that a long sum does not keep eight cores busy.
   const auto round = [&](size_t total) -> cudaError_t {
     if (total == 0) return cudaSuccess;
     cudaError_t r = st_->reserve(total);
@@ -180,14 +186,22 @@ cudaError_t StageLease::download(const HostSpan *v, int n, cudaStream_t s) {
       if (r == cudaSuccess) r = cudaEventRecord(st_->ev[c], s);
     }
     if (r != cudaSuccess) return r;
-    std::atomic<int> next{0}, ready{0};  // ready < 0: a wait failed
+    std::atomic<int> next{0}, ready{0};  // ready: chunks that landed; < 0: a wait failed
+    std::mutex mu;
+    std::condition_variable landed;
     const auto work = [&] {
+      const auto settled = [&](int c) {
+        const int k = ready.load(std::memory_order_acquire);
+        return k < 0 || k > c;
+      };
       for (int c = next.fetch_add(1); c < chunks; c = next.fetch_add(1)) {
-        int k;
-        while ((k = ready.load(std::memory_order_acquire)) <= c) {
-          if (k < 0) return;
-          std::this_thread::yield();
+        const auto until = std::chrono::steady_clock::now() + kSpin;
+        while (!settled(c) && std::chrono::steady_clock::now() < until) std::this_thread::yield();
+        if (!settled(c)) {
+          std::unique_lock<std::mutex> g(mu);
+          landed.wait(g, [&] { return settled(c); });
         }
+        if (ready.load(std::memory_order_acquire) < 0) return;
         for (int i = first[c]; i < first[c + 1]; ++i)
           std::memcpy(pieces[i].host, pin + pieces[i].off, pieces[i].bytes);
       }
@@ -201,7 +215,11 @@ cudaError_t StageLease::download(const HostSpan *v, int n, cudaStream_t s) {
     }
     for (int c = 0; c < chunks && r == cudaSuccess; ++c) {
       r = cudaEventSynchronize(st_->ev[c]);
-      ready.store(r == cudaSuccess ? c + 1 : -1, std::memory_order_release);
+      {
+        std::lock_guard<std::mutex> g(mu);
+        ready.store(r == cudaSuccess ? c + 1 : -1, std::memory_order_release);
+      }
+      landed.notify_all();
     }
     if (r == cudaSuccess) work();
     for (std::thread &x : pool) x.join();
