@@ -36,6 +36,20 @@ def test_download_is_whole(stage, mb):
     np.testing.assert_array_equal(dst, src)
 
 
+def test_copies_without_pinned_memory(stage):
+    """A system that has no pinned memory to give: the driver's own staging, as for larger inputs."""
+    stage.stage_release()
+    src = np.random.default_rng(1).integers(0, 255, 3 * 2 ** 20, dtype=np.uint8)
+    for n in (5, 2 ** 20, src.nbytes):
+        dst = np.zeros(n, dtype=np.uint8)
+        assert stage.stage_upload(src.ctypes.data, dst.ctypes.data, n, 1) == 0
+        np.testing.assert_array_equal(dst, src[:n])
+        dst[:] = 0
+        assert stage.stage_download(dst.ctypes.data, src.ctypes.data, n, 0, 1) == 0
+        np.testing.assert_array_equal(dst, src[:n])
+        assert stage.stage_last_error() == 0
+
+
 def test_waiting_takes_no_processor_time(stage):
     """Eight threads copy 16 MB out once the first chunk has landed, 0.5 s after the call. The copies take
     some 10 ms of processor time; a tenth of the wait is far above that."""

@@ -22,14 +22,17 @@ struct StageLease::Stage {
   cudaEvent_t used = nullptr;   // after the last DMA from the pinned memory
   bool pending = false;
 
-  // The pinned memory, once no DMA reads it any more.
+  // The pinned memory, once no DMA reads it any more. Where the system has none to give
+  // (cudaErrorMemoryAllocation, not left behind as the last error) copies go without.
   cudaError_t reserve(size_t bytes) {
     if (pending) {
       const cudaError_t e = cudaEventSynchronize(used);
       if (e != cudaSuccess) return e;
       pending = false;
     }
-    return pinned.ensure(bytes) ? cudaErrorMemoryAllocation : cudaSuccess;
+    if (!pinned.ensure(bytes)) return cudaSuccess;
+    cudaGetLastError();
+    return cudaErrorMemoryAllocation;
   }
   void destroy() {
     cudaSetDevice(dev);
@@ -103,9 +106,12 @@ StageLease::~StageLease() {
     std::lock_guard<std::mutex> g(g_mu);
     int kept = 0;
     for (const Stage *s : g_free) kept += s->dev == st_->dev;
-    if (kept < kKept) {
-      g_free.push_back(st_);
-      return;
+    try {
+      if (kept < kKept) {
+        g_free.push_back(st_);
+        return;
+      }
+    } catch (...) {  // no memory for the list: freed like a stage too many
     }
   }
   st_->destroy();
@@ -122,8 +128,10 @@ cudaError_t StageLease::upload(const HostSpan *v, int n, cudaStream_t s) {
   cudaError_t e = cudaSuccess;
   unsigned char *pin = nullptr;
   if (total <= kSmallUpload) {
-    if ((e = st_->reserve(total)) != cudaSuccess) return err_ = e;
-    pin = static_cast<unsigned char *>(st_->pinned.p);
+    e = st_->reserve(total);
+    if (e == cudaSuccess) pin = static_cast<unsigned char *>(st_->pinned.p);
+    else if (e != cudaErrorMemoryAllocation) return err_ = e;
+    e = cudaSuccess;
   }
   size_t off = 0, from = 0;  // staged; of it, sent
   unsigned char *to = nullptr;
@@ -166,6 +174,12 @@ cudaError_t StageLease::download(const HostSpan *v, int n, cudaStream_t s) {
   const auto round = [&](size_t total) -> cudaError_t {
     if (total == 0) return cudaSuccess;
     cudaError_t r = st_->reserve(total);
+    if (r == cudaErrorMemoryAllocation) {
+      r = cudaSuccess;
+      for (size_t i = 0; i < pieces.size() && r == cudaSuccess; ++i)
+        r = cudaMemcpyAsync(pieces[i].host, pieces[i].dev, pieces[i].bytes, cudaMemcpyDeviceToHost, s);
+      return r;
+    }
     if (r != cudaSuccess) return r;
     unsigned char *pin = static_cast<unsigned char *>(st_->pinned.p);
     const int chunks = (int)((total + kChunk - 1) / kChunk);
