@@ -856,10 +856,10 @@ static int step_impl(winds_wake_batch *b, int nsteps, int use_graph) {
       e = enqueue_post(b, l2);
       b->launches = l + l2;
       if (e != cudaSuccess) return cuda_fail(e, "wake step commit");
+      ++b->steps_done;  // the next step's: run_kj starts with the iteration's first one
     }
     b->timed_steps = nsteps;
     if (nsteps > 0) cudaEventRecord(b->ev1, b->stream);
-    b->steps_done += nsteps;
     e = cudaStreamSynchronize(b->stream);
     if (e != cudaSuccess) return cuda_fail(e, "wake step sync");
     return device_error_word(b);
