@@ -1320,7 +1320,8 @@ void winds_wake_destroy(winds_wake_batch *b) {
                     &b->h2, &b->h3, &b->uind, &b->uind_pred, &b->bound, &b->trail_prev,
                     &b->shed_cur, &b->trail_cur, &b->shed_next, &b->trail_next, &b->rc_s,
                     &b->rc_t, &b->len_old_s, &b->len_old_t, &b->len_s, &b->len_t, &b->len_ps,
-                    &b->len_pt, &b->quarter, &b->trailing, &b->wind, &b->pk, &b->ra, &b->rb, &b->tp, &b->tp_raw, &b->tgroup, &b->keys, &b->vals,
+                    &b->len_pt, &b->quarter, &b->trailing, &b->wind, &b->ser, &b->live_main,
+                    &b->live_pred, &b->live_kj, &b->pk, &b->ra, &b->rb, &b->tp, &b->tp_raw, &b->tgroup, &b->keys, &b->vals,
                     &b->perm, &b->sort_tmp, &b->groups_main, &b->groups_pred, &b->tiles,
                     &b->items, &b->order, &b->part, &b->bbox, &b->ctr, &b->err, &b->nearctr})
     x->release();
