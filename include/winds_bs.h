@@ -201,6 +201,10 @@ int winds_bs_selftest_wait_timeout(unsigned long long limit_ns);
  * the target at place k. */
 int winds_bs_selftest_order(const double *P, const int *unused, long long n, int *perm);
 
+/* Self-test of the FP64 sums' own roots: y [4][n] = their 1/sqrt(x) and 1/x, then
+ * CUDA's, of x [n] (host arrays). */
+int winds_bs_selftest_roots(const double *x, long long n, double *y);
+
 /* Frees every device buffer, stream and event of every device context
  * (the mexAtExit hook of the MEX layer). */
 void winds_bs_shutdown(void);

@@ -325,9 +325,12 @@ __device__ __forceinline__ void ref_pair(const double4 A, const double4 B, doubl
   uz = __dadd_rn(uz, __dmul_rn(ubar, __dsub_rn(__dmul_rn(pxx1, pyy2), __dmul_rn(pyy1, pxx2))));
 }
 
-// 1/sqrt(x) and 1/x to FP64 roundoff for x well inside the normal range: the
-// hardware's approximation and one third-order step, y (1 + e/2 + 3e^2/8) with
-// e = 1 - x y^2 and y (1 + e + e^2) with e = 1 - x y (Householder's method).
+// 1/sqrt(x) and 1/x for x from 2^-960 to 2^960: the hardware's approximation and one
+// third-order step, y (1 + e/2 + 3e^2/8) with e = 1 - x y^2 and y (1 + e + e^2) with
+// e = 1 - x y (Householder's method). Relative error at most 2^-52: the step leaves
+// some 2^-60, the product x y rounds e by 2^-53, of which the root takes half, and the
+// last operation rounds by 2^-53. Zero, subnormal and infinite x, NaN and, for the
+// root, negative x give no finite value. (winds_bs_selftest_roots)
 __device__ __forceinline__ double rsqrt64(double x) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));

@@ -1207,6 +1207,15 @@ __global__ void bs_wait_selftest(unsigned *err, unsigned long long limit_ns) {
   __syncthreads();
 }
 
+__global__ void bs_roots_selftest(const double *__restrict__ x, long long n, double *y) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  y[i] = rsqrt64(x[i]);
+  y[n + i] = rcp64(x[i]);
+  y[2 * n + i] = rsqrt(x[i]);
+  y[3 * n + i] = 1.0 / x[i];
+}
+
 // ============================================================ host launchers
 namespace {
 template <int T, int KF, int MODEL>
@@ -1445,6 +1454,11 @@ unsigned long long default_wait_limit_ns() { return kDefaultWaitNs; }
 
 cudaError_t launch_ffma_peak(float *out, int blocks, int iters, cudaStream_t s) {
   bs_ffma_peak<<<blocks, 256, 0, s>>>(out, iters, 0.999999f, 1e-7f);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_roots_selftest(const double *x, long long n, double *y, cudaStream_t s) {
+  bs_roots_selftest<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(x, n, y);
   return cudaGetLastError();
 }
 

@@ -109,6 +109,8 @@ cudaError_t launch_reduce(const Tile *tiles, int n_tiles, const Group *groups, c
                           const Item *items = nullptr, const GroupLive *live = nullptr);
 cudaError_t launch_ffma_peak(float *out, int blocks, int iters, cudaStream_t s);
 cudaError_t launch_wait_selftest(unsigned *err, unsigned long long limit_ns, cudaStream_t s);
+// y [4][n]: rsqrt64, rcp64 and CUDA's rsqrt and 1 / x of x [n].
+cudaError_t launch_roots_selftest(const double *x, long long n, double *y, cudaStream_t s);
 cudaError_t launch_length(const double *F1, const double *F2, long long d0, long long nf, double *L,
                           cudaStream_t s);
 

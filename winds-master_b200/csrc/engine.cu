@@ -956,6 +956,22 @@ int winds_bs_selftest_order(const double *P, const int *unused, long long n, int
   return e == cudaSuccess ? WINDS_BS_OK : cuda_fail(e, "order self-test");
 }
 
+int winds_bs_selftest_roots(const double *x, long long n, double *y) {
+  if (!x || !y || n < 1 || n > (1ll << 24)) return fail(WINDS_BS_ERR_ARG, "bad roots self-test arguments");
+  int rc;
+  Context *c = get_context(&rc);
+  if (!c) return rc;
+  cudaStream_t s = c->stream;
+  if ((rc = c->in_F.ensure(n * 5 * sizeof(double), s))) return rc;
+  double *dx = (double *)c->in_F.p, *dy = dx + n;
+  cudaError_t e = cudaMemcpyAsync(dx, x, n * sizeof(double), cudaMemcpyHostToDevice, s);
+  if (e == cudaSuccess) e = launch_roots_selftest(dx, n, dy, s);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(y, dy, 4 * n * sizeof(double), cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  return e == cudaSuccess ? WINDS_BS_OK : cuda_fail(e, "roots self-test");
+}
+
 void winds_bs_shutdown(void) {
   release_stages();
   shutdown_all();
