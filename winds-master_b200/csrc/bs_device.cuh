@@ -393,8 +393,10 @@ __device__ __forceinline__ void pair64(const double4 A, const double4 B, double 
 constexpr int kHiMin = (1023 - 480) << 20, kHiMax = (1023 + 480) << 20;    // 2^-480, 2^480
 constexpr int kHiMin2 = (1023 - 960) << 20, kHiMax2 = (1023 + 960) << 20;  // 2^-960, 2^960
 
-// High word of the reach's square; a negative reach drops every pair.
+// High word of the reach's square; a negative reach drops every pair, one that is not a
+// number none (its square's sign may be set, as in the NaN that MATLAB makes).
 __device__ __forceinline__ int reach_hi(double co) {
+  if (isnan(co)) return 0x7fffffff;
   return co < 0.0 ? -1 : __double2hiint(co * co);
 }
 
