@@ -405,8 +405,9 @@ __device__ __forceinline__ int reach_hi(double co) {
 // axis_hi: axis_limit(L^2). False, with u unchanged, for what ref_pair does
 // instead: scales far from one, the reach's edge, a point on a filament's end, and
 // where ref_pair's differences cancel, so that both agree there too: 1 + cos of the
-// angle between the ends below 2^-8 (next to the segment) and, with the Vatistas
-// core, a sine below 2^-4 or so of the angle to the filament's line.
+// angle between the ends below 2^-8 (next to the segment), with the Vatistas core a
+// sine below 2^-4 or so of the angle to the filament's line and, with a negative
+// squared cut-off, which can make it vanish, a denominator below 2^-8 of r1 r2 squared.
 constexpr int kHiE = (1023 - 8) << 20;
 __device__ __forceinline__ int axis_limit(double L2) {
   return __double2hiint(L2) - (8 << 20);
@@ -430,6 +431,7 @@ __device__ __forceinline__ bool pair64_short(const double4 A, const double4 B, c
   if (MODEL == kCoreCutoff) {
     const double q = fma(C.w, gg * gg, e);
     hq = __double2hiint(q);
+    hard = hard || hq < kHiE;  // with d >= 0 no smaller than e
     ub = (i1 + i2) * gg * rcp64(q);
   } else {
     const double c2 = fma(cx, cx, fma(cy, cy, cz * cz)), q = fma(c2, c2, C.w);
