@@ -10,6 +10,7 @@
 
 static int g_wait_ms = 0;
 static int g_fail_pinned = 0;
+static int g_copies = 0;
 static cudaError_t g_last = cudaSuccess;
 
 extern "C" {
@@ -33,15 +34,17 @@ cudaError_t cudaPointerGetAttributes(cudaPointerAttributes *a, const void *) {
 }
 cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind, cudaStream_t) {
   std::memcpy(d, s, n);
+  ++g_copies;
   return cudaSuccess;
 }
 
 // Device bytes to host through one lease, after work of `wait_ms`; pinned memory not to be had if fail_pinned.
-int stage_download(void *host, void *dev, size_t bytes, int wait_ms, int fail_pinned) {
-  g_wait_ms = wait_ms, g_fail_pinned = fail_pinned;
+int stage_download(void *host, void *dev, size_t bytes, int wait_ms, int fail_pinned,
+                   int wide) {
+  g_wait_ms = wait_ms, g_fail_pinned = fail_pinned, g_copies = 0;
   winds::StageLease stage;
   const winds::HostSpan v = {host, dev, bytes};
-  return (int)stage.download(&v, 1, (cudaStream_t)1);
+  return (int)stage.download(&v, 1, (cudaStream_t)1, wide != 0);
 }
 int stage_upload(void *host, void *dev, size_t bytes, int fail_pinned) {
   g_fail_pinned = fail_pinned;
@@ -49,6 +52,7 @@ int stage_upload(void *host, void *dev, size_t bytes, int fail_pinned) {
   const winds::HostSpan v = {host, dev, bytes};
   return (int)stage.upload(&v, 1, (cudaStream_t)1);
 }
+int stage_copies(void) { return g_copies; }
 int stage_last_error(void) { return (int)cudaGetLastError(); }
 void stage_release(void) { winds::release_stages(); }
 }

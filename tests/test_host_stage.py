@@ -3,6 +3,7 @@ CPU: whole copies, and no processor time while a transfer waits for the work bef
 from __future__ import annotations
 
 import ctypes as C
+import mmap
 import os
 import subprocess
 import time
@@ -22,7 +23,7 @@ def stage(tmp_path_factory):
                     os.path.join(CSRC, "host_stage.cu"), os.path.join(ROOT, "tests", "host_stage_fake.cpp"),
                     "-o", so, "-lpthread"], check=True, capture_output=True)
     L = C.CDLL(so)
-    L.stage_download.argtypes = [C.c_void_p, C.c_void_p, C.c_size_t, C.c_int, C.c_int]
+    L.stage_download.argtypes = [C.c_void_p, C.c_void_p, C.c_size_t, C.c_int, C.c_int, C.c_int]
     L.stage_upload.argtypes = [C.c_void_p, C.c_void_p, C.c_size_t, C.c_int]
     yield L
     L.stage_release()
@@ -31,8 +32,29 @@ def stage(tmp_path_factory):
 @pytest.mark.parametrize("mb", [0.001, 1.0, 1.5, 8.0, 40.0])
 def test_download_is_whole(stage, mb):
     src = np.random.default_rng(0).integers(0, 255, int(mb * 2 ** 20), dtype=np.uint8)
-    dst = np.zeros_like(src)
-    assert stage.stage_download(dst.ctypes.data, src.ctypes.data, src.nbytes, 0, 0) == 0
+    for wide in (0, 1):
+        dst = np.ones_like(src)  # pages in place
+        assert stage.stage_download(dst.ctypes.data, src.ctypes.data, src.nbytes, 0, 0, wide) == 0
+        np.testing.assert_array_equal(dst, src)
+        pages = mmap.mmap(-1, src.nbytes)  # none yet
+        dst = np.frombuffer(pages, dtype=np.uint8)
+        assert stage.stage_download(dst.ctypes.data, src.ctypes.data, src.nbytes, 0, 0, wide) == 0
+        np.testing.assert_array_equal(dst, src)
+
+
+@pytest.mark.parametrize("mb,there,wide,copies", [
+    (0.5, True, 0, 1), (4.5, True, 0, 5), (15.5, True, 0, 16), (40.0, True, 0, 1),
+    (0.5, False, 0, 1), (4.5, False, 0, 5), (15.5, False, 0, 16), (40.0, False, 0, 40),
+    (4.5, True, 1, 5), (40.0, True, 1, 40), (40.0, False, 1, 40)])
+def test_route(stage, mb, there, wide, copies):
+    """Chunks of 1 MB, and one plain copy for large outputs into pages that are there."""
+    src = np.ones(int(mb * 2 ** 20), dtype=np.uint8)
+    pages = mmap.mmap(-1, src.nbytes)
+    dst = np.frombuffer(pages, dtype=np.uint8)
+    if there:
+        pages.write(bytes(src.nbytes))
+    assert stage.stage_download(dst.ctypes.data, src.ctypes.data, src.nbytes, 0, 0, wide) == 0
+    assert stage.stage_copies() == copies
     np.testing.assert_array_equal(dst, src)
 
 
@@ -45,7 +67,7 @@ def test_copies_without_pinned_memory(stage):
         assert stage.stage_upload(src.ctypes.data, dst.ctypes.data, n, 1) == 0
         np.testing.assert_array_equal(dst, src[:n])
         dst[:] = 0
-        assert stage.stage_download(dst.ctypes.data, src.ctypes.data, n, 0, 1) == 0
+        assert stage.stage_download(dst.ctypes.data, src.ctypes.data, n, 0, 1, 0) == 0
         np.testing.assert_array_equal(dst, src[:n])
         assert stage.stage_last_error() == 0
 
@@ -55,9 +77,9 @@ def test_waiting_takes_no_processor_time(stage):
     some 10 ms of processor time; a tenth of the wait is far above that."""
     src = np.ones(16 * 2 ** 20, dtype=np.uint8)
     dst = np.zeros_like(src)
-    stage.stage_download(dst.ctypes.data, src.ctypes.data, src.nbytes, 0, 0)  # pages of both
+    stage.stage_download(dst.ctypes.data, src.ctypes.data, src.nbytes, 0, 0, 1)  # pages of both
     cpu, wall = time.process_time(), time.perf_counter()
-    assert stage.stage_download(dst.ctypes.data, src.ctypes.data, src.nbytes, 500, 0) == 0
+    assert stage.stage_download(dst.ctypes.data, src.ctypes.data, src.nbytes, 500, 0, 1) == 0
     cpu, wall = time.process_time() - cpu, time.perf_counter() - wall
     assert wall >= 0.5
     assert cpu <= 0.1 * wall, (cpu, wall)

@@ -11,6 +11,9 @@
 #include <thread>
 #include <vector>
 
+#include <sys/mman.h>
+#include <unistd.h>
+
 namespace winds {
 
 struct StageLease::Stage {
@@ -52,6 +55,7 @@ std::vector<StageLease::Stage *> g_free;
 
 constexpr size_t kChunk = 1u << 20;
 constexpr size_t kSmallUpload = 1u << 20;
+constexpr size_t kDirect = 16u << 20;
 constexpr std::chrono::microseconds kSpin{200};
 
 // A part of a span within one chunk of the staging memory.
@@ -60,11 +64,19 @@ struct Piece {
   size_t off, bytes;
 };
 
-// Threads that copy `bytes` out: one per MB, where starting one (some 20 us) is less
-// than what it saves, and at most 8 or half the machine's.
-int copy_threads(size_t bytes) {
+// Threads that copy `bytes` out (host_stage.h), at most half the machine's. wide: one
+// per MB, up to 8.
+int copy_threads(size_t bytes, bool wide) {
   const int hw = (int)std::thread::hardware_concurrency() / 2;
-  return std::max(1, std::min({8, hw, (int)(bytes / kChunk)}));
+  const int want = wide ? (int)(bytes / kChunk) : bytes <= 8 * kChunk ? 1 : bytes <= kDirect ? 2 : 8;
+  return std::max(1, std::min({8, hw, want}));
+}
+
+// Whether the page in the middle of these bytes is there, and not made on its first write.
+bool resident(const void *p, size_t bytes) {
+  const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE), at = (uintptr_t)p + bytes / 2;
+  unsigned char r = 0;
+  return mincore((void *)(at / page * page), 1, &r) == 0 && (r & 1);
 }
 
 bool pageable(const void *p) {
@@ -163,8 +175,13 @@ cudaError_t StageLease::upload(const HostSpan *v, int n, cudaStream_t s) {
   return e;
 }
 
-cudaError_t StageLease::download(const HostSpan *v, int n, cudaStream_t s) {
+cudaError_t StageLease::download(const HostSpan *v, int n, cudaStream_t s, bool wide) {
   if (err_ != cudaSuccess) return err_;
+  size_t bytes = 0, there = 0;  // there: to pageable memory with its pages in place
+  for (int i = 0; i < n; ++i) bytes += v[i].bytes;
+  for (int i = 0; i < n && !wide && bytes > kDirect; ++i)
+    if (v[i].bytes && pageable(v[i].host) && resident(v[i].host, v[i].bytes)) there += v[i].bytes;
+  const bool direct = there > bytes / 2;
   std::vector<Piece> pieces;
   // up to kMaxPinned bytes of pieces: a DMA per chunk and run of device memory, then
   // the threads copy each chunk once its event has passed. They start before it has,
@@ -221,7 +238,7 @@ cudaError_t StageLease::download(const HostSpan *v, int n, cudaStream_t s) {
       }
     };
     std::vector<std::thread> pool;
-    const int nthreads = copy_threads(total);
+    const int nthreads = copy_threads(bytes, wide);
     try {
       pool.reserve(nthreads);
       for (int t = 1; t < nthreads; ++t) pool.emplace_back(work);
@@ -247,7 +264,7 @@ cudaError_t StageLease::download(const HostSpan *v, int n, cudaStream_t s) {
       unsigned char *dev = static_cast<unsigned char *>(v[i].dev);
       size_t left = v[i].bytes;
       if (left == 0) continue;
-      if (!pageable(host)) {
+      if (direct || !pageable(host)) {
         e = cudaMemcpyAsync(host, dev, left, cudaMemcpyDeviceToHost, s);
         continue;
       }

@@ -294,6 +294,6 @@ extern "C" int winds_kinematics(const winds_kin_rotor *r, winds_kin_out *out) {
       span(out->bxn, k.bxn, st_n),           span(out->byn, k.byn, st_n),
       span(out->bzn, k.bzn, st_n),           span(out->vbound, k.vbound, st_n),
       span(out->vblade, k.vblade, st_n)};
-  if (e == cudaSuccess) e = stage.download(copies, 15, s);
+  if (e == cudaSuccess) e = stage.download(copies, 15, s, true);
   return e == cudaSuccess ? WINDS_BS_OK : cuda_fail(e, "kinematics");
 }
