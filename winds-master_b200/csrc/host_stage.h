@@ -16,9 +16,9 @@
 //   one thread      428   388   992   846  2213  1873  5371   4266   9967   7723
 //   two             690   630  1118   930  2020  1618  4325   3354   8336   5901
 //   one per MB      417   383  1517  1029  3261  1758  5195   3173   6243   5762
-// and a wake's state of 6.7 MB 1170, 820, 770 and 1610 us. Kinematics, in arrays of huge
-// pages and with threads that start next to the last kernel, take one per MB, up to eight
-// (28 MB: 0.94 ms, the driver 1.98, one thread 2.60).
+// and a wake's state of 6.7 MB 1170, 820, 770 and 1610 us. Kinematics, with threads that
+// start next to the last kernel, take one per MB, up to eight (28 MB: 0.9 to 1.2 ms, the
+// driver 1.98, one thread 2.60).
 #pragma once
 
 #include <cuda_runtime.h>

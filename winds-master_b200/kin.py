@@ -13,7 +13,6 @@ vbound, vblade [ns, 3, nt, nb]``).
 from __future__ import annotations
 
 import ctypes as C
-import math
 
 import numpy as np
 
@@ -55,16 +54,11 @@ def kinematics(r: dict) -> dict:
         setattr(a, f, keep[f].ctypes.data)
     for f in _SCALARS + ("ptfm_ref",):
         setattr(a, f, float(r[f]))
-    # one block for all arrays: large enough for huge pages, which first writes
-    # (15 arrays of 2 MB: 7000 page faults) are much cheaper on
+    # empty, not zeros: every value is written, and the transfer's threads make the pages
     shapes = {"hub": (nt, 3)}
     shapes.update({f: (nst, 3, nt, nb) for f in _OUT_T + _OUT_FT})
     shapes.update({f: (ns, 3, nt, nb) for f in _OUT_S + _OUT_FS})
-    block, at, out = np.empty(sum(math.prod(s) for s in shapes.values())), 0, {}
-    for f, s in shapes.items():
-        n = math.prod(s)
-        out[f] = block[at:at + n].reshape(s, order="F")
-        at += n
+    out = {f: np.empty(s, order="F") for f, s in shapes.items()}
     o = KinOutC(*[out[f].ctypes.data for f in ("hub",) + _OUT_T + _OUT_S + _OUT_FT + _OUT_FS])
     _check(_bind().winds_kinematics(C.byref(a), C.byref(o)))
     return out
