@@ -1030,8 +1030,9 @@ int winds_wake_set_kj(winds_wake_batch *b, const winds_kj_case *kj, const winds_
   }
   b->frames_n = fr, b->n_ll = tt, b->stations_n = st;
   int rc;
-  // kj_solve's vectors and matrix rows: shared memory where the largest case's
-  // fit, else a scratch; a matrix beyond kKJMatBytes is formed term by term
+  // kj_solve's vectors and matrix rows: shared memory where the largest case's fit,
+  // else a scratch; a matrix beyond kKJMatBytes (of which DevBuf allocates a quarter
+  // more), or beyond the memory that is free, is formed term by term
   const long long ctas = (long long)b->ncases * kj_cluster();
   b->kj_vec_stride = vecs, b->kj_mat_stride = mats;
   b->kj_vec_smem = vecs * 8 <= kKJSmemBytes;
@@ -1039,8 +1040,8 @@ int winds_wake_set_kj(winds_wake_batch *b, const winds_kj_case *kj, const winds_
   if (!b->kj_vec_smem && (rc = b->kj_vec.ensure(ctas * vecs * 8, s))) return rc;
   if (b->kj_mat_smem || ctas * mats * 8 > kKJMatBytes)
     b->kj_mat.release();
-  else if ((rc = b->kj_mat.ensure(ctas * mats * 8, s)))
-    return rc;
+  else if (b->kj_mat.ensure(ctas * mats * 8, s))
+    cudaGetLastError();
   for (DevBuf *x : {&b->ll, &b->bxn, &b->byn, &b->bzn, &b->vblade})
     if ((rc = x->ensure(fr * sizeof(double), s))) return rc;
   if ((rc = b->kjc_d.ensure(b->ncases * sizeof(KJCase), s)) ||
