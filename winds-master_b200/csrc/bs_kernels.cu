@@ -567,25 +567,12 @@ __device__ __forceinline__ bool f32c_item(const F32cArgs &a, const Item &it, uns
   // The FP32 sums' rounding, more than the terms', sets the error, and the chained order
   // of a wake puts the large terms of a target next to one another. So a near sum spans
   // eight filaments before it joins the others, and these join the Kahan state after
-  // each tile, and before its second half where both halves have near groups. Error
-  // against FP64 (2-norm) of a step of eight rotors: 4.7e-8 (Vatistas core) and 4.2e-8
-  // (cut-off) with one sum over 64 filaments, now 3.5e-8 and 3.2e-8 (without chains, in
-  // input order: 3.7e-8 and 3.3e-8). The sums take 1 to 4% longer for it: 11.8 -> 11.9
-  // ms on the large wake, 195 -> 203 us on 7.6k targets. (A second level of sums, over
-  // 32, or two sets for the distant form cost registers: up to 10%.)
-  const auto fold = [&] {
-#pragma unroll
-    for (int p = 0; p < NP; ++p) {
-      const int sl = lane * T + 2 * p;
-      kahan_add(s_k[0 * 32 * T + sl], s_k[1 * 32 * T + sl], ax[p].x);
-      kahan_add(s_k[2 * 32 * T + sl], s_k[3 * 32 * T + sl], ay[p].x);
-      kahan_add(s_k[4 * 32 * T + sl], s_k[5 * 32 * T + sl], az[p].x);
-      kahan_add(s_k[0 * 32 * T + sl + 1], s_k[1 * 32 * T + sl + 1], ax[p].y);
-      kahan_add(s_k[2 * 32 * T + sl + 1], s_k[3 * 32 * T + sl + 1], ay[p].y);
-      kahan_add(s_k[4 * 32 * T + sl + 1], s_k[5 * 32 * T + sl + 1], az[p].y);
-      ax[p] = ay[p] = az[p] = make_float2(0.f, 0.f);
-    }
-  };
+  // each tile. Error against FP64 (2-norm) of a step of eight rotors: 4.7e-8 (Vatistas
+  // core) and 4.2e-8 (cut-off) with one sum over 64 filaments, now 3.6e-8 and 3.3e-8, as
+  // without chains, in input order (3.7e-8 and 3.3e-8). The sums take up to 3% longer for
+  // it: 11.8 -> 11.9 ms on the large wake, 195 -> 199 us on 7.6k targets. (A second level
+  // of sums, over 32, another fold between a tile's halves or two sets for the distant
+  // form give 3.3e-8 to 3.5e-8 and cost 3 to 10%.)
 
   int i = 0;
   for (; i < ntiles; ++i) {
@@ -773,7 +760,6 @@ __device__ __forceinline__ bool f32c_item(const F32cArgs &a, const Item &it, uns
 #pragma unroll 1
       for (unsigned gm = ~gdist & kGroups; gm; gm &= gm - 1u) {
         const int gr = __ffs(gm) - 1;
-        if (KF == 64 && gr >= 8 && last < 8 && last >= 0) fold();
         const unsigned hg = group_heads(gr) | (gr != last + 1 ? 1u : 0u);
         last = gr;
         const bool near_some = (careful >> gr) & 1u;
@@ -809,7 +795,18 @@ __device__ __forceinline__ bool f32c_item(const F32cArgs &a, const Item &it, uns
       }
     }
     __syncwarp();
-    fold();
+    // into the Kahan state
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+      const int sl = lane * T + 2 * p;
+      kahan_add(s_k[0 * 32 * T + sl], s_k[1 * 32 * T + sl], ax[p].x);
+      kahan_add(s_k[2 * 32 * T + sl], s_k[3 * 32 * T + sl], ay[p].x);
+      kahan_add(s_k[4 * 32 * T + sl], s_k[5 * 32 * T + sl], az[p].x);
+      kahan_add(s_k[0 * 32 * T + sl + 1], s_k[1 * 32 * T + sl + 1], ax[p].y);
+      kahan_add(s_k[2 * 32 * T + sl + 1], s_k[3 * 32 * T + sl + 1], ay[p].y);
+      kahan_add(s_k[4 * 32 * T + sl + 1], s_k[5 * 32 * T + sl + 1], az[p].y);
+      ax[p] = ay[p] = az[p] = make_float2(0.f, 0.f);
+    }
     // Near-singular pairs of this tile: the reference formula in FP64, added to
     // the owner's Kahan state as an exact hi + lo pair. In rounds, every lane
     // lists the next kList of its pairs in the consumed stage (its groups in
