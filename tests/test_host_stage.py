@@ -18,10 +18,11 @@ CSRC = os.path.join(ROOT, "winds-master_b200", "csrc")
 @pytest.fixture(scope="module")
 def stage(tmp_path_factory):
     so = str(tmp_path_factory.mktemp("stage") / "stage.so")
+    # -Bsymbolic: the fake's functions, also after another test has loaded the CUDA runtime for all.
     subprocess.run(["g++", "-std=c++17", "-O2", "-shared", "-fPIC", "-I/usr/local/cuda/include",
                     "-I" + os.path.join(ROOT, "include"), "-I" + CSRC, "-x", "c++",
                     os.path.join(CSRC, "host_stage.cu"), os.path.join(ROOT, "tests", "host_stage_fake.cpp"),
-                    "-o", so, "-lpthread"], check=True, capture_output=True)
+                    "-o", so, "-lpthread", "-Wl,-Bsymbolic"], check=True, capture_output=True)
     L = C.CDLL(so)
     L.stage_download.argtypes = [C.c_void_p, C.c_void_p, C.c_size_t, C.c_int, C.c_int, C.c_int]
     L.stage_upload.argtypes = [C.c_void_p, C.c_void_p, C.c_size_t, C.c_int]
