@@ -173,7 +173,7 @@ int winds_bs_sync(void *stream);
  * (T = 8, eight targets per lane, and KF = 128, which runs as 64, are
  * settable). Evaluations on another stream, or with the autotuner off, use
  * the cached choice or the untuned default (T = 4, 2 below 2048 targets, 3 from
- * 49152; KF = 64; input order).
+ * 24576; KF = 64; input order).
  * set_tuning / get_tuning read and write that cache directly (e.g. to restore
  * a saved choice). */
 int winds_bs_set_autotune(int on);

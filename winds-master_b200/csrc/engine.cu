@@ -378,10 +378,12 @@ static int log2_bucket(long long n) {
 
 // Untuned tiling: more targets per lane spread a filament's loads and the screen
 // over more pairs, fewer keep the warp's ball of targets small; more items balance
-// the workers better, fewer cost less around the sum. Evaluations on the chained
-// layout: 4 targets a lane against 2 117 and 135 us on 3.1k targets, 4 against 6
-// (T = 3) 509 and 536 us on 14k, 1588 and 1552 on 30k; 16 items a worker against 32
-// 513 and 553 us on 14k, 1570 and 1599 on 30k.
+// the workers better, fewer cost less around the sum. Untuned evaluations run in
+// input order (the chained layout, 5% faster on 3k targets, 12% on 14k, 21% on 89k, is
+// the tuner's choice). There: 4 targets a lane against 2 123 and 116 us on 2.1k targets,
+// 128 and 145 on 3.2k; 6 (T = 3) against 4 634 and 620 us on 14k, 1137 and 1139 on 20k,
+// 2132 and 2215 on 30k; 16 items a worker against 32 620 and 663 us on 14k, 2132 and
+// 2166 on 30k.
 TuneChoice default_choice(long long nt) {
   TuneChoice ch;
   ch.T = nt >= 24576 ? 3 : (nt >= 2048 ? 4 : 2);

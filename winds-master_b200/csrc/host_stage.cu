@@ -114,7 +114,8 @@ StageLease::StageLease() {
 
 StageLease::~StageLease() {
   if (!st_) return;
-  if (err_ == cudaSuccess && st_->pinned.cap <= 2 * kMaxPinned && st_->scratch.cap <= kMaxDev) {
+  if (err_ == cudaSuccess && st_->pinned.cap <= kMaxPinned + kMaxPinned / 4 + 256 &&
+      st_->scratch.cap <= kMaxDev) {
     std::lock_guard<std::mutex> g(g_mu);
     int kept = 0;
     for (const Stage *s : g_free) kept += s->dev == st_->dev;

@@ -34,8 +34,8 @@ struct HostSpan {
 };
 
 // Pinned memory, a stream and device scratch for one transfer or call at a time,
-// from a pool that keeps at most kKept of them per device, each of at most
-// kMaxPinned and kMaxDev bytes; the others are freed when they come back. Any
+// from a pool that keeps at most kKept of them per device, each of at most kMaxPinned
+// bytes (and the quarter that HostBuf adds, 40 MB) and kMaxDev; the others are freed when they come back. Any
 // number of threads may hold one each.
 class StageLease {
  public:

@@ -295,8 +295,9 @@ int winds_mlp_forward_host(winds_mlp *m, const float *x, long long n, float *y) 
   if (n == 0) return WINDS_BS_OK;
   cudaSetDevice(m->dev);
   cudaStream_t s = m->stream;
-  // rows go up in pieces while the network runs on those before; results come
-  // back together, up to 4M rows at a time
+  // rows go up in pieces (the staging of one is read beside the network on the one
+  // before; its copy follows that on the stream), results come back together, up to
+  // 4M rows at a time
   const long long chunk = 1 << 15, most = 1 << 22;
   StageLease stage;
   int rc;
